@@ -62,38 +62,6 @@ __global__ void embedding_kernel(const float *__restrict__ w, const int32_t *__r
     for (int i = threadIdx.x; i < dim / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// x_out = x + delta (delta may be null); normed = x_out * (1/sqrt(mean(x_out^2)+eps)) * gamma
-__global__ void __launch_bounds__(256)
-add_rms_norm_kernel(const float *x, const float *__restrict__ delta,
-                    const float *__restrict__ gamma, float eps, int hidden,
-                    float *x_out, float *__restrict__ normed) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ float red[8];
-    const size_t base = (size_t)blockIdx.x * hidden;
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float v = x[base + i];
-        if (delta) v += delta[base + i];
-        if (x_out) x_out[base + i] = v;
-        ss = fmaf(v, v, ss);
-    }
-    const float total = block_sum(ss, red);
-    const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
-    // x_out may alias x (in-place residual update): read the sum back instead of adding twice;
-    // every thread re-reads exactly the elements it wrote
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float v;
-        if (x_out) {
-            v = x_out[base + i];
-        } else {
-            v = x[base + i];
-            if (delta) v += delta[base + i];
-        }
-        normed[base + i] = (v * inv) * gamma[i];
-    }
-}
-
 // Eight fp32 values -> bf16 in the order the packed-int4 prefill GEMM consumes its activations:
 // k = 0,4,1,5,2,6,3,7 of every group of 8 (what its nibble unpack produces), round to nearest even;
 // the same bits as its own activation pre-pass writes.
@@ -110,15 +78,71 @@ __device__ __forceinline__ uint4 pack_bf16_gemm_order(const float (&v)[8]) {
     return o;
 }
 
-// add_rms_norm_kernel with the normalised rows written as bf16 activations of the next prefill-shaped
-// linear (hidden % 8 == 0); the same arithmetic, so the bf16 values equal those the linear's own
-// pre-pass would make of the fp32 rows.
-__global__ void __launch_bounds__(256)
-add_rms_norm_act_kernel(const float *x, const float *__restrict__ delta, const float *__restrict__ gamma, float eps,
-                        int hidden, float *x_out, uint4 *__restrict__ normed_act) {
+// Position of element e of a group of 8 in that order
+__device__ __forceinline__ int gemm_order_pos(int e) { return ((e & 3) << 1) | (e >> 2); }
+
+// x_out = x + delta (delta may be null); normed = x_out * (1/sqrt(mean(x_out^2)+eps)) * gamma, written
+// as fp32 or (ACT) as the bf16 activations of the next prefill-shaped linear: the same arithmetic, so the
+// bf16 values equal those the linear's own pre-pass would make of the fp32 rows (ACT: hidden % 8 == 0).
+//
+// Latency-bound for a decode batch (a row per block, a few dozen blocks), bandwidth-bound for a prompt. A
+// thread keeps its NE elements (stride blockDim: coalesced whatever the alignment) in registers between the sum
+// of squares and the scaling, so a row costs one round trip with every load in flight; the form that walked the
+// row in a loop and re-read it took 20 us for 64 rows of 8192 and 67 us (2.5 TB/s) for 2048 of them.
+template <bool ACT, int NE>
+__global__ void __launch_bounds__(1024)
+add_rms_norm_kernel(const float *x, const float *__restrict__ delta, const float *__restrict__ gamma, float eps,
+                    int hidden, float *x_out, void *__restrict__ normed) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float red[8];
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * hidden;
+    float v[NE], g[NE];
+#pragma unroll
+    for (int j = 0; j < NE; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j] = i < hidden ? x[base + i] : 0.0f;
+        g[j] = i < hidden ? __ldg(gamma + i) : 0.0f;
+    }
+    if (delta) {
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i < hidden) v[j] += __ldg(delta + base + i);
+        }
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < NE; ++j) ss = fmaf(v[j], v[j], ss);
+    if (x_out) {
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i < hidden) x_out[base + i] = v[j];
+        }
+    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll
+    for (int j = 0; j < NE; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < hidden) {
+            const float n = (v[j] * inv) * g[j];
+            if constexpr (ACT)
+                static_cast<__nv_bfloat16 *>(normed)[base + (i & ~7) + gemm_order_pos(i & 7)] = __float2bfloat16_rn(n);
+            else
+                static_cast<float *>(normed)[base + i] = n;
+        }
+    }
+}
+
+// The same for rows longer than 16384: the row is walked in a loop and read again for the scaling
+template <bool ACT>
+__global__ void __launch_bounds__(1024)
+add_rms_norm_long_kernel(const float *x, const float *__restrict__ delta, const float *__restrict__ gamma, float eps,
+                         int hidden, float *x_out, void *__restrict__ normed) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * hidden;
     float ss = 0.0f;
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
@@ -127,43 +151,67 @@ add_rms_norm_act_kernel(const float *x, const float *__restrict__ delta, const f
         if (x_out) x_out[base + i] = v;
         ss = fmaf(v, v, ss);
     }
-    const float total = block_sum(ss, red);
-    const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
-    if (x_out) __syncthreads();   // the second pass reads elements other threads wrote
-    for (int g8 = threadIdx.x; g8 < hidden / 8; g8 += blockDim.x) {
-        float n[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int i = g8 * 8 + j;
-            float v;
-            if (x_out) {
-                v = x_out[base + i];
-            } else {
-                v = x[base + i];
-                if (delta) v += delta[base + i];
-            }
-            n[j] = (v * inv) * gamma[i];
-        }
-        normed_act[base / 8 + g8] = pack_bf16_gemm_order(n);
+    const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)hidden + eps);
+    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
+        // x_out may alias x (in-place residual update): read the sum back instead of adding twice; every
+        // thread re-reads exactly the elements it wrote
+        float v = x_out ? x_out[base + i] : x[base + i];
+        if (!x_out && delta) v += delta[base + i];
+        const float n = (v * inv) * gamma[i];
+        if constexpr (ACT)
+            static_cast<__nv_bfloat16 *>(normed)[base + (i & ~7) + gemm_order_pos(i & 7)] = __float2bfloat16_rn(n);
+        else
+            static_cast<float *>(normed)[base + i] = n;
     }
 }
 
-// swiglu_kernel with the result written as bf16 activations of the next prefill-shaped linear (inter % 8 == 0)
-__global__ void swiglu_act_kernel(const float *__restrict__ gu, uint4 *__restrict__ out_act, size_t rows, int inter) {
+// gate_up rows: [gate (inter) | up (inter)] -> silu(gate) * up, as fp32 or (ACT) as the bf16 activations of
+// the next prefill-shaped linear. Bandwidth-bound: eight values per thread and step, 128-bit accesses
+// (inter % 8 == 0, 16-byte aligned operands; swiglu_any_kernel takes the rest).
+__device__ __forceinline__ float swiglu_one(float g, float u) {
+    const float s = 1.0f / (1.0f + expf(-g));
+    return (g * s) * u;
+}
+template <bool ACT>
+__global__ void __launch_bounds__(256)
+swiglu_kernel(const float *__restrict__ gu, void *__restrict__ out, int rows, int inter) {
     pdl_wait();
     pdl_trigger();
-    const size_t total8 = rows * (size_t)(inter / 8);
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / (inter / 8);
-        const int c = (int)(i % (inter / 8)) * 8;
-        float n[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float g = gu[r * 2 * inter + c + j], u = gu[r * 2 * inter + inter + c + j];
-            const float sg = 1.0f / (1.0f + expf(-g));
-            n[j] = (g * sg) * u;
+    const int n8 = inter / 8;
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+        const float4 *grow = reinterpret_cast<const float4 *>(gu + (size_t)r * 2 * inter);
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n8; c += gridDim.x * blockDim.x) {
+            const float4 ga = __ldg(grow + 2 * c), gb = __ldg(grow + 2 * c + 1);
+            const float4 ua = __ldg(grow + 2 * (n8 + c)), ub = __ldg(grow + 2 * (n8 + c) + 1);
+            const float n[8] = {swiglu_one(ga.x, ua.x), swiglu_one(ga.y, ua.y), swiglu_one(ga.z, ua.z), swiglu_one(ga.w, ua.w),
+                                swiglu_one(gb.x, ub.x), swiglu_one(gb.y, ub.y), swiglu_one(gb.z, ub.z), swiglu_one(gb.w, ub.w)};
+            if constexpr (ACT) {
+                reinterpret_cast<uint4 *>(out)[(size_t)r * n8 + c] = pack_bf16_gemm_order(n);
+            } else {
+                float4 *o = reinterpret_cast<float4 *>(out) + 2 * ((size_t)r * n8 + c);
+                o[0] = make_float4(n[0], n[1], n[2], n[3]);
+                o[1] = make_float4(n[4], n[5], n[6], n[7]);
+            }
         }
-        out_act[i] = pack_bf16_gemm_order(n);
+    }
+}
+// any inter (ACT: a multiple of 8), any alignment of gate_up
+template <bool ACT>
+__global__ void swiglu_any_kernel(const float *__restrict__ gu, void *__restrict__ out, size_t rows, int inter) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int V = ACT ? 8 : 1;
+    const size_t total = rows * (size_t)(inter / V);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / (inter / V);
+        const int c = (int)(i % (inter / V)) * V;
+        float n[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) n[j] = swiglu_one(gu[r * 2 * inter + c + j], gu[r * 2 * inter + inter + c + j]);
+        if constexpr (ACT)
+            reinterpret_cast<uint4 *>(out)[i] = pack_bf16_gemm_order(n);
+        else
+            static_cast<float *>(out)[i] = n[0];
     }
 }
 
@@ -179,85 +227,123 @@ __device__ __forceinline__ float kv_get<int8_t>(const int8_t *row, int i, float 
     return __fmul_rn((float)row[i], scale);
 }
 
-// LayerStorage::append for KvDtype::I8 (kv_cache.rs:44-60) on one row held in `src` (global or
-// shared memory): scale = abs_max / 127 (1.0 when abs_max <= f32::EPSILON), inv = 1 / scale,
-// q = clamp(round_half_away(v * inv), -127, 127). Every thread of the block calls it.
-__device__ __forceinline__ void kv_quantize_row(const float *src, int len, int8_t *dst, float *scale_out,
-                                                float *red) {
-    float amax = 0.0f;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) amax = fmaxf(amax, fabsf(src[i]));
-    amax = block_max(amax, red);
-    const float scale = (amax <= 1.1920929e-07f) ? 1.0f : __fdiv_rn(amax, 127.0f);
-    const float inv = __fdiv_rn(1.0f, scale);
-    if (threadIdx.x == 0) *scale_out = scale;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) {
-        const float x = __fmul_rn(src[i], inv);
-        // NaN -> 0, as Rust's saturating float-to-int cast does
-        dst[i] = (x != x) ? (int8_t)0 : (int8_t)(int)fminf(fmaxf(roundf(x), -127.0f), 127.0f);
-    }
-    __syncthreads();  // `red` and `src` may be reused by the caller
-}
-
 // qkv rows: [q (n_q*d) | k (n_kv*d) | v (n_kv*d)], row r = b*seq + s at position *pos + s.
 // Rotates q in place, writes rotated k and v into the cache at [b][position][head][d]
 // (f32), or quantised per row with their scales at [b][position] (int8). A position outside
 // [0, max_seq) appends nothing and raises YSCV_DEV_POS_OVERFLOW in the status word.
-// Dynamic shared memory: d floats of rotary factors (+ n_kv*d floats of rotated keys, int8).
-template <typename KV>
-__global__ void rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d,
-                                      float theta, const int32_t *__restrict__ pos,
-                                      KV *__restrict__ kc, KV *__restrict__ vc,
-                                      float *__restrict__ kscale, float *__restrict__ vscale,
-                                      int max_seq, int *__restrict__ status) {
+//
+// Latency-bound: block (row, part) takes one part of a row: 0 its keys, 1 its values, 2.. pieces of up to
+// ROPE_ITEMS x V query pairs, so that a thread has all its loads in flight at once and a decode batch fills
+// more SMs than it has rows (one block per row, scalar accesses: 29 us for 64 rows of 64 + 16 heads of 128,
+// 10 us for 32 rows of 32 + 8 heads of 64). The frequencies need only theta and are formed while the
+// predecessor drains. V = pairs per thread and access: 4 where d % 8 == 0 and the rows are 16-byte aligned.
+//
+// int8 rows are LayerStorage::append for KvDtype::I8 (kv_cache.rs:44-60): scale = abs_max / 127 (1.0 when
+// abs_max <= f32::EPSILON), inv = 1 / scale, q = clamp(round_half_away(v * inv), -127, 127).
+// Dynamic shared memory: d floats of rotary factors (+ n_kv*d floats of the row to quantise, int8).
+constexpr int ROPE_THREADS = 256, ROPE_ITEMS = 1024;
+template <int V> struct RopeVec;
+template <> struct RopeVec<4> { using T = float4; };
+template <> struct RopeVec<1> { using T = float; };
+template <typename KV, int V>
+__global__ void __launch_bounds__(ROPE_THREADS)
+rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d, float theta,
+                      const int32_t *__restrict__ pos, KV *__restrict__ kc, KV *__restrict__ vc,
+                      float *__restrict__ kscale, float *__restrict__ vscale, int max_seq, int *__restrict__ status) {
+    constexpr bool I8 = sizeof(KV) == 1;
+    using VT = typename RopeVec<V>::T;
+    extern __shared__ __align__(16) float rsm[];
+    __shared__ float red[8];
+    const int half = d / 2, hv = half / V;
+    float *cs_tab = rsm, *sn_tab = rsm + half, *row_sm = rsm + d;
+    const int part = blockIdx.y;
+    if (part != 1)
+        for (int i = threadIdx.x; i < half; i += blockDim.x) cs_tab[i] = 1.0f / powf(theta, 2.0f * (float)i / (float)d);
     pdl_wait();
     pdl_trigger();
-    constexpr bool I8 = sizeof(KV) == 1;
-    extern __shared__ float rsm[];
-    __shared__ float red[8];
-    const int half = d / 2;
-    float *cs_tab = rsm, *sn_tab = rsm + half, *krow = rsm + d;
     const int row = blockIdx.x, b = row / seq, s = row % seq;
     const int p = *pos + s;
     const bool in_range = p >= 0 && p < max_seq;
-    if (!in_range && threadIdx.x == 0) *status = YSCV_DEV_POS_OVERFLOW;
-    const int row_w = (n_q + 2 * n_kv) * d;
-    float *r = qkv + (size_t)row * row_w;
-    const float fp = (float)p;
-    // the angle of pair i is the same for every head: one table per row
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        const float inv_freq = 1.0f / powf(theta, 2.0f * (float)i / (float)d);
-        sincosf(inv_freq * fp, &sn_tab[i], &cs_tab[i]);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < (n_q + n_kv) * half; idx += blockDim.x) {
-        const int h = idx / half, i = idx % half;
-        const float cs = cs_tab[i], sn = sn_tab[i];
-        float *v = r + (size_t)h * d;
-        const float x0 = v[i], x1 = v[i + half];
-        const float y0 = x0 * cs - x1 * sn, y1 = x0 * sn + x1 * cs;
-        if (h < n_q) {
-            v[i] = y0;
-            v[i + half] = y1;
-        } else if constexpr (I8) {
-            krow[(h - n_q) * d + i] = y0;
-            krow[(h - n_q) * d + i + half] = y1;
-        } else if (in_range) {
-            float *dst = reinterpret_cast<float *>(kc) + (((size_t)b * max_seq + p) * n_kv + (h - n_q)) * d;
-            dst[i] = y0;
-            dst[i + half] = y1;
+    if (!in_range && part == 0 && threadIdx.x == 0) *status = YSCV_DEV_POS_OVERFLOW;
+    float *r = qkv + (size_t)row * (n_q + 2 * n_kv) * d;
+    const int kv_n = n_kv * d;
+    const size_t slot = (size_t)b * max_seq + (in_range ? p : 0);
+    if (part != 1) {
+        // the angle of pair i is the same for every head: one table per block
+        const float fp = (float)p;
+        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            const float a = cs_tab[i] * fp;
+            sincosf(a, &sn_tab[i], &cs_tab[i]);
+        }
+        __syncthreads();
+        const int first = part == 0 ? 0 : (part - 2) * ROPE_ITEMS;
+        const int n_items = part == 0 ? n_kv * hv : min(n_q * hv - first, ROPE_ITEMS);
+        const float *src = part == 0 ? r + (size_t)n_q * d : r;
+        float *dst = part == 0 ? (I8 ? row_sm : reinterpret_cast<float *>(kc) + slot * kv_n) : r;
+        for (int i0 = threadIdx.x; i0 < n_items; i0 += 4 * ROPE_THREADS) {
+            VT x0[4], x1[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int idx = i0 + u * ROPE_THREADS + first;
+                if (i0 + u * ROPE_THREADS < n_items) {
+                    const float *v = src + (size_t)(idx / hv) * d + (idx % hv) * V;
+                    x0[u] = *reinterpret_cast<const VT *>(v);
+                    x1[u] = *reinterpret_cast<const VT *>(v + half);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int idx = i0 + u * ROPE_THREADS + first;
+                if (i0 + u * ROPE_THREADS < n_items && (part != 0 || I8 || in_range)) {
+                    const int i = (idx % hv) * V;
+                    VT y0, y1;
+                    const float *a0 = reinterpret_cast<const float *>(&x0[u]), *a1 = reinterpret_cast<const float *>(&x1[u]);
+                    float *o0 = reinterpret_cast<float *>(&y0), *o1 = reinterpret_cast<float *>(&y1);
+#pragma unroll
+                    for (int j = 0; j < V; ++j) {
+                        const float cs = cs_tab[i + j], sn = sn_tab[i + j];
+                        // each product rounded, as the reference rounds it (rope.rs:24-117)
+                        o0[j] = __fsub_rn(__fmul_rn(a0[j], cs), __fmul_rn(a1[j], sn));
+                        o1[j] = __fadd_rn(__fmul_rn(a0[j], sn), __fmul_rn(a1[j], cs));
+                    }
+                    float *v = dst + (size_t)(idx / hv) * d + i;
+                    *reinterpret_cast<VT *>(v) = y0;
+                    *reinterpret_cast<VT *>(v + half) = y1;
+                }
+            }
         }
     }
+    if (part > 1 || !in_range) return;   // (uniform across the block)
     const float *vsrc = r + (size_t)(n_q + n_kv) * d;
     if constexpr (I8) {
+        if (part == 1)
+            for (int i = threadIdx.x * V; i < kv_n; i += blockDim.x * V)
+                *reinterpret_cast<VT *>(row_sm + i) = *reinterpret_cast<const VT *>(vsrc + i);
         __syncthreads();
-        if (in_range) {  // (uniform across the block)
-            const size_t slot = (size_t)b * max_seq + p;
-            kv_quantize_row(krow, n_kv * d, reinterpret_cast<int8_t *>(kc) + slot * n_kv * d, kscale + slot, red);
-            kv_quantize_row(vsrc, n_kv * d, reinterpret_cast<int8_t *>(vc) + slot * n_kv * d, vscale + slot, red);
+        float amax = 0.0f;
+        for (int i = threadIdx.x; i < kv_n; i += blockDim.x) amax = fmaxf(amax, fabsf(row_sm[i]));
+        amax = block_max(amax, red);
+        const float scale = (amax <= 1.1920929e-07f) ? 1.0f : __fdiv_rn(amax, 127.0f);
+        const float inv = __fdiv_rn(1.0f, scale);
+        if (threadIdx.x == 0) (part == 0 ? kscale : vscale)[slot] = scale;
+        int8_t *dst = reinterpret_cast<int8_t *>(part == 0 ? kc : vc) + slot * kv_n;
+        for (int i = threadIdx.x * V; i < kv_n; i += blockDim.x * V) {
+            int8_t o[V];
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const float x = __fmul_rn(row_sm[i + j], inv);
+                // NaN -> 0, as Rust's saturating float-to-int cast does
+                o[j] = (x != x) ? (int8_t)0 : (int8_t)(int)fminf(fmaxf(roundf(x), -127.0f), 127.0f);
+            }
+            if constexpr (V == 4)
+                *reinterpret_cast<char4 *>(dst + i) = make_char4(o[0], o[1], o[2], o[3]);
+            else
+                dst[i] = o[0];
         }
-    } else if (in_range) {
-        float *vdst = reinterpret_cast<float *>(vc) + ((size_t)b * max_seq + p) * n_kv * d;
-        for (int i = threadIdx.x; i < n_kv * d; i += blockDim.x) vdst[i] = vsrc[i];
+    } else if (part == 1) {
+        float *vdst = reinterpret_cast<float *>(vc) + slot * kv_n;
+        for (int i = threadIdx.x * V; i < kv_n; i += blockDim.x * V)
+            *reinterpret_cast<VT *>(vdst + i) = *reinterpret_cast<const VT *>(vsrc + i);
     }
 }
 
@@ -919,22 +1005,6 @@ __global__ void attention_combine_kernel(const float *__restrict__ part, int n_s
     }
 }
 
-// gate_up rows: [gate (inter) | up (inter)] -> out = silu(gate) * up
-__global__ void swiglu_kernel(const float *__restrict__ gu, float *__restrict__ out, size_t rows,
-                              int inter) {
-    pdl_wait();
-    pdl_trigger();
-    const size_t total = rows * (size_t)inter;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / inter;
-        const int c = (int)(i % inter);
-        const float g = gu[r * 2 * inter + c], u = gu[r * 2 * inter + inter + c];
-        const float s = 1.0f / (1.0f + expf(-g));
-        out[i] = (g * s) * u;
-    }
-}
-
 // out[m][n] = sum_k x[m][k] * w[n][k]; one warp per weight row, up to 4 x rows per pass
 template <int MT>
 __global__ void __launch_bounds__(256)
@@ -1155,15 +1225,27 @@ int yscv_cuda_embedding_dev(yscv_cuda_ctx *ctx, const float *d_weight, size_t vo
     DEC_EPILOGUE(ctx, "embedding");
 }
 
+}  // extern "C"
+
+template <bool ACT>
+static int add_rms_norm_impl(yscv_cuda_ctx *ctx, const float *x, const float *delta, const float *gamma, float eps,
+                             size_t rows, size_t hidden, float *x_out, void *normed) {
+    if (rows == 0) return YSCV_CUDA_OK;
+    // eight elements per thread: 256 threads are enough up to 2048, 1024 up to 8192; sixteen up to 16384
+    const unsigned threads = hidden <= 2048 ? 256u : 1024u;
+    auto kern = hidden <= 8192 ? add_rms_norm_kernel<ACT, 8> : hidden <= 16384 ? add_rms_norm_kernel<ACT, 16> : add_rms_norm_long_kernel<ACT>;
+    YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)rows), dim3(threads), 0, ctx->stream, x, delta, gamma, eps, (int)hidden, x_out, normed));
+    DEC_EPILOGUE(ctx, ACT ? "add_rms_norm(bf16 activations out)" : "add_rms_norm");
+}
+
+extern "C" {
+
 int yscv_cuda_add_rms_norm_dev(yscv_cuda_ctx *ctx, const float *d_x, const float *d_delta,
                                const float *d_gamma, float eps, size_t rows, size_t hidden,
                                float *d_x_out, float *d_normed) {
     DEC_PROLOGUE(ctx);
     if (!d_x || !d_gamma || !d_normed) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
-    if (rows == 0) return YSCV_CUDA_OK;
-    YSCV_CUDA_TRY(launch_pdl(add_rms_norm_kernel, dim3((unsigned)rows), dim3(256), 0, ctx->stream, d_x, d_delta, d_gamma, eps, (int)hidden,
-                                                                 d_x_out, d_normed));
-    DEC_EPILOGUE(ctx, "add_rms_norm");
+    return add_rms_norm_impl<false>(ctx, d_x, d_delta, d_gamma, eps, rows, hidden, d_x_out, d_normed);
 }
 
 }  // extern "C"
@@ -1182,9 +1264,14 @@ static int rope_kv_append_impl(yscv_cuda_ctx *ctx, float *d_qkv, size_t batch, s
     const size_t smem = (d_head + (sizeof(KV) == 1 ? n_kv * d_head : 0)) * sizeof(float);
     if (smem > 48 * 1024)
         return fail(YSCV_CUDA_ERR_UNSUPPORTED, "RoPE tables for d_head=%zu, n_kv=%zu do not fit shared memory", d_head, n_kv);
-    YSCV_CUDA_TRY(launch_pdl(rope_kv_append_kernel<KV>, dim3((unsigned)(batch * seq)), dim3(128), smem, ctx->stream,
-                             d_qkv, (int)seq, (int)n_q, (int)n_kv, (int)d_head, theta, d_pos, d_kcache, d_vcache,
-                             d_kscale, d_vscale, (int)max_seq, ctx->d_status));
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(d_qkv) | reinterpret_cast<uintptr_t>(d_kcache) | reinterpret_cast<uintptr_t>(d_vcache);
+    const bool vec = d_head % 8 == 0 && (ptrs & 15) == 0;
+    const size_t q_items = n_q * (d_head / 2) / (vec ? 4 : 1);
+    const dim3 grid((unsigned)(batch * seq), (unsigned)(2 + (q_items + ROPE_ITEMS - 1) / ROPE_ITEMS));
+    auto kern = vec ? rope_kv_append_kernel<KV, 4> : rope_kv_append_kernel<KV, 1>;
+    YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(ROPE_THREADS), smem, ctx->stream, d_qkv, (int)seq, (int)n_q,
+                             (int)n_kv, (int)d_head, theta, d_pos, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq,
+                             ctx->d_status));
     DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "rope_kv_append(int8 cache)" : "rope_kv_append");
 }
 
@@ -1316,15 +1403,29 @@ int yscv_cuda_gqa_attention_i8_dev(yscv_cuda_ctx *ctx, const float *d_q, size_t 
                                       d_vscale, max_seq, d_pos, causal, d_out);
 }
 
+}  // extern "C"
+
+template <bool ACT>
+static int swiglu_impl(yscv_cuda_ctx *ctx, const float *gate_up, size_t rows, size_t inter, void *out) {
+    if (rows * inter == 0) return YSCV_CUDA_OK;
+    if (inter % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+        const dim3 grid((unsigned)((inter / 8 + 255) / 256), (unsigned)(rows < 32768 ? rows : 32768));
+        YSCV_CUDA_TRY(launch_pdl(swiglu_kernel<ACT>, grid, dim3(256), 0, ctx->stream, gate_up, out, (int)rows, (int)inter));
+    } else {
+        const size_t total = rows * (inter / (ACT ? 8 : 1));
+        const unsigned blocks = (unsigned)((total + 255) / 256 < 65535 ? (total + 255) / 256 : 65535);
+        YSCV_CUDA_TRY(launch_pdl(swiglu_any_kernel<ACT>, dim3(blocks), dim3(256), 0, ctx->stream, gate_up, out, rows, (int)inter));
+    }
+    DEC_EPILOGUE(ctx, ACT ? "swiglu(bf16 activations out)" : "swiglu");
+}
+
+extern "C" {
+
 int yscv_cuda_swiglu_dev(yscv_cuda_ctx *ctx, const float *d_gate_up, size_t rows, size_t inter,
                          float *d_out) {
     DEC_PROLOGUE(ctx);
     if (!d_gate_up || !d_out) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
-    if (rows * inter == 0) return YSCV_CUDA_OK;
-    const size_t total = rows * inter;
-    const unsigned blocks = (unsigned)((total + 255) / 256 < 65535 ? (total + 255) / 256 : 65535);
-    YSCV_CUDA_TRY(launch_pdl(swiglu_kernel, dim3(blocks), dim3(256), 0, ctx->stream, d_gate_up, d_out, rows, (int)inter));
-    DEC_EPILOGUE(ctx, "swiglu");
+    return swiglu_impl<false>(ctx, d_gate_up, rows, inter, d_out);
 }
 
 int yscv_cuda_add_rms_norm_act_dev(yscv_cuda_ctx *ctx, const float *d_x, const float *d_delta, const float *d_gamma,
@@ -1333,10 +1434,7 @@ int yscv_cuda_add_rms_norm_act_dev(yscv_cuda_ctx *ctx, const float *d_x, const f
     if (!d_x || !d_gamma || !d_normed_act) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
     if (hidden % 8 != 0 || (reinterpret_cast<uintptr_t>(d_normed_act) & 15))
         return fail(YSCV_CUDA_ERR_UNSUPPORTED, "hidden must be a multiple of 8 and the activation buffer 16-byte aligned");
-    if (rows == 0) return YSCV_CUDA_OK;
-    YSCV_CUDA_TRY(launch_pdl(add_rms_norm_act_kernel, dim3((unsigned)rows), dim3(256), 0, ctx->stream, d_x, d_delta, d_gamma, eps,
-                             (int)hidden, d_x_out, reinterpret_cast<uint4 *>(d_normed_act)));
-    DEC_EPILOGUE(ctx, "add_rms_norm(bf16 activations out)");
+    return add_rms_norm_impl<true>(ctx, d_x, d_delta, d_gamma, eps, rows, hidden, d_x_out, d_normed_act);
 }
 
 int yscv_cuda_swiglu_act_dev(yscv_cuda_ctx *ctx, const float *d_gate_up, size_t rows, size_t inter, void *d_out_act) {
@@ -1344,12 +1442,7 @@ int yscv_cuda_swiglu_act_dev(yscv_cuda_ctx *ctx, const float *d_gate_up, size_t 
     if (!d_gate_up || !d_out_act) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
     if (inter % 8 != 0 || (reinterpret_cast<uintptr_t>(d_out_act) & 15))
         return fail(YSCV_CUDA_ERR_UNSUPPORTED, "inter must be a multiple of 8 and the activation buffer 16-byte aligned");
-    if (rows * inter == 0) return YSCV_CUDA_OK;
-    const size_t total8 = rows * (inter / 8);
-    const unsigned blocks = (unsigned)((total8 + 255) / 256 < 65535 ? (total8 + 255) / 256 : 65535);
-    YSCV_CUDA_TRY(launch_pdl(swiglu_act_kernel, dim3(blocks), dim3(256), 0, ctx->stream, d_gate_up,
-                             reinterpret_cast<uint4 *>(d_out_act), rows, (int)inter));
-    DEC_EPILOGUE(ctx, "swiglu(bf16 activations out)");
+    return swiglu_impl<true>(ctx, d_gate_up, rows, inter, d_out_act);
 }
 
 int yscv_cuda_f32_matmul_dev(yscv_cuda_ctx *ctx, const float *d_w, const float *d_x, size_t m, size_t n,
