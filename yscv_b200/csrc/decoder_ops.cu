@@ -405,209 +405,6 @@ gqa_attention_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n
     }
 }
 
-// Prompt-pass attention (many query positions per sequence): the kernel above reads every key and
-// value row of a sequence once per (query position, query head), from L2: 137 GB per layer for a
-// 2048-token prompt at the 70B shape. Here a block takes QB consecutive query positions x all the
-// query heads of ONE KV head, 64 (position, head) pairs, four per warp, and walks the keys in chunks
-// of 64 rows staged in shared memory (dequantised on the way in for int8 caches), so a row is read
-// from L2 once per block. Scores: a lane per key (its row read 16 bytes at a time, the four query
-// rows broadcast from shared memory: every key value read feeds four FMAs). Weighted value sum: a
-// lane owns four consecutive elements of the head (with D = 64 the half warps take alternate keys),
-// every value read again feeds four FMAs. Each pair keeps a running maximum, exp-sum and
-// unnormalised output (the usual max-rescaling of a chunked softmax).
-// D = head size (64 or 128); dynamic shared memory: keys [64][D + 4], values [64][D], weights
-// [pairs][64], query rows [pairs][D].
-constexpr int PF_KT = 64;      // keys per chunk
-constexpr int PF_QH = 4;       // (position, head) pairs per warp
-template <typename KV, int D>
-__global__ void __launch_bounds__(512, 1)
-gqa_prefill_tiled_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n_q, int n_kv,
-                         const KV *__restrict__ kc, const KV *__restrict__ vc,
-                         const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
-                         const int32_t *__restrict__ pos, int causal, float *__restrict__ out, int QB) {
-    pdl_wait();
-    pdl_trigger();
-    constexpr bool I8 = sizeof(KV) == 1;
-    constexpr int KP = D + 4;   // key row pitch: a lane per key reads its row 16 bytes at a time without bank conflicts
-    constexpr int KPAR = 32 / (D / 4);
-    extern __shared__ __align__(16) float pf_sm[];
-    const int n_pairs = (blockDim.x >> 5) * PF_QH;
-    float *ks = pf_sm, *vs = pf_sm + PF_KT * KP, *sc_all = vs + PF_KT * D;
-    float *qs_all = sc_all + n_pairs * PF_KT;
-    const int G = n_q / n_kv;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kv_h = blockIdx.y, b = blockIdx.z;
-    const int p0 = *pos;
-    auto limit_of = [&](int s) {
-        const int l = p0 + (causal ? s + 1 : seq_q);
-        return l > max_seq ? max_seq : (l < 0 ? 0 : l);
-    };
-    // this warp's pairs: index warp * 4 + j -> head idx % G of the group, position idx / G of the tile
-    int sq[PF_QH], qh[PF_QH], lim[PF_QH];
-    bool live[PF_QH];
-    int warp_limit = 0;
-#pragma unroll
-    for (int j = 0; j < PF_QH; ++j) {
-        const int idx = warp * PF_QH + j;
-        sq[j] = blockIdx.x * QB + idx / G;
-        qh[j] = kv_h * G + idx % G;
-        live[j] = idx < G * QB && sq[j] < seq_q;
-        lim[j] = live[j] ? limit_of(sq[j]) : 0;
-        warp_limit = max(warp_limit, lim[j]);
-    }
-    const int last_sq = min(seq_q, ((int)blockIdx.x + 1) * QB) - 1;
-    const int block_limit = limit_of(last_sq);   // limits do not decrease with the position
-    const float scale = 1.0f / sqrtf((float)D);
-    const int e4 = (lane % (D / 4)) * 4, kpar = lane / (D / 4);
-    float4 acc[PF_QH];
-    float m[PF_QH], l[PF_QH];
-    float *sc = sc_all + warp * PF_QH * PF_KT, *qs = qs_all + warp * PF_QH * D;
-#pragma unroll
-    for (int j = 0; j < PF_QH; ++j) {
-        acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        m[j] = -INFINITY;
-        l[j] = 0.0f;
-        for (int i = lane; i < D; i += 32)
-            qs[j * D + i] = live[j] ? q[((size_t)b * seq_q + sq[j]) * q_stride + (size_t)qh[j] * D + i] : 0.0f;
-    }
-    __syncwarp();
-    const size_t row_elems = (size_t)n_kv * D;
-    const KV *kb = kc + (size_t)b * max_seq * row_elems + (size_t)kv_h * D;
-    const KV *vb = vc + (size_t)b * max_seq * row_elems + (size_t)kv_h * D;
-    for (int c0 = 0; c0 < block_limit; c0 += PF_KT) {
-        const int rows = min(PF_KT, block_limit - c0);
-        // stage the chunk: 4 values per thread and step
-        for (int idx = threadIdx.x; idx < rows * (D / 4); idx += blockDim.x) {
-            const int r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
-            const size_t off = (size_t)(c0 + r) * row_elems + c4;
-            float4 kv4, vv4;
-            if constexpr (I8) {
-                const float rk = kscale[(size_t)b * max_seq + c0 + r], rv = vscale[(size_t)b * max_seq + c0 + r];
-                const char4 k4 = *reinterpret_cast<const char4 *>(kb + off), v4 = *reinterpret_cast<const char4 *>(vb + off);
-                kv4 = make_float4(__fmul_rn((float)k4.x, rk), __fmul_rn((float)k4.y, rk), __fmul_rn((float)k4.z, rk), __fmul_rn((float)k4.w, rk));
-                vv4 = make_float4(__fmul_rn((float)v4.x, rv), __fmul_rn((float)v4.y, rv), __fmul_rn((float)v4.z, rv), __fmul_rn((float)v4.w, rv));
-            } else {
-                kv4 = *reinterpret_cast<const float4 *>(kb + off);
-                vv4 = *reinterpret_cast<const float4 *>(vb + off);
-            }
-            *reinterpret_cast<float4 *>(ks + r * KP + c4) = kv4;
-            *reinterpret_cast<float4 *>(vs + r * D + c4) = vv4;
-        }
-        __syncthreads();
-        const int nkw = min(rows, warp_limit - c0);   // keys of this chunk any of the warp's pairs attends to
-        if (nkw > 0) {
-            // scores: a lane per key (keys lane and lane + 32 of the chunk); a query piece read once for both keys
-            float sv[2][PF_QH];
-            {
-                float dot[2][PF_QH];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int j = 0; j < PF_QH; ++j) dot[h][j] = 0.0f;
-                const float4 *kr0 = reinterpret_cast<const float4 *>(ks + lane * KP);
-                const float4 *kr1 = reinterpret_cast<const float4 *>(ks + (lane + 32) * KP);
-                if (nkw > 32) {   // the same for the whole warp
-#pragma unroll 2
-                    for (int i = 0; i < D / 4; ++i) {
-                        const float4 k0 = kr0[i], k1 = kr1[i];
-#pragma unroll
-                        for (int j = 0; j < PF_QH; ++j) {
-                            const float4 a = reinterpret_cast<const float4 *>(qs + j * D)[i];
-                            dot[0][j] = fmaf(a.x, k0.x, dot[0][j]);
-                            dot[0][j] = fmaf(a.y, k0.y, dot[0][j]);
-                            dot[0][j] = fmaf(a.z, k0.z, dot[0][j]);
-                            dot[0][j] = fmaf(a.w, k0.w, dot[0][j]);
-                            dot[1][j] = fmaf(a.x, k1.x, dot[1][j]);
-                            dot[1][j] = fmaf(a.y, k1.y, dot[1][j]);
-                            dot[1][j] = fmaf(a.z, k1.z, dot[1][j]);
-                            dot[1][j] = fmaf(a.w, k1.w, dot[1][j]);
-                        }
-                    }
-                } else {
-#pragma unroll 4
-                    for (int i = 0; i < D / 4; ++i) {
-                        const float4 k0 = kr0[i];
-#pragma unroll
-                        for (int j = 0; j < PF_QH; ++j) {
-                            const float4 a = reinterpret_cast<const float4 *>(qs + j * D)[i];
-                            dot[0][j] = fmaf(a.x, k0.x, dot[0][j]);
-                            dot[0][j] = fmaf(a.y, k0.y, dot[0][j]);
-                            dot[0][j] = fmaf(a.z, k0.z, dot[0][j]);
-                            dot[0][j] = fmaf(a.w, k0.w, dot[0][j]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int k = lane + 32 * h;
-#pragma unroll
-                    for (int j = 0; j < PF_QH; ++j)
-                        sv[h][j] = k < lim[j] - c0 && k < rows ? dot[h][j] * scale : -INFINITY;   // rows past the limit hold stale values
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < PF_QH; ++j) {
-                float cm = fmaxf(sv[0][j], sv[1][j]);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-                const float m_new = fmaxf(m[j], cm);
-                // a pair whose limit lies before this chunk keeps its state (m_new == m, nothing added)
-                const float alpha = m_new == -INFINITY ? 1.0f : expf(m[j] - m_new);   // 0 for a pair's first chunk
-                float ps = 0.0f;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float e = sv[h][j] == -INFINITY ? 0.0f : expf(sv[h][j] - m_new);
-                    sc[j * PF_KT + lane + 32 * h] = e;
-                    ps += e;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-                l[j] = l[j] * alpha + ps;
-                acc[j].x *= alpha; acc[j].y *= alpha; acc[j].z *= alpha; acc[j].w *= alpha;
-                m[j] = m_new;
-            }
-            __syncwarp();
-            // weighted value sum: the weights of four consecutive keys of a pair come with one 16-byte read
-            // (weights past nkw are 0 or belong to rows that are not read)
-            for (int k4 = 0; k4 < nkw; k4 += 4 * KPAR) {
-                const int kq = k4 + 4 * kpar;   // this half warp's four keys
-                float4 pj[PF_QH];
-#pragma unroll
-                for (int j = 0; j < PF_QH; ++j) pj[j] = *reinterpret_cast<const float4 *>(sc + j * PF_KT + kq);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (kq + u < nkw) {
-                        const float4 v4 = *reinterpret_cast<const float4 *>(vs + (kq + u) * D + e4);
-#pragma unroll
-                        for (int j = 0; j < PF_QH; ++j) {
-                            const float pk = u == 0 ? pj[j].x : u == 1 ? pj[j].y : u == 2 ? pj[j].z : pj[j].w;
-                            acc[j].x = fmaf(pk, v4.x, acc[j].x);
-                            acc[j].y = fmaf(pk, v4.y, acc[j].y);
-                            acc[j].z = fmaf(pk, v4.z, acc[j].z);
-                            acc[j].w = fmaf(pk, v4.w, acc[j].w);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int j = 0; j < PF_QH; ++j) {
-        if constexpr (KPAR == 2) {
-            acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, 16);
-            acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, 16);
-            acc[j].z += __shfl_xor_sync(0xffffffffu, acc[j].z, 16);
-            acc[j].w += __shfl_xor_sync(0xffffffffu, acc[j].w, 16);
-        }
-        if (live[j] && kpar == 0) {
-            const float inv = l[j] > 0.0f ? 1.0f / l[j] : 0.0f;
-            float *orow = out + ((size_t)b * seq_q + sq[j]) * (size_t)n_q * D + (size_t)qh[j] * D;
-            *reinterpret_cast<float4 *>(orow + e4) = make_float4(acc[j].x * inv, acc[j].y * inv, acc[j].z * inv, acc[j].w * inv);
-        }
-    }
-}
-
 // Decode-shaped attention (one query position per sequence) with the keys split across
 // blocks so that a long cache fills the machine: block (split, kv head, b) handles keys
 // [split*chunk, ...) for ALL the query heads of its KV head's group from one pass over the
@@ -1352,24 +1149,15 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                                                                                                (int)d_head, d_out));
         DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(split-k,int8 cache)" : "gqa_attention(split-k)");
     }
-    // a prompt pass: query positions in tiles, keys and values staged once per tile
+    // a prompt pass: tiles of 128 (position, head) pairs on the tensor cores
     const size_t group = n_q / n_kv;
-    const bool rows_aligned = ((reinterpret_cast<uintptr_t>(d_kcache) | reinterpret_cast<uintptr_t>(d_vcache)) & 15) == 0;
-    if (seq_q >= 16 && (d_head == 64 || d_head == 128) && group <= 64 && rows_aligned &&
-        (reinterpret_cast<uintptr_t>(d_out) & 15) == 0) {
-        // 64 (position, head) pairs per block where the group allows, four per warp
-        const int QB = (int)(64 / group) > 0 ? (int)(64 / group) : 1;
-        const int pairs = (int)group * QB;
-        const int warps = (pairs + PF_QH - 1) / PF_QH;
-        const size_t pf_smem = (PF_KT * (d_head + 4) + PF_KT * d_head + (size_t)warps * PF_QH * (PF_KT + d_head)) * sizeof(float);
-        auto kern = d_head == 64 ? gqa_prefill_tiled_kernel<KV, 64> : gqa_prefill_tiled_kernel<KV, 128>;
-        int arc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 160 * 1024);
-        if (arc) return arc;
-        dim3 pgrid((unsigned)((seq_q + QB - 1) / QB), (unsigned)n_kv, (unsigned)batch);
-        YSCV_CUDA_TRY(launch_pdl(kern, dim3(pgrid), dim3(32 * warps), pf_smem, ctx->stream, d_q, (int)q_stride, (int)seq_q,
-                                 (int)n_q, (int)n_kv, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, causal,
-                                 d_out, QB));
-        DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(prompt tiles,int8 cache)" : "gqa_attention(prompt tiles)");
+    const uintptr_t vec_ptrs = reinterpret_cast<uintptr_t>(d_kcache) | reinterpret_cast<uintptr_t>(d_vcache) | reinterpret_cast<uintptr_t>(d_out);
+    if (seq_q >= 16 && (d_head == 64 || d_head == 128) && group <= 128 && (vec_ptrs & 15) == 0) {
+        const int rc = gqa_prefill_tc<KV>(ctx, d_q, q_stride, batch, seq_q, n_q, n_kv, d_head, d_kcache, d_vcache, d_kscale, d_vscale,
+                                          max_seq, d_pos, causal, d_out);
+        if (rc) return rc;
+        ctx->last_kernel = sizeof(KV) == 1 ? "gqa_attention(prompt tiles,tcgen05,int8 cache)" : "gqa_attention(prompt tiles,tcgen05)";
+        return YSCV_CUDA_OK;
     }
     const size_t smem = (max_seq + d_head) * sizeof(float);
     if (smem > 200 * 1024) return fail(YSCV_CUDA_ERR_UNSUPPORTED, "max_seq %zu too long for the attention kernel", max_seq);

@@ -28,6 +28,13 @@ size_t int4_prefill_scratch_bytes(size_t m, size_t k);
 int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
                       float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16 = nullptr);
 
+// gqa_prefill_tc.cu: attention of seq_q >= 16 query positions per sequence over a cache (KV = float or
+// int8_t), head size 64 or 128, at most 128 query heads per KV head, 16-byte aligned caches and output
+template <typename KV>
+int gqa_prefill_tc(yscv_cuda_ctx *ctx, const float *q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q, size_t n_kv,
+                   size_t d_head, const KV *kc, const KV *vc, const float *kscale, const float *vscale, size_t max_seq,
+                   const int32_t *pos, int causal, float *out);
+
 // int4_pack.cu
 int pack_int4(yscv_cuda_ctx *ctx, const float *d_weights, size_t m_w, size_t k, size_t gs,
               uint8_t *d_packed, float *d_scales);
