@@ -1,0 +1,81 @@
+"""The batched int4 matmul (2..128 activation rows, weights through tensor memory) at the edges of its tiles,
+stages and work split, against float64."""
+import numpy as np
+import pytest
+import torch
+
+import yscv_b200
+
+pytestmark = pytest.mark.gpu
+
+
+def _weights(g, n, k):
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = torch.rand(n, k // 32, device="cuda", generator=g) * 0.02 + 0.001
+    q = torch.stack([packed & 15, packed >> 4], -1).reshape(n, k).to(torch.int16)
+    q = torch.where(q > 7, q - 16, q).double()
+    return packed, scales, q * scales.double().repeat_interleave(32, 1)
+
+
+# (rows, outputs, depth): more work than the dispatch rule asks of each row count; n and k around the
+# 128-row tiles, the 256-k units and the CTA ranges
+CASES = [(m, n, k) for ms, shapes in [
+    ((3, 4), [(25000, 8192)]),
+    ((5, 11, 16), [(16400, 4096), (2300, 29312), (60001, 1152), (600, 110080)]),
+    ((17, 31, 32), [(10300, 2176), (700, 30080), (20000, 1152), (160000, 128)]),
+    ((33, 48, 64), [(12000, 4096), (1700, 28928), (57344, 1280)]),
+    ((65, 100, 128), [(20000, 4096), (2800, 28800), (10241, 8192)]),
+] for m in ms for n, k in shapes]
+
+
+@pytest.mark.parametrize("m,n,k", CASES)
+def test_batch_rows(m, n, k):
+    """Bounds: exact form (m <= 16) 22-bit operands (2^-23 each, relative) and fp32 sums, 1e-6; bf16 form three
+    roundings of 2^-9 (uniform: 1.13e-3 each, 2e-3 together), 4e-3."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m * 7919 + n + k)
+    with torch.cuda.stream(stream):
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g) * torch.exp(2 * torch.randn(1, k, device="cuda", generator=g))
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        first = out.clone()
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        want = x.double() @ w.T
+    stream.synchronize()
+    assert ctx.device_status() == 0
+    assert "tmem" in ctx.last_kernel(), ctx.last_kernel()
+    assert torch.equal(first, out)
+    assert torch.all(out[m] == 7.0)
+    err = float((out[:m].double() - want).norm() / want.norm())
+    assert err <= (1e-6 if m <= 16 else 4e-3), err
+    if n >= 16:
+        rows = (out[:m].double() - want).norm(dim=1) / want.norm(dim=1)
+        assert float(rows.max()) <= (2e-6 if m <= 16 else 8e-3), int(rows.argmax())
+    ctx.close()
+
+
+def test_non_finite_rows_stay_in_their_row():
+    ctx = yscv_b200.Context(0)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    n, k, m = 16400, 4096, 6
+    packed, scales, w = _weights(g, n, k)
+    x = torch.randn(m, k, device="cuda", generator=g)
+    x[1, 700] = float("nan")
+    x[3, 5] = float("inf")
+    x[4] = 0.0
+    out = torch.empty(m, n, device="cuda")
+    torch.cuda.synchronize()
+    h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+    ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+    ctx.synchronize()
+    assert not torch.isfinite(out[1]).any() and not torch.isfinite(out[3]).any()
+    assert torch.all(out[4] == 0.0)
+    keep = [0, 2, 5]
+    want = x[keep].double() @ w.T
+    assert float((out[keep].double() - want).norm() / want.norm()) <= 1e-6
+    ctx.close()

@@ -90,9 +90,17 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
         float *o = d_out + m0 * n;
         const bool aligned = ((reinterpret_cast<uintptr_t>(d_packed) | reinterpret_cast<uintptr_t>(d_scales) |
                                reinterpret_cast<uintptr_t>(a)) & 15) == 0;
-        if (aligned && int4_gemv_fast_supported(mc, n, k, gs)) {
-            rc = ctx->scratch.reserve(int4_gemv_scratch_bytes(16, k));
+        const bool batch = aligned && int4_batch_exact_wins(mc, n, k, gs);
+        if (aligned && (batch || int4_gemv_fast_supported(mc, n, k, gs))) {
+            // (one size for every m up to 16, so that a call never outgrows what another one left)
+            const size_t a_b = int4_gemv_scratch_bytes(16, k), b_b = int4_batch_exact_scratch_bytes(k);
+            rc = ctx->scratch.reserve(a_b > b_b ? a_b : b_b);
             if (rc) return rc;
+        }
+        if (batch) {
+            rc = int4_batch_gemm(ctx, d_packed, d_scales, a, nullptr, o, mc, n, k, ctx->scratch.ptr);
+            op_counters().int4_gemv_calls++;
+        } else if (aligned && int4_gemv_fast_supported(mc, n, k, gs)) {
             rc = int4_gemv_fast(ctx, d_packed, d_scales, a, o, mc, n, k, ctx->scratch.ptr);
             op_counters().int4_gemv_calls++;
         } else {
@@ -162,6 +170,11 @@ static int ctx_create_impl(int device, cudaStream_t stream, bool borrow, yscv_cu
         delete ctx;
         return fail(YSCV_CUDA_ERR_CUDA, "status word: %s", cudaGetErrorString(me));
     }
+    const int rc = ctx->batch_ws.reserve(int4_batch_ws_bytes(ctx->sm_count));
+    if (rc) {
+        yscv_cuda_ctx_destroy(ctx);
+        return rc;
+    }
     *out = ctx;
     return YSCV_CUDA_OK;
 }
@@ -189,6 +202,7 @@ void yscv_cuda_ctx_destroy(yscv_cuda_ctx *ctx) {
     ctx->tmp_bt.release();
     ctx->gemm_ws.release();
     ctx->gemm_flags.release();
+    ctx->batch_ws.release();
     ctx->tmp_colsum.release();
     if (ctx->d_status) cudaFree(ctx->d_status);
     for (auto &ev : ctx->prof_events) {

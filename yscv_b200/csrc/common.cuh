@@ -125,6 +125,9 @@ struct yscv_cuda_ctx {
     yscv::DeviceBuffer gemm_ws, gemm_flags;
     int gemm_epoch = 0;
     bool int8_tail_split = true;
+    // batched decode GEMM (int4_batch_gemm.cu): partial sums of the tiles that several CTAs share.
+    // Sized for every shape and allocated with the context: no call allocates.
+    yscv::DeviceBuffer batch_ws;
     // encoded TMA descriptors of the last few decode GEMV weight matrices (int4_gemv.cu)
     struct TmCacheEntry {
         const void *a = nullptr, *b = nullptr;

@@ -792,7 +792,8 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     p.kb_per = (p.k_blocks + p.ksplit - 1) / p.ksplit;
     p.ksplit = (p.k_blocks + p.kb_per - 1) / p.kb_per;   // no empty slice (33 blocks in 8 slices of 5: seven slices)
     float *kernel_out = out;
-    if (p.ksplit > 1) {
+    const bool batch = int4_batch_bf16_wins(m, n, k, 32);   // up to 128 rows of a large matrix
+    if (p.ksplit > 1 && !batch) {
         rc_ws = ctx->gemm_ws.reserve((size_t)p.ksplit * m * n * sizeof(float));
         if (rc_ws) return rc_ws;
         kernel_out = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
@@ -812,6 +813,8 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
         ctx->launches++;
         abf = mine;
     }
+
+    if (batch) return int4_batch_gemm(ctx, wq, scales, nullptr, abf, out, m, n, k, nullptr);
 
     CUtensorMap tm_w, tm_a;
     int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, (uint32_t)(NA * PG_BM), 32,
