@@ -406,67 +406,121 @@ gqa_attention_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n
 }
 
 // Decode-shaped attention (one query position per sequence) with the keys split across
-// blocks so that a long cache fills the machine: block (split, kv head, b) handles keys
-// [split*chunk, ...) for ALL the query heads of its KV head's group from one pass over the
-// chunk's key and value rows (a row is read once per group, not once per query head), leaves
+// blocks so that a long cache fills the machine: block (split, kv head, b) handles an equal share of
+// the keys in use (at most CH) for ALL the query heads of its KV head's group from one pass over the
+// share's key and value rows (a row is read once per group, not once per query head), leaves
 // per query head an unnormalised partial output, its running max and its exp-sum in `part`;
 // attention_combine_kernel merges the splits (the usual max-rescaling of a split softmax).
-// Query heads are taken eight at a time. d % 16 == 0, d <= 128, blockDim.x == chunk == 128.
-// Dynamic shared memory: q [8][d], weights [8][chunk], partial sums [128 / (d/4)][8][d].
-template <typename KV>
-__global__ void __launch_bounds__(128)
+// Query heads are taken eight at a time. d % 16 == 0, d <= 128, 256 threads, n_splits * CH >= max_seq.
+//
+// Bound by the latency of its phases, not by the cache's bytes (32 sequences x 200 keys of the 1B head
+// shape are 13 MB). So the whole share is brought to shared memory by asynchronous copies issued at once
+// (keys and values: one memory latency), and the softmax takes one warp per head (two block barriers in
+// all; one block-wide maximum and sum per head were 32): 25.6 -> 14.6 us for that shape.
+constexpr int DEC_HB = 8;
+constexpr int DEC_THREADS = 256;
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+
+template <typename KV> __host__ __device__ constexpr int dec_pitch(int d) { return d * (int)sizeof(KV) + 16; }   // bytes of a staged row
+template <typename KV, int CH> __host__ __device__ constexpr int dec_k_bytes(int d) {
+    // (the partial sums, 32 KB, take the keys' place)
+    return CH * dec_pitch<KV>(d) > DEC_THREADS * 4 * DEC_HB * 4 ? CH * dec_pitch<KV>(d) : DEC_THREADS * 4 * DEC_HB * 4;
+}
+template <typename KV, int CH> constexpr size_t dec_smem(int d) {
+    return (size_t)DEC_HB * d * 4 + DEC_HB * (CH + 4) * 4 + dec_k_bytes<KV, CH>(d) + (size_t)CH * dec_pitch<KV>(d);
+}
+
+template <typename KV, int CH>
+__global__ void __launch_bounds__(DEC_THREADS)
 gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv, int d,
                         const KV *__restrict__ kc, const KV *__restrict__ vc,
                         const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
-                        const int32_t *__restrict__ pos, int chunk, float *__restrict__ part) {
+                        const int32_t *__restrict__ pos, float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
     constexpr bool I8 = sizeof(KV) == 1;
-    constexpr int HB = 8;   // query heads per pass
-    extern __shared__ float sm[];
-    float *qs = sm;                    // [HB][d]
-    float *wts = qs + HB * d;          // [HB][chunk]
-    float *psum = wts + HB * chunk;    // [key groups][HB][d]
-    __shared__ float red[4];
-    const int tid = threadIdx.x;
+    constexpr int HB = DEC_HB, WP = CH + 4;
+    constexpr int HT = HB * CH / DEC_THREADS;      // heads per thread in the score phase
+    extern __shared__ __align__(16) unsigned char dsm[];
+    const int pitch = dec_pitch<KV>(d);
+    float *qs = reinterpret_cast<float *>(dsm);    // [HB][d]
+    float *wts = qs + HB * d;                      // [HB][WP]
+    unsigned char *ks = reinterpret_cast<unsigned char *>(wts + HB * WP);   // [CH][pitch]
+    unsigned char *vs = ks + dec_k_bytes<KV, CH>(d);                        // [CH][pitch]
+    float *psum = reinterpret_cast<float *>(ks);   // [key groups][HB][d], after the scores
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int split = blockIdx.x, kv_h = blockIdx.y, b = blockIdx.z, n_splits = gridDim.x;
     const int grp = n_q / n_kv;
     int limit = *pos + 1;
     limit = limit > max_seq ? max_seq : (limit < 0 ? 0 : limit);
-    const int k0 = split * chunk, k1 = min(limit, k0 + chunk);
-    const int nk = k1 - k0;
+    const int share = (limit + n_splits - 1) / n_splits;
+    const int k0 = split * share, nk = min(limit, k0 + share) - k0;
+    if (nk <= 0) {  // nothing for this split: the neutral element of the merge
+        for (int i = tid; i < grp * (d + 2); i += DEC_THREADS) {
+            const int hh = i / (d + 2), j = i - hh * (d + 2);
+            part[(((size_t)b * n_q + kv_h * grp + hh) * n_splits + split) * (d + 2) + j] = j == d ? -INFINITY : 0.0f;
+        }
+        return;
+    }
     const float scale = 1.0f / sqrtf((float)d);
-    const KV *kb = kc + (size_t)b * max_seq * n_kv * d + (size_t)kv_h * d;
-    const KV *vb = vc + (size_t)b * max_seq * n_kv * d + (size_t)kv_h * d;
-    const float *ksc = I8 ? kscale + (size_t)b * max_seq : nullptr;
-    const float *vsc = I8 ? vscale + (size_t)b * max_seq : nullptr;
-    const int quads = d / 4, kgroups = blockDim.x / quads;      // V phase: thread = (key group, 4 dims)
+    const size_t row_bytes = (size_t)n_kv * d * sizeof(KV);
+    const float *vsc = I8 ? vscale + (size_t)b * max_seq + k0 : nullptr;
+    {
+        const size_t first = (((size_t)b * max_seq + k0) * n_kv + kv_h) * d * sizeof(KV);
+        const unsigned char *kb = reinterpret_cast<const unsigned char *>(kc) + first, *vb = reinterpret_cast<const unsigned char *>(vc) + first;
+        const int pieces = d * (int)sizeof(KV) / 16;
+        const uint32_t kd = (uint32_t)__cvta_generic_to_shared(ks), vd = (uint32_t)__cvta_generic_to_shared(vs);
+        for (int i = tid; i < nk * pieces; i += DEC_THREADS) {
+            const int row = i / pieces, c = (i - row * pieces) * 16;
+            cp_async16(kd + row * pitch + c, kb + row * row_bytes + c);
+        }
+        cp_async_commit();
+        for (int i = tid; i < nk * pieces; i += DEC_THREADS) {
+            const int row = i / pieces, c = (i - row * pieces) * 16;
+            cp_async16(vd + row * pitch + c, vb + row * row_bytes + c);
+        }
+        cp_async_commit();
+    }
+    const int quads = d / 4, kgroups = DEC_THREADS / quads;      // value phase: thread = (key group, 4 dims)
     const int vq = tid % quads, vg = tid / quads;
     for (int h0 = 0; h0 < grp; h0 += HB) {
         const int nh = min(HB, grp - h0);
         const int qh0 = kv_h * grp + h0;
-        if (nk <= 0) {  // nothing for this split yet: the neutral element of the merge
-            for (int i = tid; i < nh * (d + 2); i += blockDim.x) {
-                const int hh = i / (d + 2), j = i - hh * (d + 2);
-                part[(((size_t)b * n_q + qh0 + hh) * n_splits + split) * (d + 2) + j] = j == d ? -INFINITY : 0.0f;
+        for (int i = tid; i < HB * d; i += DEC_THREADS)
+            qs[i] = i < nh * d ? q[(size_t)b * q_stride + (size_t)qh0 * d + i] : 0.0f;
+        if (h0 > 0) {
+            // the partial sums of the pass before lie where the keys were
+            __syncthreads();
+            const unsigned char *kb = reinterpret_cast<const unsigned char *>(kc) + (((size_t)b * max_seq + k0) * n_kv + kv_h) * d * sizeof(KV);
+            const int pieces = d * (int)sizeof(KV) / 16;
+            const uint32_t kd = (uint32_t)__cvta_generic_to_shared(ks);
+            for (int i = tid; i < nk * pieces; i += DEC_THREADS) {
+                const int row = i / pieces, c = (i - row * pieces) * 16;
+                cp_async16(kd + row * pitch + c, kb + row * row_bytes + c);
             }
-            continue;
+            cp_async_commit();
+            cp_async_wait<0>();
+        } else {
+            cp_async_wait<1>();
         }
-        __syncthreads();   // the previous pass is done with the shared arrays
-        for (int i = tid; i < nh * d; i += blockDim.x)
-            qs[i] = q[(size_t)b * q_stride + (size_t)(qh0 + i / d) * d + (i % d)];
         __syncthreads();
-        // ---- scores: thread j owns key k0 + j, walks its row once, 16 elements at a time ----
-        float dot[HB];
+        // ---- scores: thread = (key, HT heads) ----
+        const int key = tid % CH, hs = tid / CH * HT;
+        if (key < nk) {
+            float dot[HT];
 #pragma unroll
-        for (int h = 0; h < HB; ++h) dot[h] = 0.0f;
-        if (tid < nk) {
-            const KV *kr = kb + (size_t)(k0 + tid) * n_kv * d;
-            const float rs = I8 ? ksc[k0 + tid] : 1.0f;
+            for (int h = 0; h < HT; ++h) dot[h] = 0.0f;
+            const unsigned char *kr = ks + key * pitch;
+            const float rs = I8 ? kscale[(size_t)b * max_seq + k0 + key] : 1.0f;
+#pragma unroll 2
             for (int c = 0; c < d; c += 16) {
                 float kv[16];
                 if constexpr (I8) {
-                    const int4 w = __ldg(reinterpret_cast<const int4 *>(kr + c));
+                    const int4 w = *reinterpret_cast<const int4 *>(kr + c);
                     const int ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                     for (int t = 0; t < 16; ++t)
@@ -474,70 +528,80 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
                 } else {
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {
-                        const float4 f = __ldg(reinterpret_cast<const float4 *>(kr + c) + t);
+                        const float4 f = *reinterpret_cast<const float4 *>(kr + c * 4 + t * 16);
                         kv[4 * t] = f.x; kv[4 * t + 1] = f.y; kv[4 * t + 2] = f.z; kv[4 * t + 3] = f.w;
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < HB; ++h) {
-                    if (h < nh) {
-                        const float *qh = qs + h * d + c;
+                for (int h = 0; h < HT; ++h) {
+                    const float4 *qh = reinterpret_cast<const float4 *>(qs + (hs + h) * d + c);
 #pragma unroll
-                        for (int t = 0; t < 16; ++t) dot[h] = fmaf(qh[t], kv[t], dot[h]);
+                    for (int t = 0; t < 4; ++t) {
+                        const float4 f = qh[t];
+                        dot[h] = fmaf(f.x, kv[4 * t], dot[h]);
+                        dot[h] = fmaf(f.y, kv[4 * t + 1], dot[h]);
+                        dot[h] = fmaf(f.z, kv[4 * t + 2], dot[h]);
+                        dot[h] = fmaf(f.w, kv[4 * t + 3], dot[h]);
                     }
                 }
             }
+#pragma unroll
+            for (int h = 0; h < HT; ++h) wts[(hs + h) * WP + key] = dot[h] * scale;
         }
-        // ---- per head: local softmax over the chunk; the weights go to shared memory ----
-        for (int h = 0; h < nh; ++h) {
-            const float sc = tid < nk ? dot[h] * scale : -INFINITY;
-            const float mx = block_max(sc, red);
-            float e = tid < nk ? expf(sc - mx) : 0.0f;
-            const float se = block_sum(e, red);
-            // int8 values: fold the row scale of the value row into its weight once
-            if (I8 && tid < nk) e = e * vsc[k0 + tid];
-            wts[h * chunk + tid] = e;
-            if (tid == 0) {
-                float *po = part + (((size_t)b * n_q + qh0 + h) * n_splits + split) * (d + 2);
+        __syncthreads();
+        // ---- softmax over the share: warp = head ----
+        if (warp < nh) {
+            float e[CH / 32], mx = -INFINITY, se = 0.0f;
+#pragma unroll
+            for (int i = 0; i < CH / 32; ++i) {
+                const int j = lane + i * 32;
+                e[i] = j < nk ? wts[warp * WP + j] : -INFINITY;
+                mx = fmaxf(mx, e[i]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+            for (int i = 0; i < CH / 32; ++i) {
+                const int j = lane + i * 32;
+                e[i] = j < nk ? expf(e[i] - mx) : 0.0f;
+                se += e[i];
+                // int8 values: fold the row scale of the value row into its weight once
+                if (j < nk) wts[warp * WP + j] = I8 ? e[i] * vsc[j] : e[i];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+            if (lane == 0) {
+                float *po = part + (((size_t)b * n_q + qh0 + warp) * n_splits + split) * (d + 2);
                 po[d] = mx;
                 po[d + 1] = se;
             }
         }
+        cp_async_wait<0>();
         __syncthreads();
         // ---- weighted values: thread (key group vg, dims 4*vq..): a value row quad serves every head ----
-        float acc[HB][4];
-#pragma unroll
-        for (int h = 0; h < HB; ++h) acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.0f;
         if (vg < kgroups) {
-            // four value rows' loads in flight per thread, then the arithmetic
-            for (int j0 = vg; j0 < nk; j0 += 4 * kgroups) {
-                float v4[4][4];
+            float acc[HB][4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int j = j0 + u * kgroups;
-                    const KV *vr = vb + (size_t)(k0 + (j < nk ? j : j0)) * n_kv * d;
-                    if constexpr (I8) {
-                        const int w = __ldg(reinterpret_cast<const int *>(vr) + vq);
-                        v4[u][0] = (float)(int8_t)(w & 255); v4[u][1] = (float)(int8_t)((w >> 8) & 255);
-                        v4[u][2] = (float)(int8_t)((w >> 16) & 255); v4[u][3] = (float)(int8_t)((w >> 24) & 255);
-                    } else {
-                        const float4 f = __ldg(reinterpret_cast<const float4 *>(vr) + vq);
-                        v4[u][0] = f.x; v4[u][1] = f.y; v4[u][2] = f.z; v4[u][3] = f.w;
-                    }
+            for (int h = 0; h < HB; ++h) acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.0f;
+#pragma unroll 2
+            for (int j = vg; j < nk; j += kgroups) {
+                float v4[4];
+                if constexpr (I8) {
+                    const int w = *reinterpret_cast<const int *>(vs + j * pitch + vq * 4);
+                    v4[0] = (float)(int8_t)(w & 255); v4[1] = (float)(int8_t)((w >> 8) & 255);
+                    v4[2] = (float)(int8_t)((w >> 16) & 255); v4[3] = (float)(int8_t)((w >> 24) & 255);
+                } else {
+                    const float4 f = *reinterpret_cast<const float4 *>(vs + j * pitch + vq * 16);
+                    v4[0] = f.x; v4[1] = f.y; v4[2] = f.z; v4[3] = f.w;
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int j = j0 + u * kgroups;
-                    if (j >= nk) break;
-#pragma unroll
-                    for (int h = 0; h < HB; ++h) {
-                        if (h < nh) {
-                            const float w = wts[h * chunk + j];
-                            acc[h][0] = fmaf(w, v4[u][0], acc[h][0]);
-                            acc[h][1] = fmaf(w, v4[u][1], acc[h][1]);
-                            acc[h][2] = fmaf(w, v4[u][2], acc[h][2]);
-                            acc[h][3] = fmaf(w, v4[u][3], acc[h][3]);
-                        }
+                for (int h = 0; h < HB; ++h) {
+                    if (h < nh) {
+                        const float w = wts[h * WP + j];
+                        acc[h][0] = fmaf(w, v4[0], acc[h][0]);
+                        acc[h][1] = fmaf(w, v4[1], acc[h][1]);
+                        acc[h][2] = fmaf(w, v4[2], acc[h][2]);
+                        acc[h][3] = fmaf(w, v4[3], acc[h][3]);
                     }
                 }
             }
@@ -548,12 +612,13 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
                         make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
         }
         __syncthreads();
-        for (int i = tid; i < nh * d; i += blockDim.x) {
+        for (int i = tid; i < nh * d; i += DEC_THREADS) {
             const int h = i / d, dd = i - h * d;
             float v = 0.0f;
             for (int g = 0; g < kgroups; ++g) v += psum[((size_t)g * HB + h) * d + dd];
             part[(((size_t)b * n_q + qh0 + h) * n_splits + split) * (d + 2) + dd] = v;
         }
+        __syncthreads();   // the next pass writes the shared arrays
     }
 }
 
@@ -608,13 +673,14 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
     constexpr int SP = CH + 4;            // scores row pitch (floats)
     constexpr int PP = CH + 8;            // weight row pitch (halves)
     extern __shared__ __align__(16) unsigned char tsm[];
-    const int kp = d;                     // key row pitch (bytes); for d = 128 the 16-byte piece c of row r sits
-    const int ksw = d == 128 ? 4 : 0;     // at piece c ^ ((r & 1) * 4): the eight lanes of a read phase (two
-                                          // rows x four pieces) then touch eight different bank groups
-    const int vp = CH + 16;               // transposed value row pitch (bytes): conflict-free 32-bit reads
+    // rows of d bytes, keys and values alike. Keys: for d = 128 the 16-byte piece c of row r sits at piece
+    // c ^ ((r & 1) * 4): the eight lanes of a read phase (two rows x four pieces) then touch eight different
+    // bank groups. Values: piece c ^ (((r >> 2) & (d / 32 - 1)) * 2): the four lanes of a quad read 32-bit
+    // words of rows four apart, the eight quads 32 consecutive bytes.
+    const int ksw = d == 128 ? 4 : 0, vmask = d / 32 - 1;
     unsigned char *Ks = tsm;                                         // [CH][d]
-    unsigned char *Vt = Ks + CH * kp;                                // [d][CH + 16]
-    float *Ssm = reinterpret_cast<float *>(Vt + d * vp);             // [HB][SP]
+    unsigned char *Vs = Ks + CH * d;                                 // [CH][d]
+    float *Ssm = reinterpret_cast<float *>(Vs + CH * d);             // [HB][SP]
     __half *Ph = reinterpret_cast<__half *>(Ssm + HB * SP);          // [HB][PP] leading terms
     __half *Pl = Ph + HB * PP;                                       // [HB][PP] remainders
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -622,9 +688,10 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
     const int grp = n_q / n_kv;
     int limit = *pos + 1;
     limit = limit > max_seq ? max_seq : (limit < 0 ? 0 : limit);
-    const int k0 = split * CH, k1 = min(limit, k0 + CH);
+    const int share = (limit + n_splits - 1) / n_splits;             // at most CH: n_splits * CH >= max_seq
+    const int k0 = split * share, k1 = min(limit, k0 + share);
     const int nk = k1 - k0;
-    if (nk <= 0) {  // nothing for this split yet: the neutral element of the merge
+    if (nk <= 0) {  // nothing for this split: the neutral element of the merge
         for (int i = tid; i < grp * (d + 2); i += blockDim.x) {
             const int hh = i / (d + 2), j = i - hh * (d + 2);
             part[(((size_t)b * n_q + kv_h * grp + hh) * n_splits + split) * (d + 2) + j] = j == d ? -INFINITY : 0.0f;
@@ -636,33 +703,24 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
     const int8_t *vb = vc + (size_t)b * max_seq * n_kv * d + (size_t)kv_h * d;
     const float *ksc = kscale + (size_t)b * max_seq, *vsc = vscale + (size_t)b * max_seq;
 
-    // ---- stage the chunk: key rows as they are, value rows transposed; rows past nk are zeros ----
+    // ---- stage the share by asynchronous copies, all in flight at once; rows past nk are zeros ----
     {
         const int pieces = d / 16;        // 16-byte pieces per row
-        uint4 kw[8], vw[8];               // every load in flight before the first store
+        const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Ks), vd = (uint32_t)__cvta_generic_to_shared(Vs);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = tid + u * 128, row = i / pieces, pc = i - row * pieces;
-            kw[u] = vw[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (u < pieces && row < nk) {
-                kw[u] = __ldg(reinterpret_cast<const uint4 *>(kb + (size_t)(k0 + row) * n_kv * d) + pc);
-                vw[u] = __ldg(reinterpret_cast<const uint4 *>(vb + (size_t)(k0 + row) * n_kv * d) + pc);
+        for (int which = 0; which < 2; ++which) {
+            for (int i = tid; i < CH * pieces; i += 128) {
+                const int row = i / pieces, pc = i - row * pieces;
+                const int at = pc ^ (which == 0 ? (row & 1) * ksw : ((row >> 2) & vmask) * 2);
+                const int8_t *src = (which == 0 ? kb : vb) + (size_t)(k0 + min(row, nk - 1)) * n_kv * d + pc * 16;
+                const int live = row < nk ? 16 : 0;   // 0 source bytes: the piece is filled with zeros
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((which == 0 ? kd : vd) + row * d + (at << 4)),
+                             "l"(src), "r"(live) : "memory");
             }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = tid + u * 128, row = i / pieces, pc = i - row * pieces;
-            if (u < pieces) {
-                *reinterpret_cast<uint4 *>(Ks + row * kp + ((pc ^ ((row & 1) * ksw)) << 4)) = kw[u];
-                const uint32_t w[4] = {vw[u].x, vw[u].y, vw[u].z, vw[u].w};
-#pragma unroll
-                // (value row d keeps key k at byte k ^ ((d >> 4) << 2): the eight lanes that hold the
-                // eight pieces of one key row then store into eight different banks)
-                for (int e = 0; e < 16; ++e)
-                    Vt[(pc * 16 + e) * vp + (row ^ (pc << 2))] = (unsigned char)(w[e >> 2] >> (8 * (e & 3)));
-            }
+            cp_async_commit();
         }
     }
+    cp_async_wait<1>();
     __syncthreads();
 
     for (int h0 = 0; h0 < grp; h0 += HB) {
@@ -691,8 +749,8 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
                 if (blk * 64 < d) {
                     // (keyA and keyB = keyA + 8 have the same parity, hence the same swizzle)
                     const int pc = (blk * 4 + t) ^ ((keyA & 1) * ksw);
-                    const uint4 wa = *reinterpret_cast<const uint4 *>(Ks + keyA * kp + (pc << 4));
-                    const uint4 wb = *reinterpret_cast<const uint4 *>(Ks + keyB * kp + (pc << 4));
+                    const uint4 wa = *reinterpret_cast<const uint4 *>(Ks + keyA * d + (pc << 4));
+                    const uint4 wb = *reinterpret_cast<const uint4 *>(Ks + keyB * d + (pc << 4));
                     const uint32_t xa[4] = {wa.x, wa.y, wa.z, wa.w}, xb[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
                     for (int s4 = 0; s4 < 4; ++s4) {
@@ -747,59 +805,104 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
             *reinterpret_cast<uint2 *>(Ph + h * PP + key) = make_uint2(hi01, hi23);
             *reinterpret_cast<uint2 *>(Pl + h * PP + key) = make_uint2(lo01, lo23);
         }
+        cp_async_wait<0>();
         __syncthreads();
-        // ---- out = P x V: warp w takes d / 32 column tiles of 8; rows 8..15 of P are zero ----
-        const int ntw = d / 32;           // column tiles per warp (2 or 4)
+        // ---- out = P x V, rows 8..15 of P zero: a warp takes 32 columns as four n tiles, tile j the columns
+        // 4 g + j, so that a 32-bit word of a value row holds one column of each tile and four rows' words
+        // transpose in registers (a transposed copy in shared memory took 128 byte stores per thread).
+        // d = 64: two warps per column block, half the keys each ----
+        {
+            const int blocks = d / 32, cb = warp % blocks, part_k = warp / blocks, steps = CH / 16 * blocks / 4;
+            float o[4][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j < ntw) {
-                const int col = (warp * ntw + j) * 8 + g;     // this thread's B column (a d index)
-                float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int j = 0; j < 4; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+#pragma unroll 4
+            for (int ks = part_k * steps; ks < (part_k + 1) * steps; ++ks) {
+                const int key0 = ks * 16 + 4 * t;
+                const uint2 ah = *reinterpret_cast<const uint2 *>(Ph + g * PP + key0);
+                const uint2 al = *reinterpret_cast<const uint2 *>(Pl + g * PP + key0);
+                // (rows key0 .. key0 + 3 share the piece swizzle)
+                const unsigned char *vr = Vs + key0 * d + (((cb * 2 + (g >> 2)) ^ (((key0 >> 2) & vmask) * 2)) << 4) + (g & 3) * 4;
+                const uint32_t w0 = *reinterpret_cast<const uint32_t *>(vr), w1 = *reinterpret_cast<const uint32_t *>(vr + d);
+                const uint32_t w2 = *reinterpret_cast<const uint32_t *>(vr + 2 * d), w3 = *reinterpret_cast<const uint32_t *>(vr + 3 * d);
+                uint32_t b0[4], b1[4];
+                s8x4_to_h2x2(__byte_perm(w0, w1, 0x5140), b0[0], b0[1]);
+                s8x4_to_h2x2(__byte_perm(w0, w1, 0x7362), b0[2], b0[3]);
+                s8x4_to_h2x2(__byte_perm(w2, w3, 0x5140), b1[0], b1[1]);
+                s8x4_to_h2x2(__byte_perm(w2, w3, 0x7362), b1[2], b1[3]);
 #pragma unroll
-                for (int ks = 0; ks < CH / 16; ++ks) {
-                    const int key0 = ks * 16 + 4 * t;
-                    const uint2 ah = *reinterpret_cast<const uint2 *>(Ph + g * PP + key0);
-                    const uint2 al = *reinterpret_cast<const uint2 *>(Pl + g * PP + key0);
-                    uint32_t b0, b1;
-                    s8x4_to_h2x2(*reinterpret_cast<const uint32_t *>(Vt + col * vp + (key0 ^ ((col >> 4) << 2))), b0, b1);
-                    mma_f16(o, al.x, 0u, al.y, 0u, b0, b1);
-                    mma_f16(o, ah.x, 0u, ah.y, 0u, b0, b1);
+                for (int j = 0; j < 4; ++j) {
+                    mma_f16(o[j], al.x, 0u, al.y, 0u, b0[j], b1[j]);
+                    mma_f16(o[j], ah.x, 0u, ah.y, 0u, b0[j], b1[j]);
                 }
-                // o0, o1 = (head g, d = tile * 8 + 2t, + 1)
-                if (g < nh) {
-                    float *po = part + (((size_t)b * n_q + qh0 + g) * n_splits + split) * (d + 2) + (warp * ntw + j) * 8 + 2 * t;
-                    po[0] = o[0];
-                    po[1] = o[1];
+            }
+            // o[j][0], o[j][1] = head g, columns 32 cb + 4 * (2t) + j and 4 * (2t + 1) + j
+            if (blocks == 2) {
+                float *half = Ssm;   // [2 column blocks][32 lanes][8]; the scores are used up
+                if (part_k == 1) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        half[(cb * 32 + lane) * 9 + 2 * j] = o[j][0];
+                        half[(cb * 32 + lane) * 9 + 2 * j + 1] = o[j][1];
+                    }
                 }
+                __syncthreads();
+                if (part_k == 0) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        o[j][0] += half[(cb * 32 + lane) * 9 + 2 * j];
+                        o[j][1] += half[(cb * 32 + lane) * 9 + 2 * j + 1];
+                    }
+                }
+            }
+            if (part_k == 0 && g < nh) {
+                // (records start at multiples of d + 2 floats: 8-byte aligned)
+                float *po = part + (((size_t)b * n_q + qh0 + g) * n_splits + split) * (d + 2) + cb * 32 + 8 * t;
+                *reinterpret_cast<float2 *>(po) = make_float2(o[0][0], o[1][0]);
+                *reinterpret_cast<float2 *>(po + 2) = make_float2(o[2][0], o[3][0]);
+                *reinterpret_cast<float2 *>(po + 4) = make_float2(o[0][1], o[1][1]);
+                *reinterpret_cast<float2 *>(po + 6) = make_float2(o[2][1], o[3][1]);
             }
         }
         __syncthreads();   // the score and weight arrays are reused by the next pass
     }
 }
 
-__global__ void attention_combine_kernel(const float *__restrict__ part, int n_splits, int d,
-                                         float *__restrict__ out) {
+// Merges the splits: block per (q head, b), 128 threads; out row [b][n_q*d]. The splits' weights are
+// worked out once per block, a thread per split, then a thread per column adds with its loads in flight
+// (a serial walk that evaluated every weight in every thread: 27 us for 64 x 64 heads x 18 splits).
+constexpr int COMBINE_BATCH = 128;
+__global__ void __launch_bounds__(128)
+attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, float *__restrict__ out) {
     pdl_wait();
     pdl_trigger();
-    // block per (q head, b); out row [b][n_q*d]
+    __shared__ float red[4], wt[COMBINE_BATCH];
+    const int tid = threadIdx.x;
     const size_t hb = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
     const float *p = part + hb * n_splits * (d + 2);
     float M = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) M = fmaxf(M, p[(size_t)s * (d + 2) + d]);
-    float L = 0.0f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float m = p[(size_t)s * (d + 2) + d];
-        if (m > -INFINITY) L += expf(m - M) * p[(size_t)s * (d + 2) + d + 1];
-    }
-    const float inv = L > 0.0f ? 1.0f / L : 0.0f;
-    for (int i = threadIdx.x; i < d; i += blockDim.x) {
-        float acc = 0.0f;
-        for (int s = 0; s < n_splits; ++s) {
+    for (int s = tid; s < n_splits; s += 128) M = fmaxf(M, p[(size_t)s * (d + 2) + d]);
+    M = block_max(M, red);
+    float L = 0.0f, acc = 0.0f;
+    for (int s0 = 0; s0 < n_splits; s0 += COMBINE_BATCH) {
+        const int s = s0 + tid, ns = min(COMBINE_BATCH, n_splits - s0);
+        float w = 0.0f;
+        if (s < n_splits) {
             const float m = p[(size_t)s * (d + 2) + d];
-            if (m > -INFINITY) acc = fmaf(expf(m - M), p[(size_t)s * (d + 2) + i], acc);
+            if (m > -INFINITY) w = expf(m - M);
+            L += w * (w > 0.0f ? p[(size_t)s * (d + 2) + d + 1] : 0.0f);
         }
-        out[hb * d + i] = acc * inv;
+        __syncthreads();
+        wt[tid] = w;
+        __syncthreads();
+        if (tid < d) {
+#pragma unroll 6
+            for (int i = 0; i < ns; ++i) acc = fmaf(wt[i], p[(size_t)(s0 + i) * (d + 2) + tid], acc);
+        }
     }
+    L = block_sum(L, red);
+    const float inv = L > 0.0f ? 1.0f / L : 0.0f;
+    if (tid < d) out[hb * d + tid] = acc * inv;
 }
 
 // out[m][n] = sum_k x[m][k] * w[n][k]; one warp per weight row, up to 4 x rows per pass
@@ -1114,7 +1217,7 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
         // key and value rows are read with 128-bit loads
         if (((reinterpret_cast<uintptr_t>(d_kcache) | reinterpret_cast<uintptr_t>(d_vcache)) & 15) != 0)
             return fail(YSCV_CUDA_ERR_UNSUPPORTED, "the key and value caches must be 16-byte aligned");
-        const int chunk = 128;
+        const int chunk = sizeof(KV) == 4 && d_head > 64 ? 64 : 128;   // (what fits shared memory twice)
         const int n_splits = (int)((max_seq + chunk - 1) / chunk);
         const size_t need = batch * n_q * (size_t)n_splits * (d_head + 2) * sizeof(float);
         int rc = ctx->scratch_attn.reserve(need);
@@ -1122,12 +1225,10 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
         float *part = reinterpret_cast<float *>(ctx->scratch_attn.ptr);
         // one block per (key chunk, KV head, sequence): it serves every query head of the group
         dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)batch);
-        const size_t kgroups = 128 / (d_head / 4);
-        const size_t split_smem = (8 * d_head + 8 * chunk + kgroups * 8 * d_head) * sizeof(float);
         if constexpr (sizeof(KV) == 1) {
             // int8 caches with head sizes of 64 or 128: both contractions on the tensor cores
             if ((d_head == 64 || d_head == 128) && ctx->attn_tensor_cores) {
-                const size_t tc_smem = 128 * d_head + d_head * (128 + 16) + 8 * (128 + 4) * sizeof(float) +
+                const size_t tc_smem = 2 * 128 * d_head + 8 * (128 + 4) * sizeof(float) +
                                        2 * 8 * (128 + 8) * sizeof(uint16_t);
                 YSCV_CUDA_TRY(launch_pdl(gqa_decode_split_tc_kernel, dim3(grid), dim3(128), tc_smem, ctx->stream, d_q,
                                          (int)q_stride, (int)n_q, (int)n_kv, (int)d_head,
@@ -1140,9 +1241,17 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                 DEC_EPILOGUE(ctx, "gqa_attention(split-k,int8 cache,mma)");
             }
         }
-        YSCV_CUDA_TRY(launch_pdl(gqa_decode_split_kernel<KV>, dim3(grid), dim3(128), split_smem,
-                                 ctx->stream, d_q, (int)q_stride, (int)n_q, (int)n_kv, (int)d_head, d_kcache, d_vcache,
-                                 d_kscale, d_vscale, (int)max_seq, d_pos, chunk, part));
+        auto kern = gqa_decode_split_kernel<KV, 128>;
+        size_t split_smem = dec_smem<KV, 128>((int)d_head);
+        if constexpr (sizeof(KV) == 4) {
+            if (chunk == 64) {
+                kern = gqa_decode_split_kernel<KV, 64>;
+                split_smem = dec_smem<KV, 64>((int)d_head);
+            }
+        }
+        if ((rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 80 * 1024))) return rc;
+        YSCV_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(DEC_THREADS), split_smem, ctx->stream, d_q, (int)q_stride, (int)n_q, (int)n_kv,
+                                 (int)d_head, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, part));
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
         YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel, dim3(dim3((unsigned)n_q, (unsigned)batch)), dim3(128), 0, ctx->stream, part, n_splits,
