@@ -79,3 +79,33 @@ def test_non_finite_rows_stay_in_their_row():
     want = x[keep].double() @ w.T
     assert float((out[keep].double() - want).norm() / want.norm()) <= 1e-6
     ctx.close()
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 19456, 4096), (515, 13001, 2112), (400, 24000, 8192), (257, 19301, 4096)])
+def test_split_last_round(m, n, k):
+    """The CTA-pair GEMM with few tiles in its last round (their k blocks are cut over all pairs): ragged rows
+    and tokens, both stage depths. Bound as above, for every 512-row column of tiles too."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    with torch.cuda.stream(stream):
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g)
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        report = ctx.dispatch_report()
+        first = out.clone()
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        want = x.double() @ w.T
+    stream.synchronize()
+    assert ctx.device_status() == 0
+    assert "split over k" in report and " 0 split over k" not in report, report
+    assert torch.equal(first, out)
+    assert torch.all(out[m] == 7.0)
+    diff = out[:m].double() - want
+    assert float(diff.norm() / want.norm()) <= 4e-3
+    for n0 in range(0, n, 512):
+        assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 5e-3, n0
+    ctx.close()

@@ -55,6 +55,10 @@ struct PGParams {
     // MMAs are short and a hand-over (dequantised tile -> MMA -> buffer back) costs ~1000 cycles
     // whatever the work: two sub-blocks per hand-over halve their number. k_blocks, kb_per count stages.
     int ksub;
+    // CTA-pair form: tiles [0, full_tiles) go to the pairs whole; the k blocks of the rest are numbered
+    // through and every pair takes an equal range, parts of tiles to `parts` (see PPWalk)
+    int full_tiles;
+    float *parts;
 };
 
 __device__ __forceinline__ void pg_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
@@ -427,6 +431,37 @@ __device__ __forceinline__ void pp_commit(uint32_t bar) {
                  : "memory");
 }
 
+// One pair's work: whole tiles round by round, then its share of the last round, which would leave most
+// pairs idle when few tiles remain (2048 x 8192 x 10240: 160 tiles on 74 pairs): the remaining tiles'
+// k blocks in one sequence, cut into equal ranges. A range is shorter than a tile, so it meets at most
+// two; the part of tile i (of the remaining ones) done by pair c is slot c + i of `parts`,
+// [256 tokens][512 rows] fp32, and pp_join_kernel adds a tile's parts in pair order.
+struct PPWalk {
+    int t, full, pairs, kb, pair, u, u1;
+    __device__ PPWalk(const PGParams &p, int pair_, int n_pairs, int tiles)
+        : t(pair_), full(p.full_tiles), pairs(n_pairs), kb(p.k_blocks), pair(pair_) {
+        const int rest = (tiles - p.full_tiles) * p.k_blocks;
+        u = (int)((long long)pair_ * rest / n_pairs);
+        u1 = (int)((long long)(pair_ + 1) * rest / n_pairs);
+    }
+    // slot < 0: a whole tile
+    __device__ bool next(int &tile, int &k0, int &k1, int &slot) {
+        if (t < full) {
+            tile = t; k0 = 0; k1 = kb; slot = -1;
+            t += pairs;
+            return true;
+        }
+        if (u >= u1) return false;
+        const int i = u / kb;
+        tile = full + i;
+        k0 = u - i * kb;
+        k1 = min(kb, k0 + u1 - u);
+        slot = k1 - k0 == kb ? -1 : pair + i;
+        u += k1 - k0;
+        return true;
+    }
+};
+
 template <int KSUB>
 __global__ void __launch_bounds__(PG_THREADS, 1)
 int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
@@ -473,6 +508,8 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     pdl_wait();      // as in the one-CTA kernel
     pdl_trigger();
 
+    PPWalk walk(p, pair, n_pairs, tiles);
+    int t, kb0, kb1, part;
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         if (lane == 0) {
@@ -482,9 +519,9 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             uint32_t phase = 0;
             bool alive = true;
             const uint32_t leader_full_act = map_to_cta(bar_full_act, 0);
-            for (int t = pair; t < tiles && alive; t += n_pairs) {
+            while (alive && walk.next(t, kb0, kb1, part)) {
                 const int nt_i = t % p.n_tiles, tc = t / p.n_tiles;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     alive = mbar_wait(bar_empty + slot * 8, phase ^ 1u, status);
                     if (!alive) break;
                     const uint32_t st = ring + (uint32_t)slot * PP_STAGE;
@@ -511,11 +548,11 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             bool alive = true;
             const uint32_t peer_empty = map_to_cta(bar_empty, 1), peer_aempty = map_to_cta(bar_aempty, 1);
             const uint32_t peer_tfull = map_to_cta(bar_tfull, 1);
-            for (int t = pair; t < tiles && alive; t += n_pairs) {
+            while (alive && walk.next(t, kb0, kb1, part)) {
                 alive = mbar_spin_cluster(bar_tempty, tphase ^ 1u, status);
                 if (!alive) break;
                 pg_fence_after();
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     alive = mbar_wait_cluster(bar_full_act + slot * 8, phase, status) &&
                             mbar_spin_cluster(bar_afull + abuf * 8, aphase, status);
                     if (!alive) break;
@@ -529,7 +566,7 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 #pragma unroll
                             for (int kk = 0; kk < PG_BK / 16; ++kk)  // K = 16 per instruction: +32 bytes
                                 pp_mma_bf16(tmem_base + a * 256, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc,
-                                            (kb > 0 || sub > 0 || kk > 0) ? 1u : 0u);
+                                            (kb > kb0 || sub > 0 || kk > 0) ? 1u : 0u);
                         }
                     }
                     pp_commit(bar_empty + slot * 8);
@@ -554,7 +591,7 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         bool alive = true;
         const __nv_bfloat162 bias = __float2bfloat162_rn(136.0f);
         const uint32_t leader_afull = map_to_cta(bar_afull, 0);
-        for (int t = pair; t < tiles && alive; t += n_pairs) {
+        while (alive && walk.next(t, kb0, kb1, part)) {
             const int nt_i = t % p.n_tiles;
             const float *srow[2];
             bool live_row[2];
@@ -565,9 +602,9 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                 live_row[a] = row < p.N;
                 srow[a] = scales + (size_t)(live_row[a] ? row : 0) * groups + half;
 #pragma unroll
-                for (int sub = 0; sub < KSUB; ++sub) sc_next[sub][a] = live_row[a] ? __ldg(srow[a] + sub * 2) : 0.0f;
+                for (int sub = 0; sub < KSUB; ++sub) sc_next[sub][a] = live_row[a] ? __ldg(srow[a] + (kb0 * KSUB + sub) * 2) : 0.0f;
             }
-            for (int kb = 0; kb < p.k_blocks; ++kb) {
+            for (int kb = kb0; kb < kb1; ++kb) {
                 float sc[KSUB][2];
 #pragma unroll
                 for (int sub = 0; sub < KSUB; ++sub) {
@@ -575,7 +612,7 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                     for (int a = 0; a < 2; ++a) {
                         sc[sub][a] = sc_next[sub][a];
                         // the next stage's scales travel while this one is converted
-                        if (kb + 1 < p.k_blocks && live_row[a]) sc_next[sub][a] = __ldg(srow[a] + ((kb + 1) * KSUB + sub) * 2);
+                        if (kb + 1 < kb1 && live_row[a]) sc_next[sub][a] = __ldg(srow[a] + ((kb + 1) * KSUB + sub) * 2);
                     }
                 }
                 alive = mbar_wait(bar_full_w + slot * 8, phase, status) &&
@@ -625,7 +662,7 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         uint32_t tphase = 0;
         bool alive = true;
         const uint32_t leader_tempty = map_to_cta(bar_tempty, 0);
-        for (int t = pair; t < tiles && alive; t += n_pairs) {
+        while (alive && walk.next(t, kb0, kb1, part)) {
             const int nt_i = t % p.n_tiles, tc = t / p.n_tiles;
             alive = mbar_wait(bar_tfull, tphase, status);
             if (!alive) break;
@@ -639,7 +676,11 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                     uint32_t rr[32];
                     pg_tmem_ld32(taddr + c0, rr);
                     const int tok0 = tc * 256 + c0;
-                    if (n < p.N) {
+                    if (part >= 0) {
+                        float *dst = p.parts + ((size_t)part * 256 + c0) * 512 + rank * 256 + a * PG_BM + q * 32 + lane;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) dst[j * 512] = __uint_as_float(rr[j]);
+                    } else if (n < p.N) {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
                             if (tok0 + j < p.M) out[(size_t)(tok0 + j) * p.N + n] = __uint_as_float(rr[j]);
@@ -676,6 +717,43 @@ __global__ void __launch_bounds__(256) add_kslices_kernel(const float4 *__restri
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
         out[i] = a;
+    }
+}
+
+// The tiles of the CTA-pair kernel's last round that several pairs share. Block (tile, 8 tokens), a
+// thread four rows.
+__global__ void __launch_bounds__(128) pp_join_kernel(PGParams p, int n_pairs, int vec, float *__restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x, tile = p.full_tiles + i, rest = (int)gridDim.x * p.k_blocks;
+    // pairs of the tile's first and last k block
+    const int c0 = (int)((((long long)i * p.k_blocks + 1) * n_pairs - 1) / rest);
+    const int c1 = (int)((((long long)(i + 1) * p.k_blocks) * n_pairs - 1) / rest);
+    if (c0 == c1) return;
+    const int n0 = tile % p.n_tiles * 512 + threadIdx.x * 4, tok0 = tile / p.n_tiles * 256 + blockIdx.y * 8;
+    float4 sum[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c = c0; c <= c1; ++c) {
+        const float4 *src = reinterpret_cast<const float4 *>(p.parts + ((size_t)(c + i) * 256 + blockIdx.y * 8) * 512) + threadIdx.x;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 v = __ldcg(src + j * 128);
+            sum[j].x += v.x; sum[j].y += v.y; sum[j].z += v.z; sum[j].w += v.w;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (tok0 + j >= p.M) break;
+        float *dst = out + (size_t)(tok0 + j) * p.N + n0;
+        if (vec && n0 + 3 < p.N) {
+            *reinterpret_cast<float4 *>(dst) = sum[j];
+        } else {
+            if (n0 < p.N) dst[0] = sum[j].x;
+            if (n0 + 1 < p.N) dst[1] = sum[j].y;
+            if (n0 + 2 < p.N) dst[2] = sum[j].z;
+            if (n0 + 3 < p.N) dst[3] = sum[j].w;
+        }
     }
 }
 
@@ -726,14 +804,38 @@ static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, con
     const int tiles = p.n_tiles * p.t_chunks;
     const int pairs = tiles < ctx->max_prefill_pairs ? tiles : ctx->max_prefill_pairs;
     cfg.gridDim = dim3(2 * pairs);
+    // Split the last round where that saves more than the parts cost: a round takes about 0.9 us per 64 k,
+    // a part (512 KB written and read back) 0.125 us from L2 and up to twice that from HBM, the second launch
+    // 3 us: 2048 x 8192 x 10240 (12 tiles left for 74 pairs) 345 -> 281 us, 2048 x 8192 x 57344 (8 left) 1675 ->
+    // 1592; with 54 left (2048 x 8192 x 8192) nothing is gained. The workspace is never grown
+    // inside a capture: there (without an earlier call of the size) the last round stays whole.
+    const int rest = tiles % pairs;
+    p.full_tiles = tiles;
+    if (tiles > pairs && rest > 0 && 0.9 * (p.K / 64) * (pairs - rest) / pairs > 2.0 * (0.125 * (pairs + rest) + 3.0)) {
+        const size_t need = (size_t)(pairs + rest) * 256 * 512 * sizeof(float);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        YSCV_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
+        if (ctx->gemm_ws.bytes >= need || (cap == cudaStreamCaptureStatusNone && ctx->gemm_ws.reserve(need) == YSCV_CUDA_OK)) {
+            p.full_tiles = tiles - rest;
+            p.parts = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
+        } else {
+            cudaGetLastError();   // (no memory for it: not this call's failure)
+        }
+    }
     ctx->prof_begin();
     YSCV_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tm_w, tm_a, scales, out, p, ctx->d_status));
     ctx->prof_end();
     YSCV_CUDA_TRY(cudaGetLastError());
     ctx->launches++;
+    if (p.full_tiles < tiles) {
+        const int vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+        YSCV_CUDA_TRY(launch_pdl(pp_join_kernel, dim3((unsigned)rest, 32), dim3(128), 0, ctx->stream, p, pairs, vec, out));
+        ctx->launches++;
+    }
     snprintf(ctx->report_int4, sizeof(ctx->report_int4),
              "int4_prefill_gemm m=%d n=%d k=%d: tcgen05 bf16 cta_group::2, pair tile 512 rows x 256 tokens, %d k per stage, "
-             "%d stages of %d KB per CTA, %d tiles on %d CTA pairs", p.M, p.N, p.K, KSUB * PG_BK, p.stages, G::STAGE / 1024, tiles, pairs);
+             "%d stages of %d KB per CTA, %d tiles on %d CTA pairs, %d split over k", p.M, p.N, p.K, KSUB * PG_BK, p.stages, G::STAGE / 1024,
+             tiles, pairs, tiles - p.full_tiles);
     ctx->last_kernel = "int4_prefill_gemm(tcgen05,bf16,cta_group::2)";
     return YSCV_CUDA_OK;
 }
