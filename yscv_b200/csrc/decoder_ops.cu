@@ -416,7 +416,7 @@ gqa_attention_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n
 // Bound by the latency of its phases, not by the cache's bytes (32 sequences x 200 keys of the 1B head
 // shape are 13 MB). So the whole share is brought to shared memory by asynchronous copies issued at once
 // (keys and values: one memory latency), and the softmax takes one warp per head (two block barriers in
-// all; one block-wide maximum and sum per head were 32): 25.6 -> 14.6 us for that shape.
+// all; one block-wide maximum and sum per head were 32): 25.6 -> 11.0 us for that shape.
 constexpr int DEC_HB = 8;
 constexpr int DEC_THREADS = 256;
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
@@ -434,9 +434,10 @@ template <typename KV, int CH> constexpr size_t dec_smem(int d) {
     return (size_t)DEC_HB * d * 4 + DEC_HB * (CH + 4) * 4 + dec_k_bytes<KV, CH>(d) + (size_t)CH * dec_pitch<KV>(d);
 }
 
-template <typename KV, int CH>
-__global__ void __launch_bounds__(DEC_THREADS)
-gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv, int d,
+// D = 64 or 128: the head size, known to the compiler (index arithmetic without divisions); 0: any
+template <typename KV, int CH, int D>
+__global__ void __launch_bounds__(DEC_THREADS, 3)
+gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv, int d_,
                         const KV *__restrict__ kc, const KV *__restrict__ vc,
                         const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
                         const int32_t *__restrict__ pos, float *__restrict__ part) {
@@ -444,6 +445,7 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
     pdl_trigger();
     constexpr bool I8 = sizeof(KV) == 1;
     constexpr int HB = DEC_HB, WP = CH + 4;
+    const int d = D ? D : d_;
     constexpr int HT = HB * CH / DEC_THREADS;      // heads per thread in the score phase
     extern __shared__ __align__(16) unsigned char dsm[];
     const int pitch = dec_pitch<KV>(d);
@@ -633,10 +635,12 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
 //   scores^T [16 keys x 8 heads] = K tile [16 keys x d] (A, straight from the staged rows) x
 //                                  Q^T [d x 8 heads] (B, two terms)
 //   out [8 heads x d]            = P [8 (of 16 rows) x 128 keys] (A, two terms) x V [128 keys x d]
-//                                  (B, read from a transposed copy of the chunk's value rows)
+//                                  (B, four value rows' words transposed in registers)
 // The k order inside an MMA is free as long as both operands agree: a thread takes 4 consecutive
 // d (or keys) for the four k slots it owns, so its K bytes are one 16-byte read per 64 d and its V
-// bytes one 32-bit read per 16 keys. d is 64 or 128.
+// bytes four 32-bit reads per 16 keys and 32 columns. d is 64 or 128, a template argument: the kernel is bound by
+// the instructions it issues (2.7 per cycle), and index divisions by a run-time d were a quarter of them: 64 x 2049
+// keys, 64 / 8 heads of 128: 144 us with transposed byte stores, 119 without, 95 with d known (its bytes: 41).
 __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                         uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -662,14 +666,15 @@ __device__ __forceinline__ void split_h2(float a, float b, uint32_t &hi, uint32_
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+template <int D>
 __global__ void __launch_bounds__(128)
-gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv, int d,
+gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv,
                            const int8_t *__restrict__ kc, const int8_t *__restrict__ vc,
                            const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
                            const int32_t *__restrict__ pos, float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
-    constexpr int CH = 128, HB = 8;
+    constexpr int CH = 128, HB = 8, d = D;
     constexpr int SP = CH + 4;            // scores row pitch (floats)
     constexpr int PP = CH + 8;            // weight row pitch (halves)
     extern __shared__ __align__(16) unsigned char tsm[];
@@ -677,7 +682,7 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
     // c ^ ((r & 1) * 4): the eight lanes of a read phase (two rows x four pieces) then touch eight different
     // bank groups. Values: piece c ^ (((r >> 2) & (d / 32 - 1)) * 2): the four lanes of a quad read 32-bit
     // words of rows four apart, the eight quads 32 consecutive bytes.
-    const int ksw = d == 128 ? 4 : 0, vmask = d / 32 - 1;
+    constexpr int ksw = d == 128 ? 4 : 0, vmask = d / 32 - 1;
     unsigned char *Ks = tsm;                                         // [CH][d]
     unsigned char *Vs = Ks + CH * d;                                 // [CH][d]
     float *Ssm = reinterpret_cast<float *>(Vs + CH * d);             // [HB][SP]
@@ -705,12 +710,14 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
 
     // ---- stage the share by asynchronous copies, all in flight at once; rows past nk are zeros ----
     {
-        const int pieces = d / 16;        // 16-byte pieces per row
+        constexpr int pieces = d / 16;    // 16-byte pieces per row
         const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Ks), vd = (uint32_t)__cvta_generic_to_shared(Vs);
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
-            for (int i = tid; i < CH * pieces; i += 128) {
-                const int row = i / pieces, pc = i - row * pieces;
+            // (piece and swizzle of a thread stay the same from step to step: rows advance by 128 / pieces)
+#pragma unroll
+            for (int i0 = 0; i0 < CH * pieces; i0 += 128) {
+                const int i = i0 + tid, row = i / pieces, pc = i % pieces;
                 const int at = pc ^ (which == 0 ? (row & 1) * ksw : ((row >> 2) & vmask) * 2);
                 const int8_t *src = (which == 0 ? kb : vb) + (size_t)(k0 + min(row, nk - 1)) * n_kv * d + pc * 16;
                 const int live = row < nk ? 16 : 0;   // 0 source bytes: the piece is filled with zeros
@@ -720,8 +727,15 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
             cp_async_commit();
         }
     }
-    cp_async_wait<1>();
-    __syncthreads();
+    // what else a thread reads from memory travels with them: the scales of its four keys in the scores
+    // (rows 32 warp + 16 i + g and + 8) and of its four in the weights, and (below) the query operands
+    float ks4[4], vs4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int key = warp * 32 + (i >> 1) * 16 + (i & 1) * 8 + g;
+        ks4[i] = key < nk ? __ldg(ksc + k0 + key) * scale : 0.0f;
+        vs4[i] = 4 * lane + i < nk ? __ldg(vsc + k0 + 4 * lane + i) : 0.0f;
+    }
 
     for (int h0 = 0; h0 < grp; h0 += HB) {
         const int nh = min(HB, grp - h0);
@@ -738,6 +752,10 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
                 split_h2(v.x, v.y, qh[ks][0], ql[ks][0]);
                 split_h2(v.z, v.w, qh[ks][1], ql[ks][1]);
             }
+        }
+        if (h0 == 0) {
+            cp_async_wait<1>();
+            __syncthreads();
         }
         // ---- scores^T: warp w takes keys 32 w .. 32 w + 31 as two tiles of 16 ----
 #pragma unroll
@@ -764,8 +782,7 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
                 }
             }
             // c0, c1 = (keyA, heads 2t, 2t+1); c2, c3 = (keyB, same heads)
-            const float sa = keyA < nk ? __ldg(ksc + k0 + keyA) * scale : 0.0f;
-            const float sb = keyB < nk ? __ldg(ksc + k0 + keyB) * scale : 0.0f;
+            const float sa = ks4[mt * 2], sb = ks4[mt * 2 + 1];
             Ssm[(2 * t) * SP + keyA] = keyA < nk ? c[0] * sa : -INFINITY;
             Ssm[(2 * t + 1) * SP + keyA] = keyA < nk ? c[1] * sa : -INFINITY;
             Ssm[(2 * t) * SP + keyB] = keyB < nk ? c[2] * sb : -INFINITY;
@@ -797,11 +814,8 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
             }
             // the value row's scale is folded into its weight; two fp16 terms per weight
             uint32_t hi01, lo01, hi23, lo23;
-            const float4 vs = key < nk ? make_float4(__ldg(vsc + k0 + min(key, nk - 1)), __ldg(vsc + k0 + min(key + 1, nk - 1)),
-                                                     __ldg(vsc + k0 + min(key + 2, nk - 1)), __ldg(vsc + k0 + min(key + 3, nk - 1)))
-                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            split_h2(e[0] * vs.x, e[1] * vs.y, hi01, lo01);
-            split_h2(e[2] * vs.z, e[3] * vs.w, hi23, lo23);
+            split_h2(e[0] * vs4[0], e[1] * vs4[1], hi01, lo01);
+            split_h2(e[2] * vs4[2], e[3] * vs4[3], hi23, lo23);
             *reinterpret_cast<uint2 *>(Ph + h * PP + key) = make_uint2(hi01, hi23);
             *reinterpret_cast<uint2 *>(Pl + h * PP + key) = make_uint2(lo01, lo23);
         }
@@ -812,13 +826,14 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
         // transpose in registers (a transposed copy in shared memory took 128 byte stores per thread).
         // d = 64: two warps per column block, half the keys each ----
         {
-            const int blocks = d / 32, cb = warp % blocks, part_k = warp / blocks, steps = CH / 16 * blocks / 4;
+            constexpr int blocks = d / 32, steps = CH / 16 * blocks / 4;
+            const int cb = warp % blocks, part_k = warp / blocks;
             float o[4][4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
-#pragma unroll 4
-            for (int ks = part_k * steps; ks < (part_k + 1) * steps; ++ks) {
-                const int key0 = ks * 16 + 4 * t;
+#pragma unroll
+            for (int k_ = 0; k_ < steps; ++k_) {
+                const int key0 = (part_k * steps + k_) * 16 + 4 * t;
                 const uint2 ah = *reinterpret_cast<const uint2 *>(Ph + g * PP + key0);
                 const uint2 al = *reinterpret_cast<const uint2 *>(Pl + g * PP + key0);
                 // (rows key0 .. key0 + 3 share the piece swizzle)
@@ -1230,8 +1245,8 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
             if ((d_head == 64 || d_head == 128) && ctx->attn_tensor_cores) {
                 const size_t tc_smem = 2 * 128 * d_head + 8 * (128 + 4) * sizeof(float) +
                                        2 * 8 * (128 + 8) * sizeof(uint16_t);
-                YSCV_CUDA_TRY(launch_pdl(gqa_decode_split_tc_kernel, dim3(grid), dim3(128), tc_smem, ctx->stream, d_q,
-                                         (int)q_stride, (int)n_q, (int)n_kv, (int)d_head,
+                auto kern = d_head == 128 ? gqa_decode_split_tc_kernel<128> : gqa_decode_split_tc_kernel<64>;
+                YSCV_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(128), tc_smem, ctx->stream, d_q, (int)q_stride, (int)n_q, (int)n_kv,
                                          reinterpret_cast<const int8_t *>(d_kcache), reinterpret_cast<const int8_t *>(d_vcache),
                                          d_kscale, d_vscale, (int)max_seq, d_pos, part));
                 YSCV_CUDA_TRY(cudaGetLastError());
@@ -1241,11 +1256,11 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                 DEC_EPILOGUE(ctx, "gqa_attention(split-k,int8 cache,mma)");
             }
         }
-        auto kern = gqa_decode_split_kernel<KV, 128>;
+        auto kern = d_head == 64 ? gqa_decode_split_kernel<KV, 128, 64> : gqa_decode_split_kernel<KV, 128, 0>;
         size_t split_smem = dec_smem<KV, 128>((int)d_head);
         if constexpr (sizeof(KV) == 4) {
             if (chunk == 64) {
-                kern = gqa_decode_split_kernel<KV, 64>;
+                kern = d_head == 128 ? gqa_decode_split_kernel<KV, 64, 128> : gqa_decode_split_kernel<KV, 64, 0>;
                 split_smem = dec_smem<KV, 64>((int)d_head);
             }
         }

@@ -466,6 +466,7 @@ bg_join_kernel(BGParams p, int NA, int grid, float *__restrict__ out) {
     float sum[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t) sum[t] = 0.0f;
+#pragma unroll 4
     for (int c = c0; c <= c1; ++c) {
         const float *part = p.ws + ((size_t)(2 * c + (c == c1 ? 0 : 1)) * NA + a) * p.BT * 128 + (size_t)t0 * 128 + r;
 #pragma unroll
