@@ -182,6 +182,7 @@ class Int4Decoder:
             self.wdown.append(self._linear(*sharding.shard_cols(pd, sd, g, r, G)))
 
     _keep_full = False
+    _chain_step = False
 
     @classmethod
     def with_full_weights(cls, *args, **kw):
@@ -225,7 +226,7 @@ class Int4Decoder:
         if act16:
             h16 = self._buf("h16", rows, H, dtype=torch.bfloat16)
             a16 = self._buf("a16", rows, self.mlp_l, dtype=torch.bfloat16)
-        fused = self.plan is not None and seq == 1
+        fused = self.plan is not None and seq == 1 and not self._chain_step
         if fused:
             # the whole step in one launch: layers, final norm, LM head, greedy token, position
             logits = self._buf("logits", B, c.vocab)
@@ -315,11 +316,17 @@ class Int4Decoder:
         """Record one decode step (reads self.next_tokens, writes it back) as a CUDA graph."""
         with torch.cuda.stream(self.stream):
             saved = self.pos.clone(), self.next_tokens.clone()
+            # Batches of 2..8 sequences: replayed from a graph, where a launch costs no host time, the operator
+            # chain is the faster step (1B shape, us, chain / one launch: batch 2 979 / 1353, 4 1162 / 1400, 8 1220 /
+            # 1783; after 1500 tokens 1008 / 1625, 1233 / 1895, 1438 / 2795). Small models, whose operators
+            # are all launch latency, and eager steps keep the one launch.
+            self._chain_step = self.batch > 1 and self.cfg.hidden >= 2048
             self.forward(self.next_tokens, 1)  # warm-up: sizes every buffer outside the capture
             self.stream.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=self.stream, capture_error_mode="thread_local"):
                 self.forward(self.next_tokens, 1)
+            self._chain_step = False
             self.pos.copy_(saved[0])
             self.next_tokens.copy_(saved[1])
         self.stream.synchronize()
