@@ -364,57 +364,64 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             // D fp32, A and B fp16, both K-major, M = 128
             const uint32_t id_s = (1u << 4) | ((uint32_t)(AT_KT >> 3) << 17) | ((uint32_t)(AT_ROWS >> 4) << 24);
             const uint32_t id_o = (1u << 4) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(AT_ROWS >> 4) << 24);
             bool alive = true;
             auto scores = [&](int i) {
                 const int st = i % STAGES, s = i & 1;
-                alive = mbar_wait(kfull + st * 8, (uint32_t)(i / STAGES) & 1u, status) &&
-                        mbar_wait(sfree + s * 8, ((uint32_t)(i >> 1) & 1u) ^ 1u, status);
+                alive = __all_sync(0xffffffffu, mbar_wait(kfull + st * 8, (uint32_t)(i / STAGES) & 1u, status) &&
+                                                    mbar_wait(sfree + s * 8, ((uint32_t)(i >> 1) & 1u) ^ 1u, status));
                 if (!alive) return;
                 at_fence_after();
                 const uint32_t ks = base + G::RING + (uint32_t)st * ATImage<D>::BYTES;
-                uint32_t acc = 0;
+                if (elect_one()) {
+                    uint32_t acc = 0;
 #pragma unroll
-                for (int term = 0; term < 3; ++term) {      // lo hi, hi lo, hi hi
-                    const uint32_t qa = base + (term == 0 ? G::Q_TERM : 0), kb = ks + (term == 1 ? ATImage<D>::K_TERM : 0);
+                    for (int term = 0; term < 3; ++term) {      // lo hi, hi lo, hi hi
+                        const uint32_t qa = base + (term == 0 ? G::Q_TERM : 0), kb = ks + (term == 1 ? ATImage<D>::K_TERM : 0);
 #pragma unroll
-                    for (int sub = 0; sub < D / 64; ++sub) {
-                        const uint64_t da = at_desc(qa + sub * (AT_ROWS * 128)), db = at_desc(kb + sub * (AT_KT * 128));
+                        for (int sub = 0; sub < D / 64; ++sub) {
+                            const uint64_t da = at_desc(qa + sub * (AT_ROWS * 128)), db = at_desc(kb + sub * (AT_KT * 128));
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {     // K = 16 per instruction: +32 bytes
-                            at_mma_ss(t_s + s * 64, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), id_s, acc);
-                            acc = 1;
+                            for (int kk = 0; kk < 4; ++kk) {     // K = 16 per instruction: +32 bytes
+                                at_mma_ss(t_s + s * 64, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), id_s, acc);
+                                acc = 1;
+                            }
                         }
                     }
+                    at_commit(kempty + st * 8);
+                    at_commit(sfull + s * 8);
                 }
-                at_commit(kempty + st * 8);
-                at_commit(sfull + s * 8);
+                __syncwarp();
             };
             auto values = [&](int i) {
                 const int st = i % STAGES, s = i & 1;
                 const uint32_t par = (uint32_t)(i >> 1) & 1u;
-                alive = mbar_wait(vfull + st * 8, (uint32_t)(i / STAGES) & 1u, status) &&
-                        mbar_wait(pfull + s * 8, par, status) && mbar_wait(ofree + s * 8, par ^ 1u, status);
+                alive = __all_sync(0xffffffffu, mbar_wait(vfull + st * 8, (uint32_t)(i / STAGES) & 1u, status) &&
+                                                    mbar_wait(pfull + s * 8, par, status) &&
+                                                    mbar_wait(ofree + s * 8, par ^ 1u, status));
                 if (!alive) return;
                 at_fence_after();
                 const uint32_t vs = base + G::RING + (uint32_t)st * ATImage<D>::BYTES + ATImage<D>::K_BYTES;
-                uint32_t acc = 0;
+                if (elect_one()) {
+                    uint32_t acc = 0;
 #pragma unroll
-                for (int term = 0; term < 3; ++term) {
-                    const uint32_t pa = t_p + s * 64 + (term == 0 ? 32 : 0);
-                    const uint64_t db = at_desc(vs + (term == 1 ? ATImage<D>::V_TERM : 0));
+                    for (int term = 0; term < 3; ++term) {
+                        const uint32_t pa = t_p + s * 64 + (term == 0 ? 32 : 0);
+                        const uint64_t db = at_desc(vs + (term == 1 ? ATImage<D>::V_TERM : 0));
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {         // 16 keys: 8 columns of the weights
-                        at_mma_ts(t_o + s * 128, pa + kk * 8, db + (uint64_t)(kk * 2), id_o, acc);
-                        acc = 1;
+                        for (int kk = 0; kk < 4; ++kk) {         // 16 keys: 8 columns of the weights
+                            at_mma_ts(t_o + s * 128, pa + kk * 8, db + (uint64_t)(kk * 2), id_o, acc);
+                            acc = 1;
+                        }
                     }
+                    at_commit(vempty + st * 8);
+                    at_commit(pfree + s * 8);
+                    at_commit(ofull + s * 8);
                 }
-                at_commit(vempty + st * 8);
-                at_commit(pfree + s * 8);
-                at_commit(ofull + s * 8);
+                __syncwarp();
             };
             for (int i = 0; i < n && alive; ++i) {
                 scores(i);

@@ -63,13 +63,6 @@ __device__ __forceinline__ uint64_t bg_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
            (uint64_t)2 << 61;
 }
-// The issuing warp runs its loop converged and elects one lane around the instructions: with the whole
-// loop in one lane's branch the operands travel through ordinary registers and an MMA costs 65 cycles.
-__device__ __forceinline__ bool bg_elect() {
-    uint32_t p;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ void bg_mma(uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -236,7 +229,7 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
                     const uint32_t ta = t_a + slot * 64;
                     const uint64_t db = bg_desc(act + half * 2 * act_rows * 128);
                     const uint64_t sub_step = (uint64_t)(act_rows * 128 >> 4);
-                    if (bg_elect()) {
+                    if (elect_one()) {
                         if constexpr (EXACT) {
                             // rows 16..31 of an activation tile are the low terms (16 x 128 bytes further on);
                             // group g of 32 k: columns g * 16 of A, its own accumulator of 16 columns

@@ -212,7 +212,7 @@ int4_prefill_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        {
             // D fp32, A and B bf16, both K-major, N = BT, M = 128
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.BT >> 3) << 17) |
                                    ((uint32_t)(PG_BM >> 4) << 24);
@@ -220,39 +220,43 @@ int4_prefill_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             uint32_t phase = 0, aphase = 0, tphase = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < tiles && alive; t += gridDim.x) {
-                alive = mbar_wait(bar_tempty + tbuf * 8, tphase ^ 1u, status);
+                alive = __all_sync(0xffffffffu, mbar_wait(bar_tempty + tbuf * 8, tphase ^ 1u, status));
                 if (!alive) break;
                 pg_fence_after();
                 const uint32_t tacc = tmem_base + (uint32_t)tbuf * 256;
                 const int kb0 = SPLITK ? ((t / p.n_tiles) % p.ksplit) * p.kb_per : 0;
                 const int kb1 = SPLITK ? min(p.k_blocks, kb0 + p.kb_per) : p.k_blocks;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    alive = mbar_wait(bar_full + slot * 8, phase, status) &&
-                            mbar_wait(bar_afull + abuf * 8, aphase, status);
+                    alive = __all_sync(0xffffffffu, mbar_wait(bar_full + slot * 8, phase, status) &&
+                                                        mbar_wait(bar_afull + abuf * 8, aphase, status));
                     if (!alive) break;
                     pg_fence_after();
                     const uint32_t st = ring + (uint32_t)slot * p.stage_bytes;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int sub = 0; sub < KSUB; ++sub) {
+                        for (int sub = 0; sub < KSUB; ++sub) {
 #pragma unroll
-                        for (int a = 0; a < NA; ++a) {
-                            const uint64_t da = pg_desc_sw128(a_tiles + abuf * A_BUF + (sub * NA + a) * A_TILE);
-                            for (int j = 0; j < p.NT; ++j) {
-                                const uint64_t db = pg_desc_sw128(st + sub * act_bytes + j * (p.BT * 128));
+                            for (int a = 0; a < NA; ++a) {
+                                const uint64_t da = pg_desc_sw128(a_tiles + abuf * A_BUF + (sub * NA + a) * A_TILE);
+                                for (int j = 0; j < p.NT; ++j) {
+                                    const uint64_t db = pg_desc_sw128(st + sub * act_bytes + j * (p.BT * 128));
 #pragma unroll
-                                for (int kk = 0; kk < PG_BK / 16; ++kk)  // K = 16 per instruction: +32 bytes
-                                    pg_mma_bf16(tacc + a * acc_cols + j * p.BT, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2),
-                                                idesc, (kb > kb0 || sub > 0 || kk > 0) ? 1u : 0u);
+                                    for (int kk = 0; kk < PG_BK / 16; ++kk)  // K = 16 per instruction: +32 bytes
+                                        pg_mma_bf16(tacc + a * acc_cols + j * p.BT, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2),
+                                                    idesc, (kb > kb0 || sub > 0 || kk > 0) ? 1u : 0u);
+                                }
                             }
                         }
+                        pg_commit(bar_empty + slot * 8);
+                        pg_commit(bar_aempty + abuf * 8);
                     }
-                    pg_commit(bar_empty + slot * 8);
-                    pg_commit(bar_aempty + abuf * 8);
+                    __syncwarp();
                     if (++slot == p.stages) { slot = 0; phase ^= 1u; }
                     if (++abuf == 2) { abuf = 0; aphase ^= 1u; }
                 }
                 if (!alive) break;
-                pg_commit(bar_tfull + tbuf * 8);
+                if (elect_one()) pg_commit(bar_tfull + tbuf * 8);
+                __syncwarp();
                 if (++tbuf == p.acc_bufs) { tbuf = 0; tphase ^= 1u; }
             }
         }
