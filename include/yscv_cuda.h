@@ -95,8 +95,8 @@ const char *yscv_cuda_dispatch_report(const yscv_cuda_ctx *ctx);
  * (crates/yscv-onnx/src/runner/quant_stats.rs:21-92): how many calls each kernel family
  * served since the last reset. cpu_fallbacks is always 0: this library has no CPU path. */
 typedef struct {
-    uint64_t int4_gemv_calls;      /* m <= 16 passes on the integer-MMA decode kernel */
-    uint64_t int4_gemm_calls;      /* m > 16 calls on the tensor-core prefill GEMM */
+    uint64_t int4_gemv_calls;      /* m <= 16 passes on the fp32-exact decode kernels */
+    uint64_t int4_gemm_calls;      /* m > 16 calls on the bf16 tensor-core GEMMs */
     uint64_t int4_generic_calls;   /* passes on the warp-per-row kernel (odd group / k / alignment) */
     uint64_t int8_gemm_calls;      /* every int8 GEMM launch, whatever the epilogue */
     uint64_t qlinear_matmul_calls;
@@ -195,7 +195,8 @@ void yscv_cuda_int4_weight_free(yscv_cuda_int4_weight *w);
 /* The int4 branch of exec_matmul (crates/yscv-onnx/src/runner/linear.rs:223-278) on
  * device memory: d_activation [m,k] f32 -> d_output [m,n] f32. One pass over the
  * weights for any m (the reference re-reads them m times when m < 8). m <= 16 takes
- * the bandwidth-bound decode kernel, larger m the tensor-core prefill GEMM. */
+ * an fp32-exact decode kernel (integer MMA; 3..16 rows of a large matrix: two-term fp16 products
+ * with dequantised weights in tensor memory), larger m a bf16 tensor-core GEMM. */
 int yscv_cuda_int4_matmul_dev(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w,
                               const float *d_activation, float *d_output, size_t m);
 
