@@ -159,8 +159,8 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
     BGWalk walk(p);
     int tile, k0, k1;
     bool alive = true;
-    // The weights are the caller's constants: the first stages' are fetched while the predecessor
-    // drains. Everything else may be its output, or (workspace, `out`) still in its use.
+    // The weights are the caller's constants (the kernels that pack them are ordinary launches, complete
+    // before a dependent one starts): the first stages' are fetched while the predecessor drains. Everything else may be its output, or (workspace, `out`) still in its use.
     if (warp != 0) pdl_wait();
 
     if (warp == 0) {
@@ -197,6 +197,9 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
                     if (++st == p.stages) { st = 0; ph ^= 1u; }
                 }
             }
+            // a consumer gave up: no stage's copies may be in flight when the CTA leaves (bounded)
+            if (!alive)
+                for (int i = 0; i < p.stages; ++i) mbar_wait(full + i * 8, i < st ? ph : ph ^ 1u, nullptr);
         } else {
             pdl_wait();
         }
