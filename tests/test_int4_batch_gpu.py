@@ -109,3 +109,42 @@ def test_split_last_round(m, n, k):
     for n0 in range(0, n, 512):
         assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 5e-3, n0
     ctx.close()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (2048, 14336, 4096), (257, 19301, 4096),                       # two tiles left, 64 k blocks for 74 pairs
+    (200, 38400, 1792), (200, 38300, 4096),                        # one tile left, 14 and 32 k blocks
+    (130, 38400, 9344), (130, 38400, 9472), (130, 38400, 9600),    # one tile left, 73, 74 and 75 k blocks
+    (513, 13312, 2112),                                            # 78 tiles, four left, 64 k per stage
+])
+def test_split_last_round_reads_only_what_it_wrote(m, n, k):
+    """The same GEMM with fewer left-over k blocks than CTA pairs (some pairs then have no part of the last
+    round), behind a GEMM that left large values all over the workspace. Bound as above, column by column of
+    tiles."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k + m)
+    with torch.cuda.stream(stream):
+        packed, scales, _ = _weights(g, 10240, 8192)
+        x = torch.full((2048, 8192), 1e6, device="cuda")
+        out = torch.empty(2048, 10240, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), 10240, 8192, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), 2048)
+        report = ctx.dispatch_report()
+        assert "split over k" in report and " 0 split over k" not in report, report
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g)
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        report = ctx.dispatch_report()
+        want = x.double() @ w.T
+    stream.synchronize()
+    assert ctx.device_status() == 0
+    assert "split over k" in report and " 0 split over k" not in report, report
+    assert torch.all(out[m] == 7.0)
+    diff = out[:m].double() - want
+    for n0 in range(0, n, 512):
+        assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 5e-3, n0
+    ctx.close()

@@ -739,6 +739,8 @@ __global__ void __launch_bounds__(128) pp_join_kernel(PGParams p, int n_pairs, i
 #pragma unroll
     for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int c = c0; c <= c1; ++c) {
+        // (with fewer k blocks left than pairs some pairs have an empty range and wrote no part)
+        if ((long long)c * rest / n_pairs == (long long)(c + 1) * rest / n_pairs) continue;
         const float4 *src = reinterpret_cast<const float4 *>(p.parts + ((size_t)(c + i) * 256 + blockIdx.y * 8) * 512) + threadIdx.x;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
