@@ -28,9 +28,11 @@
  *    same device.
  *  - "_dev" entry points only enqueue work, with one exception: the first call
  *    for a shape larger than any seen before may grow the context's scratch
- *    buffers (a cudaFree and a cudaMalloc, which synchronise the device and are
+ *    buffers (a cudaMalloc and a cudaFree, which synchronise the device and are
  *    not allowed inside a stream capture). Run one call of every shape before
- *    capturing a CUDA graph.
+ *    capturing a CUDA graph. Calls after the capture may be larger: a buffer that
+ *    a captured call used stays allocated, outgrown or not, until the context is
+ *    destroyed, so the context has to outlive the graph's replays.
  *  - Pointers given to "_dev" entry points must be aligned as the natural
  *    vector width of the operand asks (16 bytes for f32 rows read with 128-bit
  *    loads); a pointer that is not is rejected with YSCV_CUDA_ERR_UNSUPPORTED or

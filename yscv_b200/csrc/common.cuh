@@ -42,12 +42,25 @@ struct OpCounters {
 };
 OpCounters &op_counters();
 
-// Grow-only device buffer owned by a context.
+// Grow-only device buffer owned by a context. A CUDA graph keeps the address that a captured call used, so a
+// buffer that was handed out inside a capture is not freed when a later call outgrows it: it goes to
+// `captured` and lives until release(). Such a buffer grows by half at least, so that what is kept stays below
+// twice the buffer in use.
 struct DeviceBuffer {
     void *ptr = nullptr;
     size_t bytes = 0;
-    int reserve(size_t want);
+    bool in_graph = false;           // handed out inside a capture since it was allocated
+    std::vector<void *> captured;    // outgrown, but a graph may still use them
+    // `stream`: the stream of the call that asks
+    int reserve(size_t want, cudaStream_t stream);
+    // The same for a buffer that a call can do without: false (and no error) where it would have to grow
+    // inside a capture or the memory is not there.
+    bool try_reserve(size_t want, cudaStream_t stream);
     void release();
+
+  private:
+    cudaError_t grow(size_t want);
+    bool note_capture(cudaStream_t stream);
 };
 
 }  // namespace yscv

@@ -1235,7 +1235,7 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
         const int chunk = sizeof(KV) == 4 && d_head > 64 ? 64 : 128;   // (what fits shared memory twice)
         const int n_splits = (int)((max_seq + chunk - 1) / chunk);
         const size_t need = batch * n_q * (size_t)n_splits * (d_head + 2) * sizeof(float);
-        int rc = ctx->scratch_attn.reserve(need);
+        int rc = ctx->scratch_attn.reserve(need, ctx->stream);
         if (rc) return rc;
         float *part = reinterpret_cast<float *>(ctx->scratch_attn.ptr);
         // one block per (key chunk, KV head, sequence): it serves every query head of the group
@@ -1368,7 +1368,7 @@ int yscv_cuda_f32_matmul_dev(yscv_cuda_ctx *ctx, const float *d_w, const float *
     const unsigned blocks = (unsigned)((n + 7) / 8 < (size_t)(16 * ctx->sm_count) ? (n + 7) / 8 : 16 * ctx->sm_count);
     if (m > 8 && ctx->f32_tensor_cores && f32_gemm_tc_supported(d_w, d_x, m, n, k)) {
         // wide batch: three TF32 products per fp32 product on the tensor cores, weights read once
-        int rc = ctx->scratch.reserve(f32_gemm_tc_scratch_bytes(m, k));
+        int rc = ctx->scratch.reserve(f32_gemm_tc_scratch_bytes(m, k), ctx->stream);
         if (rc) return rc;
         rc = f32_gemm_tc(ctx, d_w, d_x, m, n, k, d_out, ctx->scratch.ptr);
         if (rc) return rc;
@@ -1403,7 +1403,7 @@ int yscv_cuda_argmax_last_dev(yscv_cuda_ctx *ctx, const float *d_logits, size_t 
     if (vocab == 0) return fail(YSCV_CUDA_ERR_BAD_ARG, "empty vocabulary");
     if (vocab >= 8192) {
         const int nb = 64;
-        int rc = ctx->scratch_attn.reserve(rows * nb * 8);
+        int rc = ctx->scratch_attn.reserve(rows * nb * 8, ctx->stream);
         if (rc) return rc;
         float *pv = reinterpret_cast<float *>(ctx->scratch_attn.ptr);
         int32_t *pi = reinterpret_cast<int32_t *>(pv + rows * nb);

@@ -551,7 +551,7 @@ static int prefill_tc_launch(yscv_cuda_ctx *ctx, const float *q, size_t q_stride
     // the images of as many sequences as fit 256 MB at a time (at least one), so that the scratch stays bounded
     size_t bg = (256u << 20) / per_seq;
     bg = bg < 1 ? 1 : (bg > batch ? batch : bg);
-    int rc = ctx->scratch_attn.reserve(bg * per_seq);
+    int rc = ctx->scratch_attn.reserve(bg * per_seq, ctx->stream);
     if (rc) return rc;
     unsigned char *images = reinterpret_cast<unsigned char *>(ctx->scratch_attn.ptr);
     float *inv = reinterpret_cast<float *>(images + bg * n_kv * n_tiles * ATImage<D>::BYTES);

@@ -813,19 +813,14 @@ static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, con
     // Split the last round where that saves more than the parts cost: a round takes about 0.9 us per 64 k,
     // a part (512 KB written and read back) 0.125 us from L2 and up to twice that from HBM, the second launch
     // 3 us: 2048 x 8192 x 10240 (12 tiles left for 74 pairs) 345 -> 281 us, 2048 x 8192 x 57344 (8 left) 1675 ->
-    // 1592; with 54 left (2048 x 8192 x 8192) nothing is gained. The workspace is never grown
-    // inside a capture: there (without an earlier call of the size) the last round stays whole.
+    // 1592; with 54 left (2048 x 8192 x 8192) nothing is gained. Without memory for the parts, or inside a
+    // capture without an earlier call of the size, the last round stays whole.
     const int rest = tiles % pairs;
     p.full_tiles = tiles;
     if (tiles > pairs && rest > 0 && 0.9 * (p.K / 64) * (pairs - rest) / pairs > 2.0 * (0.125 * (pairs + rest) + 3.0)) {
-        const size_t need = (size_t)(pairs + rest) * 256 * 512 * sizeof(float);
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        YSCV_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
-        if (ctx->gemm_ws.bytes >= need || (cap == cudaStreamCaptureStatusNone && ctx->gemm_ws.reserve(need) == YSCV_CUDA_OK)) {
+        if (ctx->gemm_ws.try_reserve((size_t)(pairs + rest) * 256 * 512 * sizeof(float), ctx->stream)) {
             p.full_tiles = tiles - rest;
             p.parts = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
-        } else {
-            cudaGetLastError();   // (no memory for it: not this call's failure)
         }
     }
     ctx->prof_begin();
@@ -902,7 +897,7 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     float *kernel_out = out;
     const bool batch = int4_batch_bf16_wins(m, n, k, 32);   // up to 128 rows of a large matrix
     if (p.ksplit > 1 && !batch) {
-        rc_ws = ctx->gemm_ws.reserve((size_t)p.ksplit * m * n * sizeof(float));
+        rc_ws = ctx->gemm_ws.reserve((size_t)p.ksplit * m * n * sizeof(float), ctx->stream);
         if (rc_ws) return rc_ws;
         kernel_out = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
     }

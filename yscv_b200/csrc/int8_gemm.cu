@@ -763,10 +763,10 @@ static int launch_g8(yscv_cuda_ctx *ctx, const void *d_a, size_t lda, const yscv
         int units = (int)((tail_blocks + sms - 1) / sms);
         if (units < 4) units = 4;  // at most k_blocks / 4 + 1 parts per tile
         const int ctas = (int)((tail_blocks + units - 1) / units);
-        rc = ctx->gemm_ws.reserve((size_t)sms * G8_BM * 256 * sizeof(int32_t));
+        rc = ctx->gemm_ws.reserve((size_t)sms * G8_BM * 256 * sizeof(int32_t), ctx->stream);
         if (rc) return rc;
         if (!ctx->gemm_flags.ptr) {
-            rc = ctx->gemm_flags.reserve((size_t)sms * 4 * sizeof(int));
+            rc = ctx->gemm_flags.reserve((size_t)sms * 4 * sizeof(int), ctx->stream);
             if (rc) return rc;
             YSCV_CUDA_TRY(cudaMemsetAsync(ctx->gemm_flags.ptr, 0, (size_t)sms * 4 * sizeof(int), ctx->stream));
         }
@@ -872,7 +872,7 @@ int int8_gemm(yscv_cuda_ctx *ctx, const void *d_a, const yscv_cuda_i8b *b, size_
     p.b_zp = b->b_zp;
     p.k_true = (int)b->k;
     if (b->b_zp != 0) {
-        int rc = ctx->rowsum.reserve(m * sizeof(int32_t));
+        int rc = ctx->rowsum.reserve(m * sizeof(int32_t), ctx->stream);
         if (rc) return rc;
         rowsum_a_kernel<<<(unsigned)((m + 7) / 8), 256, 0, ctx->stream>>>(
             reinterpret_cast<const uint8_t *>(d_a), reinterpret_cast<int32_t *>(ctx->rowsum.ptr), (int)m,
@@ -885,7 +885,7 @@ int int8_gemm(yscv_cuda_ctx *ctx, const void *d_a, const yscv_cuda_i8b *b, size_
     size_t lda = b->k;
     if (b->k != b->kp || (reinterpret_cast<uintptr_t>(d_a) & 15)) {
         // TMA needs a 16-byte aligned base and row pitch: stage A into a padded copy
-        int rc = ctx->scratch.reserve(m * b->kp);
+        int rc = ctx->scratch.reserve(m * b->kp, ctx->stream);
         if (rc) return rc;
         const size_t total = m * b->kp;
         const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
