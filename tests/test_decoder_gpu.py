@@ -163,6 +163,7 @@ def run_parity(tctx, oracle, cfg, n_layers, batch, prompt_len, steps, seed, logi
         flip_margin = 1e-2
     dec = Int4Decoder.with_full_weights(ctx, cfg, batch, prompt_len + steps + 1, s, seed=seed, layers=n_layers,
                                         fused_step=fused_step, kv_int8=kv_int8, plan_options=plan_options)
+    dec.one_launch = dec.plan is not None   # the form that the caller asked for, also where the chain is the default
     assert (dec.plan is not None) == (fused_step and (batch == 1 or (batch <= 8 and not kv_int8 and cfg.hidden <= 2048)))
     from oracle_decoder import OracleDecoder
     ref = OracleDecoder(oracle, cfg, n_layers, export_weights(dec), dec.embedding.cpu().numpy(),

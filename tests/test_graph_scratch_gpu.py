@@ -90,3 +90,35 @@ def test_outgrown_buffers_are_given_back():
         ctx.close()
         del x, out
     assert abs(used[0] - used[1]) <= 8 << 20, used
+
+
+@pytest.mark.parametrize("hidden,batch,launches", [(512, 1, 1), (512, 4, 1), (1024, 4, None), (2048, 1, 1), (2048, 2, None),
+                                                    (2048, 8, None)])
+def test_eager_and_replayed_steps_take_the_same_form(hidden, batch, launches):
+    """Bit for bit the same logits and tokens, whichever form (one launch, or None: the operator chain) the
+    shape takes; a program that chooses the other form gets it in both."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    cfg = DecoderConfig(layers=2, hidden=hidden, mlp=2 * hidden, n_q=hidden // 64, n_kv=4, head_dim=64, vocab=9000)
+    rows = [synth.uniform_int(80 + b, 7, 20, 0, cfg.vocab - 1) for b in range(batch)]
+    prompt = torch.from_numpy(np.stack(rows).astype(np.int32)).cuda()
+    for other in (False, True):
+        want = not other if launches else other
+        got = []
+        for graph in (False, True):
+            dec = Int4Decoder(ctx, cfg, batch, 64, stream, seed=6)
+            assert dec.plan is not None and dec.one_launch == (launches is not None)
+            dec.one_launch = want
+            dec.prefill(prompt)
+            if graph:
+                dec.capture_decode_step()
+            before = ctx.launch_count()
+            toks = dec.decode(5, use_graph=graph)
+            stream.synchronize()
+            if not graph:
+                assert (ctx.launch_count() - before == 5) == want
+            got.append((toks, dec._buf("logits", batch, cfg.vocab).clone()))
+            dec.close()
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert ctx.device_status() == 0
+    ctx.close()

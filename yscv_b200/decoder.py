@@ -45,6 +45,14 @@ class DecoderConfig:
     weight_std: float = 0.02
 
 
+# Steps of 2..8 sequences run as the operator chain from this hidden size on, as one launch below: the line lies
+# where the chain is the faster form eagerly too (a launch costs host time there). us per step, chain / one launch,
+# 200 cached positions, replayed and eager: hidden 512 (8 layers) batch 2 251 / 286 and 360 / 287, batch 8 318 / 351
+# and 442 / 351; 1024 (16 layers) batch 2 574 / 754 and 689 / 754, batch 8 713 / 884 and 846 / 884; 2048 (22
+# layers) batch 2 983 / 1363 and 1043 / 1362, batch 8 1252 / 1782 and 1320 / 1781. Longer caches favour the chain:
+# after 1500 positions 1427 / 2809 and 1494 / 2810 there. (Above 2048 the batch form has no plan.)
+CHAIN_HIDDEN = 1024
+
 TINYLLAMA_1B = DecoderConfig(22, 2048, 5632, 32, 4, 64, 32000, 1e-5, 10000.0)
 LLAMA3_70B = DecoderConfig(80, 8192, 28672, 64, 8, 128, 128256, 1e-5, 500000.0)
 
@@ -120,6 +128,10 @@ class Int4Decoder:
                 if int(ok.item()) == 0 and self.plan is not None:
                     self.plan.free()
                     self.plan = None
+        # Whether single-token steps, eager and captured alike, run as that one launch or as the operator chain
+        # (a program may choose before its first step). Batches of 2..8 sequences take the chain from hidden
+        # CHAIN_HIDDEN on.
+        self.one_launch = self.plan is not None and (batch == 1 or cfg.hidden < CHAIN_HIDDEN)
 
     def _connect_tp(self):
         """Create this rank's exchange region, gather every rank's IPC handle, map the peers."""
@@ -182,7 +194,6 @@ class Int4Decoder:
             self.wdown.append(self._linear(*sharding.shard_cols(pd, sd, g, r, G)))
 
     _keep_full = False
-    _chain_step = False
 
     @classmethod
     def with_full_weights(cls, *args, **kw):
@@ -226,7 +237,7 @@ class Int4Decoder:
         if act16:
             h16 = self._buf("h16", rows, H, dtype=torch.bfloat16)
             a16 = self._buf("a16", rows, self.mlp_l, dtype=torch.bfloat16)
-        fused = self.plan is not None and seq == 1 and not self._chain_step
+        fused = self.one_launch and seq == 1
         if fused:
             # the whole step in one launch: layers, final norm, LM head, greedy token, position
             logits = self._buf("logits", B, c.vocab)
@@ -287,6 +298,7 @@ class Int4Decoder:
         before the process group is destroyed: a graph that holds NCCL nodes must go first."""
         self.stream.synchronize()
         self.graph = None
+        self.one_launch = False
         if self.plan is not None:
             self.plan.free()
             self.plan = None
@@ -316,17 +328,11 @@ class Int4Decoder:
         """Record one decode step (reads self.next_tokens, writes it back) as a CUDA graph."""
         with torch.cuda.stream(self.stream):
             saved = self.pos.clone(), self.next_tokens.clone()
-            # Batches of 2..8 sequences: replayed from a graph, where a launch costs no host time, the operator
-            # chain is the faster step (1B shape, us, chain / one launch: batch 2 979 / 1353, 4 1162 / 1400, 8 1220 /
-            # 1783; after 1500 tokens 1008 / 1625, 1233 / 1895, 1438 / 2795). Small models, whose operators
-            # are all launch latency, and eager steps keep the one launch.
-            self._chain_step = self.batch > 1 and self.cfg.hidden >= 2048
             self.forward(self.next_tokens, 1)  # warm-up: sizes every buffer outside the capture
             self.stream.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=self.stream, capture_error_mode="thread_local"):
                 self.forward(self.next_tokens, 1)
-            self._chain_step = False
             self.pos.copy_(saved[0])
             self.next_tokens.copy_(saved[1])
         self.stream.synchronize()

@@ -126,7 +126,7 @@ def run(model="tinyllama", batch=1, prompt_len=128, max_tokens=256, warmup=1, la
         "cuda_graph": bool(use_graph), "prefill": "fp32-exact" if exact_prefill else "bf16 tensor-core",
         "decode_step": ("one persistent kernel per token" + (" per GPU, partial sums exchanged through peer memory "
                                                               "inside it" if world > 1 else ""))
-        if dec.plan is not None else ("operator chain" + (" + NCCL all-reduce" if world > 1 else "")),
+        if dec.one_launch else ("operator chain" + (" + NCCL all-reduce" if world > 1 else "")),
         "kv_cache": ("int8 rows + f32 scale per token" if kv_int8 else "f32") +
                     (", first prompt_len positions filled with random rows instead of a prompt pass" if synthetic_cache else ""),
         "first_tokens": toks[:8, 0].cpu().tolist(),
