@@ -50,3 +50,51 @@ def test_decode_shares(d, n_kv, group, max_seq, cached, kv_int8):
     assert torch.all(out[-8:] == 3.0)
     assert float((got - want).norm() / want.norm()) <= (4e-5 if kv_int8 else 4e-6)
     ctx.close()
+
+
+@pytest.mark.parametrize("d", [48, 64, 128])
+@pytest.mark.parametrize("kv_int8", [False, True])
+def test_shares_of_infinite_scores(d, kv_int8):
+    """A whole share of keys with scores of -inf weighs nothing in the merge; a NaN score reaches the output of
+    its head and of no other."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d)
+    n_q, n_kv, max_seq, cached = 6, 2, 400, 390
+    with torch.cuda.stream(stream):
+        q = torch.rand(1, n_q * d, device="cuda", generator=g) + 0.1     # (positive: the sign of a score is its key's)
+        shape = (1, max_seq, n_kv, d)
+        pos = torch.full((1,), cached, dtype=torch.int32, device="cuda")
+        out = torch.empty(n_q, d, device="cuda")
+        if kv_int8:
+            k, v = (torch.randint(-127, 128, shape, dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+            k[0, :200] = -torch.randint(1, 128, (200, n_kv, d), device="cuda", generator=g).to(torch.int8)
+            ks, vs = (torch.rand(1, max_seq, device="cuda", generator=g) * 0.01 + 0.005 for _ in range(2))
+            ks[0, :200] = float("inf")
+        else:
+            k, v = (torch.randn(shape, device="cuda", generator=g) for _ in range(2))
+            k[0, :200, :, 0] = -float("inf")
+
+        def call():
+            if kv_int8:
+                ctx.gqa_attention_i8_dev(q.data_ptr(), n_q * d, 1, 1, n_q, n_kv, d, k.data_ptr(), ks.data_ptr(), v.data_ptr(),
+                                         vs.data_ptr(), max_seq, pos.data_ptr(), True, out.data_ptr())
+            else:
+                ctx.gqa_attention_dev(q.data_ptr(), n_q * d, 1, 1, n_q, n_kv, d, k.data_ptr(), v.data_ptr(), max_seq,
+                                      pos.data_ptr(), True, out.data_ptr())
+            return out.clone()
+
+        got = call()
+        kd, vd = (k * ks[:, :, None, None], v * vs[:, :, None, None]) if kv_int8 else (k, v)
+        kd, vd = kd[0, 200:cached + 1].double(), vd[0, 200:cached + 1].double()
+        p = torch.softmax(torch.einsum("hgd,shd->hgs", q.double().view(n_kv, -1, d), kd) / math.sqrt(d), -1)
+        want = torch.einsum("hgs,shd->hgd", p, vd).reshape(n_q, d)
+        q[0, 2 * d] = float("nan")
+        poisoned = call()
+    stream.synchronize()
+    assert float((got.double() - want).norm() / want.norm()) <= (4e-5 if kv_int8 else 4e-6)
+    assert torch.isnan(poisoned[2]).all()
+    keep = [0, 1, 3, 4, 5]
+    assert torch.equal(poisoned[keep], got[keep])
+    ctx.close()

@@ -562,10 +562,11 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float ref = mx == -INFINITY ? 0.0f : mx;   // a share of -inf scores weighs nothing (and is no -inf + inf)
 #pragma unroll
             for (int i = 0; i < CH / 32; ++i) {
                 const int j = lane + i * 32;
-                e[i] = j < nk ? expf(e[i] - mx) : 0.0f;
+                e[i] = j < nk ? expf(e[i] - ref) : 0.0f;
                 se += e[i];
                 // int8 values: fold the row scale of the value row into its weight once
                 if (j < nk) wts[warp * WP + j] = I8 ? e[i] * vsc[j] : e[i];
@@ -800,9 +801,10 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
             const int key = 4 * lane;
             float e[4] = {sv.x, sv.y, sv.z, sv.w};
             float se = 0.0f;
+            const float ref = mx == -INFINITY ? 0.0f : mx;   // (as above)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                e[i] = (key + i < nk && h < nh) ? expf(e[i] - mx) : 0.0f;
+                e[i] = (key + i < nk && h < nh) ? expf(e[i] - ref) : 0.0f;
                 se += e[i];
             }
 #pragma unroll
