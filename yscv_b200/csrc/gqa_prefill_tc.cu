@@ -112,7 +112,14 @@ __device__ __forceinline__ void at_split(float a, float b, uint32_t &hi, uint32_
 
 // ---- keys and values of one layer -> fp16 hi / lo images ---------------------------------------
 // Block (tile of 64 keys, KV head, sequence). Image of a tile: keys {hi, lo} x [D / 64][64 rows][128 B],
-// values {hi, lo} x [D rows][128 B]; rows past the last key in use are zeros.
+// values {hi, lo} x [D rows][128 B]; rows past the last key in use are zeros. inv_scales: the inverse scales
+// {keys, values} of the tile; 0 for the keys says that the tile cannot be had in two terms:
+//   - a row with an infinity or NaN (it would reach, as 0 x NaN, positions that do not attend to its key),
+//   - a row whose largest magnitude is below 2^-12 of the tile's (its absolute error, 2^-39 of the tile's
+//     maximum, would come near 2^-24 of the row's own, which is what an fp32 operand has),
+//   - a tile maximum outside [2^-50, 2^50] (the product of the inverse scales would leave the fp32 range).
+constexpr float AT_ROW_RANGE = 1.0f / 4096.0f, AT_LEAST = 8.8817842e-16f, AT_MOST = 1.1258999e15f;
+__device__ __forceinline__ bool at_in_range(float amax) { return (amax == 0.0f) | ((amax >= AT_LEAST) & (amax <= AT_MOST)); }
 template <int D> struct ATImage {
     static constexpr int K_TERM = AT_KT * D * 2;          // one term of the keys, in bytes
     static constexpr int V_TERM = AT_KT * D * 2;
@@ -120,11 +127,24 @@ template <int D> struct ATImage {
     static constexpr int BYTES = K_BYTES + V_BYTES;
 };
 
+// What both kernels know of a call. A (sequence, KV head) pair is b * n_kv + head.
+template <typename KV> struct ATCall {
+    const float *q;
+    int q_stride, q_vec, seq_q, n_q, n_kv, max_seq, causal;
+    const KV *kc, *vc;
+    const float *kscale, *vscale;
+    const int32_t *pos;
+    float *out;
+    int QB;                       // query positions per CTA
+    int n_tiles;                  // key tiles of max_seq
+    int pair0, pairs;             // pairs of this launch
+    unsigned char *images;        // [pairs][n_tiles]
+    float *inv_scales;            // [pairs][n_tiles][2]
+};
+
+// Block (pair, tile), then every gridDim.y-th tile of the pair up to the last key in use
 template <typename KV, int D>
-__global__ void __launch_bounds__(256)
-kv_split_kernel(const KV *__restrict__ kc, const KV *__restrict__ vc, const float *__restrict__ kscale,
-                const float *__restrict__ vscale, int n_kv, int max_seq, int seq_q, const int32_t *__restrict__ pos,
-                unsigned char *__restrict__ images, float *__restrict__ inv_scales) {
+__global__ void __launch_bounds__(256, 3) kv_split_kernel(const __grid_constant__ ATCall<KV> a) {
     pdl_wait();
     pdl_trigger();
     constexpr bool I8 = sizeof(KV) == 1;
@@ -132,95 +152,111 @@ kv_split_kernel(const KV *__restrict__ kc, const KV *__restrict__ vc, const floa
     constexpr int ITEMS = AT_KT * CPR / 256;      // such groups per thread
     __shared__ float vt[AT_KT][D + 1];
     __shared__ float red[2][8];
-    const int tile = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
-    int limit = *pos + seq_q;
-    limit = limit > max_seq ? max_seq : limit;
-    const int k0 = tile * AT_KT;
-    if (k0 >= limit) return;
-    const size_t row_elems = (size_t)n_kv * D;
-    const KV *kb = kc + ((size_t)b * max_seq + k0) * row_elems + (size_t)h * D;
-    const KV *vb = vc + ((size_t)b * max_seq + k0) * row_elems + (size_t)h * D;
-    float k[ITEMS][8], v[ITEMS][8];
+    const int b = (a.pair0 + blockIdx.x) / a.n_kv, h = (a.pair0 + blockIdx.x) % a.n_kv, tid = threadIdx.x;
+    const int limit = min(*a.pos + a.seq_q, a.max_seq);
+    const size_t row_elems = (size_t)a.n_kv * D;
+    for (int tile = blockIdx.y; tile * AT_KT < limit; tile += gridDim.y) {
+        const int k0 = tile * AT_KT;
+        const size_t row0 = (size_t)b * a.max_seq + k0;
+        const KV *kb = a.kc + row0 * row_elems + (size_t)h * D, *vb = a.vc + row0 * row_elems + (size_t)h * D;
+        float k[ITEMS][8], v[ITEMS][8];
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-        const int idx = tid + it * 256, r = idx / CPR, c = (idx % CPR) * 8;
-        const bool live = k0 + r < limit;
-        if constexpr (I8) {
-            const float rk = live ? kscale[(size_t)b * max_seq + k0 + r] : 0.0f, rv = live ? vscale[(size_t)b * max_seq + k0 + r] : 0.0f;
-            uint2 kw = make_uint2(0u, 0u), vw = make_uint2(0u, 0u);
-            if (live) {
-                kw = *reinterpret_cast<const uint2 *>(kb + r * row_elems + c);
-                vw = *reinterpret_cast<const uint2 *>(vb + r * row_elems + c);
+        for (int it = 0; it < ITEMS; ++it) {
+            const int idx = tid + it * 256, r = idx / CPR, c = (idx % CPR) * 8;
+            const bool live = k0 + r < limit;
+            if constexpr (I8) {
+                const float rk = live ? a.kscale[row0 + r] : 0.0f, rv = live ? a.vscale[row0 + r] : 0.0f;
+                uint2 kw = make_uint2(0u, 0u), vw = make_uint2(0u, 0u);
+                if (live) {
+                    kw = *reinterpret_cast<const uint2 *>(kb + r * row_elems + c);
+                    vw = *reinterpret_cast<const uint2 *>(vb + r * row_elems + c);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t wk = j < 4 ? kw.x : kw.y, wv = j < 4 ? vw.x : vw.y;
+                    k[it][j] = __fmul_rn((float)(int8_t)(wk >> (8 * (j & 3))), rk);
+                    v[it][j] = __fmul_rn((float)(int8_t)(wv >> (8 * (j & 3))), rv);
+                }
+            } else {
+                float4 ka = make_float4(0.f, 0.f, 0.f, 0.f), kd = ka, va = ka, vd = ka;
+                if (live) {
+                    const float4 *kp = reinterpret_cast<const float4 *>(kb + r * row_elems + c);
+                    const float4 *vp = reinterpret_cast<const float4 *>(vb + r * row_elems + c);
+                    ka = kp[0]; kd = kp[1]; va = vp[0]; vd = vp[1];
+                }
+                k[it][0] = ka.x; k[it][1] = ka.y; k[it][2] = ka.z; k[it][3] = ka.w;
+                k[it][4] = kd.x; k[it][5] = kd.y; k[it][6] = kd.z; k[it][7] = kd.w;
+                v[it][0] = va.x; v[it][1] = va.y; v[it][2] = va.z; v[it][3] = va.w;
+                v[it][4] = vd.x; v[it][5] = vd.y; v[it][6] = vd.z; v[it][7] = vd.w;
             }
+        }
+        float km = 0.0f, vm = 0.0f, krow[ITEMS], vrow[ITEMS];   // of the tile, of this thread's rows (CPR lanes each)
+        float nan = 0.0f;                                        // 0 x value, summed: NaN behind an infinity or NaN
+#pragma unroll
+        for (int it = 0; it < ITEMS; ++it) {
+            const int idx = tid + it * 256, r = idx / CPR, c = (idx % CPR) * 8;
+            krow[it] = vrow[it] = 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const uint32_t wk = j < 4 ? kw.x : kw.y, wv = j < 4 ? vw.x : vw.y;
-                k[it][j] = __fmul_rn((float)(int8_t)(wk >> (8 * (j & 3))), rk);
-                v[it][j] = __fmul_rn((float)(int8_t)(wv >> (8 * (j & 3))), rv);
+                krow[it] = fmaxf(krow[it], fabsf(k[it][j]));
+                vrow[it] = fmaxf(vrow[it], fabsf(v[it][j]));
+                nan = fmaf(k[it][j], 0.0f, fmaf(v[it][j], 0.0f, nan));
+                vt[r][c + j] = v[it][j];
             }
-        } else {
-            float4 ka = make_float4(0.f, 0.f, 0.f, 0.f), kd = ka, va = ka, vd = ka;
-            if (live) {
-                const float4 *kp = reinterpret_cast<const float4 *>(kb + r * row_elems + c);
-                const float4 *vp = reinterpret_cast<const float4 *>(vb + r * row_elems + c);
-                ka = kp[0]; kd = kp[1]; va = vp[0]; vd = vp[1];
+#pragma unroll
+            for (int o = CPR / 2; o > 0; o >>= 1) {
+                krow[it] = fmaxf(krow[it], __shfl_xor_sync(0xffffffffu, krow[it], o));
+                vrow[it] = fmaxf(vrow[it], __shfl_xor_sync(0xffffffffu, vrow[it], o));
             }
-            k[it][0] = ka.x; k[it][1] = ka.y; k[it][2] = ka.z; k[it][3] = ka.w;
-            k[it][4] = kd.x; k[it][5] = kd.y; k[it][6] = kd.z; k[it][7] = kd.w;
-            v[it][0] = va.x; v[it][1] = va.y; v[it][2] = va.z; v[it][3] = va.w;
-            v[it][4] = vd.x; v[it][5] = vd.y; v[it][6] = vd.z; v[it][7] = vd.w;
+            km = fmaxf(km, krow[it]);
+            vm = fmaxf(vm, vrow[it]);
         }
-    }
-    float km = 0.0f, vm = 0.0f;
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-        const int idx = tid + it * 256, r = idx / CPR, c = (idx % CPR) * 8;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            km = fmaxf(km, fabsf(k[it][j]));
-            vm = fmaxf(vm, fabsf(v[it][j]));
-            vt[r][c + j] = v[it][j];
+        for (int o = 16; o >= CPR; o >>= 1) {
+            km = fmaxf(km, __shfl_xor_sync(0xffffffffu, km, o));
+            vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
         }
-    }
+        if ((tid & 31) == 0) { red[0][tid >> 5] = km; red[1][tid >> 5] = vm; }
+        __syncthreads();
+        for (int i = 0; i < 8; ++i) { km = fmaxf(km, red[0][i]); vm = fmaxf(vm, red[1][i]); }
+        bool wide = (nan != 0.0f) | !at_in_range(km) | !at_in_range(vm);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        km = fmaxf(km, __shfl_xor_sync(0xffffffffu, km, o));
-        vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
-    }
-    if ((tid & 31) == 0) { red[0][tid >> 5] = km; red[1][tid >> 5] = vm; }
-    __syncthreads();
-    for (int i = 0; i < 8; ++i) { km = fmaxf(km, red[0][i]); vm = fmaxf(vm, red[1][i]); }
-    float kup, kdown, vup, vdown;
-    at_scale(km, kup, kdown);
-    at_scale(vm, vup, vdown);
-    const size_t t_idx = ((size_t)b * n_kv + h) * gridDim.x + tile;
-    unsigned char *img = images + t_idx * ATImage<D>::BYTES;
-    if (tid == 0) { inv_scales[2 * t_idx] = kdown; inv_scales[2 * t_idx + 1] = vdown; }
+        for (int it = 0; it < ITEMS; ++it)
+            wide |= ((krow[it] > 0.0f) & (krow[it] < km * AT_ROW_RANGE)) | ((vrow[it] > 0.0f) & (vrow[it] < vm * AT_ROW_RANGE));
+        wide = __syncthreads_or(wide);
+        float kup, kdown, vup, vdown;
+        at_scale(km, kup, kdown);
+        at_scale(vm, vup, vdown);
+        const size_t t_idx = (size_t)blockIdx.x * a.n_tiles + tile;
+        unsigned char *img = a.images + t_idx * ATImage<D>::BYTES;
+        if (tid == 0) { a.inv_scales[2 * t_idx] = wide ? 0.0f : kdown; a.inv_scales[2 * t_idx + 1] = vdown; }
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-        const int idx = tid + it * 256, r = idx / CPR, c8 = idx % CPR;
-        uint4 hi, lo;
-        at_split(k[it][0] * kup, k[it][1] * kup, hi.x, lo.x);
-        at_split(k[it][2] * kup, k[it][3] * kup, hi.y, lo.y);
-        at_split(k[it][4] * kup, k[it][5] * kup, hi.z, lo.z);
-        at_split(k[it][6] * kup, k[it][7] * kup, hi.w, lo.w);
-        // 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 64-element sub-tile
-        unsigned char *dst = img + (c8 >> 3) * (AT_KT * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4);
-        *reinterpret_cast<uint4 *>(dst) = hi;
-        *reinterpret_cast<uint4 *>(dst + ATImage<D>::K_TERM) = lo;
-    }
-    unsigned char *vimg = img + ATImage<D>::K_BYTES;
+        for (int it = 0; it < ITEMS; ++it) {
+            const int idx = tid + it * 256, r = idx / CPR, c8 = idx % CPR;
+            uint4 hi, lo;
+            at_split(k[it][0] * kup, k[it][1] * kup, hi.x, lo.x);
+            at_split(k[it][2] * kup, k[it][3] * kup, hi.y, lo.y);
+            at_split(k[it][4] * kup, k[it][5] * kup, hi.z, lo.z);
+            at_split(k[it][6] * kup, k[it][7] * kup, hi.w, lo.w);
+            // 16-byte chunk c of row r sits at chunk c ^ (r & 7) of its 64-element sub-tile
+            unsigned char *dst = img + (c8 >> 3) * (AT_KT * 128) + r * 128 + (((c8 & 7) ^ (r & 7)) << 4);
+            *reinterpret_cast<uint4 *>(dst) = hi;
+            *reinterpret_cast<uint4 *>(dst + ATImage<D>::K_TERM) = lo;
+        }
+        unsigned char *vimg = img + ATImage<D>::K_BYTES;
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-        const int idx = tid + it * 256, d = idx % D, g = idx / D;   // element d of keys 8 g .. 8 g + 7
-        uint4 hi, lo;
-        at_split(vt[8 * g][d] * vup, vt[8 * g + 1][d] * vup, hi.x, lo.x);
-        at_split(vt[8 * g + 2][d] * vup, vt[8 * g + 3][d] * vup, hi.y, lo.y);
-        at_split(vt[8 * g + 4][d] * vup, vt[8 * g + 5][d] * vup, hi.z, lo.z);
-        at_split(vt[8 * g + 6][d] * vup, vt[8 * g + 7][d] * vup, hi.w, lo.w);
-        unsigned char *dst = vimg + d * 128 + ((g ^ (d & 7)) << 4);
-        *reinterpret_cast<uint4 *>(dst) = hi;
-        *reinterpret_cast<uint4 *>(dst + ATImage<D>::V_TERM) = lo;
+        for (int it = 0; it < ITEMS; ++it) {
+            const int idx = tid + it * 256, d = idx % D, g = idx / D;   // element d of keys 8 g .. 8 g + 7
+            uint4 hi, lo;
+            at_split(vt[8 * g][d] * vup, vt[8 * g + 1][d] * vup, hi.x, lo.x);
+            at_split(vt[8 * g + 2][d] * vup, vt[8 * g + 3][d] * vup, hi.y, lo.y);
+            at_split(vt[8 * g + 4][d] * vup, vt[8 * g + 5][d] * vup, hi.z, lo.z);
+            at_split(vt[8 * g + 6][d] * vup, vt[8 * g + 7][d] * vup, hi.w, lo.w);
+            unsigned char *dst = vimg + d * 128 + ((g ^ (d & 7)) << 4);
+            *reinterpret_cast<uint4 *>(dst) = hi;
+            *reinterpret_cast<uint4 *>(dst + ATImage<D>::V_TERM) = lo;
+        }
+        __syncthreads();   // the next tile writes vt and red
     }
 }
 
@@ -234,13 +270,137 @@ template <int D> struct ATGeom {
     static constexpr int SMEM = BARS + 272;
 };
 
-template <int D>
-__global__ void __launch_bounds__(AT_THREADS, 1)
-gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int seq_q, int n_q, int n_kv, int max_seq,
-                      const int32_t *__restrict__ pos, int causal, const unsigned char *__restrict__ images,
-                      const float *__restrict__ inv_scales, int n_tiles, float *__restrict__ out, int QB,
-                      int *__restrict__ status) {
+// The query tile in fp32 throughout, for what two fp16 terms cannot hold (see kv_split_kernel): FMAs over 64-key chunks staged in shared memory, four (position, head) pairs per warp. A key
+// that a pair does not attend to is not multiplied at all. 2048 tokens, 64 / 8 heads of 128: 3.5 ms a layer
+// against 0.28 on the tensor cores.
+template <typename KV, int D>
+__device__ __noinline__ void at_fp32_tile(const ATCall<KV> &a, float *sm, int b, int kv_h, int qt, int p0) {
+    constexpr bool I8 = sizeof(KV) == 1;
+    constexpr int KP = D + 4;   // key row pitch: a lane per key reads its row 16 bytes at a time without bank conflicts
+    constexpr int KPAR = 32 / (D / 4), WARPS = AT_THREADS / 32, QH = 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *ks = sm, *vs = ks + AT_KT * KP, *sc = vs + AT_KT * D + warp * QH * AT_KT;
+    float *qs = vs + AT_KT * D + WARPS * QH * AT_KT + warp * QH * D;
+    const int group = a.n_q / a.n_kv;
+    const float scale = 1.0f / sqrtf((float)D);
+    const int e4 = (lane % (D / 4)) * 4, kpar = lane / (D / 4);
+    const size_t row_elems = (size_t)a.n_kv * D, seq_row = (size_t)b * a.max_seq;
+    for (int r0 = 0; r0 < group * a.QB; r0 += WARPS * QH) {
+        int sq[QH], qh[QH], lim[QH];
+        bool live[QH];
+        float4 acc[QH];
+        float m[QH], l[QH];
+        int warp_limit = 0;
+#pragma unroll
+        for (int j = 0; j < QH; ++j) {
+            const int idx = r0 + warp * QH + j;
+            sq[j] = qt * a.QB + idx / group;
+            qh[j] = kv_h * group + idx % group;
+            live[j] = idx < group * a.QB && sq[j] < a.seq_q;
+            lim[j] = live[j] ? max(0, min(a.max_seq, p0 + (a.causal ? sq[j] + 1 : a.seq_q))) : 0;
+            warp_limit = max(warp_limit, lim[j]);
+            acc[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            m[j] = -INFINITY;
+            l[j] = 0.0f;
+            for (int i = lane; i < D; i += 32)
+                qs[j * D + i] = live[j] ? a.q[((size_t)b * a.seq_q + sq[j]) * a.q_stride + (size_t)qh[j] * D + i] : 0.0f;
+        }
+        const int last = min(a.seq_q, qt * a.QB + (min(r0 + WARPS * QH, group * a.QB) - 1) / group + 1);
+        const int block_limit = max(0, min(a.max_seq, p0 + (a.causal ? last : a.seq_q)));
+        for (int c0 = 0; c0 < block_limit; c0 += AT_KT) {
+            const int rows = min(AT_KT, block_limit - c0);
+            __syncthreads();
+            for (int idx = threadIdx.x; idx < rows * (D / 4); idx += AT_THREADS) {
+                const int r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
+                const size_t off = (seq_row + c0 + r) * row_elems + (size_t)kv_h * D + c4;
+                float4 k4, v4;
+                if constexpr (I8) {
+                    const float rk = a.kscale[seq_row + c0 + r], rv = a.vscale[seq_row + c0 + r];
+                    const char4 kw = *reinterpret_cast<const char4 *>(a.kc + off), vw = *reinterpret_cast<const char4 *>(a.vc + off);
+                    k4 = make_float4(__fmul_rn((float)kw.x, rk), __fmul_rn((float)kw.y, rk), __fmul_rn((float)kw.z, rk), __fmul_rn((float)kw.w, rk));
+                    v4 = make_float4(__fmul_rn((float)vw.x, rv), __fmul_rn((float)vw.y, rv), __fmul_rn((float)vw.z, rv), __fmul_rn((float)vw.w, rv));
+                } else {
+                    k4 = *reinterpret_cast<const float4 *>(a.kc + off);
+                    v4 = *reinterpret_cast<const float4 *>(a.vc + off);
+                }
+                *reinterpret_cast<float4 *>(ks + r * KP + c4) = k4;
+                *reinterpret_cast<float4 *>(vs + r * D + c4) = v4;
+            }
+            __syncthreads();
+            const int nkw = min(rows, warp_limit - c0);   // keys of this chunk that any of the warp's pairs attends to
+            if (nkw <= 0) continue;
+            // scores: a lane per key (lane and lane + 32), each piece of a query read once for both
+            float s[2][QH];
+#pragma unroll
+            for (int j = 0; j < QH; ++j) s[0][j] = s[1][j] = 0.0f;
+            const float4 *kr = reinterpret_cast<const float4 *>(ks + lane * KP);
+#pragma unroll 2
+            for (int i = 0; i < D / 4; ++i) {
+                const float4 k0 = kr[i], k1 = kr[i + 32 * KP / 4];
+#pragma unroll
+                for (int j = 0; j < QH; ++j) {
+                    const float4 x = reinterpret_cast<const float4 *>(qs + j * D)[i];
+                    s[0][j] = fmaf(x.w, k0.w, fmaf(x.z, k0.z, fmaf(x.y, k0.y, fmaf(x.x, k0.x, s[0][j]))));
+                    s[1][j] = fmaf(x.w, k1.w, fmaf(x.z, k1.z, fmaf(x.y, k1.y, fmaf(x.x, k1.x, s[1][j]))));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < QH; ++j) {
+                // (rows past the limit hold stale values)
+                const float s0 = lane < lim[j] - c0 ? s[0][j] * scale : -INFINITY, s1 = lane + 32 < lim[j] - c0 ? s[1][j] * scale : -INFINITY;
+                float cm = fmaxf(s0, s1);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+                const float m_new = fmaxf(m[j], cm);
+                const float alpha = m_new == -INFINITY ? 1.0f : expf(m[j] - m_new);   // 0 for a pair's first chunk
+                const float e0 = s0 == -INFINITY ? 0.0f : expf(s0 - m_new), e1 = s1 == -INFINITY ? 0.0f : expf(s1 - m_new);
+                sc[j * AT_KT + lane] = e0;
+                sc[j * AT_KT + lane + 32] = e1;
+                float ps = e0 + e1;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
+                l[j] = l[j] * alpha + ps;
+                acc[j].x *= alpha; acc[j].y *= alpha; acc[j].z *= alpha; acc[j].w *= alpha;
+                m[j] = m_new;
+            }
+            __syncwarp();
+            // weighted values: a lane owns four columns (D = 64: the half warps take alternate keys)
+            for (int k = kpar; k < nkw; k += KPAR) {
+                const float4 v4 = *reinterpret_cast<const float4 *>(vs + k * D + e4);
+#pragma unroll
+                for (int j = 0; j < QH; ++j) {
+                    if (k < lim[j] - c0) {
+                        const float p = sc[j * AT_KT + k];
+                        acc[j].x = fmaf(p, v4.x, acc[j].x);
+                        acc[j].y = fmaf(p, v4.y, acc[j].y);
+                        acc[j].z = fmaf(p, v4.z, acc[j].z);
+                        acc[j].w = fmaf(p, v4.w, acc[j].w);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < QH; ++j) {
+            if constexpr (KPAR == 2) {
+                acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, 16);
+                acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, 16);
+                acc[j].z += __shfl_xor_sync(0xffffffffu, acc[j].z, 16);
+                acc[j].w += __shfl_xor_sync(0xffffffffu, acc[j].w, 16);
+            }
+            if (live[j] && kpar == 0) {
+                const float inv = l[j] == 0.0f ? 0.0f : 1.0f / l[j];
+                float *row = a.out + ((size_t)b * a.seq_q + sq[j]) * (size_t)a.n_q * D + (size_t)qh[j] * D;
+                *reinterpret_cast<float4 *>(row + e4) = make_float4(acc[j].x * inv, acc[j].y * inv, acc[j].z * inv, acc[j].w * inv);
+            }
+        }
+        __syncthreads();   // the next pairs' queries
+    }
+}
+
+template <typename KV, int D>
+__global__ void __launch_bounds__(AT_THREADS, 1) gqa_prefill_tc_kernel(const __grid_constant__ ATCall<KV> a, int *__restrict__ status) {
     using G = ATGeom<D>;
+    const int q_stride = a.q_stride, seq_q = a.seq_q, n_q = a.n_q, n_kv = a.n_kv, max_seq = a.max_seq, QB = a.QB;
     constexpr int STAGES = G::STAGES;
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -252,8 +412,8 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
     const uint32_t ofull = bars + 192, ofree = bars + 208, afull = bars + 224;                        // [2], [2], [4]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + G::BARS + 256);
     const int group = n_q / n_kv;
-    const int kv_h = blockIdx.x % n_kv, b = blockIdx.x / n_kv;
-    const int qt = gridDim.y - 1 - blockIdx.y;      // the longest key ranges first
+    const int pair = blockIdx.x % a.pairs, kv_h = (a.pair0 + pair) % n_kv, b = (a.pair0 + pair) / n_kv;
+    const int qt = (gridDim.x - 1 - blockIdx.x) / a.pairs;      // the longest key ranges first
 
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) {
@@ -279,15 +439,16 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
     }
     pdl_wait();
     pdl_trigger();
-    const int p0 = *pos;
+    const int p0 = *a.pos;
     auto limit_of = [&](int s) {
-        const int l = p0 + (causal ? s + 1 : seq_q);
+        const int l = p0 + (a.causal ? s + 1 : seq_q);
         return l > max_seq ? max_seq : (l < 0 ? 0 : l);
     };
     const int block_limit = limit_of(min(seq_q, (qt + 1) * QB) - 1);   // limits do not decrease with the position
     const int n = (block_limit + AT_KT - 1) / AT_KT;                   // key tiles of this CTA
-    const unsigned char *img = images + (size_t)blockIdx.x * n_tiles * ATImage<D>::BYTES;
-    const float *inv = inv_scales + (size_t)blockIdx.x * n_tiles * 2;
+    const unsigned char *img = a.images + (size_t)pair * a.n_tiles * ATImage<D>::BYTES;
+    const float *inv = a.inv_scales + (size_t)pair * a.n_tiles * 2;
+    bool wide = false;                                                 // this CTA takes the fp32 path
 
     // ---- query tile: pair r -> head r % group of the group, position r / group of the tile ----
     {
@@ -303,10 +464,10 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[it][j] = 0.0f;
             if (live) {
-                const float *src = q + ((size_t)b * seq_q + s) * q_stride + (size_t)(kv_h * group + r % group) * D + c8 * 8;
-                if (q_vec) {
-                    const float4 a = __ldg(reinterpret_cast<const float4 *>(src)), d = __ldg(reinterpret_cast<const float4 *>(src) + 1);
-                    v[it][0] = a.x; v[it][1] = a.y; v[it][2] = a.z; v[it][3] = a.w;
+                const float *src = a.q + ((size_t)b * seq_q + s) * q_stride + (size_t)(kv_h * group + r % group) * D + c8 * 8;
+                if (a.q_vec) {
+                    const float4 c = __ldg(reinterpret_cast<const float4 *>(src)), d = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+                    v[it][0] = c.x; v[it][1] = c.y; v[it][2] = c.z; v[it][3] = c.w;
                     v[it][4] = d.x; v[it][5] = d.y; v[it][6] = d.z; v[it][7] = d.w;
                 } else {
 #pragma unroll
@@ -314,17 +475,23 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
                 }
             }
         }
+        // (here the position, on which n hangs, is there as well: in front of the query loads this took 1 %)
+        for (int i = tid; i < n; i += AT_THREADS) wide |= inv[2 * i] == 0.0f;
 #pragma unroll
         for (int it = 0; it < STEPS; ++it) {
             const int r = (it * 12 + warp) * RPW + lane / LPR;
-            float m = 0.0f;
+            float m = 0.0f, nan = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(v[it][j]));
+            for (int j = 0; j < 8; ++j) {
+                m = fmaxf(m, fabsf(v[it][j]));
+                nan = fmaf(v[it][j], 0.0f, nan);
+            }
 #pragma unroll
             for (int o = LPR / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (r < AT_ROWS) {
                 float up, down;
                 at_scale(m, up, down);
+                wide |= (nan != 0.0f) | !at_in_range(m);
                 if (c8 == 0) qinv_sm[r] = down;
                 uint4 hi, lo;
                 at_split(v[it][0] * up, v[it][1] * up, hi.x, lo.x);
@@ -339,13 +506,15 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     at_fence_before();
-    __syncthreads();
+    wide = __syncthreads_or(wide);
     at_fence_after();
     const uint32_t tmem = *tmem_slot;
     // TMEM columns: scores [2] x 64, weights [2] x {hi 32, lo 32}, value sums [2] x 128
     const uint32_t t_s = tmem, t_p = tmem + 128, t_o = tmem + 256;
 
-    if (warp == 0) {
+    if (wide) {
+        at_fp32_tile<KV, D>(a, reinterpret_cast<float *>(smem), b, kv_h, qt, p0);
+    } else if (warp == 0) {
         if (lane == 0) {
             uint32_t phase = 0;
             bool alive = true;
@@ -528,7 +697,7 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
         if (live && alive) {
             const float l = n > 0 ? l_sm[row] : 0.0f;
             const float f = l > 0.0f ? 1.0f / l : 0.0f;
-            float4 *dst = reinterpret_cast<float4 *>(out + ((size_t)b * seq_q + s_pos) * (size_t)n_q * D + (size_t)(kv_h * group + row % group) * D);
+            float4 *dst = reinterpret_cast<float4 *>(a.out + ((size_t)b * seq_q + s_pos) * (size_t)n_q * D + (size_t)(kv_h * group + row % group) * D);
 #pragma unroll
             for (int j = 0; j < D / 4; ++j) dst[j] = make_float4(o[4 * j] * f, o[4 * j + 1] * f, o[4 * j + 2] * f, o[4 * j + 3] * f);
         }
@@ -541,35 +710,31 @@ gqa_prefill_tc_kernel(const float *__restrict__ q, int q_stride, int q_vec, int 
     }
 }
 
-template <typename KV, int D>
-static int prefill_tc_launch(yscv_cuda_ctx *ctx, const float *q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q,
-                             size_t n_kv, const KV *kc, const KV *vc, const float *kscale, const float *vscale,
-                             size_t max_seq, const int32_t *pos, int causal, float *out) {
+template <typename KV, int D> static int prefill_tc_launch(yscv_cuda_ctx *ctx, size_t batch, ATCall<KV> a) {
     using G = ATGeom<D>;
-    const size_t n_tiles = (max_seq + AT_KT - 1) / AT_KT;
-    const size_t per_seq = n_kv * n_tiles * (ATImage<D>::BYTES + 2 * sizeof(float));
+    a.n_tiles = (a.max_seq + AT_KT - 1) / AT_KT;
+    a.QB = AT_ROWS / (a.n_q / a.n_kv);
+    const size_t per_pair = (size_t)a.n_tiles * (ATImage<D>::BYTES + 2 * sizeof(float)), pairs = batch * a.n_kv;
     // the images of as many sequences as fit 256 MB at a time (at least one), so that the scratch stays bounded
-    size_t bg = (256u << 20) / per_seq;
-    bg = bg < 1 ? 1 : (bg > batch ? batch : bg);
-    int rc = ctx->scratch_attn.reserve(bg * per_seq, ctx->stream);
+    size_t group = (256u << 20) / (per_pair * a.n_kv);
+    group = (group < 1 ? 1 : (group > batch ? batch : group)) * a.n_kv;
+    int rc = ctx->scratch_attn.reserve(group * per_pair, ctx->stream);
     if (rc) return rc;
-    unsigned char *images = reinterpret_cast<unsigned char *>(ctx->scratch_attn.ptr);
-    float *inv = reinterpret_cast<float *>(images + bg * n_kv * n_tiles * ATImage<D>::BYTES);
-    auto kern = gqa_prefill_tc_kernel<D>;
+    a.images = reinterpret_cast<unsigned char *>(ctx->scratch_attn.ptr);
+    a.inv_scales = reinterpret_cast<float *>(a.images + group * a.n_tiles * ATImage<D>::BYTES);
+    auto kern = gqa_prefill_tc_kernel<KV, D>;
     rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 227 * 1024);
     if (rc) return rc;
-    const int QB = (int)(AT_ROWS / (n_q / n_kv));
-    const int q_vec = ((reinterpret_cast<uintptr_t>(q) & 15) == 0 && q_stride % 4 == 0) ? 1 : 0;
-    for (size_t b0 = 0; b0 < batch; b0 += bg) {
-        const size_t nb = batch - b0 < bg ? batch - b0 : bg;
-        const size_t row0 = b0 * max_seq, cache0 = row0 * n_kv * D;
-        YSCV_CUDA_TRY(launch_pdl(kv_split_kernel<KV, D>, dim3((unsigned)n_tiles, (unsigned)n_kv, (unsigned)nb), dim3(256), 0, ctx->stream,
-                                 kc + cache0, vc + cache0, kscale ? kscale + row0 : nullptr, vscale ? vscale + row0 : nullptr,
-                                 (int)n_kv, (int)max_seq, (int)seq_q, pos, images, inv));
+    const size_t q_tiles = ((size_t)a.seq_q + a.QB - 1) / a.QB;
+    for (size_t p0 = 0; p0 < pairs; p0 += group) {
+        a.pair0 = (int)p0;
+        a.pairs = (int)(pairs - p0 < group ? pairs - p0 : group);
+        // blocks for two or three rounds of the SMs: a cache is mostly longer than the keys in use
+        const int rounds = 16 * ctx->sm_count / a.pairs + 1;
+        YSCV_CUDA_TRY(launch_pdl(kv_split_kernel<KV, D>, dim3((unsigned)a.pairs, (unsigned)(a.n_tiles < rounds ? a.n_tiles : rounds)),
+                                 dim3(256), 0, ctx->stream, a));
         ctx->launches++;
-        YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)(n_kv * nb), (unsigned)((seq_q + QB - 1) / QB)), dim3(AT_THREADS), (size_t)G::SMEM,
-                                 ctx->stream, q + b0 * seq_q * q_stride, (int)q_stride, q_vec, (int)seq_q, (int)n_q, (int)n_kv, (int)max_seq,
-                                 pos, causal, images, inv, (int)n_tiles, out + b0 * seq_q * n_q * D, QB, ctx->d_status));
+        YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)(a.pairs * q_tiles)), dim3(AT_THREADS), (size_t)G::SMEM, ctx->stream, a, ctx->d_status));
         ctx->launches++;
     }
     YSCV_CUDA_TRY(cudaGetLastError());
@@ -580,8 +745,22 @@ template <typename KV>
 int gqa_prefill_tc(yscv_cuda_ctx *ctx, const float *q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q, size_t n_kv,
                    size_t d_head, const KV *kc, const KV *vc, const float *kscale, const float *vscale, size_t max_seq,
                    const int32_t *pos, int causal, float *out) {
-    auto f = d_head == 64 ? prefill_tc_launch<KV, 64> : prefill_tc_launch<KV, 128>;
-    return f(ctx, q, q_stride, batch, seq_q, n_q, n_kv, kc, vc, kscale, vscale, max_seq, pos, causal, out);
+    ATCall<KV> a = {};
+    a.q = q;
+    a.q_stride = (int)q_stride;
+    a.q_vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0 && q_stride % 4 == 0;
+    a.seq_q = (int)seq_q;
+    a.n_q = (int)n_q;
+    a.n_kv = (int)n_kv;
+    a.max_seq = (int)max_seq;
+    a.causal = causal;
+    a.kc = kc;
+    a.vc = vc;
+    a.kscale = kscale;
+    a.vscale = vscale;
+    a.pos = pos;
+    a.out = out;
+    return d_head == 64 ? prefill_tc_launch<KV, 64>(ctx, batch, a) : prefill_tc_launch<KV, 128>(ctx, batch, a);
 }
 template int gqa_prefill_tc<float>(yscv_cuda_ctx *, const float *, size_t, size_t, size_t, size_t, size_t, size_t, const float *,
                                    const float *, const float *, const float *, size_t, const int32_t *, int, float *);
