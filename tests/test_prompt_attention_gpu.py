@@ -161,3 +161,57 @@ def test_a_query_row_stays_in_its_row(d):
     want = _exact(torch.nan_to_num(q, nan=0.0, posinf=0.0), k, v, 0)
     _check(got[~bad], want[~bad])
     ctx.close()
+
+
+@pytest.mark.parametrize("B,n_kv,max_seq,launches", [(3, 2, 80000, 4), (2, 3, 100000, 4), (3, 1, 100000, 4)])
+def test_images_of_a_long_cache_in_groups(B, n_kv, max_seq, launches):
+    """Caches whose images pass 256 MB: (sequence, KV head) pairs are taken in groups, here six in threes (the
+    middle sequence in both), six in whole sequences of three, and two and one."""
+    ctx, _ = _context()
+    g = _generator(9)
+    seq, p0, n_q, d = 20, 1000, 4 * n_kv, 128
+    q = torch.randn(B, seq, n_q, d, device="cuda", generator=g)
+    k, v = (torch.zeros(B, max_seq, n_kv, d, device="cuda") for _ in range(2))
+    for t in (k, v):
+        t[:, :p0 + seq] = torch.randn(B, p0 + seq, n_kv, d, device="cuda", generator=g)
+    before = ctx.launch_count()
+    got = _call(ctx, q, k, v, p0)
+    assert ctx.launch_count() - before == launches
+    _check(got, _exact(q, k, v, p0))
+    ctx.close()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("kv_int8", [False, True])
+def test_first_call_inside_a_capture(d, kv_int8):
+    """A context that has no scratch for the images yet and may not allocate: the call takes the fp32 path."""
+    ctx, stream = _context()
+    g = _generator(d)
+    B, seq, p0, n_q, n_kv, max_seq = 2, 100, 70, 24, 4, 200
+    q = torch.randn(B, seq, n_q, d, device="cuda", generator=g)
+    pos = torch.full((1,), p0, dtype=torch.int32, device="cuda")
+    out = torch.zeros(B, seq, n_q, d, device="cuda")
+    if kv_int8:
+        k8, v8 = (torch.randint(-127, 128, (B, max_seq, n_kv, d), dtype=torch.int8, device="cuda", generator=g) for _ in range(2))
+        ks, vs = (torch.rand(B, max_seq, device="cuda", generator=g) * 0.01 + 0.01 for _ in range(2))
+        k, v = k8.float() * ks[:, :, None, None], v8.float() * vs[:, :, None, None]
+    else:
+        k, v = (torch.randn(B, max_seq, n_kv, d, device="cuda", generator=g) for _ in range(2))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        if kv_int8:
+            ctx.gqa_attention_i8_dev(q.data_ptr(), n_q * d, B, seq, n_q, n_kv, d, k8.data_ptr(), ks.data_ptr(), v8.data_ptr(),
+                                     vs.data_ptr(), max_seq, pos.data_ptr(), True, out.data_ptr())
+        else:
+            ctx.gqa_attention_dev(q.data_ptr(), n_q * d, B, seq, n_q, n_kv, d, k.data_ptr(), v.data_ptr(), max_seq,
+                                  pos.data_ptr(), True, out.data_ptr())
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        _check(out, _exact(q, k, v, p0))
+    assert ctx.device_status() == 0
+    del graph
+    ctx.close()

@@ -138,7 +138,7 @@ template <typename KV> struct ATCall {
     int QB;                       // query positions per CTA
     int n_tiles;                  // key tiles of max_seq
     int pair0, pairs;             // pairs of this launch
-    unsigned char *images;        // [pairs][n_tiles]
+    unsigned char *images;        // [pairs][n_tiles]; null: no scratch, every CTA takes the fp32 path
     float *inv_scales;            // [pairs][n_tiles][2]
 };
 
@@ -270,7 +270,8 @@ template <int D> struct ATGeom {
     static constexpr int SMEM = BARS + 272;
 };
 
-// The query tile in fp32 throughout, for what two fp16 terms cannot hold (see kv_split_kernel): FMAs over 64-key chunks staged in shared memory, four (position, head) pairs per warp. A key
+// The query tile in fp32 throughout, for what two fp16 terms cannot hold (see kv_split_kernel) and for calls
+// without scratch: FMAs over 64-key chunks staged in shared memory, four (position, head) pairs per warp. A key
 // that a pair does not attend to is not multiplied at all. 2048 tokens, 64 / 8 heads of 128: 3.5 ms a layer
 // against 0.28 on the tensor cores.
 template <typename KV, int D>
@@ -448,7 +449,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) gqa_prefill_tc_kernel(const __g
     const int n = (block_limit + AT_KT - 1) / AT_KT;                   // key tiles of this CTA
     const unsigned char *img = a.images + (size_t)pair * a.n_tiles * ATImage<D>::BYTES;
     const float *inv = a.inv_scales + (size_t)pair * a.n_tiles * 2;
-    bool wide = false;                                                 // this CTA takes the fp32 path
+    bool wide = a.images == nullptr;                                   // this CTA takes the fp32 path
 
     // ---- query tile: pair r -> head r % group of the group, position r / group of the tile ----
     {
@@ -476,7 +477,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) gqa_prefill_tc_kernel(const __g
             }
         }
         // (here the position, on which n hangs, is there as well: in front of the query loads this took 1 %)
-        for (int i = tid; i < n; i += AT_THREADS) wide |= inv[2 * i] == 0.0f;
+        if (!wide)
+            for (int i = tid; i < n; i += AT_THREADS) wide |= inv[2 * i] == 0.0f;
 #pragma unroll
         for (int it = 0; it < STEPS; ++it) {
             const int r = (it * 12 + warp) * RPW + lane / LPR;
@@ -714,26 +716,35 @@ template <typename KV, int D> static int prefill_tc_launch(yscv_cuda_ctx *ctx, s
     using G = ATGeom<D>;
     a.n_tiles = (a.max_seq + AT_KT - 1) / AT_KT;
     a.QB = AT_ROWS / (a.n_q / a.n_kv);
+    // The images of as many (sequence, KV head) pairs at a time as fit 256 MB, but of a whole sequence up to
+    // 1.25 GB where that much is free: one head after another takes 16 positions on an empty cache of 131072 x 8 x
+    // 128 from 28 to 117 us.
     const size_t per_pair = (size_t)a.n_tiles * (ATImage<D>::BYTES + 2 * sizeof(float)), pairs = batch * a.n_kv;
-    // the images of as many sequences as fit 256 MB at a time (at least one), so that the scratch stays bounded
-    size_t group = (256u << 20) / (per_pair * a.n_kv);
-    group = (group < 1 ? 1 : (group > batch ? batch : group)) * a.n_kv;
-    int rc = ctx->scratch_attn.reserve(group * per_pair, ctx->stream);
-    if (rc) return rc;
-    a.images = reinterpret_cast<unsigned char *>(ctx->scratch_attn.ptr);
-    a.inv_scales = reinterpret_cast<float *>(a.images + group * a.n_tiles * ATImage<D>::BYTES);
+    const size_t fit = (256u << 20) / per_pair > 1 ? (256u << 20) / per_pair : 1, all = (1280u << 20) / per_pair;
+    size_t group = fit < (size_t)a.n_kv && all >= (size_t)a.n_kv ? a.n_kv : fit;
+    if (group > pairs) group = pairs;
+    bool split = ctx->scratch_attn.try_reserve(group * per_pair, ctx->stream);
+    if (!split && fit < group) split = ctx->scratch_attn.try_reserve((group = fit) * per_pair, ctx->stream);
+    if (split) {
+        a.images = reinterpret_cast<unsigned char *>(ctx->scratch_attn.ptr);
+        a.inv_scales = reinterpret_cast<float *>(a.images + group * a.n_tiles * ATImage<D>::BYTES);
+    } else {
+        group = pairs;
+    }
     auto kern = gqa_prefill_tc_kernel<KV, D>;
-    rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 227 * 1024);
+    const int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 227 * 1024);
     if (rc) return rc;
     const size_t q_tiles = ((size_t)a.seq_q + a.QB - 1) / a.QB;
     for (size_t p0 = 0; p0 < pairs; p0 += group) {
         a.pair0 = (int)p0;
         a.pairs = (int)(pairs - p0 < group ? pairs - p0 : group);
-        // blocks for two or three rounds of the SMs: a cache is mostly longer than the keys in use
-        const int rounds = 16 * ctx->sm_count / a.pairs + 1;
-        YSCV_CUDA_TRY(launch_pdl(kv_split_kernel<KV, D>, dim3((unsigned)a.pairs, (unsigned)(a.n_tiles < rounds ? a.n_tiles : rounds)),
-                                 dim3(256), 0, ctx->stream, a));
-        ctx->launches++;
+        if (split) {
+            // blocks for two or three rounds of the SMs: a cache is mostly longer than the keys in use
+            const int rounds = 16 * ctx->sm_count / a.pairs + 1;
+            YSCV_CUDA_TRY(launch_pdl(kv_split_kernel<KV, D>, dim3((unsigned)a.pairs, (unsigned)(a.n_tiles < rounds ? a.n_tiles : rounds)),
+                                     dim3(256), 0, ctx->stream, a));
+            ctx->launches++;
+        }
         YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)(a.pairs * q_tiles)), dim3(AT_THREADS), (size_t)G::SMEM, ctx->stream, a, ctx->d_status));
         ctx->launches++;
     }
