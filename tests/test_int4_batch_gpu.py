@@ -148,3 +148,38 @@ def test_split_last_round_reads_only_what_it_wrote(m, n, k):
     for n0 in range(0, n, 512):
         assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 5e-3, n0
     ctx.close()
+
+
+def test_workspace_is_taken_by_the_first_call():
+    """A context that runs no such call does not hold its 39 MB; inside a capture, where nothing may be allocated,
+    a first call takes the kernel for smaller matrices."""
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    assert free - torch.cuda.mem_get_info()[0] <= 8 << 20
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    n, k, m = 16400, 4096, 8
+    with torch.cuda.stream(stream):
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g)
+        out = torch.empty(m, n, device="cuda")
+        small = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), 64, k, 32)
+        large = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(small, x.data_ptr(), out.data_ptr(), m)     # sizes the scratch of this k
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            ctx.int4_matmul_dev(large, x.data_ptr(), out.data_ptr(), m)
+        assert "tmem" not in ctx.last_kernel()
+        want = x.double() @ w.T
+        for again in range(2):
+            out.zero_()
+            graph.replay() if not again else ctx.int4_matmul_dev(large, x.data_ptr(), out.data_ptr(), m)
+            stream.synchronize()
+            assert float((out.double() - want).norm() / want.norm()) <= 2e-6
+    assert "tmem" in ctx.last_kernel()
+    assert ctx.device_status() == 0
+    del graph
+    ctx.close()

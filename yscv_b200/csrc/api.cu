@@ -138,7 +138,7 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
         float *o = d_out + m0 * n;
         const bool aligned = ((reinterpret_cast<uintptr_t>(d_packed) | reinterpret_cast<uintptr_t>(d_scales) |
                                reinterpret_cast<uintptr_t>(a)) & 15) == 0;
-        const bool batch = aligned && int4_batch_exact_wins(mc, n, k, gs);
+        const bool batch = aligned && int4_batch_exact_wins(mc, n, k, gs) && int4_batch_ready(ctx);
         if (aligned && (batch || int4_gemv_fast_supported(mc, n, k, gs))) {
             // (one size for every m up to 16, so that a call never outgrows what another one left)
             const size_t a_b = int4_gemv_scratch_bytes(16, k), b_b = int4_batch_exact_scratch_bytes(k);
@@ -217,11 +217,6 @@ static int ctx_create_impl(int device, cudaStream_t stream, bool borrow, yscv_cu
         if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
         return fail(YSCV_CUDA_ERR_CUDA, "status word: %s", cudaGetErrorString(me));
-    }
-    const int rc = ctx->batch_ws.reserve(int4_batch_ws_bytes(ctx->sm_count), ctx->stream);
-    if (rc) {
-        yscv_cuda_ctx_destroy(ctx);
-        return rc;
     }
     *out = ctx;
     return YSCV_CUDA_OK;

@@ -138,8 +138,8 @@ struct yscv_cuda_ctx {
     yscv::DeviceBuffer gemm_ws, gemm_flags;
     int gemm_epoch = 0;
     bool int8_tail_split = true;
-    // batched decode GEMM (int4_batch_gemm.cu): partial sums of the tiles that several CTAs share.
-    // Sized for every shape and allocated with the context: no call allocates.
+    // batched decode GEMM (int4_batch_gemm.cu): partial sums of the tiles that several CTAs share,
+    // sized for every shape by the first call that takes it
     yscv::DeviceBuffer batch_ws;
     // encoded TMA descriptors of the last few decode GEMV weight matrices (int4_gemv.cu)
     struct TmCacheEntry {

@@ -521,7 +521,11 @@ act_split16_kernel(const float *__restrict__ act, int M, int K, int kb, __half *
     if (lane == 0) inv[u * 16 + m] = __uint_as_float((254u - s) << 23);
 }
 
-size_t int4_batch_ws_bytes(int sm_count) { return (size_t)sm_count * 2 * 2 * 128 * 128 * sizeof(float); }
+// 39 MB, whatever the shape. Where it cannot be had (a first call inside a capture, no memory) the call takes the
+// kernel that it took before there was this one.
+bool int4_batch_ready(yscv_cuda_ctx *ctx) {
+    return ctx->batch_ws.try_reserve((size_t)ctx->sm_count * 2 * 2 * 128 * 128 * sizeof(float), ctx->stream);
+}
 size_t int4_batch_exact_scratch_bytes(size_t k) { return 32 * k * 2 + (k + BG_UNIT - 1) / BG_UNIT * 64 + 512; }
 
 // k % 128: the scale rows (k / 32 floats) are TMA rows, whose pitch must be a multiple of 16 bytes.

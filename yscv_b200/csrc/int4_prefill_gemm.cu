@@ -895,7 +895,7 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     p.kb_per = (p.k_blocks + p.ksplit - 1) / p.ksplit;
     p.ksplit = (p.k_blocks + p.kb_per - 1) / p.kb_per;   // no empty slice (33 blocks in 8 slices of 5: seven slices)
     float *kernel_out = out;
-    const bool batch = int4_batch_bf16_wins(m, n, k, 32);   // up to 128 rows of a large matrix
+    const bool batch = int4_batch_bf16_wins(m, n, k, 32) && int4_batch_ready(ctx);   // up to 128 rows of a large matrix
     if (p.ksplit > 1 && !batch) {
         rc_ws = ctx->gemm_ws.reserve((size_t)p.ksplit * m * n * sizeof(float), ctx->stream);
         if (rc_ws) return rc_ws;

@@ -31,10 +31,10 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
 // int4_batch_gemm.cu: 1..128 activation rows, k % 128 == 0, 16-byte aligned operands. act_bf16 == nullptr:
 // at most 16 rows, fp32-exact, `act` fp32 and scratch of int4_batch_exact_scratch_bytes(k); otherwise bf16
 // activations in the prefill GEMM's k order. The two predicates say where each form is the faster kernel.
-size_t int4_batch_ws_bytes(int sm_count);
 size_t int4_batch_exact_scratch_bytes(size_t k);
 bool int4_batch_bf16_wins(size_t m, size_t n, size_t k, size_t gs);
 bool int4_batch_exact_wins(size_t m, size_t n, size_t k, size_t gs);
+bool int4_batch_ready(yscv_cuda_ctx *ctx);   // its workspace is there, or could be allocated now
 int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act, const void *act_bf16, float *out,
                     size_t m, size_t n, size_t k, void *scratch);
 
