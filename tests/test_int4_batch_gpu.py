@@ -183,3 +183,33 @@ def test_workspace_is_taken_by_the_first_call():
     assert ctx.device_status() == 0
     del graph
     ctx.close()
+
+
+@pytest.mark.parametrize("n,k", [(16400, 4096), (16400, 4224)])
+def test_infinite_and_tiny_activations(n, k):
+    """Up to 16 rows, what a sum of fp32 products gives: an infinity times a weight of 0 is NaN, else the weight's
+    sign says which infinity, whatever else the row holds; rows of 1e-30 and of subnormals keep their values
+    (the bound for subnormals, which have 2^-149 as their last place: 1e-3)."""
+    ctx = yscv_b200.Context(0)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    packed, scales, w = _weights(g, n, k)
+    x = torch.randn(5, k, device="cuda", generator=g)
+    x[0, 700] = float("inf")
+    x[0, 701] = -3e38
+    x[1, k - 1] = -float("inf")
+    x[2] *= 1e-30
+    x[3] *= 1e-40
+    out = torch.empty(5, n, device="cuda")
+    torch.cuda.synchronize()
+    h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+    ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), 5)
+    ctx.synchronize()
+    assert "tmem" in ctx.last_kernel()
+    for row, col, sign in ((0, 700, 1.0), (1, k - 1, -1.0)):
+        want = torch.where(w[:, col] == 0, torch.nan, torch.sign(w[:, col]) * sign * torch.inf).float()
+        assert torch.equal(torch.nan_to_num(out[row], 7.0, 1.0, -1.0), torch.nan_to_num(want, 7.0, 1.0, -1.0))
+    for row, bound in ((2, 1e-6), (3, 1e-3), (4, 1e-6)):
+        want = x[row].double() @ w.T
+        assert float((out[row].double() - want).norm() / want.norm()) <= bound, row
+    ctx.close()

@@ -497,12 +497,18 @@ act_split16_kernel(const float *__restrict__ act, int M, int K, int kb, __half *
     for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    // power of two that brings the block's maximum into [2^13, 2^14) (1 for zero, subnormal and
-    // non-finite maxima: those keep their infinities and NaNs), and its inverse
+    // power of two that brings the block's maximum into [2^13, 2^14) (2^126 at most), and its inverse. A block with
+    // an infinity keeps its scale of 1 and its infinities, whose remainder is 0 (not inf - inf); what else it holds
+    // only has to stay finite, since the row's sums no longer are.
     const uint32_t e = (__float_as_uint(mx) >> 23) & 255u;
-    uint32_t s = 267u - e;
-    s = (e == 0u || e == 255u) ? 127u : (s > 253u ? 253u : s);
+    const bool inf = e == 255u;
+    const uint32_t s = inf ? 127u : min(267u - e, 253u);
     const float up = __uint_as_float(s << 23);
+    if (inf) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (fabsf(v[i]) < INFINITY) v[i] = fminf(fmaxf(v[i], -65504.0f), 65504.0f);
+    }
     uint4 hi, lo;
     uint32_t *h = &hi.x, *l = &lo.x;
 #pragma unroll
@@ -510,7 +516,7 @@ act_split16_kernel(const float *__restrict__ act, int M, int K, int kb, __half *
         const float x = v[2 * i] * up, y = v[2 * i + 1] * up;
         const __half2 hh = __floats2half2_rn(x, y);
         const float2 f = __half22float2(hh);
-        const __half2 ll = __floats2half2_rn(x - f.x, y - f.y);
+        const __half2 ll = __floats2half2_rn(inf && f.x == x ? 0.0f : x - f.x, inf && f.y == y ? 0.0f : y - f.y);
         h[i] = *reinterpret_cast<const uint32_t *>(&hh);
         l[i] = *reinterpret_cast<const uint32_t *>(&ll);
     }
