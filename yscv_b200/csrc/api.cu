@@ -77,11 +77,16 @@ cudaError_t DeviceBuffer::grow(size_t want) {
     return e;
 }
 
+int DeviceBuffer::reserve(size_t want) {
+    if (want > bytes || !ptr) YSCV_CUDA_TRY(grow(want));
+    return YSCV_CUDA_OK;
+}
+
 int DeviceBuffer::reserve(size_t want, cudaStream_t stream) {
     const bool capturing = note_capture(stream);
-    if (want > bytes || !ptr) YSCV_CUDA_TRY(grow(want));
-    in_graph = in_graph || capturing;
-    return YSCV_CUDA_OK;
+    const int rc = reserve(want);
+    in_graph = in_graph || (capturing && rc == YSCV_CUDA_OK);
+    return rc;
 }
 
 bool DeviceBuffer::try_reserve(size_t want, cudaStream_t stream) {
@@ -142,7 +147,8 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
         if (aligned && (batch || int4_gemv_fast_supported(mc, n, k, gs))) {
             // (one size for every m up to 16, so that a call never outgrows what another one left)
             const size_t a_b = int4_gemv_scratch_bytes(16, k), b_b = int4_batch_exact_scratch_bytes(k);
-            rc = ctx->scratch.reserve(a_b > b_b ? a_b : b_b, ctx->stream);
+            const size_t want = a_b > b_b ? a_b : b_b;
+            rc = batch || int4_gemv_uses_scratch(mc, k) ? ctx->scratch.reserve(want, ctx->stream) : ctx->scratch.reserve(want);
             if (rc) return rc;
         }
         if (batch) {
@@ -359,8 +365,8 @@ int yscv_cuda_packed_int4_gemm(yscv_cuda_ctx *ctx, const uint8_t *weight_packed,
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t wb = n * k / 2, sb = n * (k / group_size) * sizeof(float);
     const size_t ab = m * k * sizeof(float), ob = m * n * sizeof(float);
-    if ((rc = ctx->in0.reserve(wb, ctx->stream)) || (rc = ctx->in1.reserve(sb, ctx->stream)) || (rc = ctx->in2.reserve(ab, ctx->stream)) ||
-        (rc = ctx->out0.reserve(ob, ctx->stream)))
+    if ((rc = ctx->in0.reserve(wb)) || (rc = ctx->in1.reserve(sb)) || (rc = ctx->in2.reserve(ab)) ||
+        (rc = ctx->out0.reserve(ob)))
         return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, weight_packed, wb, cudaMemcpyHostToDevice, ctx->stream));
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in1.ptr, scales, sb, cudaMemcpyHostToDevice, ctx->stream));
@@ -414,7 +420,7 @@ int yscv_cuda_pack_int4_symmetric_per_group(yscv_cuda_ctx *ctx, const float *wei
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t wb = m_w * k * sizeof(float), pb = m_w * k / 2;
     const size_t sb = m_w * (k / group_size) * sizeof(float);
-    if ((rc = ctx->in0.reserve(wb, ctx->stream)) || (rc = ctx->out0.reserve(pb, ctx->stream)) || (rc = ctx->out1.reserve(sb, ctx->stream)))
+    if ((rc = ctx->in0.reserve(wb)) || (rc = ctx->out0.reserve(pb)) || (rc = ctx->out1.reserve(sb)))
         return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, weights, wb, cudaMemcpyHostToDevice, ctx->stream));
     rc = pack_int4(ctx, (const float *)ctx->in0.ptr, m_w, k, group_size, (uint8_t *)ctx->out0.ptr,
@@ -538,7 +544,7 @@ int yscv_cuda_int4_matmul(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w,
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t ab = m * w->k * sizeof(float), ob = m * w->m_w * sizeof(float);
     int rc;
-    if ((rc = ctx->in2.reserve(ab, ctx->stream))) return rc;
+    if ((rc = ctx->in2.reserve(ab))) return rc;
     // A page-locked output buffer is written by the kernel itself (posted writes over PCIe, no
     // copy-engine pass behind the kernel); a pageable one goes through the staging buffer. The
     // activations are always copied in: every CTA reads all of them, which must not cross PCIe
@@ -546,7 +552,7 @@ int yscv_cuda_int4_matmul(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w,
     float *d_out = m <= 16 ? static_cast<float *>(mapped_alias(output)) : nullptr;
     const bool direct = d_out != nullptr && (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
     if (!direct) {
-        if ((rc = ctx->out0.reserve(ob, ctx->stream))) return rc;
+        if ((rc = ctx->out0.reserve(ob))) return rc;
         d_out = (float *)ctx->out0.ptr;
     }
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in2.ptr, activation, ab, cudaMemcpyHostToDevice, ctx->stream));
@@ -611,7 +617,7 @@ int yscv_cuda_pack_i8_b_for_matmul(yscv_cuda_ctx *ctx, const int8_t *b, size_t k
     int rc = check_i8_shape(k, n);
     if (rc) return rc;
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
-    if ((rc = ctx->in1.reserve(k * n, ctx->stream))) return rc;
+    if ((rc = ctx->in1.reserve(k * n))) return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in1.ptr, b, k * n, cudaMemcpyHostToDevice, ctx->stream));
     rc = i8b_create(ctx, (const int8_t *)ctx->in1.ptr, k, n, out);
     if (rc) return rc;
@@ -665,7 +671,7 @@ static int i8_gemm_host(yscv_cuda_ctx *ctx, const void *a, const yscv_cuda_i8b *
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t ab = m * b->k, ob = m * b->n * elem_bytes;
     int rc;
-    if ((rc = ctx->in0.reserve(ab, ctx->stream)) || (rc = ctx->out0.reserve(ob, ctx->stream))) return rc;
+    if ((rc = ctx->in0.reserve(ab)) || (rc = ctx->out0.reserve(ob))) return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, a, ab, cudaMemcpyHostToDevice, ctx->stream));
     rc = i8_gemm_dev(ctx, ctx->in0.ptr, b, m, ctx->out0.ptr, a_unsigned, a_zp, rq);
     if (rc) return rc;
@@ -699,8 +705,8 @@ int yscv_cuda_int8_matmul(yscv_cuda_ctx *ctx, const int8_t *a, const int8_t *b, 
     // B^T and its column sums live in buffers the context keeps (grow-only): no allocation
     // per call once the largest shape has been seen
     const size_t kp = (k + 15) / 16 * 16;
-    if ((rc = ctx->in1.reserve(k * n, ctx->stream)) || (rc = ctx->tmp_bt.reserve(n * kp, ctx->stream)) ||
-        (rc = ctx->tmp_colsum.reserve(n * sizeof(int32_t), ctx->stream)))
+    if ((rc = ctx->in1.reserve(k * n)) || (rc = ctx->tmp_bt.reserve(n * kp)) ||
+        (rc = ctx->tmp_colsum.reserve(n * sizeof(int32_t))))
         return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in1.ptr, b, k * n, cudaMemcpyHostToDevice, ctx->stream));
     rc = pack_i8_b(ctx, (const int8_t *)ctx->in1.ptr, k, n, (int8_t *)ctx->tmp_bt.ptr,
@@ -766,8 +772,8 @@ static int i8_requant_i8_host(yscv_cuda_ctx *ctx, const int8_t *a, const yscv_cu
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t ab = m * b->k, ob = m * b->n, vb = b->n * 4;
     int rc;
-    if ((rc = ctx->in0.reserve(ab, ctx->stream)) || (rc = ctx->out0.reserve(ob, ctx->stream)) || (rc = ctx->in1.reserve(vb, ctx->stream)) ||
-        (rc = ctx->in2.reserve(vb, ctx->stream)))
+    if ((rc = ctx->in0.reserve(ab)) || (rc = ctx->out0.reserve(ob)) || (rc = ctx->in1.reserve(vb)) ||
+        (rc = ctx->in2.reserve(vb)))
         return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, a, ab, cudaMemcpyHostToDevice, ctx->stream));
     if (corr) YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in1.ptr, corr, vb, cudaMemcpyHostToDevice, ctx->stream));

@@ -51,8 +51,11 @@ struct DeviceBuffer {
     size_t bytes = 0;
     bool in_graph = false;           // handed out inside a capture since it was allocated
     std::vector<void *> captured;    // outgrown, but a graph may still use them
-    // `stream`: the stream of the call that asks
+    // For a kernel of a call on `stream`, which may be under capture
     int reserve(size_t want, cudaStream_t stream);
+    // For what no capture can hold: staging of the calls that synchronise, space that this call does not use
+    // (asking the stream takes 0.15 us, which calls that launch one kernel and nothing else would feel)
+    int reserve(size_t want);
     // The same for a buffer that a call can do without: false (and no error) where it would have to grow
     // inside a capture or the memory is not there.
     bool try_reserve(size_t want, cudaStream_t stream);

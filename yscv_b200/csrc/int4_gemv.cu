@@ -475,6 +475,14 @@ bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs) {
 
 // Largest resident digit copy the fused-quantisation variant keeps in shared memory.
 constexpr int FUSEQ_MAX_DIGIT_BYTES = 72 * 1024;
+// few activation rows: every CTA quantises them itself, no separate launch
+static bool fused_quant(int mp, int gs, int k) {
+    return mp <= 4 && (k / (32 * gs)) * quant_layout(mp, gs).blob_bytes <= FUSEQ_MAX_DIGIT_BYTES;
+}
+bool int4_gemv_uses_scratch(size_t m, size_t k) {
+    const int mp = padded_m((int)m);
+    return !fused_quant(mp, stage_groups(mp, (int)k), (int)k);
+}
 
 template <int MP, int GS, int TP2, bool FUSEQ>
 static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
@@ -556,8 +564,7 @@ static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *sc
     const int rows_per_cta = (N + ctx->sm_count - 1) / ctx->sm_count;
     const bool small = rows_per_cta <= 32;
     if constexpr (MP <= 4) {
-        // few activation rows: every CTA quantises them itself, no separate launch
-        if ((K / (32 * GS)) * q.blob_bytes <= FUSEQ_MAX_DIGIT_BYTES) {
+        if (fused_quant(MP, GS, K)) {
             ctx->last_kernel = "int4_gemv_fast(imma,tma,fused-quant)";
             return small ? launch_fast<MP, GS, 2, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q)
                          : launch_fast<MP, GS, 8, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q);

@@ -114,7 +114,7 @@ int yscv_cuda_requant_i32_row_to_i8(yscv_cuda_ctx *ctx, const int32_t *acc, cons
     if (!acc || !out) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     int rc;
-    if ((rc = ctx->in0.reserve(len * 4, ctx->stream)) || (rc = ctx->in1.reserve(c * 4, ctx->stream)) || (rc = ctx->out0.reserve(len, ctx->stream))) return rc;
+    if ((rc = ctx->in0.reserve(len * 4)) || (rc = ctx->in1.reserve(c * 4)) || (rc = ctx->out0.reserve(len))) return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, acc, len * 4, cudaMemcpyHostToDevice, ctx->stream));
     if (bias) YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in1.ptr, bias, c * 4, cudaMemcpyHostToDevice, ctx->stream));
     rc = yscv_cuda_requant_i32_row_to_i8_dev(ctx, (const int32_t *)ctx->in0.ptr, bias ? (const int32_t *)ctx->in1.ptr : nullptr,
@@ -144,8 +144,8 @@ int yscv_cuda_int4_weight_from_f32(yscv_cuda_ctx *ctx, const float *weight, size
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
     const size_t wb = m_w * k * sizeof(float);
     int rc;
-    if ((rc = ctx->in0.reserve(wb, ctx->stream))) return rc;
-    if (transposed_source && (rc = ctx->scratch.reserve(wb, ctx->stream))) return rc;
+    if ((rc = ctx->in0.reserve(wb))) return rc;
+    if (transposed_source && (rc = ctx->scratch.reserve(wb))) return rc;
     YSCV_CUDA_TRY(cudaMemcpyAsync(ctx->in0.ptr, weight, wb, cudaMemcpyHostToDevice, ctx->stream));
     const float *src = (const float *)ctx->in0.ptr;
     if (transposed_source) {
