@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("d,n_kv,group", [(16, 2, 3), (48, 1, 8), (64, 2, 12), (64, 3, 1), (80, 2, 5), (128, 2, 8), (128, 1, 17)])
-@pytest.mark.parametrize("max_seq,cached", [(129, 0), (130, 129), (300, 127), (300, 128), (300, 256), (700, 699), (2100, 5)])
+@pytest.mark.parametrize("max_seq,cached", [(129, 0), (130, 129), (300, 127), (300, 128), (300, 256), (700, 699), (2100, 5), (9000, 63),
+                                            (9000, 64), (9000, 200), (9000, 1300), (20000, 19000), (2178, 1999)])
 @pytest.mark.parametrize("kv_int8", [False, True])
 def test_decode_shares(d, n_kv, group, max_seq, cached, kv_int8):
     """Scores of a few units. f32: 32-bit products and sums leave 1e-6 of the output's norm; the bound is 4e-6.

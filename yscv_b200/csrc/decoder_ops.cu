@@ -407,10 +407,10 @@ gqa_attention_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n
 
 // Decode-shaped attention (one query position per sequence) with the keys split across
 // blocks so that a long cache fills the machine: block (split, kv head, b) handles an equal share of
-// the keys in use (at most CH) for ALL the query heads of its KV head's group from one pass over the
+// the keys in use (dec_share) for ALL the query heads of its KV head's group from one pass over the
 // share's key and value rows (a row is read once per group, not once per query head), leaves
 // per query head an unnormalised partial output, its running max and its exp-sum in `part`;
-// attention_combine_kernel merges the splits (the usual max-rescaling of a split softmax).
+// attention_combine_kernel merges the splits that have keys (the usual max-rescaling of a split softmax).
 // Query heads are taken eight at a time. d % 16 == 0, d <= 128, 256 threads, n_splits * CH >= max_seq.
 //
 // Bound by the latency of its phases, not by the cache's bytes (32 sequences x 200 keys of the 1B head
@@ -419,6 +419,17 @@ gqa_attention_kernel(const float *__restrict__ q, int q_stride, int seq_q, int n
 // all; one block-wide maximum and sum per head were 32): 25.6 -> 11.0 us for that shape.
 constexpr int DEC_HB = 8;
 constexpr int DEC_THREADS = 256;
+__device__ __forceinline__ int dec_limit(const int32_t *pos, int max_seq) { return max(0, min(max_seq, *pos + 1)); }
+// Keys per split. A cache is mostly longer than the conversation in it, and a block costs about as much for a
+// few keys as for CH: equal shares over as few splits as hold the keys in use in shares of up to CH, or, while
+// that is fewer than `want` (two blocks per SM), in shares of down to 64. 200 keys in a cache of 8192, 32
+// sequences, 64 / 8 heads of 128, f32 / int8: 59 / 28 us, spread over all splits 318 / 140. A nearly full cache
+// keeps all its splits (32 / 4 heads of 64, 8 sequences, 2049 keys: 16.1 us in 18 shares, 19.6 in 17).
+template <int CH> __device__ __forceinline__ int dec_share(int limit, int n_splits, int want) {
+    int used = max(1, max((limit + CH - 1) / CH, min(min((limit + 63) / 64, want), n_splits)));
+    if (used * 8 >= n_splits * 7) used = n_splits;
+    return (limit + used - 1) / used;
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
@@ -440,7 +451,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 3)
 gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv, int d_,
                         const KV *__restrict__ kc, const KV *__restrict__ vc,
                         const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
-                        const int32_t *__restrict__ pos, float *__restrict__ part) {
+                        const int32_t *__restrict__ pos, int want, float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
     constexpr bool I8 = sizeof(KV) == 1;
@@ -457,17 +468,9 @@ gqa_decode_split_kernel(const float *__restrict__ q, int q_stride, int n_q, int 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int split = blockIdx.x, kv_h = blockIdx.y, b = blockIdx.z, n_splits = gridDim.x;
     const int grp = n_q / n_kv;
-    int limit = *pos + 1;
-    limit = limit > max_seq ? max_seq : (limit < 0 ? 0 : limit);
-    const int share = (limit + n_splits - 1) / n_splits;
+    const int limit = dec_limit(pos, max_seq), share = dec_share<CH>(limit, n_splits, want);
     const int k0 = split * share, nk = min(limit, k0 + share) - k0;
-    if (nk <= 0) {  // nothing for this split: the neutral element of the merge
-        for (int i = tid; i < grp * (d + 2); i += DEC_THREADS) {
-            const int hh = i / (d + 2), j = i - hh * (d + 2);
-            part[(((size_t)b * n_q + kv_h * grp + hh) * n_splits + split) * (d + 2) + j] = j == d ? -INFINITY : 0.0f;
-        }
-        return;
-    }
+    if (nk <= 0) return;   // (the merge does not read this split)
     const float scale = 1.0f / sqrtf((float)d);
     const size_t row_bytes = (size_t)n_kv * d * sizeof(KV);
     const float *vsc = I8 ? vscale + (size_t)b * max_seq + k0 : nullptr;
@@ -672,7 +675,7 @@ __global__ void __launch_bounds__(128)
 gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, int n_kv,
                            const int8_t *__restrict__ kc, const int8_t *__restrict__ vc,
                            const float *__restrict__ kscale, const float *__restrict__ vscale, int max_seq,
-                           const int32_t *__restrict__ pos, float *__restrict__ part) {
+                           const int32_t *__restrict__ pos, int want, float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
     constexpr int CH = 128, HB = 8, d = D;
@@ -692,18 +695,9 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int split = blockIdx.x, kv_h = blockIdx.y, b = blockIdx.z, n_splits = gridDim.x;
     const int grp = n_q / n_kv;
-    int limit = *pos + 1;
-    limit = limit > max_seq ? max_seq : (limit < 0 ? 0 : limit);
-    const int share = (limit + n_splits - 1) / n_splits;             // at most CH: n_splits * CH >= max_seq
-    const int k0 = split * share, k1 = min(limit, k0 + share);
-    const int nk = k1 - k0;
-    if (nk <= 0) {  // nothing for this split: the neutral element of the merge
-        for (int i = tid; i < grp * (d + 2); i += blockDim.x) {
-            const int hh = i / (d + 2), j = i - hh * (d + 2);
-            part[(((size_t)b * n_q + kv_h * grp + hh) * n_splits + split) * (d + 2) + j] = j == d ? -INFINITY : 0.0f;
-        }
-        return;
-    }
+    const int limit = dec_limit(pos, max_seq), share = dec_share<CH>(limit, n_splits, want);
+    const int k0 = split * share, nk = min(limit, k0 + share) - k0;
+    if (nk <= 0) return;   // (the merge does not read this split)
     const float scale = 1.0f / sqrtf((float)d);
     const int8_t *kb = kc + (size_t)b * max_seq * n_kv * d + (size_t)kv_h * d;
     const int8_t *vb = vc + (size_t)b * max_seq * n_kv * d + (size_t)kv_h * d;
@@ -889,32 +883,49 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
 // worked out once per block, a thread per split, then a thread per column adds with its loads in flight
 // (a serial walk that evaluated every weight in every thread: 27 us for 64 x 64 heads x 18 splits).
 constexpr int COMBINE_BATCH = 128;
+constexpr int PRE = 16;   // loads of a column in flight
+template <int CH>
 __global__ void __launch_bounds__(128)
-attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, float *__restrict__ out) {
+attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, int max_seq, const int32_t *__restrict__ pos,
+                         int want, float *__restrict__ out) {
     pdl_wait();
     pdl_trigger();
     __shared__ float red[4], wt[COMBINE_BATCH];
     const int tid = threadIdx.x;
     const size_t hb = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
     const float *p = part + hb * n_splits * (d + 2);
-    float M = -INFINITY;
-    for (int s = tid; s < n_splits; s += 128) M = fmaxf(M, p[(size_t)s * (d + 2) + d]);
+    // what the first splits left is fetched while the position, which says how many count, is on its way
+    float v[PRE];
+    const float m0 = tid < n_splits ? p[(size_t)tid * (d + 2) + d] : -INFINITY, l0 = tid < n_splits ? p[(size_t)tid * (d + 2) + d + 1] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < PRE; ++u) v[u] = tid < d && u < n_splits ? p[(size_t)u * (d + 2) + tid] : 0.0f;
+    const int limit = dec_limit(pos, max_seq), share = dec_share<CH>(limit, n_splits, want);
+    const int used = limit > 0 ? (limit + share - 1) / share : 0;
+    float M = tid < used ? m0 : -INFINITY;
+    for (int s = tid + 128; s < used; s += 128) M = fmaxf(M, p[(size_t)s * (d + 2) + d]);
     M = block_max(M, red);
     float L = 0.0f, acc = 0.0f;
-    for (int s0 = 0; s0 < n_splits; s0 += COMBINE_BATCH) {
-        const int s = s0 + tid, ns = min(COMBINE_BATCH, n_splits - s0);
+    for (int s0 = 0; s0 < used; s0 += COMBINE_BATCH) {
+        const int s = s0 + tid, ns = min(COMBINE_BATCH, used - s0);
         float w = 0.0f;
-        if (s < n_splits) {
-            const float m = p[(size_t)s * (d + 2) + d];
+        if (s < used) {
+            const float m = s0 == 0 ? m0 : p[(size_t)s * (d + 2) + d];
             if (m > -INFINITY) w = expf(m - M);
-            L += w * (w > 0.0f ? p[(size_t)s * (d + 2) + d + 1] : 0.0f);
+            if (w > 0.0f) L += w * (s0 == 0 ? l0 : p[(size_t)s * (d + 2) + d + 1]);
         }
         __syncthreads();
         wt[tid] = w;
         __syncthreads();
         if (tid < d) {
-#pragma unroll 6
-            for (int i = 0; i < ns; ++i) acc = fmaf(wt[i], p[(size_t)(s0 + i) * (d + 2) + tid], acc);
+            for (int i = 0; i < ns; i += PRE) {
+                if (s0 + i > 0) {
+#pragma unroll
+                    for (int u = 0; u < PRE; ++u) v[u] = i + u < ns ? p[(size_t)(s0 + i + u) * (d + 2) + tid] : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < PRE; ++u)
+                    if (i + u < ns) acc = fmaf(wt[i + u], v[u], acc);
+            }
         }
     }
     L = block_sum(L, red);
@@ -1236,6 +1247,7 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
             return fail(YSCV_CUDA_ERR_UNSUPPORTED, "the key and value caches must be 16-byte aligned");
         const int chunk = sizeof(KV) == 4 && d_head > 64 ? 64 : 128;   // (what fits shared memory twice)
         const int n_splits = (int)((max_seq + chunk - 1) / chunk);
+        const int want = (2 * ctx->sm_count + (int)(batch * n_kv) - 1) / (int)(batch * n_kv);
         const size_t need = batch * n_q * (size_t)n_splits * (d_head + 2) * sizeof(float);
         int rc = ctx->scratch_attn.reserve(need, ctx->stream);
         if (rc) return rc;
@@ -1250,11 +1262,11 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                 auto kern = d_head == 128 ? gqa_decode_split_tc_kernel<128> : gqa_decode_split_tc_kernel<64>;
                 YSCV_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(128), tc_smem, ctx->stream, d_q, (int)q_stride, (int)n_q, (int)n_kv,
                                          reinterpret_cast<const int8_t *>(d_kcache), reinterpret_cast<const int8_t *>(d_vcache),
-                                         d_kscale, d_vscale, (int)max_seq, d_pos, part));
+                                         d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
                 YSCV_CUDA_TRY(cudaGetLastError());
                 ctx->launches++;
-                YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel, dim3(dim3((unsigned)n_q, (unsigned)batch)), dim3(128), 0,
-                                         ctx->stream, part, n_splits, (int)d_head, d_out));
+                YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel<128>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part,
+                                         n_splits, (int)d_head, (int)max_seq, d_pos, want, d_out));
                 DEC_EPILOGUE(ctx, "gqa_attention(split-k,int8 cache,mma)");
             }
         }
@@ -1268,11 +1280,11 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
         }
         if ((rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 80 * 1024))) return rc;
         YSCV_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(DEC_THREADS), split_smem, ctx->stream, d_q, (int)q_stride, (int)n_q, (int)n_kv,
-                                 (int)d_head, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, part));
+                                 (int)d_head, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
-        YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel, dim3(dim3((unsigned)n_q, (unsigned)batch)), dim3(128), 0, ctx->stream, part, n_splits,
-                                                                                               (int)d_head, d_out));
+        YSCV_CUDA_TRY(launch_pdl(chunk == 64 ? attention_combine_kernel<64> : attention_combine_kernel<128>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part, n_splits,
+                                 (int)d_head, (int)max_seq, d_pos, want, d_out));
         DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(split-k,int8 cache)" : "gqa_attention(split-k)");
     }
     // a prompt pass: tiles of 128 (position, head) pairs on the tensor cores
