@@ -20,10 +20,11 @@ def _weights(g, n, k):
 # (rows, outputs, depth): more work than the dispatch rule asks of each row count; n and k around the
 # 128-row tiles, the 256-k units and the CTA ranges
 CASES = [(m, n, k) for ms, shapes in [
-    ((3, 4), [(25000, 8192)]),
-    ((5, 11, 16), [(16400, 4096), (2300, 29312), (60001, 1152), (600, 110080)]),
-    ((17, 31, 32), [(10300, 2176), (700, 30080), (20000, 1152), (160000, 128)]),
-    ((33, 48, 64), [(12000, 4096), (1700, 28928), (57344, 1280)]),
+    ((3, 4), [(43000, 8192), (25000, 8064)]),
+    ((5, 8), [(20000, 4096), (2300, 29312), (60001, 1152), (600, 135168)]),
+    ((11, 16), [(16400, 4096), (2300, 29312), (60001, 1152), (600, 110080)]),
+    ((17, 31, 32), [(23000, 2176), (1650, 30080), (42000, 1152), (380000, 128)]),
+    ((33, 48, 64), [(20000, 4096), (2800, 28928), (63000, 1280)]),
     ((65, 100, 128), [(20000, 4096), (2800, 28800), (10241, 8192)]),
 ] for m in ms for n, k in shapes]
 
@@ -62,7 +63,7 @@ def test_non_finite_rows_stay_in_their_row():
     ctx = yscv_b200.Context(0)
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
-    n, k, m = 16400, 4096, 6
+    n, k, m = 20000, 4096, 6
     packed, scales, w = _weights(g, n, k)
     x = torch.randn(m, k, device="cuda", generator=g)
     x[1, 700] = float("nan")
@@ -160,7 +161,7 @@ def test_workspace_is_taken_by_the_first_call():
     assert free - torch.cuda.mem_get_info()[0] <= 8 << 20
     g = torch.Generator(device="cuda")
     g.manual_seed(3)
-    n, k, m = 16400, 4096, 8
+    n, k, m = 20000, 4096, 8
     with torch.cuda.stream(stream):
         packed, scales, w = _weights(g, n, k)
         x = torch.randn(m, k, device="cuda", generator=g)
@@ -185,7 +186,7 @@ def test_workspace_is_taken_by_the_first_call():
     ctx.close()
 
 
-@pytest.mark.parametrize("n,k", [(16400, 4096), (16400, 4224)])
+@pytest.mark.parametrize("n,k", [(20000, 4096), (16400, 4224)])
 def test_infinite_and_tiny_activations(n, k):
     """Up to 16 rows, what a sum of fp32 products gives: an infinity times a weight of 0 is NaN, else the weight's
     sign says which infinity, whatever else the row holds; rows of 1e-30 and of subnormals keep their values

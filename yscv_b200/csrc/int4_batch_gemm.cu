@@ -540,20 +540,24 @@ static bool bg_shape(size_t n, size_t k, size_t gs) {
 }
 
 // Which calls gain. Three launches, a TMEM hand-over and the join cost about 10 us whatever the size,
-// so small matrices stay where they are (us, here against the other kernel):
-//   bf16, against int4_prefill_gemm_kernel: 57344 x 8192: 32 rows 80 / 191, 64 rows 90 / 202, 128 rows
-//   135 / 235; 8192 x 28672: 51 / 91, 55 / 93, 82 / 98; 10240 x 8192: 27 / 38, 34 / 41, 40 / 46;
-//   14336 x 4096: 23 / 30, 28 / 30, 34 / 32; 11264 x 2048: 15.6 / 17.0, 20 / 17.5, 25 / 19
+// so small matrices stay where they are (us per call in a graph that walks copies of the weights, 500 MB together,
+// here against the other kernel):
+//   bf16, against int4_prefill_gemm_kernel, 32 / 64 / 128 rows: 57344 x 8192 81 / 148, 92 / 173, 138 / 194;
+//   8192 x 28672 52 / 76, 56 / 80, 75 / 88; 22016 x 4096 30 / 36, 34 / 40, 44 / 47; 10240 x 8192 27 / 33, 31 / 36,
+//   40 / 41; 14336 x 4096 23 / 26, 27 / 26, 34 / 29; 4096 x 14336 24 / 25, 26 / 26, 33 / 31; 16384 x 2048 18 / 15,
+//   22 / 16, 27 / 18; 6144 x 4096 17 / 14, 20 / 16, 26 / 21; 11264 x 2048 15.8 / 15.2, 20 / 15, 25 / 17
 bool int4_batch_bf16_wins(size_t m, size_t n, size_t k, size_t gs) {
     const size_t weights = n * k;
-    return m > 16 && m <= 128 && bg_shape(n, k, gs) && weights >= (m <= 32 ? 20000000u : m <= 64 ? 48000000u : 80000000u);
+    return m > 16 && m <= 128 && bg_shape(n, k, gs) && weights >= (m <= 32 ? 40000000u : 80000000u);
 }
-//   exact, against the integer-MMA GEMV: 57344 x 8192: 16 rows 78 / 152; 8192 x 28672: 16 rows 47 / 83,
-//   8 rows 47 / 60, 4 rows 47 / 49, 2 rows 47 / 34; 10240 x 8192: 25 / 39, 25 / 27, 25 / 25, 25 / 17;
-//   14336 x 4096: 16 rows 23 / 23
+//   exact, against the integer-MMA GEMV, 4 / 8 / 16 rows: 57344 x 8192 79 / 85, 80 / 95, 78 / 143; 8192 x 28672
+//   49 / 49, 50 / 60, 50 / 83; 28672 x 8192 47 / 46, 47 / 51, 47 / 74; 22016 x 4096 27 / 29, 27 / 28, 27 / 41; 10240 x
+//   8192 25 / 24, 25.1 / 26.5, 25 / 39; 14336 x 4096 22 / 18, 23 / 16, 23 / 22; 2 rows: everywhere behind. Depths that
+//   are no multiple of 256 would take the fp32 FMA kernel, several times slower: earlier lines.
 bool int4_batch_exact_wins(size_t m, size_t n, size_t k, size_t gs) {
     const size_t weights = n * k;
-    return m > 2 && m <= 16 && bg_shape(n, k, gs) && weights >= (m > 4 ? 64000000u : 200000000u);
+    const bool gemv = k % 256 == 0;
+    return m > 2 && m <= 16 && bg_shape(n, k, gs) && weights >= (m > 8 ? 64000000u : m > 4 ? (gemv ? 80000000u : 64000000u) : gemv ? 350000000u : 200000000u);
 }
 
 template <int NA, bool EXACT>
@@ -634,7 +638,7 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
         ctx->launches++;
         rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, terms, 32, k, k * 2, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        return NA == 2 ? launch_batch<2, true>(ctx, tm_w, tm_s, tm_a, out, p, grid) : launch_batch<1, true>(ctx, tm_w, tm_s, tm_a, out, p, grid);
+        return launch_batch<2, true>(ctx, tm_w, tm_s, tm_a, out, p, grid);
     }
     rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, act_bf16, m, k, k * 2, (uint32_t)p.BT, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
