@@ -380,3 +380,43 @@ def test_tail_split_is_bit_identical(ctx, oracle, m, k, n, splits):
     assert np.array_equal(outs[True][0][rows], oracle.requant_range(acc, 2e-4, 128.0, 0, 255).astype(np.uint8))
     pk.free()
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n", [(64, 11008, 4096), (100, 8192, 300)])
+def test_tail_split_replayed_from_a_graph(m, k, n):
+    """Every replay publishes the same word in the flags of the split: the owner of a tile must still wait for
+    this replay's parts, which a new A makes different from the last one's."""
+    import torch
+    import yscv_b200
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    with torch.cuda.stream(stream):
+        b = torch.randint(-127, 128, (k, n), dtype=torch.int8, device="cuda", generator=g)
+        a = torch.zeros(m, k, dtype=torch.int8, device="cuda")
+        out = torch.empty(m, n, dtype=torch.int32, device="cuda")
+        packed = ctx.pack_i8_b_dev(b.data_ptr(), k, n)
+
+        def call():
+            ctx.matmul_integer_dev(a.data_ptr(), False, 0, packed, m, out.data_ptr())
+
+        call()
+        assert "tail split" in ctx.dispatch_report()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            call()
+        for i in range(20):
+            a.copy_(torch.randint(-127, 128, (m, k), dtype=torch.int8, device="cuda", generator=g))
+            want = (a.double() @ b.double()).to(torch.int32)
+            if i % 3 == 2:
+                call()
+            else:
+                graph.replay()
+            stream.synchronize()
+            assert torch.equal(out, want), i
+    assert ctx.device_status() == 0
+    del graph
+    packed.free()
+    ctx.close()

@@ -137,7 +137,7 @@ struct yscv_cuda_ctx {
     yscv::DeviceBuffer rowsum;        // row sums of A (int8 GEMM with a zero point on B)
     yscv::DeviceBuffer tmp_bt, tmp_colsum;  // B^T and column sums of the non-prepacked int8 entry point
     // int8 GEMM with a split tail: one slot of partial sums per CTA, four flags per CTA; every
-    // launch that splits publishes a new epoch in the flags, so they are never reset
+    // launch that splits publishes a new epoch in the flags, and who waited for a flag sets it back to 0
     yscv::DeviceBuffer gemm_ws, gemm_flags;
     int gemm_epoch = 0;
     bool int8_tail_split = true;

@@ -62,8 +62,8 @@ struct G8Params {
     // the tiles from `tail_first` on are cut into runs of `tail_units` K blocks, one run per CTA,
     // laid end to end over those tiles. The CTA that holds a tile's first K block owns the tile;
     // the others leave their int32 partial sums in slot blockIdx.x of `ws` and publish `epoch`
-    // in ws_flag[4 * blockIdx.x + epilogue warp]. Integer addition is exact and commutative, so
-    // the result does not depend on the split. tail_first == tiles: no split.
+    // in ws_flag[4 * blockIdx.x + epilogue warp], which the owner sets back to 0. Integer addition
+    // is exact and commutative, so the result does not depend on the split. tail_first == tiles: no split.
     int tail_first, tail_units;
     int32_t *ws;
     int *ws_flag;
@@ -466,6 +466,10 @@ int8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                     }
                 }
                 alive = __all_sync(0xffffffffu, alive);
+                // no other warp reads these flags: taken back, so that a graph, whose replays all publish the
+                // word of the captured launch, waits for the parts of the replay at hand
+                if (lane == 0)
+                    for (int c = c_first; c <= c_last; ++c) p.ws_flag[4 * c + q] = 0;
                 if (alive) epilogue_row<BN>(p, colsum, out, row, taddr, nb, xpose, rt, c_first, c_last);
             } else {
                 epilogue_row<BN>(p, colsum, out, row, taddr, nb, xpose);
