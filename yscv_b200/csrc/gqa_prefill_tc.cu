@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) gqa_prefill_tc_kernel(const __g
         if (lane == 0) {
             uint32_t phase = 0;
             bool alive = true;
+            int keys = 0, values = 0;   // tiles whose copies were issued
             for (int i = 0, st = 0; i < n && alive; ++i) {
                 const uint32_t dst = base + G::RING + (uint32_t)st * ATImage<D>::BYTES;
                 const unsigned char *src = img + (size_t)i * ATImage<D>::BYTES;
@@ -527,11 +528,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) gqa_prefill_tc_kernel(const __g
                 if (!alive) break;
                 mbar_expect_tx(kfull + st * 8, ATImage<D>::K_BYTES);
                 bulk_load(dst, src, ATImage<D>::K_BYTES, kfull + st * 8);
+                ++keys;
                 alive = mbar_wait(vempty + st * 8, phase ^ 1u, status);
                 if (!alive) break;
                 mbar_expect_tx(vfull + st * 8, ATImage<D>::V_BYTES);
                 bulk_load(dst + ATImage<D>::K_BYTES, src + ATImage<D>::K_BYTES, ATImage<D>::V_BYTES, vfull + st * 8);
+                ++values;
                 if (++st == STAGES) { st = 0; phase ^= 1u; }
+            }
+            // a consumer gave up: no copy may be in flight when the CTA leaves (bounded)
+            if (!alive) {
+                for (int i = max(0, keys - STAGES); i < keys; ++i) mbar_wait(kfull + i % STAGES * 8, (uint32_t)(i / STAGES) & 1u, nullptr);
+                for (int i = max(0, values - STAGES); i < values; ++i) mbar_wait(vfull + i % STAGES * 8, (uint32_t)(i / STAGES) & 1u, nullptr);
             }
         }
     } else if (warp == 1) {
