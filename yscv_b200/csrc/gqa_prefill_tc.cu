@@ -144,7 +144,7 @@ template <typename KV> struct ATCall {
 
 // Block (pair, tile), then every gridDim.y-th tile of the pair up to the last key in use
 template <typename KV, int D>
-__global__ void __launch_bounds__(256, 3) kv_split_kernel(const __grid_constant__ ATCall<KV> a) {
+__global__ void __launch_bounds__(256, 2) kv_split_kernel(const __grid_constant__ ATCall<KV> a) {
     pdl_wait();
     pdl_trigger();
     constexpr bool I8 = sizeof(KV) == 1;
