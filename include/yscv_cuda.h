@@ -118,7 +118,8 @@ int yscv_cuda_ctx_set_int4_prefill_exact(yscv_cuda_ctx *ctx, int exact);
 /* Kernel-selection switch of the bf16 prefill GEMM: enable != 0 (the default) lets prefills
  * with at least one 512-row x 256-token tile per CTA pair run on CTA pairs (tcgen05
  * cta_group::2: each CTA dequantises 256 weight rows and stages half of the activation tile);
- * 0 keeps the one-CTA kernel. Same products, same summation order over k. */
+ * 0 keeps the one-CTA kernel. Same products, and the same summation order over k except for the
+ * tiles of a last round that is split over k (the report says how many), which are added in parts. */
 int yscv_cuda_ctx_set_int4_prefill_cta_pairs(yscv_cuda_ctx *ctx, int enable);
 /* Kernel-selection switch of the int8 GEMM, like the reference's environment gates on its
  * int8 paths (crates/yscv-onnx/src/runner/quant_stats.rs:68-71). The GEMM has a one-CTA kernel

@@ -1,4 +1,4 @@
-"""The batched int4 matmul (2..128 activation rows, weights through tensor memory) at the edges of its tiles,
+"""The batched int4 matmul (3..128 activation rows, weights through tensor memory) at the edges of its tiles,
 stages and work split, against float64."""
 import numpy as np
 import pytest

@@ -1,4 +1,4 @@
-// Packed-int4 x fp32 matmul for a batch of 2..128 activation rows on the 5th-generation tensor cores,
+// Packed-int4 x fp32 matmul for a batch of 3..128 activation rows on the 5th-generation tensor cores,
 // dequantised weights through tensor memory: packed_int4_gemm_dispatch
 // (crates/yscv-kernels/src/ops/int4_matmul.rs:387-435, 548-605) between the few-row GEMV and the
 // prompt-sized GEMM. The weight rows are the MMA's M side (128 per tile), the activation rows its N side.
@@ -6,12 +6,12 @@
 // Two forms of one kernel:
 //   bf16   17..128 rows: weights q * scale and activations rounded to bf16, fp32 accumulators (the
 //          contract and the products of int4_prefill_gemm.cu)
-//   exact  2..16 rows: the int4 values themselves as fp16 (exact), activations as two fp16 terms
+//   exact  3..16 rows: the int4 values themselves as fp16 (exact), activations as two fp16 terms
 //          hi + lo of the value scaled by a power of two per row and 256 k (22 significant bits, absolute
 //          error below 2^-38 of that block's maximum). One accumulator holds one group of 32 k (the
 //          tensor core adds by truncation: nothing accumulates longer), and the drain multiplies it by
 //          the fp32 group scale and adds in fp32 registers, rounded. Relative error against float64
-//          1.3e-7 (the integer-MMA GEMV's 21-bit blocks: 5.4e-7; with outliers of 10^4: 1.2e-7 and 1.2e-6).
+//          1.2e-7 (the integer-MMA GEMV's 21-bit blocks: 5.4e-7; with outliers of 10^4: 1.2e-7 and 1.2e-6).
 //
 // What bounds it: the weights' HBM stream (0.625 B per weight). A dequantised tile that goes through
 // shared memory costs 4 B of shared-memory traffic per weight and a round trip; here the thread that
