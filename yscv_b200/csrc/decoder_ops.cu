@@ -423,7 +423,7 @@ __device__ __forceinline__ int dec_limit(const int32_t *pos, int max_seq) { retu
 // Keys per split. A cache is mostly longer than the conversation in it, and a block costs about as much for a
 // few keys as for CH: equal shares over as few splits as hold the keys in use in shares of up to CH, or, while
 // that is fewer than `want` (two blocks per SM), in shares of down to 64. 200 keys in a cache of 8192, 32
-// sequences, 64 / 8 heads of 128, f32 / int8: 59 / 28 us, spread over all splits 318 / 140. A nearly full cache
+// sequences, 64 / 8 heads of 128, f32 / int8: 59 / 27 us, spread over all splits 318 / 139. A nearly full cache
 // keeps all its splits (32 / 4 heads of 64, 8 sequences, 2049 keys: 16.1 us in 18 shares, 19.6 in 17).
 template <int CH> __device__ __forceinline__ int dec_share(int limit, int n_splits, int want) {
     int used = max(1, max((limit + CH - 1) / CH, min(min((limit + 63) / 64, want), n_splits)));
@@ -882,10 +882,12 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
 // Merges the splits: block per (q head, b), 128 threads; out row [b][n_q*d]. The splits' weights are
 // worked out once per block, a thread per split, then a thread per column adds with its loads in flight
 // (a serial walk that evaluated every weight in every thread: 27 us for 64 x 64 heads x 18 splits).
+// PRE: loads of a column in flight, BLOCKS: per SM. Sixteen and ten behind the f32 kernel (8 sequences, 64 / 8 heads of
+// 128, 2049 keys in 2178: 62.4 us both kernels, with eight and sixteen 65.2), eight and sixteen behind the int8
+// kernels, which leave it half the time (32 sequences, 32 / 4 heads of 64, 200 keys in 330: 8.0 us, the other way 12.2).
 constexpr int COMBINE_BATCH = 128;
-constexpr int PRE = 16;   // loads of a column in flight
-template <int CH>
-__global__ void __launch_bounds__(128)
+template <int CH, int PRE, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS)
 attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, int max_seq, const int32_t *__restrict__ pos,
                          int want, float *__restrict__ out) {
     pdl_wait();
@@ -1265,7 +1267,7 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                                          d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
                 YSCV_CUDA_TRY(cudaGetLastError());
                 ctx->launches++;
-                YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel<128>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part,
+                YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel<128, 8, 16>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part,
                                          n_splits, (int)d_head, (int)max_seq, d_pos, want, d_out));
                 DEC_EPILOGUE(ctx, "gqa_attention(split-k,int8 cache,mma)");
             }
@@ -1283,7 +1285,10 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                                  (int)d_head, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
-        YSCV_CUDA_TRY(launch_pdl(chunk == 64 ? attention_combine_kernel<64> : attention_combine_kernel<128>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part, n_splits,
+        auto merge = sizeof(KV) == 1 ? attention_combine_kernel<128, 8, 16>
+                     : chunk == 64   ? attention_combine_kernel<64, 16, 10>
+                                     : attention_combine_kernel<128, 16, 10>;
+        YSCV_CUDA_TRY(launch_pdl(merge, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part, n_splits,
                                  (int)d_head, (int)max_seq, d_pos, want, d_out));
         DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(split-k,int8 cache)" : "gqa_attention(split-k)");
     }
