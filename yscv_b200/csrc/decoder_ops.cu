@@ -935,41 +935,73 @@ attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, in
     if (tid < d) out[hb * d + tid] = acc * inv;
 }
 
-// out[m][n] = sum_k x[m][k] * w[n][k]; one warp per weight row, up to 4 x rows per pass
-template <int MT>
+// out[m][n] = sum_k x[m][k] * w[n][k] for m <= MT: one warp per R weight rows, which share the x rows it reads.
+// Bound by the weights' HBM stream: enough loads in flight per warp (R rows, unrolled) and one pass whatever m.
+// The weights skip L1, which holds the x rows. With a row per warp, four loads in flight and a pass per 4 x rows
+// 32000 x 2048 took 54.1 / 57.3 / 119 us at 1 / 4 / 8 x rows, now 41.2 / 49 / 67 (6.4, 5.3 and 3.9 TB/s; from five rows
+// on the x rows' L1 reads bound it); 128256 x 8192 at one row 770 -> 600 us.
+__device__ __forceinline__ float4 ldg_stream(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+template <int MT, int R, int UNROLL>
 __global__ void __launch_bounds__(256)
-f32_matmul_kernel(const float *__restrict__ w, const float *__restrict__ x, float *__restrict__ out,
-                  int m0, int M, int N, int K) {
+f32_matmul_kernel(const float *__restrict__ w, const float *__restrict__ x, float *__restrict__ out, int M, int N, int K) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const int wpb = blockDim.x >> 5;
-    const int mt = min(MT, M - m0);
-    for (int n = blockIdx.x * wpb + (threadIdx.x >> 5); n < N; n += gridDim.x * wpb) {
-        const float4 *wr = reinterpret_cast<const float4 *>(w + (size_t)n * K);
-        float acc[MT];
+    const int wpb = blockDim.x >> 5, K4 = K / 4;
+    for (int n = (blockIdx.x * wpb + (threadIdx.x >> 5)) * R; n < N; n += gridDim.x * wpb * R) {
+        const float4 *wr[R];
 #pragma unroll
-        for (int i = 0; i < MT; ++i) acc[i] = 0.0f;
-#pragma unroll 4
-        for (int c = lane; c < K / 4; c += 32) {
-            const float4 wv = __ldg(wr + c);
+        for (int j = 0; j < R; ++j) wr[j] = reinterpret_cast<const float4 *>(w + (size_t)min(n + j, N - 1) * K);
+        float acc[R][MT];
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+            for (int i = 0; i < MT; ++i) acc[j][i] = 0.0f;
+        // (no branch on i: x rows past M repeat the last one, so that a step's loads are issued together)
+        auto step = [&](const float4 (&wv)[R], int c) {
+            float4 xv[MT];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) xv[i] = __ldg(reinterpret_cast<const float4 *>(x + (size_t)min(i, M - 1) * K) + c);
 #pragma unroll
             for (int i = 0; i < MT; ++i) {
-                if (i < mt) {
-                    const float4 xv = __ldg(reinterpret_cast<const float4 *>(x + (size_t)(m0 + i) * K) + c);
-                    acc[i] = fmaf(wv.x, xv.x, acc[i]);
-                    acc[i] = fmaf(wv.y, xv.y, acc[i]);
-                    acc[i] = fmaf(wv.z, xv.z, acc[i]);
-                    acc[i] = fmaf(wv.w, xv.w, acc[i]);
+#pragma unroll
+                for (int j = 0; j < R; ++j) {
+                    acc[j][i] = fmaf(wv[j].x, xv[i].x, acc[j][i]);
+                    acc[j][i] = fmaf(wv[j].y, xv[i].y, acc[j][i]);
+                    acc[j][i] = fmaf(wv[j].z, xv[i].z, acc[j][i]);
+                    acc[j][i] = fmaf(wv[j].w, xv[i].w, acc[j][i]);
                 }
             }
+        };
+        int c = lane;
+        for (; c + (UNROLL - 1) * 32 < K4; c += UNROLL * 32) {
+            float4 wv[UNROLL][R];
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+                for (int j = 0; j < R; ++j) wv[u][j] = ldg_stream(wr[j] + c + u * 32);
+#pragma unroll
+            for (int u = 0; u < UNROLL; ++u) step(wv[u], c + u * 32);
+        }
+        for (; c < K4; c += 32) {
+            float4 wv[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) wv[j] = ldg_stream(wr[j] + c);
+            step(wv, c);
         }
 #pragma unroll
-        for (int i = 0; i < MT; ++i) {
-            float v = acc[i];
+        for (int j = 0; j < R; ++j) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0 && i < mt) out[(size_t)(m0 + i) * N + n] = v;
+            for (int i = 0; i < MT; ++i) {
+                float v = acc[j][i];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0 && i < M && n + j < N) out[(size_t)i * N + n + j] = v;
+            }
         }
     }
 }
@@ -1109,14 +1141,23 @@ argmax_final_kernel(const float *__restrict__ pv, const int32_t *__restrict__ pi
                     int32_t *__restrict__ out) {
     pdl_wait();
     pdl_trigger();
-    // partials are in increasing index order: scan them in order, later wins ties
-    if (threadIdx.x != 0) return;
+    // partials are in increasing index order: scan them in order, later wins ties (staged first: a scan that
+    // loads as it goes waits for L2 again and again)
+    __shared__ float sv[64];
+    __shared__ int32_t si[64];
     const int row = blockIdx.x;
+    if (threadIdx.x < nb) {
+        sv[threadIdx.x] = pv[row * nb + threadIdx.x];
+        si[threadIdx.x] = pi[row * nb + threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     float best = -INFINITY;
     int idx = -1;
+#pragma unroll 8
     for (int j = 0; j < nb; ++j) {
-        const int i = pi[row * nb + j];
-        const float v = pv[row * nb + j];
+        const int i = si[j];
+        const float v = sv[j];
         if (i >= 0 && (idx < 0 || !(v < best))) { best = v; idx = i; }
     }
     out[row] = idx < 0 ? 0 : idx;
@@ -1384,7 +1425,6 @@ int yscv_cuda_f32_matmul_dev(yscv_cuda_ctx *ctx, const float *d_w, const float *
     if ((reinterpret_cast<uintptr_t>(d_w) | reinterpret_cast<uintptr_t>(d_x)) & 15)
         return fail(YSCV_CUDA_ERR_UNSUPPORTED, "weights and activations must be 16-byte aligned");
     if (m * n == 0) return YSCV_CUDA_OK;
-    const unsigned blocks = (unsigned)((n + 7) / 8 < (size_t)(16 * ctx->sm_count) ? (n + 7) / 8 : 16 * ctx->sm_count);
     if (m > 8 && ctx->f32_tensor_cores && f32_gemm_tc_supported(d_w, d_x, m, n, k)) {
         // wide batch: three TF32 products per fp32 product on the tensor cores, weights read once
         int rc = ctx->scratch.reserve(f32_gemm_tc_scratch_bytes(m, k), ctx->stream);
@@ -1404,12 +1444,13 @@ int yscv_cuda_f32_matmul_dev(yscv_cuda_ctx *ctx, const float *d_w, const float *
         ctx->last_kernel = "f32_matmul(tiled)";
         return YSCV_CUDA_OK;
     }
-    // one pass over the weights per 4 activation rows
-    for (size_t m0 = 0; m0 < m; m0 += 4) {
-        YSCV_CUDA_TRY(launch_pdl(f32_matmul_kernel<4>, dim3(blocks), dim3(256), 0, ctx->stream, d_w, d_x, d_out, (int)m0, (int)m, (int)n, (int)k));
-        YSCV_CUDA_TRY(cudaGetLastError());
-        ctx->launches++;
-    }
+    // one pass over the weights: rows per warp and unroll with enough loads in flight for the registers that m takes
+    auto kern = m == 1 ? f32_matmul_kernel<1, 2, 4> : m == 2 ? f32_matmul_kernel<2, 2, 4> : m <= 4 ? f32_matmul_kernel<4, 4, 2> : f32_matmul_kernel<8, 4, 1>;
+    const size_t rows = m <= 2 ? 2 : 4, need = (n + 8 * rows - 1) / (8 * rows), most = (size_t)16 * ctx->sm_count;
+    const unsigned blocks = (unsigned)(need < most ? need : most);
+    YSCV_CUDA_TRY(launch_pdl(kern, dim3(blocks), dim3(256), 0, ctx->stream, d_w, d_x, d_out, (int)m, (int)n, (int)k));
+    YSCV_CUDA_TRY(cudaGetLastError());
+    ctx->launches++;
     ctx->last_kernel = "f32_matmul";
     return YSCV_CUDA_OK;
 }
