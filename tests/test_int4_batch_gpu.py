@@ -26,6 +26,8 @@ CASES = [(m, n, k) for ms, shapes in [
     ((17, 31, 32), [(23000, 2176), (1650, 30080), (42000, 1152), (380000, 128)]),
     ((33, 48, 64), [(20000, 4096), (2800, 28928), (63000, 1280)]),
     ((65, 100, 128), [(20000, 4096), (2800, 28800), (10241, 8192)]),
+    # slices of k: one tile and many, more slices than CTAs of a round, units that do not divide, an odd number of outputs
+    ((17, 32, 33, 64, 97, 128), [(1, 128), (127, 384), (129, 256), (300, 16384), (1001, 1152), (2560, 2176), (2048, 5632), (11264, 2048)]),
 ] for m in ms for n, k in shapes]
 
 

@@ -18,9 +18,21 @@
 // owns a weight row writes its values to TMEM (tcgen05.st), where the MMA reads its A operand. A stage
 // is 256 k (128 contiguous bytes of every row), so that DRAM sees whole lines.
 //
-// Work split: the units (tile, 256 k) are numbered through and every CTA takes an equal contiguous
+// Work split, large matrices: the units (tile, 256 k) are numbered through and every CTA takes an equal contiguous
 // range, so that no tile count leaves SMs idle. The parts of a tile whose units lie in several CTAs go
 // to a workspace as fp32 partial sums; a second kernel adds them in CTA order (the same result every time).
+// Smaller ones (bf16, SLICED): a CTA takes whole items (tile, slice of k) and stores the slice's sums as
+// [slice][M][N] rows, which add_kslices_kernel adds in slice order; nothing to add with one slice.
+// bg_split chooses.
+//
+// A small call is a chain of latencies: launch, weights from HBM, dequantisation, activations, MMA, drain, and the
+// next kernel's wait. So a stage has a barrier for its weights and one for its activations, and the weights are
+// fetched and dequantised into the A slots while the predecessor still runs; no more stages than a CTA has units, so
+// that its blocks fit beside it; the drain steps one pointer (with an address and two bounds per element it took 1.1
+// us for 32 columns, now 0.35). us per call with its activation pass, 32 / 64 / 128 rows, against
+// int4_prefill_gemm_kernel with K slices: 2560 x 2048 8.0 / 8.6 / 9.8 (9.7 / 12.5 / 16.5), 11264 x 2048 12.2 / 12.9 / 15.3
+// (15.4 / 15.4 / 17.3), 2048 x 5632 10.1 / 10.7 / 12.2 (11.8 / 13.4 / 23.5), 4096 x 4096 10.8 / 11.6 / 13.2 (12.7 / 13.6 /
+// 20.3). The drain alone: 57344 x 8192 at 64 rows 90 -> 84.
 //
 // Warps: 0 TMA producer, 1 (and 2) MMA issuer of tile half 0 (and 1), 4..11 dequantise (two groups of
 // four warps: a tile half each, or every other slot), 12.. drain and store. A hand-over between the
@@ -50,6 +62,8 @@ struct BGParams {
     int M, N, K;
     int BT;                 // activation rows of the MMA (multiple of 16); exact: 16
     int kb, units;          // units per tile, units in all
+    int per, rest;          // units / CTAs, units % CTAs
+    int slices, tiles;      // sliced form: k slices per tile, tiles
     int stages, stage_bytes;
     int acc_bufs;           // bf16: accumulator sets in TMEM
     float *ws;              // [CTA][2: part with its tile's last unit, part without][NA][BT][128]
@@ -97,23 +111,37 @@ __device__ __forceinline__ void bg_st32(uint32_t taddr, const uint32_t *r) {
         "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
         : "memory");
 }
-// One CTA's walk over its units, last one first: every call yields a tile and its range of k units.
-struct BGWalk {
-    int end, first, kb;
+// First unit of CTA c: c * units / CTAs without the 64-bit division (a third of a small call's set-up)
+__host__ __device__ inline int bg_first_unit(const BGParams &p, int c, int grid) { return c * p.per + c * p.rest / grid; }
+// One CTA's walk: every call yields a tile and its range of k units. Equal ranges of the units, last one first, or
+// (SLICED) the items (slice, tile) CTA by CTA.
+template <bool SLICED> struct BGWalk {
+    int end, first, kb, slice;
     __device__ BGWalk(const BGParams &p)
-        : end((int)((long long)(blockIdx.x + 1) * p.units / gridDim.x)), first((int)((long long)blockIdx.x * p.units / gridDim.x)), kb(p.kb) {}
-    __device__ bool next(int &tile, int &k0, int &k1) {
+        : end(SLICED ? (int)blockIdx.x : bg_first_unit(p, blockIdx.x + 1, gridDim.x)), first(SLICED ? p.tiles : bg_first_unit(p, blockIdx.x, gridDim.x)),
+          kb(p.kb), slice(SLICED ? p.slices : 0) {}
+    __device__ bool next(int &tile, int &k0, int &k1, int &sl) {
+        if (SLICED) {
+            if (end >= first * slice) return false;
+            sl = end / first;
+            tile = end - sl * first;
+            k0 = sl * kb / slice;
+            k1 = (sl + 1) * kb / slice;
+            end += gridDim.x;
+            return true;
+        }
         if (end <= first) return false;
         tile = (end - 1) / kb;
         const int start = max(first, tile * kb);
         k0 = start - tile * kb;
         k1 = end - tile * kb;
         end = start;
+        sl = 0;
         return true;
     }
 };
 
-template <int NA, bool EXACT>
+template <int NA, bool EXACT, bool SLICED>
 __global__ void __launch_bounds__(bg_threads<NA, EXACT>(), 1)
 int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s,
                        const __grid_constant__ CUtensorMap tm_a, float *__restrict__ out, BGParams p, int *__restrict__ status) {
@@ -126,13 +154,14 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
     const int act_rows = EXACT ? 32 : p.BT;
     constexpr int S_OFF = NA * BG_W, A_OFF = NA * (BG_W + BG_S);
     const uint32_t bars = base + (uint32_t)p.stages * p.stage_bytes;
-    const uint32_t full = bars, empty = bars + 64, afull = bars + 128, mdone = bars + 160, dempty = bars + 192;
-    const uint32_t tfull = bars + 224, tempty = bars + 240;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)p.stages * p.stage_bytes + 256);
+    const uint32_t wfull = bars, xfull = bars + 64, empty = bars + 128, afull = bars + 192, mdone = bars + 224, dempty = bars + 256;
+    const uint32_t tfull = bars + 288, tempty = bars + 304;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)p.stages * p.stage_bytes + 320);
 
     if (tid == 0) {
         for (int i = 0; i < p.stages; ++i) {
-            mbar_init(full + i * 8, 1);
+            mbar_init(wfull + i * 8, 1);   // nibbles and scales have landed
+            mbar_init(xfull + i * 8, 1);   // activations (and inverse scales) have landed
             mbar_init(empty + i * 8, NA + (EXACT ? EPI_WARPS : 0));
         }
         for (int i = 0; i < BG_SLOTS; ++i) {
@@ -156,40 +185,41 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
     pdl_trigger();
     const uint32_t tmem = *tmem_slot;
     const uint32_t t_a = tmem + 256;                 // columns 0..255: accumulators, 256..511: A slots
-    BGWalk walk(p);
-    int tile, k0, k1;
+    BGWalk<SLICED> walk(p);
+    int tile, k0, k1, sl;
     bool alive = true;
     // The weights are the caller's constants (the kernels that pack them are ordinary launches, complete
-    // before a dependent one starts): the first stages' are fetched while the predecessor drains. Everything else may be its output, or (workspace, `out`) still in its use.
-    if (warp != 0) pdl_wait();
+    // before a dependent one starts): the first stages' are fetched, and dequantised into the A slots, while the
+    // predecessor drains. The producer waits before it fetches activations, which may be its output, the drain
+    // before it writes the workspace and `out`, which may still be in its use.
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t bytes = NA * (BG_W + BG_S) + 4 * act_rows * 128 + (EXACT ? 64 : 0);
             auto weights = [&](int st, int tl, int u) {
-                const uint32_t dst = base + (uint32_t)st * p.stage_bytes, bar = full + st * 8;
-                mbar_expect_tx(bar, bytes);
+                const uint32_t dst = base + (uint32_t)st * p.stage_bytes, bar = wfull + st * 8;
+                mbar_expect_tx(bar, NA * (BG_W + BG_S));
 #pragma unroll
                 for (int a = 0; a < NA; ++a) {
                     tma_load_2d(dst + a * BG_W, &tm_w, u * (BG_UNIT / 2), (tl * NA + a) * 128, bar);
                     tma_load_2d(dst + S_OFF + a * BG_S, &tm_s, u * (BG_UNIT / 32), (tl * NA + a) * 128, bar);
                 }
             };
-            BGWalk ahead(p);
+            BGWalk<SLICED> ahead(p);
             int early = 0;
-            while (early < p.stages && ahead.next(tile, k0, k1))
+            while (early < p.stages && ahead.next(tile, k0, k1, sl))
                 for (int u = k0; u < k1 && early < p.stages; ++u) weights(early++, tile, u);
             pdl_wait();
             int st = 0, cnt = 0;
             uint32_t ph = 0;
-            while (alive && walk.next(tile, k0, k1)) {
+            while (alive && walk.next(tile, k0, k1, sl)) {
                 for (int u = k0; u < k1; ++u) {
                     if (cnt++ >= early) {
                         alive = mbar_wait(empty + st * 8, ph ^ 1u, status);
                         if (!alive) break;
                         weights(st, tile, u);
                     }
-                    const uint32_t dst = base + (uint32_t)st * p.stage_bytes, bar = full + st * 8;
+                    const uint32_t dst = base + (uint32_t)st * p.stage_bytes, bar = xfull + st * 8;
+                    mbar_expect_tx(bar, 4 * act_rows * 128 + (EXACT ? 64 : 0));
 #pragma unroll
                     for (int s = 0; s < 4; ++s)
                         tma_load_2d(dst + A_OFF + s * act_rows * 128, &tm_a, u * BG_UNIT + s * 64, 0, bar);
@@ -199,9 +229,10 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
             }
             // a consumer gave up: no stage's copies may be in flight when the CTA leaves (bounded)
             if (!alive)
-                for (int i = 0; i < p.stages; ++i) mbar_wait(full + i * 8, i < st ? ph : ph ^ 1u, nullptr);
-        } else {
-            pdl_wait();
+                for (int i = 0; i < p.stages; ++i) {
+                    mbar_wait(wfull + i * 8, i < st ? ph : ph ^ 1u, nullptr);
+                    mbar_wait(xfull + i * 8, i < st ? ph : ph ^ 1u, nullptr);
+                }
         }
         __syncwarp();
     } else if (warp <= NA) {
@@ -212,14 +243,14 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
                                ((uint32_t)(128 >> 4) << 24);
         int st = 0, ring = 0, buf = 0;
         uint32_t ph = 0, rph = 0, bph = 0;
-        while (alive && walk.next(tile, k0, k1)) {
+        while (alive && walk.next(tile, k0, k1, sl)) {
             if (!EXACT) {
                 alive = __all_sync(0xffffffffu, mbar_wait(tempty + buf * 8, bph ^ 1u, status));
                 if (!alive) break;
             }
             const uint32_t acc = tmem + (buf * NA + a) * p.BT;
             for (int u = k0; u < k1 && alive; ++u) {
-                alive = __all_sync(0xffffffffu, mbar_wait(full + st * 8, ph, status));
+                alive = __all_sync(0xffffffffu, mbar_wait(xfull + st * 8, ph, status));
                 if (!alive) break;
                 const uint32_t act = base + (uint32_t)st * p.stage_bytes + A_OFF;
 #pragma unroll
@@ -270,9 +301,9 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         int st = 0, ring = NA == 2 ? 0 : g;
         uint32_t ph = 0, rph = 0;
-        while (alive && walk.next(tile, k0, k1)) {
+        while (alive && walk.next(tile, k0, k1, sl)) {
             for (int u = k0; u < k1 && alive; ++u) {
-                alive = mbar_wait(full + st * 8, ph, status);
+                alive = mbar_wait(wfull + st * 8, ph, status);
                 if (!alive) break;
                 const unsigned char *stage = smem + (size_t)st * p.stage_bytes;
                 const unsigned char *row = stage + a * BG_W + r * 128;
@@ -350,8 +381,9 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
         const uint32_t lane_base = (uint32_t)((w & 3) * 32) << 16;
         int st = 0, buf = 0, ring = 0;
         uint32_t ph = 0, bph = 0, rph = 0;
-        while (alive && walk.next(tile, k0, k1)) {
-            const bool whole = k0 == 0 && k1 == p.kb;
+        pdl_wait();
+        while (alive && walk.next(tile, k0, k1, sl)) {
+            const bool whole = SLICED || (k0 == 0 && k1 == p.kb);
             float *const mine = p.ws + (size_t)(2 * blockIdx.x + (k1 == p.kb ? 0 : 1)) * NA * p.BT * 128 + r;
             if constexpr (EXACT) {
                 const int a = w >> 2;
@@ -360,7 +392,7 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
                 for (int t = 0; t < 16; ++t) acc[t] = 0.0f;
                 for (int u = k0; u < k1 && alive; ++u) {
                     const unsigned char *stage = smem + (size_t)st * p.stage_bytes;
-                    alive = mbar_wait(full + st * 8, ph, status);
+                    alive = mbar_wait(wfull + st * 8, ph, status) && mbar_wait(xfull + st * 8, ph, status);
                     if (!alive) break;
                     const unsigned char *srow = stage + S_OFF + a * BG_S + r * 32;
                     float part[16];
@@ -418,17 +450,18 @@ int4_batch_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
 #pragma unroll 1
                 for (int a = 0; a < NA; ++a) {
                     const int n = (tile * NA + a) * 128 + r;
+                    // a column of the result, or of this CTA's part of the tile
+                    float *o = whole ? out + (size_t)sl * p.M * p.N + n : mine + (size_t)a * p.BT * 128;
+                    const size_t pitch = whole ? p.N : 128;
+                    const int rows = whole ? (n < p.N ? p.M : 0) : p.BT;
 #pragma unroll 1
                     for (int t0 = 0; t0 < p.BT; t0 += 32) {
                         uint32_t d[32];
                         bg_ld32(tmem + (buf * NA + a) * p.BT + t0 + lane_base, d);
 #pragma unroll
                         for (int t = 0; t < 32; ++t) {
-                            if (!whole) {
-                                if (t0 + t < p.BT) mine[((size_t)a * p.BT + t0 + t) * 128] = __uint_as_float(d[t]);
-                            } else if (n < p.N && t0 + t < p.M) {
-                                out[(size_t)(t0 + t) * p.N + n] = __uint_as_float(d[t]);
-                            }
+                            if (t0 + t < rows) *o = __uint_as_float(d[t]);
+                            o += pitch;
                         }
                     }
                 }
@@ -539,17 +572,11 @@ static bool bg_shape(size_t n, size_t k, size_t gs) {
     return tensor_map_encoder() != nullptr && gs == 32 && k % 128 == 0 && k >= 128 && n >= 1 && n < (1u << 22) && k < (1u << 22);
 }
 
-// Which calls gain. Three launches, a TMEM hand-over and the join cost about 10 us whatever the size,
-// so small matrices stay where they are (us per call in a graph that walks copies of the weights, 500 MB together,
-// here against the other kernel):
-//   bf16, against int4_prefill_gemm_kernel, 32 / 64 / 128 rows: 57344 x 8192 81 / 148, 92 / 173, 138 / 194;
-//   8192 x 28672 52 / 76, 56 / 80, 75 / 88; 22016 x 4096 30 / 36, 34 / 40, 44 / 47; 10240 x 8192 27 / 33, 31 / 36,
-//   40 / 41; 14336 x 4096 23 / 26, 27 / 26, 34 / 29; 4096 x 14336 24 / 25, 26 / 26, 33 / 31; 16384 x 2048 18 / 15,
-//   22 / 16, 27 / 18; 6144 x 4096 17 / 14, 20 / 16, 26 / 21; 11264 x 2048 15.8 / 15.2, 20 / 15, 25 / 17
-bool int4_batch_bf16_wins(size_t m, size_t n, size_t k, size_t gs) {
-    const size_t weights = n * k;
-    return m > 16 && m <= 128 && bg_shape(n, k, gs) && weights >= (m <= 32 ? 40000000u : 80000000u);
-}
+// Which calls gain.
+//   bf16: every one of 17..128 rows, against int4_prefill_gemm_kernel (figures at the top; large ones, 32 / 64 / 128
+//   rows: 57344 x 8192 77 / 148, 84 / 173, 130 / 194; 8192 x 28672 50 / 76, 52 / 81, 68 / 89; 10240 x 8192 26 / 33, 29 / 36,
+//   35 / 42; 14336 x 4096 20 / 27, 21 / 26, 26 / 29; the closest 16384 x 2048 at 128 rows 15.9 / 18.0)
+bool int4_batch_bf16_wins(size_t m, size_t n, size_t k, size_t gs) { return m > 16 && m <= 128 && bg_shape(n, k, gs); }
 //   exact, against the integer-MMA GEMV, 4 / 8 / 16 rows: 57344 x 8192 79 / 85, 80 / 95, 78 / 143; 8192 x 28672
 //   49 / 49, 50 / 60, 50 / 83; 28672 x 8192 47 / 46, 47 / 51, 47 / 74; 22016 x 4096 27 / 29, 27 / 28, 27 / 41; 10240 x
 //   8192 25 / 24, 25.1 / 26.5, 25 / 39; 14336 x 4096 22 / 18, 23 / 16, 23 / 22; 2 rows: everywhere behind. Depths that
@@ -560,15 +587,19 @@ bool int4_batch_exact_wins(size_t m, size_t n, size_t k, size_t gs) {
     return m > 2 && m <= 16 && bg_shape(n, k, gs) && weights >= (m > 8 ? 64000000u : m > 4 ? (gemv ? 80000000u : 64000000u) : gemv ? 350000000u : 200000000u);
 }
 
-template <int NA, bool EXACT>
+template <int NA, bool EXACT, bool SLICED>
 static int launch_batch(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, const CUtensorMap &tm_s, const CUtensorMap &tm_a, float *out,
                         BGParams p, int grid) {
     const int act = EXACT ? 4 * 32 * 128 + BG_INV : 4 * p.BT * 128;
     p.stage_bytes = NA * (BG_W + BG_S) + act;
     p.stages = (227 * 1024 - 1024) / p.stage_bytes;
     if (p.stages > BG_MAX_STAGES) p.stages = BG_MAX_STAGES;
+    const int longest = SLICED ? (p.tiles * p.slices + grid - 1) / grid * ((p.kb + p.slices - 1) / p.slices) : (p.units + grid - 1) / grid;
+    if (p.stages > longest) p.stages = longest;   // units of a CTA
     const int smem = p.stages * p.stage_bytes + 512;
-    auto kern = int4_batch_gemm_kernel<NA, EXACT>;
+    auto kern = int4_batch_gemm_kernel<NA, EXACT, SLICED>;
+    p.per = p.units / grid;
+    p.rest = p.units % grid;
     int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kern), ctx->device, 227 * 1024);
     if (rc) return rc;
     ctx->prof_begin();
@@ -578,13 +609,13 @@ static int launch_batch(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, const CUten
     YSCV_CUDA_TRY(cudaGetLastError());
     ctx->launches++;
     bool shared = false;
-    for (int c = 1; c < grid && !shared; ++c) shared = (long long)c * p.units / grid % p.kb != 0;
+    for (int c = 1; c < grid && !shared && !SLICED; ++c) shared = bg_first_unit(p, c, grid) % p.kb != 0;
     if (shared) {
         YSCV_CUDA_TRY(launch_pdl(bg_join_kernel, dim3((unsigned)(p.units / p.kb * NA), (unsigned)(p.BT / 8)), dim3(128), 0, ctx->stream, p,
                                  NA, grid, out));
         ctx->launches++;
     }
-    const int splits = (grid + (p.units / p.kb) - 1) / (p.units / p.kb);
+    const int splits = SLICED ? p.slices : (grid + (p.units / p.kb) - 1) / (p.units / p.kb);
     if (EXACT) {
         snprintf(ctx->report_int4, sizeof(ctx->report_int4),
                  "int4_fast m=%d n=%d k=%d: tcgen05 fp16 two-term, CTA tile %d rows x 16, 256 k per stage, %d stages, %d units on %d CTAs",
@@ -597,6 +628,25 @@ static int launch_batch(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, const CUten
         ctx->last_kernel = "int4_prefill_gemm(tcgen05,bf16,tmem)";
     }
     return YSCV_CUDA_OK;
+}
+
+// K slices of the sliced form, or 0 for equal ranges over the CTAs, by the modelled time in us: units one after another
+// in a CTA, a round's drain, the launch that adds slices and their traffic; equal ranges cost a second drain and the
+// join. The constants are a fit to 24 shapes from 512 x 2048 to 8192 x 28672 at 20 / 32 / 64 / 128 rows with every
+// choice forced in turn; its choice is 0.15 % behind the best of them on average and 3 % at worst.
+static int bg_split(const BGParams &p, int NA, int grid, int sms, bool slices_ok, size_t ws_bytes) {
+    const double unit = 0.64 + 0.002 * p.BT, mb = 0.07e-6;
+    double best = 3.2 + (p.units + grid - 1) / grid * unit * (NA == 2 ? 1.75 : 1.0) + 2.0 * grid * NA * 128 * p.BT * 4 * mb;
+    int slices = 0;
+    const int tiles = (p.N + 127) / 128;
+    for (int s = 1; s <= 8 && s <= p.kb; ++s) {
+        const double bytes = (double)s * p.M * p.N * 4;
+        if (s > 1 && (!slices_ok || bytes > (double)ws_bytes)) break;
+        const double rounds = (int)(((long long)tiles * s + sms - 1) / sms);
+        const double cost = rounds * ((p.kb + s - 1) / s * unit + 0.55) + (s > 1 ? 0.97 + 0.022 * s + bytes * mb : 0.0);
+        if (cost < best) { best = cost; slices = s; }
+    }
+    return slices;
 }
 
 // exact: act = fp32 rows, scratch of int4_batch_exact_scratch_bytes(k). Otherwise act_bf16 = bf16 rows
@@ -623,6 +673,7 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
     int grid = p.units < sms ? p.units : sms;
     if (grid > tiles * 4) grid = tiles * 4;
     p.acc_bufs = NA * p.BT > 128 ? 1 : 2;
+    p.slices = exact ? 0 : bg_split(p, NA, grid, sms, (m * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0, ctx->batch_ws.bytes);
 
     CUtensorMap tm_w, tm_s, tm_a;
     int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -638,11 +689,19 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
         ctx->launches++;
         rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, terms, 32, k, k * 2, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        return launch_batch<2, true>(ctx, tm_w, tm_s, tm_a, out, p, grid);
+        return launch_batch<2, true, false>(ctx, tm_w, tm_s, tm_a, out, p, grid);
     }
     rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, act_bf16, m, k, k * 2, (uint32_t)p.BT, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    return NA == 2 ? launch_batch<2, false>(ctx, tm_w, tm_s, tm_a, out, p, grid) : launch_batch<1, false>(ctx, tm_w, tm_s, tm_a, out, p, grid);
+    if (p.slices > 0) {
+        p.tiles = tiles1;
+        p.units = tiles1 * p.kb;
+        p.acc_bufs = 2;
+        const int items = tiles1 * p.slices;
+        rc = launch_batch<1, false, true>(ctx, tm_w, tm_s, tm_a, p.slices > 1 ? p.ws : out, p, items < sms ? items : sms);
+        return rc || p.slices == 1 ? rc : add_kslices(ctx, p.ws, out, m * n, p.slices);
+    }
+    return NA == 2 ? launch_batch<2, false, false>(ctx, tm_w, tm_s, tm_a, out, p, grid) : launch_batch<1, false, false>(ctx, tm_w, tm_s, tm_a, out, p, grid);
 }
 
 }  // namespace yscv

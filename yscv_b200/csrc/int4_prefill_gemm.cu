@@ -724,6 +724,16 @@ __global__ void __launch_bounds__(256) add_kslices_kernel(const float4 *__restri
     }
 }
 
+// parts: [slices][elements], 16-byte aligned, elements % 4 == 0
+int add_kslices(yscv_cuda_ctx *ctx, const float *parts, float *out, size_t elements, int slices) {
+    const size_t n4 = elements / 4;
+    const unsigned blocks = (unsigned)((n4 + 255) / 256 < 1184 ? (n4 + 255) / 256 : 1184);
+    YSCV_CUDA_TRY(launch_pdl(add_kslices_kernel, dim3(blocks), dim3(256), 0, ctx->stream, reinterpret_cast<const float4 *>(parts),
+                             reinterpret_cast<float4 *>(out), n4, slices));
+    ctx->launches++;
+    return YSCV_CUDA_OK;
+}
+
 // The tiles of the CTA-pair kernel's last round that several pairs share. Block (tile, 8 tokens), a
 // thread four rows.
 __global__ void __launch_bounds__(128) pp_join_kernel(PGParams p, int n_pairs, int vec, float *__restrict__ out) {
@@ -947,11 +957,8 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     YSCV_CUDA_TRY(cudaGetLastError());
     ctx->launches++;
     if (p.ksplit > 1) {
-        const size_t n4 = m * n / 4;
-        const unsigned blocks = (unsigned)((n4 + 255) / 256 < 1184 ? (n4 + 255) / 256 : 1184);
-        YSCV_CUDA_TRY(launch_pdl(add_kslices_kernel, dim3(blocks), dim3(256), 0, ctx->stream,
-                                 reinterpret_cast<const float4 *>(kernel_out), reinterpret_cast<float4 *>(out), n4, p.ksplit));
-        ctx->launches++;
+        const int arc = add_kslices(ctx, kernel_out, out, m * n, p.ksplit);
+        if (arc) return arc;
     }
     snprintf(ctx->report_int4, sizeof(ctx->report_int4),
              "int4_prefill_gemm m=%zu n=%zu k=%zu: tcgen05 bf16, CTA tile %d rows x %d tokens, %d k per stage, %d stages, "
