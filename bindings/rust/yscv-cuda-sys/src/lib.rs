@@ -195,4 +195,6 @@ extern "C" {
     pub fn yscv_cuda_decode_plan_step_token_dev(ctx: *mut yscv_cuda_ctx, plan: *const yscv_cuda_decode_plan, d_embedding: *const f32, vocab: usize, d_token: *mut i32, d_pos: *mut i32, d_final_gamma: *const f32, d_lm_head: *const f32, d_x: *mut f32, d_logits: *mut f32) -> c_int;
     pub fn yscv_cuda_decode_plan_step_token_shard_dev(ctx: *mut yscv_cuda_ctx, plan: *const yscv_cuda_decode_plan, d_embedding: *const f32, vocab: usize, d_token: *mut i32, d_pos: *mut i32, d_final_gamma: *const f32, d_lm_head_rows: *const f32, lm_row0: usize, lm_rows: usize, d_x: *mut f32, d_logits: *mut f32) -> c_int;
     pub fn yscv_cuda_decode_plan_free(plan: *mut yscv_cuda_decode_plan);
+    pub fn yscv_cuda_decoder_layers_workspace(ctx: *mut yscv_cuda_ctx, layers: *const yscv_cuda_decode_layer, n_layers: usize, hidden: usize, inter: usize, n_q: usize, n_kv: usize, d_head: usize, batch: usize, seq: usize, bytes: *mut usize) -> c_int;
+    pub fn yscv_cuda_decoder_layers_dev(ctx: *mut yscv_cuda_ctx, layers: *const yscv_cuda_decode_layer, n_layers: usize, hidden: usize, inter: usize, n_q: usize, n_kv: usize, d_head: usize, max_seq: usize, eps: f32, rope_theta: f32, kv_int8: c_int, batch: usize, seq: usize, d_pos: *const i32, d_x: *mut f32, d_final_gamma: *const f32, d_last: *mut f32, d_workspace: *mut c_void, workspace_bytes: usize) -> c_int;
 }

@@ -636,6 +636,29 @@ int yscv_cuda_decode_plan_step_token_shard_dev(yscv_cuda_ctx *ctx, const yscv_cu
 
 void yscv_cuda_decode_plan_free(yscv_cuda_decode_plan *plan);
 
+/* ---- the layers of a decoder in one call -----------------------------------------------
+ * The same sequence of operators as above for any number of sequences and positions (a decode step
+ * with seq == 1, a prompt pass), as a chain of kernels: the arithmetic of the stand-alone entry
+ * points, with the activations handed over in the form the next matmul takes and the K slices of a
+ * matmul added by the operator behind it. d_x [batch * seq][hidden] f32 holds the embedded tokens
+ * (row b * seq + s at position *d_pos + s) and is overwritten; the caches are
+ * [batch][max_seq][n_kv][d_head] (kv_int8: int8 with scale tables [batch][max_seq]); d_last
+ * [batch][hidden] receives RMSNorm(final residual) * final_gamma of every sequence's last position.
+ * _workspace says how many bytes of device memory a pass needs (its first call may allocate the
+ * library's own workspace, so ask outside a capture); passes that overlap need one each. hidden, inter and
+ * d_head must be multiples of 8, hidden at most 8192, d_x, the gammas, d_last and the workspace 16-byte aligned
+ * (else YSCV_CUDA_ERR_UNSUPPORTED). */
+int yscv_cuda_decoder_layers_workspace(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers,
+                                       size_t n_layers, size_t hidden, size_t inter, size_t n_q,
+                                       size_t n_kv, size_t d_head, size_t batch, size_t seq,
+                                       size_t *bytes);
+int yscv_cuda_decoder_layers_dev(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers,
+                                 size_t n_layers, size_t hidden, size_t inter, size_t n_q,
+                                 size_t n_kv, size_t d_head, size_t max_seq, float eps,
+                                 float rope_theta, int kv_int8, size_t batch, size_t seq,
+                                 const int32_t *d_pos, float *d_x, const float *d_final_gamma,
+                                 float *d_last, void *d_workspace, size_t workspace_bytes);
+
 #ifdef __cplusplus
 }
 #endif

@@ -168,6 +168,35 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
     return YSCV_CUDA_OK;
 }
 
+int int4_act_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, size_t m) {
+    const size_t n = w->m_w, k = w->k, gs = w->group_size;
+    if (m == 0 || ((reinterpret_cast<uintptr_t>(w->d_packed) | reinterpret_cast<uintptr_t>(w->d_scales)) & 15)) return ACT_F32;
+    if (m > 16) return !ctx->prefill_exact && int4_prefill_supported(m, n, k, gs) ? ACT_BF16 : ACT_F32;
+    if (int4_batch_exact_wins(m, n, k, gs) && int4_batch_ready(ctx)) return ACT_TERMS;
+    return int4_gemv_fast_supported(m, n, k, gs) && int4_gemv_uses_scratch(m, k) ? ACT_DIGITS : ACT_F32;
+}
+
+int int4_form_parts(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, int form, size_t m) {
+    return form == ACT_BF16 && int4_batch_bf16_wins(m, w->m_w, w->k, w->group_size) && int4_batch_ready(ctx) ? int4_batch_parts(ctx, m, w->m_w, w->k) : 1;
+}
+
+int int4_matmul_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, const ActOut &a, float *out, int *parts) {
+    const size_t n = w->m_w, k = w->k, m = (size_t)a.rows;
+    if (parts && a.form != ACT_BF16) *parts = 1;
+    switch (a.form) {
+        case ACT_BF16:
+            op_counters().int4_gemm_calls++;
+            return int4_prefill_gemm(ctx, w->d_packed, w->d_scales, nullptr, out, m, n, k, nullptr, a.ptr, parts);
+        case ACT_DIGITS:
+            op_counters().int4_gemv_calls++;
+            return int4_gemv_digits(ctx, w->d_packed, w->d_scales, a.ptr, out, m, n, k);
+        case ACT_TERMS:
+            op_counters().int4_gemv_calls++;
+            return int4_batch_gemm(ctx, w->d_packed, w->d_scales, nullptr, nullptr, out, m, n, k, a.ptr);
+        default: return int4_matmul_dev(ctx, w->d_packed, w->d_scales, n, k, w->group_size, static_cast<const float *>(a.ptr), out, m);
+    }
+}
+
 }  // namespace yscv
 
 // The event pairs are created by yscv_cuda_ctx_profile_enable, never here: a launch path

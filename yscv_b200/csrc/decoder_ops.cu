@@ -17,9 +17,10 @@
 // whole decode step stays on the device and can be replayed as one CUDA graph: the
 // sequence position and the token ids are read from device memory, never passed as
 // kernel arguments.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <cuda_bf16.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -62,33 +63,115 @@ __global__ void embedding_kernel(const float *__restrict__ w, const int32_t *__r
     for (int i = threadIdx.x; i < dim / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// Eight fp32 values -> bf16 in the order the packed-int4 prefill GEMM consumes its activations:
-// k = 0,4,1,5,2,6,3,7 of every group of 8 (what its nibble unpack produces), round to nearest even;
-// the same bits as its own activation pre-pass writes.
-__device__ __forceinline__ uint4 pack_bf16_gemm_order(const float (&v)[8]) {
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(v[0], v[4]);
-    __nv_bfloat162 p1 = __floats2bfloat162_rn(v[1], v[5]);
-    __nv_bfloat162 p2 = __floats2bfloat162_rn(v[2], v[6]);
-    __nv_bfloat162 p3 = __floats2bfloat162_rn(v[3], v[7]);
-    uint4 o;
-    o.x = *reinterpret_cast<uint32_t *>(&p0);
-    o.y = *reinterpret_cast<uint32_t *>(&p1);
-    o.z = *reinterpret_cast<uint32_t *>(&p2);
-    o.w = *reinterpret_cast<uint32_t *>(&p3);
-    return o;
+// Eight consecutive values that are the sum of `parts` arrays `pitch` floats apart, added in that order
+__device__ __forceinline__ void load8(const float *p, int parts, size_t pitch, float (&v)[8]) {
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+#pragma unroll 4
+    for (int s = 1; s < parts; ++s) {
+        const float4 *q = reinterpret_cast<const float4 *>(p + s * pitch);
+        const float4 c = __ldg(q), d = __ldg(q + 1);
+        v[0] += c.x; v[1] += c.y; v[2] += c.z; v[3] += c.w;
+        v[4] += d.x; v[5] += d.y; v[6] += d.z; v[7] += d.w;
+    }
 }
 
 // Position of element e of a group of 8 in that order
 __device__ __forceinline__ int gemm_order_pos(int e) { return ((e & 3) << 1) | (e >> 2); }
 
-// x_out = x + delta (delta may be null); normed = x_out * (1/sqrt(mean(x_out^2)+eps)) * gamma, written
-// as fp32 or (ACT) as the bf16 activations of the next prefill-shaped linear: the same arithmetic, so the
-// bf16 values equal those the linear's own pre-pass would make of the fp32 rows (ACT: hidden % 8 == 0).
+// x_out = x + delta (delta may be null), delta the sum of `parts` arrays `pitch` floats apart; the row normalised,
+// (x_out / sqrt(mean(x_out^2) + eps)) * gamma, in the form that the matmul behind it takes. Input row of block b:
+// row0 + b * row_step (blocks past the rows of `o` write padding).
 //
-// Latency-bound for a decode batch (a row per block, a few dozen blocks), bandwidth-bound for a prompt. A
-// thread keeps its NE elements (stride blockDim: coalesced whatever the alignment) in registers between the sum
-// of squares and the scaling, so a row costs one round trip with every load in flight; the form that walked the
-// row in a loop and re-read it took 20 us for 64 rows of 8192 and 67 us (2.5 TB/s) for 2048 of them.
+// Latency-bound for a decode batch (a block per row), bandwidth-bound for a prompt. A thread keeps eight consecutive
+// values in registers between the sum of squares and the scaling: one round trip with every load in
+// flight, 128-bit accesses, and what the activation forms want a lane to hold. The sum of squares goes through shared
+// memory so that its order is that of the kernel below (thread t: elements t, t + T, ...): the same result for every form and
+// alignment. With 32-bit accesses 2048 rows of 8192 to bf16 took 95 us, now 68 (4.3 TB/s); the passes it stands for
+// (partial sums added, conversion to digit planes) were launches of their own, 1.5 to 1.8 us each behind a decode batch.
+// T = 256 up to 2048 values, else 1024 (hidden <= 8 T). P pieces of eight per thread, T / P threads: one for a few rows,
+// more for a prompt, whose blocks then share an SM and keep the values in shared memory meanwhile.
+template <int FORM, int T, int P>
+__global__ void __launch_bounds__(T / P, P > 1 ? 1536 * P / T : 1)
+norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, const float *__restrict__ gamma, float eps, int hidden,
+                 size_t row0, size_t row_step, float *x_out, ActOut o) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int TH = T / P;
+    __shared__ float red[32];
+    __shared__ __align__(16) float sm[8 * T];
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    if (FORM == ACT_DIGITS && row >= o.rows) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const int i = (tid + p * TH) * 8;
+            store_act_padding(o, row, i < hidden ? i : 0, i < hidden);
+        }
+        return;
+    }
+    const size_t base = (row0 + row * row_step) * hidden;
+    float v[8] = {};
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const int i = (tid + p * TH) * 8;
+        if (i < hidden) {   // (x not through the read-only path: x_out may be x)
+            const float4 a = *reinterpret_cast<const float4 *>(x + base + i), b = *reinterpret_cast<const float4 *>(x + base + i + 4);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            if (delta) {
+                float d[8];
+                load8(delta + base + i, parts, pitch, d);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) v[t] += d[t];
+            }
+            const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+            *reinterpret_cast<float4 *>(sm + i) = lo;
+            *reinterpret_cast<float4 *>(sm + i + 4) = hi;
+            if (x_out) {
+                *reinterpret_cast<float4 *>(x_out + base + i) = lo;
+                *reinterpret_cast<float4 *>(x_out + base + i + 4) = hi;
+            }
+        }
+    }
+    float g[8] = {};
+    if (P == 1 && tid * 8 < hidden) load8(gamma + tid * 8, 1, 0, g);
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = tid + p * TH + j * T;
+            const float y = e < hidden ? sm[e] : 0.0f;
+            ss = fmaf(y, y, ss);
+        }
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, s);
+        if (lane == 0) red[(tid + p * TH) >> 5] = ss;
+    }
+    __syncthreads();
+    float total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) total += red[w];
+    const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const int i = (tid + p * TH) * 8;
+        const bool on = i < hidden;
+        if (P > 1 && on) {
+            load8(gamma + i, 1, 0, g);
+            const float4 a = *reinterpret_cast<const float4 *>(sm + i), b = *reinterpret_cast<const float4 *>(sm + i + 4);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) v[t] = (v[t] * inv) * g[t];
+        store_act<FORM>(o, v, row, i, on);
+    }
+}
+
+// The same for operands that are not 16-byte aligned and rows that are no multiple of 8, up to 16384
 template <bool ACT, int NE>
 __global__ void __launch_bounds__(1024)
 add_rms_norm_kernel(const float *x, const float *__restrict__ delta, const float *__restrict__ gamma, float eps,
@@ -172,26 +255,28 @@ __device__ __forceinline__ float swiglu_one(float g, float u) {
     const float s = 1.0f / (1.0f + expf(-g));
     return (g * s) * u;
 }
-template <bool ACT>
+template <int FORM>
 __global__ void __launch_bounds__(256)
-swiglu_kernel(const float *__restrict__ gu, void *__restrict__ out, int rows, int inter) {
+swiglu_form_kernel(const float *__restrict__ gu, int parts, size_t pitch, int rows, int inter, ActOut o) {
     pdl_wait();
     pdl_trigger();
     const int n8 = inter / 8;
     for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-        const float4 *grow = reinterpret_cast<const float4 *>(gu + (size_t)r * 2 * inter);
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n8; c += gridDim.x * blockDim.x) {
-            const float4 ga = __ldg(grow + 2 * c), gb = __ldg(grow + 2 * c + 1);
-            const float4 ua = __ldg(grow + 2 * (n8 + c)), ub = __ldg(grow + 2 * (n8 + c) + 1);
-            const float n[8] = {swiglu_one(ga.x, ua.x), swiglu_one(ga.y, ua.y), swiglu_one(ga.z, ua.z), swiglu_one(ga.w, ua.w),
-                                swiglu_one(gb.x, ub.x), swiglu_one(gb.y, ub.y), swiglu_one(gb.z, ub.z), swiglu_one(gb.w, ub.w)};
-            if constexpr (ACT) {
-                reinterpret_cast<uint4 *>(out)[(size_t)r * n8 + c] = pack_bf16_gemm_order(n);
-            } else {
-                float4 *o = reinterpret_cast<float4 *>(out) + 2 * ((size_t)r * n8 + c);
-                o[0] = make_float4(n[0], n[1], n[2], n[3]);
-                o[1] = make_float4(n[4], n[5], n[6], n[7]);
+        for (int c0 = blockIdx.x * blockDim.x; c0 < n8; c0 += gridDim.x * blockDim.x) {   // (whole warps reach store_act)
+            const int c = c0 + threadIdx.x;
+            const bool on = c < n8;
+            if (FORM == ACT_DIGITS && r >= o.rows) {
+                store_act_padding(o, r, on ? c * 8 : 0, on);
+                continue;
             }
+            float g[8] = {}, u[8] = {}, n[8];
+            if (on) {
+                load8(gu + (size_t)r * 2 * inter + c * 8, parts, pitch, g);
+                load8(gu + (size_t)r * 2 * inter + inter + c * 8, parts, pitch, u);
+            }
+#pragma unroll
+            for (int t = 0; t < 8; ++t) n[t] = swiglu_one(g[t], u[t]);
+            store_act<FORM>(o, n, r, c * 8, on);
         }
     }
 }
@@ -228,7 +313,8 @@ __device__ __forceinline__ float kv_get<int8_t>(const int8_t *row, int i, float 
 }
 
 // qkv rows: [q (n_q*d) | k (n_kv*d) | v (n_kv*d)], row r = b*seq + s at position *pos + s.
-// Rotates q in place, writes rotated k and v into the cache at [b][position][head][d]
+// The rows are the sum of `parts` arrays `pitch` floats apart. Writes rotated q to q_out (which may be the q of qkv,
+// in place), rotated k and v into the cache at [b][position][head][d]
 // (f32), or quantised per row with their scales at [b][position] (int8). A position outside
 // [0, max_seq) appends nothing and raises YSCV_DEV_POS_OVERFLOW in the status word.
 //
@@ -247,7 +333,7 @@ template <> struct RopeVec<4> { using T = float4; };
 template <> struct RopeVec<1> { using T = float; };
 template <typename KV, int V>
 __global__ void __launch_bounds__(ROPE_THREADS)
-rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d, float theta,
+rope_kv_append_kernel(const float *qkv, int parts, size_t pitch, float *q_out, int q_out_stride, int seq, int n_q, int n_kv, int d, float theta,
                       const int32_t *__restrict__ pos, KV *__restrict__ kc, KV *__restrict__ vc,
                       float *__restrict__ kscale, float *__restrict__ vscale, int max_seq, int *__restrict__ status) {
     constexpr bool I8 = sizeof(KV) == 1;
@@ -265,8 +351,20 @@ rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d
     const int p = *pos + s;
     const bool in_range = p >= 0 && p < max_seq;
     if (!in_range && part == 0 && threadIdx.x == 0) *status = YSCV_DEV_POS_OVERFLOW;
-    float *r = qkv + (size_t)row * (n_q + 2 * n_kv) * d;
+    const float *r = qkv + (size_t)row * (n_q + 2 * n_kv) * d;
     const int kv_n = n_kv * d;
+    auto load = [&](const float *v) {
+        VT x = *reinterpret_cast<const VT *>(v);
+        float *a = reinterpret_cast<float *>(&x);
+#pragma unroll 4
+        for (int s = 1; s < parts; ++s) {
+            const VT y = *reinterpret_cast<const VT *>(v + s * pitch);
+            const float *b = reinterpret_cast<const float *>(&y);
+#pragma unroll
+            for (int j = 0; j < V; ++j) a[j] += b[j];
+        }
+        return x;
+    };
     const size_t slot = (size_t)b * max_seq + (in_range ? p : 0);
     if (part != 1) {
         // the angle of pair i is the same for every head: one table per block
@@ -279,7 +377,7 @@ rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d
         const int first = part == 0 ? 0 : (part - 2) * ROPE_ITEMS;
         const int n_items = part == 0 ? n_kv * hv : min(n_q * hv - first, ROPE_ITEMS);
         const float *src = part == 0 ? r + (size_t)n_q * d : r;
-        float *dst = part == 0 ? (I8 ? row_sm : reinterpret_cast<float *>(kc) + slot * kv_n) : r;
+        float *dst = part == 0 ? (I8 ? row_sm : reinterpret_cast<float *>(kc) + slot * kv_n) : q_out + (size_t)row * q_out_stride;
         for (int i0 = threadIdx.x; i0 < n_items; i0 += 4 * ROPE_THREADS) {
             VT x0[4], x1[4];
 #pragma unroll
@@ -287,8 +385,8 @@ rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d
                 const int idx = i0 + u * ROPE_THREADS + first;
                 if (i0 + u * ROPE_THREADS < n_items) {
                     const float *v = src + (size_t)(idx / hv) * d + (idx % hv) * V;
-                    x0[u] = *reinterpret_cast<const VT *>(v);
-                    x1[u] = *reinterpret_cast<const VT *>(v + half);
+                    x0[u] = load(v);
+                    x1[u] = load(v + half);
                 }
             }
 #pragma unroll
@@ -318,7 +416,7 @@ rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d
     if constexpr (I8) {
         if (part == 1)
             for (int i = threadIdx.x * V; i < kv_n; i += blockDim.x * V)
-                *reinterpret_cast<VT *>(row_sm + i) = *reinterpret_cast<const VT *>(vsrc + i);
+                *reinterpret_cast<VT *>(row_sm + i) = load(vsrc + i);
         __syncthreads();
         float amax = 0.0f;
         for (int i = threadIdx.x; i < kv_n; i += blockDim.x) amax = fmaxf(amax, fabsf(row_sm[i]));
@@ -343,7 +441,7 @@ rope_kv_append_kernel(float *__restrict__ qkv, int seq, int n_q, int n_kv, int d
     } else if (part == 1) {
         float *vdst = reinterpret_cast<float *>(vc) + slot * kv_n;
         for (int i = threadIdx.x * V; i < kv_n; i += blockDim.x * V)
-            *reinterpret_cast<VT *>(vdst + i) = *reinterpret_cast<const VT *>(vsrc + i);
+            *reinterpret_cast<VT *>(vdst + i) = load(vsrc + i);
     }
 }
 
@@ -886,14 +984,19 @@ gqa_decode_split_tc_kernel(const float *__restrict__ q, int q_stride, int n_q, i
 // 128, 2049 keys in 2178: 62.4 us both kernels, with eight and sixteen 65.2), eight and sixteen behind the int8
 // kernels, which leave it half the time (32 sequences, 32 / 4 heads of 64, 200 keys in 330: 8.0 us, the other way 12.2).
 constexpr int COMBINE_BATCH = 128;
-template <int CH, int PRE, int BLOCKS>
+// The row goes out in the form of the matmul behind it; rows past those of `o` are its padding.
+template <int CH, int PRE, int BLOCKS, int FORM>
 __global__ void __launch_bounds__(128, BLOCKS)
 attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, int max_seq, const int32_t *__restrict__ pos,
-                         int want, float *__restrict__ out) {
+                         int want, ActOut o) {
     pdl_wait();
     pdl_trigger();
     __shared__ float red[4], wt[COMBINE_BATCH];
     const int tid = threadIdx.x;
+    if (FORM == ACT_DIGITS && (int)blockIdx.y >= o.rows) {
+        if (tid < 32) store_act_padding(o, blockIdx.y, blockIdx.x * d + (tid * 8 < d ? tid * 8 : 0), tid * 8 < d);
+        return;
+    }
     const size_t hb = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
     const float *p = part + hb * n_splits * (d + 2);
     // what the first splits left is fetched while the position, which says how many count, is on its way
@@ -932,7 +1035,19 @@ attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, in
     }
     L = block_sum(L, red);
     const float inv = L > 0.0f ? 1.0f / L : 0.0f;
-    if (tid < d) out[hb * d + tid] = acc * inv;
+    if constexpr (FORM == ACT_F32) {
+        if (tid < d) static_cast<float *>(o.ptr)[hb * d + tid] = acc * inv;
+    } else {
+        __shared__ __align__(16) float row[128];
+        row[tid] = acc * inv;
+        __syncthreads();
+        if (tid < 32) {
+            float v[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v[t] = row[tid * 8 < d ? tid * 8 + t : 0];
+            store_act<FORM>(o, v, blockIdx.y, blockIdx.x * d + tid * 8, tid * 8 < d);
+        }
+    }
 }
 
 // out[m][n] = sum_k x[m][k] * w[n][k] for m <= MT: one warp per R weight rows, which share the x rows it reads.
@@ -1198,10 +1313,36 @@ int yscv_cuda_embedding_dev(yscv_cuda_ctx *ctx, const float *d_weight, size_t vo
 
 }  // extern "C"
 
+namespace yscv {
+// hidden % 8 == 0 and at most 8192, operands (and `pitch` floats) 16-byte aligned
+int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
+              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out) {
+    const bool prompt = rows > 512 && (out.form == ACT_F32 || out.form == ACT_BF16);
+    const unsigned threads = hidden <= 2048 ? (prompt ? 128u : 256u) : (prompt ? 256u : 1024u);
+    auto pick = [&](auto form) {
+        constexpr int F = decltype(form)::value;
+        if constexpr (F == ACT_F32 || F == ACT_BF16)
+            if (prompt) return hidden <= 2048 ? norm_form_kernel<F, 256, 2> : norm_form_kernel<F, 1024, 4>;
+        return hidden <= 2048 ? norm_form_kernel<F, 256, 1> : norm_form_kernel<F, 1024, 1>;
+    };
+    auto kern = out.form == ACT_BF16     ? pick(std::integral_constant<int, ACT_BF16>())
+                : out.form == ACT_DIGITS ? pick(std::integral_constant<int, ACT_DIGITS>())
+                : out.form == ACT_TERMS  ? pick(std::integral_constant<int, ACT_TERMS>())
+                                         : pick(std::integral_constant<int, ACT_F32>());
+    YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)out.slots()), dim3(threads), 0, ctx->stream, x, delta, parts, pitch, gamma, eps, (int)hidden,
+                             row0, row_step, x_out, out));
+    DEC_EPILOGUE(ctx, out.form == ACT_F32 ? "add_rms_norm" : "add_rms_norm(bf16 activations out)");
+}
+}  // namespace yscv
+
 template <bool ACT>
 static int add_rms_norm_impl(yscv_cuda_ctx *ctx, const float *x, const float *delta, const float *gamma, float eps,
                              size_t rows, size_t hidden, float *x_out, void *normed) {
     if (rows == 0) return YSCV_CUDA_OK;
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(gamma) |
+                           reinterpret_cast<uintptr_t>(x_out) | reinterpret_cast<uintptr_t>(normed);
+    if (hidden % 8 == 0 && hidden <= 8192 && (ptrs & 15) == 0)
+        return norm_form(ctx, x, delta, 1, 0, gamma, eps, rows, 0, 1, hidden, x_out, act_out(ACT ? ACT_BF16 : ACT_F32, rows, hidden, normed));
     // eight elements per thread: 256 threads are enough up to 2048, 1024 up to 8192; sixteen up to 16384
     const unsigned threads = hidden <= 2048 ? 256u : 1024u;
     auto kern = hidden <= 8192 ? add_rms_norm_kernel<ACT, 8> : hidden <= 16384 ? add_rms_norm_kernel<ACT, 16> : add_rms_norm_long_kernel<ACT>;
@@ -1221,6 +1362,30 @@ int yscv_cuda_add_rms_norm_dev(yscv_cuda_ctx *ctx, const float *d_x, const float
 
 }  // extern "C"
 
+namespace yscv {
+template <typename KV>
+int rope_append_form(yscv_cuda_ctx *ctx, const float *qkv, int parts, size_t pitch, float *q_out, size_t q_out_stride, size_t batch,
+                     size_t seq, size_t n_q, size_t n_kv, size_t d_head, float theta, const int32_t *d_pos, KV *kcache, KV *vcache,
+                     float *kscale, float *vscale, size_t max_seq) {
+    const size_t smem = (d_head + (sizeof(KV) == 1 ? n_kv * d_head : 0)) * sizeof(float);
+    if (smem > 48 * 1024)
+        return fail(YSCV_CUDA_ERR_UNSUPPORTED, "RoPE tables for d_head=%zu, n_kv=%zu do not fit shared memory", d_head, n_kv);
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kcache) |
+                           reinterpret_cast<uintptr_t>(vcache);
+    const bool vec = d_head % 8 == 0 && (ptrs & 15) == 0 && pitch % 4 == 0 && q_out_stride % 4 == 0;
+    const size_t q_items = n_q * (d_head / 2) / (vec ? 4 : 1);
+    const dim3 grid((unsigned)(batch * seq), (unsigned)(2 + (q_items + ROPE_ITEMS - 1) / ROPE_ITEMS));
+    auto kern = vec ? rope_kv_append_kernel<KV, 4> : rope_kv_append_kernel<KV, 1>;
+    YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(ROPE_THREADS), smem, ctx->stream, qkv, parts, pitch, q_out, (int)q_out_stride, (int)seq,
+                             (int)n_q, (int)n_kv, (int)d_head, theta, d_pos, kcache, vcache, kscale, vscale, (int)max_seq, ctx->d_status));
+    DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "rope_kv_append(int8 cache)" : "rope_kv_append");
+}
+template int rope_append_form<float>(yscv_cuda_ctx *, const float *, int, size_t, float *, size_t, size_t, size_t, size_t, size_t, size_t,
+                                     float, const int32_t *, float *, float *, float *, float *, size_t);
+template int rope_append_form<int8_t>(yscv_cuda_ctx *, const float *, int, size_t, float *, size_t, size_t, size_t, size_t, size_t, size_t,
+                                      float, const int32_t *, int8_t *, int8_t *, float *, float *, size_t);
+}  // namespace yscv
+
 template <typename KV>
 static int rope_kv_append_impl(yscv_cuda_ctx *ctx, float *d_qkv, size_t batch, size_t seq, size_t n_q,
                                size_t n_kv, size_t d_head, float theta, const int32_t *d_pos,
@@ -1232,25 +1397,9 @@ static int rope_kv_append_impl(yscv_cuda_ctx *ctx, float *d_qkv, size_t batch, s
     if (d_head == 0 || d_head % 2 != 0) return fail(YSCV_CUDA_ERR_BAD_ARG, "d_head must be even for RoPE");
     if (n_kv == 0 || max_seq == 0) return fail(YSCV_CUDA_ERR_BAD_ARG, "n_kv and max_seq must be positive");
     if (batch * seq == 0) return YSCV_CUDA_OK;
-    const size_t smem = (d_head + (sizeof(KV) == 1 ? n_kv * d_head : 0)) * sizeof(float);
-    if (smem > 48 * 1024)
-        return fail(YSCV_CUDA_ERR_UNSUPPORTED, "RoPE tables for d_head=%zu, n_kv=%zu do not fit shared memory", d_head, n_kv);
-    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(d_qkv) | reinterpret_cast<uintptr_t>(d_kcache) | reinterpret_cast<uintptr_t>(d_vcache);
-    const bool vec = d_head % 8 == 0 && (ptrs & 15) == 0;
-    const size_t q_items = n_q * (d_head / 2) / (vec ? 4 : 1);
-    const dim3 grid((unsigned)(batch * seq), (unsigned)(2 + (q_items + ROPE_ITEMS - 1) / ROPE_ITEMS));
-    auto kern = vec ? rope_kv_append_kernel<KV, 4> : rope_kv_append_kernel<KV, 1>;
-    YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(ROPE_THREADS), smem, ctx->stream, d_qkv, (int)seq, (int)n_q,
-                             (int)n_kv, (int)d_head, theta, d_pos, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq,
-                             ctx->d_status));
-    DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "rope_kv_append(int8 cache)" : "rope_kv_append");
+    return rope_append_form(ctx, d_qkv, 1, 0, d_qkv, (n_q + 2 * n_kv) * d_head, batch, seq, n_q, n_kv, d_head, theta, d_pos, d_kcache, d_vcache,
+                            d_kscale, d_vscale, max_seq);
 }
-
-template <typename KV>
-static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch,
-                              size_t seq_q, size_t n_q, size_t n_kv, size_t d_head, const KV *d_kcache,
-                              const KV *d_vcache, const float *d_kscale, const float *d_vscale,
-                              size_t max_seq, const int32_t *d_pos, int causal, float *d_out);
 
 extern "C" {
 
@@ -1271,17 +1420,30 @@ int yscv_cuda_rope_kv_append_i8_dev(yscv_cuda_ctx *ctx, float *d_qkv, size_t bat
 
 }  // extern "C"
 
+namespace yscv {
+static bool decode_attention(size_t seq_q, int causal, size_t max_seq) { return seq_q == 1 && causal && max_seq > 128; }
+bool gqa_attention_writes(int form, size_t seq_q, size_t d_head, size_t max_seq) {
+    return (form == ACT_BF16 || (form == ACT_DIGITS && d_head % 32 == 0)) && decode_attention(seq_q, 1, max_seq);
+}
+
+// Merge of the splits, in the form of `out`
+template <int CH, int PRE, int BLOCKS>
+static int launch_combine(yscv_cuda_ctx *ctx, const float *part, int n_splits, size_t n_q, size_t d_head, size_t max_seq, const int32_t *d_pos,
+                          int want, const ActOut &out) {
+    auto kern = out.form == ACT_BF16     ? attention_combine_kernel<CH, PRE, BLOCKS, ACT_BF16>
+                : out.form == ACT_DIGITS ? attention_combine_kernel<CH, PRE, BLOCKS, ACT_DIGITS>
+                                         : attention_combine_kernel<CH, PRE, BLOCKS, ACT_F32>;
+    YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)n_q, (unsigned)out.slots()), dim3(128), 0, ctx->stream, part, n_splits, (int)d_head, (int)max_seq,
+                             d_pos, want, out));
+    return YSCV_CUDA_OK;
+}
+
 template <typename KV>
-static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch,
-                              size_t seq_q, size_t n_q, size_t n_kv, size_t d_head, const KV *d_kcache,
-                              const KV *d_vcache, const float *d_kscale, const float *d_vscale,
-                              size_t max_seq, const int32_t *d_pos, int causal, float *d_out) {
-    DEC_PROLOGUE(ctx);
-    if (!d_q || !d_kcache || !d_vcache || !d_pos || !d_out) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
-    if (sizeof(KV) == 1 && (!d_kscale || !d_vscale)) return fail(YSCV_CUDA_ERR_BAD_ARG, "null scale table");
-    if (n_kv == 0 || n_q % n_kv != 0) return fail(YSCV_CUDA_ERR_BAD_ARG, "n_q must be a multiple of n_kv");
-    if (batch * seq_q == 0) return YSCV_CUDA_OK;
-    if (seq_q == 1 && causal && max_seq > 128) {
+int gqa_attention_form(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q, size_t n_kv,
+                       size_t d_head, const KV *d_kcache, const KV *d_vcache, const float *d_kscale, const float *d_vscale,
+                       size_t max_seq, const int32_t *d_pos, int causal, const ActOut &out) {
+    float *d_out = static_cast<float *>(out.ptr);   // (ACT_F32 everywhere but behind the merge)
+    if (decode_attention(seq_q, causal, max_seq)) {
         // decode over a long cache: split the keys across blocks, then merge
         if (d_head % 16 != 0 || d_head > 128)
             return fail(YSCV_CUDA_ERR_UNSUPPORTED, "d_head %zu not supported by the decode attention", d_head);
@@ -1308,8 +1470,7 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                                          d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
                 YSCV_CUDA_TRY(cudaGetLastError());
                 ctx->launches++;
-                YSCV_CUDA_TRY(launch_pdl(attention_combine_kernel<128, 8, 16>, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part,
-                                         n_splits, (int)d_head, (int)max_seq, d_pos, want, d_out));
+                if ((rc = launch_combine<128, 8, 16>(ctx, part, n_splits, n_q, d_head, max_seq, d_pos, want, out))) return rc;
                 DEC_EPILOGUE(ctx, "gqa_attention(split-k,int8 cache,mma)");
             }
         }
@@ -1326,11 +1487,10 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                                  (int)d_head, d_kcache, d_vcache, d_kscale, d_vscale, (int)max_seq, d_pos, want, part));
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
-        auto merge = sizeof(KV) == 1 ? attention_combine_kernel<128, 8, 16>
-                     : chunk == 64   ? attention_combine_kernel<64, 16, 10>
-                                     : attention_combine_kernel<128, 16, 10>;
-        YSCV_CUDA_TRY(launch_pdl(merge, dim3((unsigned)n_q, (unsigned)batch), dim3(128), 0, ctx->stream, part, n_splits,
-                                 (int)d_head, (int)max_seq, d_pos, want, d_out));
+        rc = sizeof(KV) == 1 ? launch_combine<128, 8, 16>(ctx, part, n_splits, n_q, d_head, max_seq, d_pos, want, out)
+             : chunk == 64   ? launch_combine<64, 16, 10>(ctx, part, n_splits, n_q, d_head, max_seq, d_pos, want, out)
+                             : launch_combine<128, 16, 10>(ctx, part, n_splits, n_q, d_head, max_seq, d_pos, want, out);
+        if (rc) return rc;
         DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(split-k,int8 cache)" : "gqa_attention(split-k)");
     }
     // a prompt pass: tiles of 128 (position, head) pairs on the tensor cores
@@ -1355,6 +1515,25 @@ static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_str
                              d_pos, causal, d_out));
     DEC_EPILOGUE(ctx, sizeof(KV) == 1 ? "gqa_attention(int8 cache)" : "gqa_attention");
 }
+template int gqa_attention_form<float>(yscv_cuda_ctx *, const float *, size_t, size_t, size_t, size_t, size_t, size_t, const float *,
+                                       const float *, const float *, const float *, size_t, const int32_t *, int, const ActOut &);
+template int gqa_attention_form<int8_t>(yscv_cuda_ctx *, const float *, size_t, size_t, size_t, size_t, size_t, size_t, const int8_t *,
+                                        const int8_t *, const float *, const float *, size_t, const int32_t *, int, const ActOut &);
+}  // namespace yscv
+
+template <typename KV>
+static int gqa_attention_impl(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch,
+                              size_t seq_q, size_t n_q, size_t n_kv, size_t d_head, const KV *d_kcache,
+                              const KV *d_vcache, const float *d_kscale, const float *d_vscale,
+                              size_t max_seq, const int32_t *d_pos, int causal, float *d_out) {
+    DEC_PROLOGUE(ctx);
+    if (!d_q || !d_kcache || !d_vcache || !d_pos || !d_out) return fail(YSCV_CUDA_ERR_BAD_ARG, "null operand");
+    if (sizeof(KV) == 1 && (!d_kscale || !d_vscale)) return fail(YSCV_CUDA_ERR_BAD_ARG, "null scale table");
+    if (n_kv == 0 || n_q % n_kv != 0) return fail(YSCV_CUDA_ERR_BAD_ARG, "n_q must be a multiple of n_kv");
+    if (batch * seq_q == 0) return YSCV_CUDA_OK;
+    return gqa_attention_form(ctx, d_q, q_stride, batch, seq_q, n_q, n_kv, d_head, d_kcache, d_vcache, d_kscale, d_vscale, max_seq, d_pos,
+                              causal, act_out(ACT_F32, batch * seq_q, n_q * d_head, d_out));
+}
 
 extern "C" {
 
@@ -1377,12 +1556,25 @@ int yscv_cuda_gqa_attention_i8_dev(yscv_cuda_ctx *ctx, const float *d_q, size_t 
 
 }  // extern "C"
 
+namespace yscv {
+// inter % 8 == 0, operands (and `pitch` floats) 16-byte aligned
+int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out) {
+    const size_t visit = out.slots();
+    const dim3 grid((unsigned)((inter / 8 + 255) / 256), (unsigned)(visit < 32768 ? visit : 32768));
+    auto kern = out.form == ACT_BF16     ? swiglu_form_kernel<ACT_BF16>
+                : out.form == ACT_DIGITS ? swiglu_form_kernel<ACT_DIGITS>
+                : out.form == ACT_TERMS  ? swiglu_form_kernel<ACT_TERMS>
+                                         : swiglu_form_kernel<ACT_F32>;
+    YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(256), 0, ctx->stream, gate_up, parts, pitch, (int)visit, (int)inter, out));
+    DEC_EPILOGUE(ctx, out.form == ACT_F32 ? "swiglu" : "swiglu(bf16 activations out)");
+}
+}  // namespace yscv
+
 template <bool ACT>
 static int swiglu_impl(yscv_cuda_ctx *ctx, const float *gate_up, size_t rows, size_t inter, void *out) {
     if (rows * inter == 0) return YSCV_CUDA_OK;
     if (inter % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-        const dim3 grid((unsigned)((inter / 8 + 255) / 256), (unsigned)(rows < 32768 ? rows : 32768));
-        YSCV_CUDA_TRY(launch_pdl(swiglu_kernel<ACT>, grid, dim3(256), 0, ctx->stream, gate_up, out, (int)rows, (int)inter));
+        return swiglu_form(ctx, gate_up, 1, 0, rows, inter, act_out(ACT ? ACT_BF16 : ACT_F32, rows, inter, out));
     } else {
         const size_t total = rows * (inter / (ACT ? 8 : 1));
         const unsigned blocks = (unsigned)((total + 255) / 256 < 65535 ? (total + 255) / 256 : 65535);

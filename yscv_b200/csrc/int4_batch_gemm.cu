@@ -39,9 +39,6 @@
 // roles costs about 330 cycles of barrier traffic whatever it carries and an MMA here 40 to 60, so a
 // slot (one hand-over) is 128 rows x 128 k and the two halves have an issuer each: with 64-k slots and
 // one issuer 57344 x 8192 at 64 rows took 126 us, without any work in the roles still 72.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include "common.cuh"
 #include "kernels.cuh"
 #include "tma.cuh"
@@ -508,9 +505,7 @@ bg_join_kernel(BGParams p, int NA, int grid, float *__restrict__ out) {
     }
 }
 
-// fp32 activations -> fp16 terms [hi: 16 rows][k], [lo: 16 rows][k] (k order of every group of 8:
-// 0,4,1,5,2,6,3,7, the order in which the nibbles of a weight word come out) and the inverse block
-// scales [256-k block][16]. A warp takes one row and 256 k.
+// fp32 activations -> the exact form's fp16 terms (store_terms). A warp takes one row and 256 k.
 __global__ void __launch_bounds__(128)
 act_split16_kernel(const float *__restrict__ act, int M, int K, int kb, __half *__restrict__ terms, float *__restrict__ inv) {
     pdl_wait();
@@ -524,48 +519,32 @@ act_split16_kernel(const float *__restrict__ act, int M, int K, int kb, __half *
         a = __ldg(src);
         b = __ldg(src + 1);
     }
-    float v[8] = {a.x, b.x, a.y, b.y, a.z, b.z, a.w, b.w};
-    float mx = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    // power of two that brings the block's maximum into [2^13, 2^14) (2^126 at most), and its inverse. A block with
-    // an infinity keeps its scale of 1 and its infinities, whose remainder is 0 (not inf - inf); what else it holds
-    // only has to stay finite, since the row's sums no longer are.
-    const uint32_t e = (__float_as_uint(mx) >> 23) & 255u;
-    const bool inf = e == 255u;
-    const uint32_t s = inf ? 127u : min(267u - e, 253u);
-    const float up = __uint_as_float(s << 23);
-    if (inf) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (fabsf(v[i]) < INFINITY) v[i] = fminf(fmaxf(v[i], -65504.0f), 65504.0f);
-    }
-    uint4 hi, lo;
-    uint32_t *h = &hi.x, *l = &lo.x;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float x = v[2 * i] * up, y = v[2 * i + 1] * up;
-        const __half2 hh = __floats2half2_rn(x, y);
-        const float2 f = __half22float2(hh);
-        const __half2 ll = __floats2half2_rn(inf && f.x == x ? 0.0f : x - f.x, inf && f.y == y ? 0.0f : y - f.y);
-        h[i] = *reinterpret_cast<const uint32_t *>(&hh);
-        l[i] = *reinterpret_cast<const uint32_t *>(&ll);
-    }
-    if (k < K) {
-        *reinterpret_cast<uint4 *>(terms + (size_t)m * K + k) = hi;
-        *reinterpret_cast<uint4 *>(terms + (size_t)(16 + m) * K + k) = lo;
-    }
-    if (lane == 0) inv[u * 16 + m] = __uint_as_float((254u - s) << 23);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    store_terms(v, terms, inv, K, m, k, k < K);
 }
 
 // 39 MB, whatever the shape. Where it cannot be had (a first call inside a capture, no memory) the call takes the
 // kernel that it took before there was this one.
-bool int4_batch_ready(yscv_cuda_ctx *ctx) {
-    return ctx->batch_ws.try_reserve((size_t)ctx->sm_count * 2 * 2 * 128 * 128 * sizeof(float), ctx->stream);
+static size_t bg_ws_bytes(const yscv_cuda_ctx *ctx) { return (size_t)ctx->sm_count * 2 * 2 * 128 * 128 * sizeof(float); }
+bool int4_batch_ready(yscv_cuda_ctx *ctx) { return ctx->batch_ws.try_reserve(bg_ws_bytes(ctx), ctx->stream); }
+static size_t bg_inv_offset(size_t k) { return (32 * k * 2 + 255) / 256 * 256; }   // of the inverse scales behind the terms
+size_t int4_batch_exact_scratch_bytes(size_t k) { return bg_inv_offset(k) + (k + BG_UNIT - 1) / BG_UNIT * 64 + 256; }
+
+size_t act_bytes(int form, size_t m, size_t k) {
+    if (form == ACT_DIGITS) return int4_gemv_scratch_bytes(m, k);
+    if (form == ACT_TERMS) return int4_batch_exact_scratch_bytes(k);
+    return m * k * (form == ACT_BF16 ? 2 : 4);
 }
-size_t int4_batch_exact_scratch_bytes(size_t k) { return 32 * k * 2 + (k + BG_UNIT - 1) / BG_UNIT * 64 + 512; }
+ActOut act_out(int form, size_t m, size_t k, void *buffer) {
+    ActOut o;
+    o.form = form;
+    o.rows = (int)m;
+    o.k = (int)k;
+    o.ptr = buffer;
+    if (form == ACT_DIGITS) o.q = int4_gemv_layout(m, k);
+    if (form == ACT_TERMS) o.inv = reinterpret_cast<float *>(static_cast<unsigned char *>(buffer) + bg_inv_offset(k));
+    return o;
+}
 
 // k % 128: the scale rows (k / 32 floats) are TMA rows, whose pitch must be a multiple of 16 bytes.
 static bool bg_shape(size_t n, size_t k, size_t gs) {
@@ -633,8 +612,9 @@ static int launch_batch(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, const CUten
 // K slices of the sliced form, or 0 for equal ranges over the CTAs, by the modelled time in us: units one after another
 // in a CTA, a round's drain, the launch that adds slices and their traffic; equal ranges cost a second drain and the
 // join. The constants are a fit to 24 shapes from 512 x 2048 to 8192 x 28672 at 20 / 32 / 64 / 128 rows with every
-// choice forced in turn; its choice is 0.15 % behind the best of them on average and 3 % at worst.
-static int bg_split(const BGParams &p, int NA, int grid, int sms, bool slices_ok, size_t ws_bytes) {
+// choice forced in turn; its choice is 0.15 % behind the best of them on average and 3 % at worst. left_apart: the
+// caller's next kernel adds the slices, which costs it their reads.
+static int bg_split(const BGParams &p, int NA, int grid, int sms, bool slices_ok, size_t ws_bytes, bool left_apart) {
     const double unit = 0.64 + 0.002 * p.BT, mb = 0.07e-6;
     double best = 3.2 + (p.units + grid - 1) / grid * unit * (NA == 2 ? 1.75 : 1.0) + 2.0 * grid * NA * 128 * p.BT * 4 * mb;
     int slices = 0;
@@ -643,17 +623,17 @@ static int bg_split(const BGParams &p, int NA, int grid, int sms, bool slices_ok
         const double bytes = (double)s * p.M * p.N * 4;
         if (s > 1 && (!slices_ok || bytes > (double)ws_bytes)) break;
         const double rounds = (int)(((long long)tiles * s + sms - 1) / sms);
-        const double cost = rounds * ((p.kb + s - 1) / s * unit + 0.55) + (s > 1 ? 0.97 + 0.022 * s + bytes * mb : 0.0);
+        const double cost = rounds * ((p.kb + s - 1) / s * unit + 0.55) + (s == 1 ? 0.0 : left_apart ? 0.1 * s + bytes * mb / 2 : 0.97 + 0.022 * s + bytes * mb);
         if (cost < best) { best = cost; slices = s; }
     }
     return slices;
 }
 
-// exact: act = fp32 rows, scratch of int4_batch_exact_scratch_bytes(k). Otherwise act_bf16 = bf16 rows
-// in the permuted k order.
-int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act, const void *act_bf16, float *out,
-                    size_t m, size_t n, size_t k, void *scratch) {
-    const bool exact = act_bf16 == nullptr;
+struct BGPlan {
+    BGParams p;
+    int NA, grid;
+};
+static BGPlan bg_plan(yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k, bool exact, bool slices_ok, bool left_apart) {
     BGParams p = {};
     p.M = (int)m;
     p.N = (int)n;
@@ -673,7 +653,37 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
     int grid = p.units < sms ? p.units : sms;
     if (grid > tiles * 4) grid = tiles * 4;
     p.acc_bufs = NA * p.BT > 128 ? 1 : 2;
-    p.slices = exact ? 0 : bg_split(p, NA, grid, sms, (m * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0, ctx->batch_ws.bytes);
+    if (!exact) p.slices = bg_split(p, NA, grid, sms, slices_ok, bg_ws_bytes(ctx), left_apart);
+    if (p.slices > 0) {
+        p.tiles = tiles1;
+        p.units = tiles1 * p.kb;
+        p.acc_bufs = 2;
+        const int items = tiles1 * p.slices;
+        return {p, 1, items < sms ? items : sms};
+    }
+    return {p, NA, grid};
+}
+int int4_batch_parts(yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) {
+    const int s = bg_plan(ctx, m, n, k, false, true, true).p.slices;
+    return s > 1 ? s : 1;
+}
+
+// exact: act = fp32 rows (null: terms and inverse scales are in `scratch`), scratch of int4_batch_exact_scratch_bytes(k).
+// Otherwise act_bf16 = bf16 rows in the permuted k order.
+int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act, const void *act_bf16, float *out,
+                    size_t m, size_t n, size_t k, void *scratch, int *parts) {
+    const bool exact = act_bf16 == nullptr;
+    // (add_kslices reads 16 bytes at a time)
+    const bool join_ok = (m * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    bool left_apart = parts && *parts > 1;
+    BGPlan plan = bg_plan(ctx, m, n, k, exact, left_apart || join_ok, left_apart);
+    if (left_apart && plan.p.slices > *parts) {
+        left_apart = false;
+        plan = bg_plan(ctx, m, n, k, exact, join_ok, false);
+    }
+    BGParams p = plan.p;
+    const int NA = plan.NA, grid = plan.grid;
+    if (parts) *parts = left_apart && p.slices > 1 ? p.slices : 1;
 
     CUtensorMap tm_w, tm_s, tm_a;
     int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -682,11 +692,13 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
     if (rc) return rc;
     if (exact) {
         __half *terms = reinterpret_cast<__half *>(scratch);
-        float *inv = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + ((32 * k * 2 + 255) / 256) * 256);
+        float *inv = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + bg_inv_offset(k));
         p.inv = inv;
-        const unsigned blocks = (unsigned)((m * p.kb + 3) / 4);
-        YSCV_CUDA_TRY(launch_pdl(act_split16_kernel, dim3(blocks), dim3(128), 0, ctx->stream, act, p.M, p.K, p.kb, terms, inv));
-        ctx->launches++;
+        if (act) {
+            const unsigned blocks = (unsigned)((m * p.kb + 3) / 4);
+            YSCV_CUDA_TRY(launch_pdl(act_split16_kernel, dim3(blocks), dim3(128), 0, ctx->stream, act, p.M, p.K, p.kb, terms, inv));
+            ctx->launches++;
+        }
         rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, terms, 32, k, k * 2, 32, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
         return launch_batch<2, true, false>(ctx, tm_w, tm_s, tm_a, out, p, grid);
@@ -694,12 +706,9 @@ int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, 
     rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, act_bf16, m, k, k * 2, (uint32_t)p.BT, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     if (p.slices > 0) {
-        p.tiles = tiles1;
-        p.units = tiles1 * p.kb;
-        p.acc_bufs = 2;
-        const int items = tiles1 * p.slices;
-        rc = launch_batch<1, false, true>(ctx, tm_w, tm_s, tm_a, p.slices > 1 ? p.ws : out, p, items < sms ? items : sms);
-        return rc || p.slices == 1 ? rc : add_kslices(ctx, p.ws, out, m * n, p.slices);
+        const bool join = p.slices > 1 && !left_apart;
+        rc = launch_batch<1, false, true>(ctx, tm_w, tm_s, tm_a, join ? p.ws : out, p, grid);
+        return rc || !join ? rc : add_kslices(ctx, p.ws, out, m * n, p.slices);
     }
     return NA == 2 ? launch_batch<2, false, false>(ctx, tm_w, tm_s, tm_a, out, p, grid) : launch_batch<1, false, false>(ctx, tm_w, tm_s, tm_a, out, p, grid);
 }

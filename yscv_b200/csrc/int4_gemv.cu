@@ -557,6 +557,7 @@ static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scale
     return YSCV_CUDA_OK;
 }
 
+// act == nullptr: the digit planes are in `scratch`
 template <int MP, int GS>
 static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
                           const float *act, float *out, int M, int N, int K, void *scratch) {
@@ -564,17 +565,19 @@ static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *sc
     const int rows_per_cta = (N + ctx->sm_count - 1) / ctx->sm_count;
     const bool small = rows_per_cta <= 32;
     if constexpr (MP <= 4) {
-        if (fused_quant(MP, GS, K)) {
+        if (act && fused_quant(MP, GS, K)) {
             ctx->last_kernel = "int4_gemv_fast(imma,tma,fused-quant)";
             return small ? launch_fast<MP, GS, 2, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q)
                          : launch_fast<MP, GS, 8, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q);
         }
     }
     unsigned char *blobs = reinterpret_cast<unsigned char *>(scratch);
-    const int items = (K / 32) * quant_slots(q);
-    YSCV_CUDA_TRY(launch_pdl(act_quant_kernel, dim3((items * 4 + 127) / 128), dim3(128), 0, ctx->stream, act, blobs, M, K, q));
-    YSCV_CUDA_TRY(cudaGetLastError());
-    ctx->launches++;
+    if (act) {
+        const int items = (K / 32) * quant_slots(q);
+        YSCV_CUDA_TRY(launch_pdl(act_quant_kernel, dim3((items * 4 + 127) / 128), dim3(128), 0, ctx->stream, act, blobs, M, K, q));
+        YSCV_CUDA_TRY(cudaGetLastError());
+        ctx->launches++;
+    }
     ctx->last_kernel = "int4_gemv_fast(imma,tma)";
     return small ? launch_fast<MP, GS, 2, false>(ctx, wq, scales, blobs, act, out, M, N, K, q)
                  : launch_fast<MP, GS, 8, false>(ctx, wq, scales, blobs, act, out, M, N, K, q);
@@ -595,6 +598,14 @@ int int4_gemv_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, c
         case 8: return launch_fast_tp<8, 8>(ctx, wq, scales, act, out, M, N, K, scratch);
         default: return launch_fast_tp<16, 8>(ctx, wq, scales, act, out, M, N, K, scratch);
     }
+}
+
+QuantLayout int4_gemv_layout(size_t m, size_t k) {
+    const int mp = padded_m((int)m);
+    return quant_layout(mp, stage_groups(mp, (int)k));
+}
+int int4_gemv_digits(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const void *digits, float *out, size_t m, size_t n, size_t k) {
+    return int4_gemv_fast(ctx, wq, scales, nullptr, out, m, n, k, const_cast<void *>(digits));
 }
 
 // ---------------------------------------------------------------------------

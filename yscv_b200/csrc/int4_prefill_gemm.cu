@@ -854,7 +854,7 @@ static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, con
 // act_bf16 != nullptr: the activations are already bf16 in the GEMM's k order (what the pre-pass
 // below writes; the decoder's norm and SwiGLU kernels can emit it): `act` and `scratch` are not used.
 int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
-                      float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16) {
+                      float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16, int *parts) {
     PGParams p = {};
     int rc_ws = 0;
     p.M = (int)m;
@@ -927,7 +927,8 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
         abf = mine;
     }
 
-    if (batch) return int4_batch_gemm(ctx, wq, scales, nullptr, abf, out, m, n, k, nullptr);
+    if (batch) return int4_batch_gemm(ctx, wq, scales, nullptr, abf, out, m, n, k, nullptr, parts);
+    if (parts) *parts = 1;
 
     CUtensorMap tm_w, tm_a;
     int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, (uint32_t)(NA * PG_BM), 32,

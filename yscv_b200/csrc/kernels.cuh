@@ -3,8 +3,11 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "act_forms.cuh"
+
 struct yscv_cuda_ctx;
 struct yscv_cuda_i8b;
+struct yscv_cuda_int4_weight;
 
 namespace yscv {
 
@@ -20,6 +23,9 @@ int f32_gemm_tc(yscv_cuda_ctx *ctx, const float *d_w, const float *d_x, size_t m
                 float *d_out, void *scratch);
 int int4_gemv_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
                    float *out, size_t m, size_t n, size_t k, void *scratch);
+// the same with digit planes that the caller wrote (ActForm ACT_DIGITS, act_out())
+int int4_gemv_digits(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const void *digits, float *out, size_t m, size_t n, size_t k);
+QuantLayout int4_gemv_layout(size_t m, size_t k);
 int int4_gemv_generic(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
                       const float *act, float *out, size_t m, size_t n, size_t k, size_t gs);
 
@@ -27,7 +33,7 @@ int int4_gemv_generic(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
 bool int4_prefill_supported(size_t m, size_t n, size_t k, size_t gs);
 size_t int4_prefill_scratch_bytes(size_t m, size_t k);
 int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
-                      float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16 = nullptr);
+                      float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16 = nullptr, int *parts = nullptr);
 
 int add_kslices(yscv_cuda_ctx *ctx, const float *parts, float *out, size_t elements, int slices);
 
@@ -38,8 +44,34 @@ size_t int4_batch_exact_scratch_bytes(size_t k);
 bool int4_batch_bf16_wins(size_t m, size_t n, size_t k, size_t gs);
 bool int4_batch_exact_wins(size_t m, size_t n, size_t k, size_t gs);
 bool int4_batch_ready(yscv_cuda_ctx *ctx);   // its workspace is there, or could be allocated now
+// With *parts > 1 (bf16 form; int4_batch_parts() says how many are wanted) `out` has room for so many partial sums
+// [part][m][n], whose sum in that order is the result; *parts then says how many there are. act == nullptr: `scratch` holds the exact form's terms already.
 int int4_batch_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act, const void *act_bf16, float *out,
-                    size_t m, size_t n, size_t k, void *scratch);
+                    size_t m, size_t n, size_t k, void *scratch, int *parts = nullptr);
+int int4_batch_parts(yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k);
+
+// A matmul's activations in the form it takes them best, written by the operator in front of it (act_forms.cuh).
+int int4_act_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, size_t m);
+size_t act_bytes(int form, size_t m, size_t k);
+ActOut act_out(int form, size_t m, size_t k, void *buffer);
+// Partial sums that int4_matmul_form leaves where there is room for them (1: the result itself); its `parts` is
+// the room, and then what there is.
+int int4_form_parts(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, int form, size_t m);
+int int4_matmul_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, const ActOut &act, float *out, int *parts);
+
+// decoder_ops.cu, the operators between the matmuls. Inputs that are `parts` partial sums lie `pitch` floats apart.
+int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
+              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out);
+int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out);
+template <typename KV>
+int rope_append_form(yscv_cuda_ctx *ctx, const float *qkv, int parts, size_t pitch, float *q_out, size_t q_out_stride, size_t batch,
+                     size_t seq, size_t n_q, size_t n_kv, size_t d_head, float theta, const int32_t *d_pos, KV *kcache, KV *vcache,
+                     float *kscale, float *vscale, size_t max_seq);
+template <typename KV>
+int gqa_attention_form(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q, size_t n_kv,
+                       size_t d_head, const KV *d_kcache, const KV *d_vcache, const float *d_kscale, const float *d_vscale,
+                       size_t max_seq, const int32_t *d_pos, int causal, const ActOut &out);
+bool gqa_attention_writes(int form, size_t seq_q, size_t d_head, size_t max_seq);   // forms other than ACT_F32
 
 // gqa_prefill_tc.cu: attention of seq_q >= 16 query positions per sequence over a cache (KV = float or
 // int8_t), head size 64 or 128, at most 128 query heads per KV head, 16-byte aligned caches and output

@@ -93,6 +93,17 @@ class Int4Decoder:
         self._bufs = {}
         self.graph = None
         stream.synchronize()
+        layers_of = [dict(qkv=self.wqkv[l].handle, o=self.wo[l].handle, gate_up=self.wgu[l].handle,
+                          down=self.wdown[l].handle, gamma_attn=self.gamma.data_ptr(),
+                          gamma_mlp=self.gamma.data_ptr(), kcache=self.kcache[l].data_ptr(),
+                          vcache=self.vcache[l].data_ptr(),
+                          kscale=self.kscale[l].data_ptr() if kv_int8 else None,
+                          vscale=self.vscale[l].data_ptr() if kv_int8 else None) for l in range(self.n_layers)]
+        # one GPU: the chain of a step or prompt pass as one library call (a collective between the operators
+        # needs them one by one)
+        self.layers = None
+        if tp_size == 1 and self.n_layers > 0 and cfg.hidden % 8 == 0 and cfg.hidden <= 8192 and self.mlp_l % 8 == 0 and cfg.head_dim % 8 == 0:
+            self.layers = ctx.decode_layers(layers_of)
         # batch 1: the whole single-token step as one persistent kernel per GPU, when the
         # shapes allow it (the library says which do). With tensor parallelism the ranks'
         # kernels exchange their partial sums through exchange regions mapped with CUDA IPC;
@@ -110,12 +121,7 @@ class Int4Decoder:
                     self.lm_rows = cfg.vocab // tp_size
                     self.lm_row0 = tp_rank * self.lm_rows
                 self.plan = ctx.decode_plan(
-                    [dict(qkv=self.wqkv[l].handle, o=self.wo[l].handle, gate_up=self.wgu[l].handle,
-                          down=self.wdown[l].handle, gamma_attn=self.gamma.data_ptr(),
-                          gamma_mlp=self.gamma.data_ptr(), kcache=self.kcache[l].data_ptr(),
-                          vcache=self.vcache[l].data_ptr(),
-                          kscale=self.kscale[l].data_ptr() if kv_int8 else None,
-                          vscale=self.vscale[l].data_ptr() if kv_int8 else None) for l in range(self.n_layers)],
+                    layers_of,
                     cfg.hidden, self.mlp_l, self.nq_l, self.nkv_l, cfg.head_dim, max_seq, cfg.eps, cfg.rope_theta,
                     tp=self.tp_comm, kv_int8=kv_int8, batch=batch, **(plan_options or {}))
             except YscvCudaError as e:
@@ -224,6 +230,16 @@ class Int4Decoder:
         rows = B * seq
         qkv_w = (self.nq_l + 2 * self.nkv_l) * d
         x = self._buf("x", rows, H)
+        if self.layers is not None and not (self.one_launch and seq == 1):
+            shape = (H, self.mlp_l, self.nq_l, self.nkv_l, d)
+            need = ctx.decoder_layers_workspace(self.layers, *shape, B, seq)
+            ws = self._buf("layers", need, dtype=torch.uint8)
+            last = self._buf("last", B, H)
+            logits = self._buf("logits", B, c.vocab)
+            ctx.embedding_dev(self.embedding.data_ptr(), c.vocab, H, tokens.data_ptr(), rows, x.data_ptr())
+            ctx.decoder_layers_dev(self.layers, *shape, self.max_seq, c.eps, c.rope_theta, self.kv_int8, B, seq, self.pos.data_ptr(),
+                                   x.data_ptr(), self.gamma.data_ptr(), last.data_ptr(), ws.data_ptr(), need)
+            return self._head(last, logits, seq)
         h = self._buf("h", rows, H)
         qkv = self._buf("qkv", rows, qkv_w)
         attn = self._buf("attn", rows, self.nq_l * d)
@@ -287,8 +303,11 @@ class Int4Decoder:
             delta = down.data_ptr()
         ctx.add_rms_norm_dev(x.data_ptr(), delta, self.gamma.data_ptr(), c.eps, rows, H, x.data_ptr(), h.data_ptr())
         last = h if seq == 1 else h.view(B, seq, H)[:, seq - 1, :].contiguous()
-        logits = self._buf("logits", B, c.vocab)
-        ctx.f32_matmul_dev(self.lm_head.data_ptr(), last.data_ptr(), B, c.vocab, H, logits.data_ptr())
+        return self._head(last, self._buf("logits", B, c.vocab), seq)
+
+    def _head(self, last: torch.Tensor, logits: torch.Tensor, seq: int) -> torch.Tensor:
+        c, ctx, B = self.cfg, self.ctx, self.batch
+        ctx.f32_matmul_dev(self.lm_head.data_ptr(), last.data_ptr(), B, c.vocab, c.hidden, logits.data_ptr())
         ctx.argmax_last_dev(logits.data_ptr(), B, c.vocab, self.next_tokens.data_ptr())
         ctx.advance_pos_dev(self.pos.data_ptr(), seq)
         return logits
@@ -310,6 +329,7 @@ class Int4Decoder:
             self.tp_comm.close()
             self.tp_comm = None
         self._bufs.clear()
+        self.layers = None
         self.kcache, self.vcache = [], []
         self.wqkv, self.wo, self.wgu, self.wdown = [], [], [], []
         torch.cuda.synchronize()

@@ -92,6 +92,8 @@ SIGNATURES = {
                                                C.POINTER(_vp)]),
     "yscv_cuda_decode_plan_step_dev": (C.c_int, [_vp, _vp, _vp, _sz, _vp, _vp, _vp]),
     "yscv_cuda_decode_plan_step_token_dev": (C.c_int, [_vp, _vp, _vp, _sz, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "yscv_cuda_decoder_layers_workspace": (C.c_int, [_vp, _vp] + [_sz] * 8 + [C.POINTER(_sz)]),
+    "yscv_cuda_decoder_layers_dev": (C.c_int, [_vp, _vp] + [_sz] * 7 + [C.c_float, C.c_float, C.c_int, _sz, _sz] + [_vp] * 5 + [_sz]),
     "yscv_cuda_decode_plan_free": (None, [_vp]),
     "yscv_cuda_decode_plan_create_ex": (C.c_int, [_vp, _vp, _sz, _sz, _sz, _sz, _sz, _sz, _sz, C.c_float, C.c_float,
                                                   _vp, C.POINTER(_vp)]),
@@ -752,13 +754,9 @@ class Context:
                                                        _vp(d_kc), _vp(d_ks), _vp(d_vc), _vp(d_vs), max_seq, _vp(d_pos),
                                                        int(causal), _vp(d_out)))
 
-    def decode_plan(self, layers, hidden, inter, n_q, n_kv, d_head, max_seq, eps, rope_theta, *, variant=-1,
-                    max_tiles=0, k_chunk=0, attention_form=-1, spin_limit=0, tp: "TpComm | None" = None,
-                    kv_int8=False, batch=1) -> DecodePlan:
-        """layers: list of dicts with Int4Weight `qkv`, `o`, `gate_up`, `down` and device
-        pointers `gamma_attn`, `gamma_mlp`, `kcache`, `vcache` (with kv_int8 also `kscale`,
-        `vscale`). The keyword arguments are the fields of yscv_cuda_decode_options (defaults: the
-        library's own choices)."""
+    @staticmethod
+    def decode_layers(layers):
+        """Array of yscv_cuda_decode_layer from the dicts that decode_plan takes; it does not keep them alive."""
         arr = (DecodeLayer * len(layers))()
         for dst, l in zip(arr, layers):
             dst.qkv, dst.o, dst.gate_up, dst.down = (l["qkv"].handle, l["o"].handle, l["gate_up"].handle,
@@ -766,6 +764,30 @@ class Context:
             dst.d_gamma_attn, dst.d_gamma_mlp = l["gamma_attn"], l["gamma_mlp"]
             dst.d_kcache, dst.d_vcache = l["kcache"], l["vcache"]
             dst.d_kscale, dst.d_vscale = l.get("kscale"), l.get("vscale")
+        return arr
+
+    def decoder_layers_workspace(self, layers, hidden, inter, n_q, n_kv, d_head, batch, seq) -> int:
+        """Bytes of device memory a decoder_layers_dev call needs; `layers` as decode_layers() makes them."""
+        n = _sz()
+        _check(self.lib.yscv_cuda_decoder_layers_workspace(self.handle, layers, len(layers), hidden, inter, n_q, n_kv,
+                                                           d_head, batch, seq, C.byref(n)))
+        return n.value
+
+    def decoder_layers_dev(self, layers, hidden, inter, n_q, n_kv, d_head, max_seq, eps, rope_theta, kv_int8, batch, seq, d_pos, d_x,
+                           d_final_gamma, d_last, d_workspace, workspace_bytes):
+        """All layers and the final norm of the last positions as one chain of kernels."""
+        _check(self.lib.yscv_cuda_decoder_layers_dev(self.handle, layers, len(layers), hidden, inter, n_q, n_kv, d_head,
+                                                     max_seq, eps, rope_theta, int(kv_int8), batch, seq, _vp(d_pos), _vp(d_x),
+                                                     _vp(d_final_gamma), _vp(d_last), _vp(d_workspace), workspace_bytes))
+
+    def decode_plan(self, layers, hidden, inter, n_q, n_kv, d_head, max_seq, eps, rope_theta, *, variant=-1,
+                    max_tiles=0, k_chunk=0, attention_form=-1, spin_limit=0, tp: "TpComm | None" = None,
+                    kv_int8=False, batch=1) -> DecodePlan:
+        """layers: list of dicts with Int4Weight `qkv`, `o`, `gate_up`, `down` and device
+        pointers `gamma_attn`, `gamma_mlp`, `kcache`, `vcache` (with kv_int8 also `kscale`,
+        `vscale`). The keyword arguments are the fields of yscv_cuda_decode_options (defaults: the
+        library's own choices)."""
+        arr = self.decode_layers(layers)
         h = _vp()
         opt = DecodeOptions(variant, max_tiles, k_chunk, attention_form, spin_limit, tp.handle if tp else None,
                             1 if kv_int8 else 0, int(batch))
