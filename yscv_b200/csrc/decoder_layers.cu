@@ -4,7 +4,7 @@
 // single calls cannot is hand results over as they are: an operator writes the activations in the form that the
 // matmul behind it takes (act_forms.cuh), and a matmul whose k was cut into slices leaves them for the operator behind
 // it to add. A launch of a small decode batch is 1.5 to 2 us of latency whatever it does: 32 sequences at the 1B shape
-// (22 layers) had 15 launches per layer, 8 sequences 13; now 9.
+// (22 layers) had 15 launches per layer, 8 sequences 13; now 7 (9 over long caches).
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -73,6 +73,10 @@ int check(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_lay
     return YSCV_CUDA_OK;
 }
 
+bool caches_aligned(const yscv_cuda_decode_layer &l) {
+    return ((reinterpret_cast<uintptr_t>(l.d_kcache) | reinterpret_cast<uintptr_t>(l.d_vcache)) & 15) == 0;
+}
+
 template <typename KV>
 int run(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_layers, const Shape &s, const Layout &o, size_t max_seq, float eps,
         float theta, const int32_t *pos, float *x, const float *final_gamma, float *last, unsigned char *ws) {
@@ -89,15 +93,22 @@ int run(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_layer
         if ((rc = norm_form(ctx, x, delta, parts, m * H, l.d_gamma_attn, eps, m, 0, 1, H, x, a))) return rc;
         parts = o.parts_qkv;
         if ((rc = int4_matmul_form(ctx, l.qkv, a, qkv, &parts))) return rc;
-        float *const q = parts > 1 ? reinterpret_cast<float *>(ws + o.q) : qkv;
-        const size_t q_stride = parts > 1 ? nq : s.qkv();
-        if ((rc = rope_append_form<KV>(ctx, qkv, parts, m * s.qkv(), q, q_stride, s.batch, s.seq, s.n_q, s.n_kv, s.d, theta, pos, kc, vc,
-                                       l.d_kscale, l.d_vscale, max_seq)))
-            return rc;
         const int form = int4_act_form(ctx, l.o, m);
-        a = act_out(gqa_attention_writes(form, s.seq, s.d, max_seq) ? form : (int)ACT_F32, m, nq, act);
-        if ((rc = gqa_attention_form<KV>(ctx, q, q_stride, s.batch, s.seq, s.n_q, s.n_kv, s.d, kc, vc, l.d_kscale, l.d_vscale, max_seq, pos, 1, a)))
-            return rc;
+        const int own = form == ACT_TERMS ? (int)ACT_F32 : form;   // (a block of terms spans heads)
+        if (s.seq == 1 && caches_aligned(l) && gqa_decode_fused_wins(ctx, own, sizeof(KV) == 1, s.batch, s.n_q, s.n_kv, s.d, max_seq)) {
+            a = act_out(own, m, nq, act);
+            if ((rc = gqa_decode_fused<KV>(ctx, qkv, parts, m * s.qkv(), s.batch, s.n_q, s.n_kv, s.d, theta, pos, kc, vc, l.d_kscale, l.d_vscale, max_seq, a)))
+                return rc;
+        } else {
+            float *const q = parts > 1 ? reinterpret_cast<float *>(ws + o.q) : qkv;
+            const size_t q_stride = parts > 1 ? nq : s.qkv();
+            if ((rc = rope_append_form<KV>(ctx, qkv, parts, m * s.qkv(), q, q_stride, s.batch, s.seq, s.n_q, s.n_kv, s.d, theta, pos, kc, vc,
+                                           l.d_kscale, l.d_vscale, max_seq)))
+                return rc;
+            a = act_out(gqa_attention_writes(form, s.seq, s.d, max_seq) ? form : (int)ACT_F32, m, nq, act);
+            if ((rc = gqa_attention_form<KV>(ctx, q, q_stride, s.batch, s.seq, s.n_q, s.n_kv, s.d, kc, vc, l.d_kscale, l.d_vscale, max_seq, pos, 1, a)))
+                return rc;
+        }
         parts = o.parts_o;
         if ((rc = int4_matmul_form(ctx, l.o, a, down, &parts))) return rc;
         a = act_out(int4_act_form(ctx, l.gate_up, m), m, H, act);

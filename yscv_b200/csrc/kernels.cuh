@@ -71,6 +71,12 @@ template <typename KV>
 int gqa_attention_form(yscv_cuda_ctx *ctx, const float *d_q, size_t q_stride, size_t batch, size_t seq_q, size_t n_q, size_t n_kv,
                        size_t d_head, const KV *d_kcache, const KV *d_vcache, const float *d_kscale, const float *d_vscale,
                        size_t max_seq, const int32_t *d_pos, int causal, const ActOut &out);
+// gqa_decode_fused.cu: RoPE, cache append and attention of one position per sequence, for a chain in which nothing
+// between the two kernels in front of it and the end of the step before touches the caches or the position
+bool gqa_decode_fused_wins(const yscv_cuda_ctx *ctx, int form, bool kv_int8, size_t batch, size_t n_q, size_t n_kv, size_t d_head, size_t max_seq);
+template <typename KV>
+int gqa_decode_fused(yscv_cuda_ctx *ctx, const float *qkv, int parts, size_t pitch, size_t batch, size_t n_q, size_t n_kv, size_t d_head,
+                     float theta, const int32_t *d_pos, KV *kcache, KV *vcache, float *kscale, float *vscale, size_t max_seq, const ActOut &out);
 bool gqa_attention_writes(int form, size_t seq_q, size_t d_head, size_t max_seq);   // forms other than ACT_F32
 
 // gqa_prefill_tc.cu: attention of seq_q >= 16 query positions per sequence over a cache (KV = float or
