@@ -216,3 +216,41 @@ def test_infinite_and_tiny_activations(n, k):
         want = x[row].double() @ w.T
         assert float((out[row].double() - want).norm() / want.norm()) <= bound, row
     ctx.close()
+
+
+@pytest.mark.parametrize("m,n,k,form", [
+    (129, 1000, 4096, "slices"), (200, 8192, 4096, "slices"), (300, 2048, 2112, "slices"), (700, 520, 8192, "slices"), (1000, 2048, 2048, "slices"),
+    (257, 14336, 1088, "pairs"), (300, 14336, 4096, "pairs"), (700, 8200, 2048, "pairs"), (1000, 14336, 2112, "pairs"), (1001, 14335, 1024, "pairs"),
+    (600, 57344, 1024, "pairs"), (1030, 38400, 2048, "pairs"),
+])
+def test_prompt_tiles(m, n, k, form):
+    """Prompt matmuls that leave SMs idle with tiles of 256 tokens: k in slices (one or more tiles of tokens), CTA-pair tiles of
+    fewer tokens, fewer pair tiles than pairs, a split last round of narrow tiles; bounds as above, row by row too."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + m)
+    with torch.cuda.stream(stream):
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g)
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        report = ctx.dispatch_report()
+        first = out.clone()
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        want = x.double() @ w.T
+    stream.synchronize()
+    assert ctx.device_status() == 0
+    if form == "slices":
+        assert "K slice(s)" in report and " 1 K slice(s)" not in report, report
+    else:
+        assert "cta_group::2" in report and "rows x 256 tokens" not in report, report
+    assert torch.equal(first, out)
+    assert torch.all(out[m] == 7.0)
+    diff = out[:m].double() - want
+    assert float(diff.norm() / want.norm()) <= 4e-3
+    assert float((diff.norm(dim=1) / want.norm(dim=1)).max()) <= 8e-3
+    for n0 in range(0, n, 512):
+        assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 8e-3, n0
+    ctx.close()

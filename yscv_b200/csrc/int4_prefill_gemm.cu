@@ -358,15 +358,16 @@ int4_prefill_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             for (int a = 0; a < NA; ++a) {
                 const int n = nt_i * (NA * PG_BM) + a * PG_BM + q * 32 + lane;   // output channel of this lane
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)tbuf * 256 + (uint32_t)(a * acc_cols);
+                float *o = o_base + (size_t)tc * acc_cols * p.N + n;   // stepped token by token
+                const int rows = n < p.N ? p.M - tc * acc_cols : 0;
 #pragma unroll 1
                 for (int c0 = 0; c0 < acc_cols; c0 += 32) {
                     uint32_t rr[32];
                     pg_tmem_ld32(taddr + c0, rr);
-                    const int tok0 = tc * acc_cols + c0;
-                    if (n < p.N) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (tok0 + j < p.M) o_base[(size_t)(tok0 + j) * p.N + n] = __uint_as_float(rr[j]);
+                    for (int j = 0; j < 32; ++j) {
+                        if (c0 + j < rows) *o = __uint_as_float(rr[j]);
+                        o += p.N;
                     }
                 }
             }
@@ -389,9 +390,9 @@ int4_prefill_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 // CTA-pair form for large prefills: tcgen05.mma.cta_group::2
 // ---------------------------------------------------------------------------
 //
-// Two CTAs on the two SMs of a TPC (a cluster of 2) share a tile of 512 weight rows x 256 tokens.
+// Two CTAs on the two SMs of a TPC (a cluster of 2) share a tile of 512 weight rows x BT tokens (up to 256).
 // Each CTA dequantises its own 256 weight rows (two 128-row tiles, as the NA = 2 form above) and
-// stages HALF of the activation tile of a k block (128 tokens); the leader (cluster rank 0) issues
+// stages HALF of the activation tile of a k block (BT / 2 tokens); the leader (cluster rank 0) issues
 // MMAs of M = 256, N = 256 that read both CTAs' shared memory and leave rows 0..127 in its own
 // TMEM and rows 128..255 in the peer's. Per k block an SM then pulls 8 KB of nibbles + 16 KB of
 // activations from L2 instead of 8 + 32 KB, and its tensor core reads half the activation bytes
@@ -484,7 +485,7 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     const uint32_t bar_full_w = bars, bar_full_act = bars + 64, bar_empty = bars + 128;
     const uint32_t bar_afull = bars + 192, bar_aempty = bars + 224, bar_tfull = bars + 256, bar_tempty = bars + 264;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + PP_ABUFS * PP_A_BUF + (size_t)p.stages * PP_STAGE + 272);
-    const int tiles = p.n_tiles * p.t_chunks;   // pair tiles: 512 weight rows x 256 tokens
+    const int tiles = p.n_tiles * p.t_chunks;   // pair tiles: 512 weight rows x BT tokens
 
     if (tid == 0) {
         for (int i = 0; i < p.stages; ++i) {
@@ -529,12 +530,12 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
                     alive = mbar_wait(bar_empty + slot * 8, phase ^ 1u, status);
                     if (!alive) break;
                     const uint32_t st = ring + (uint32_t)slot * PP_STAGE;
-                    if (rank == 0) mbar_expect_tx(bar_full_act + slot * 8, 2 * KSUB * PP_ACT);
+                    if (rank == 0) mbar_expect_tx(bar_full_act + slot * 8, KSUB * p.BT * 128);
                     mbar_expect_tx(bar_full_w + slot * 8, KSUB * PP_W);
 #pragma unroll
                     for (int sub = 0; sub < KSUB; ++sub) {
                         const int kx = kb * KSUB + sub;   // 64-k block
-                        tma_load_2d_pair(st + sub * PP_ACT, &tm_a, kx * PG_BK, tc * 256 + (int)rank * 128, leader_full_act + slot * 8);
+                        tma_load_2d_pair(st + sub * PP_ACT, &tm_a, kx * PG_BK, tc * p.BT + (int)rank * (p.BT / 2), leader_full_act + slot * 8);
                         tma_load_2d(st + KSUB * PP_ACT + sub * PP_W, &tm_w, kx * 32, nt_i * 512 + (int)rank * 256, bar_full_w + slot * 8);
                     }
                     if (++slot == p.stages) { slot = 0; phase ^= 1u; }
@@ -544,8 +545,8 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
     } else if (warp == 1) {
         // ---------------- MMA issuer (leader only) ----------------
         if (lane == 0 && rank == 0) {
-            // D fp32, A and B bf16, both K-major, N = 256, M = 256 over the pair
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
+            // D fp32, A and B bf16, both K-major, N = BT, M = 256 over the pair
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.BT >> 3) << 17) |
                                    ((uint32_t)(256 >> 4) << 24);
             int slot = 0, abuf = 0;
             uint32_t phase = 0, aphase = 0, tphase = 0;
@@ -675,19 +676,19 @@ int4_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
             for (int a = 0; a < 2; ++a) {
                 const int n = nt_i * 512 + (int)rank * 256 + a * PG_BM + q * 32 + lane;   // output channel of this lane
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * 256);
+                // a column of the result or of the part, stepped token by token (nothing overlaps this: an address and
+                // two bounds per element took 2 us more of a tile's 8)
+                float *o = part >= 0 ? p.parts + (size_t)part * 256 * 512 + rank * 256 + a * PG_BM + q * 32 + lane : out + (size_t)tc * p.BT * p.N + n;
+                const size_t pitch = part >= 0 ? 512 : p.N;
+                const int rows = part >= 0 ? p.BT : n < p.N ? min(p.BT, p.M - tc * p.BT) : 0;
 #pragma unroll 1
-                for (int c0 = 0; c0 < 256; c0 += 32) {
+                for (int c0 = 0; c0 < p.BT; c0 += 32) {
                     uint32_t rr[32];
                     pg_tmem_ld32(taddr + c0, rr);
-                    const int tok0 = tc * 256 + c0;
-                    if (part >= 0) {
-                        float *dst = p.parts + ((size_t)part * 256 + c0) * 512 + rank * 256 + a * PG_BM + q * 32 + lane;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) dst[j * 512] = __uint_as_float(rr[j]);
-                    } else if (n < p.N) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (tok0 + j < p.M) out[(size_t)(tok0 + j) * p.N + n] = __uint_as_float(rr[j]);
+                    for (int j = 0; j < 32; ++j) {
+                        if (c0 + j < rows) *o = __uint_as_float(rr[j]);
+                        o += pitch;
                     }
                 }
             }
@@ -744,7 +745,7 @@ __global__ void __launch_bounds__(128) pp_join_kernel(PGParams p, int n_pairs, i
     const int c0 = (int)((((long long)i * p.k_blocks + 1) * n_pairs - 1) / rest);
     const int c1 = (int)((((long long)(i + 1) * p.k_blocks) * n_pairs - 1) / rest);
     if (c0 == c1) return;
-    const int n0 = tile % p.n_tiles * 512 + threadIdx.x * 4, tok0 = tile / p.n_tiles * 256 + blockIdx.y * 8;
+    const int n0 = tile % p.n_tiles * 512 + threadIdx.x * 4, tok0 = tile / p.n_tiles * p.BT + blockIdx.y * 8;
     float4 sum[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -780,12 +781,60 @@ bool int4_prefill_supported(size_t m, size_t n, size_t k, size_t gs) {
            m < (1u << 30) && n < (1u << 30) && k < (1u << 30);
 }
 
+// Split the last round of pair tiles where that saves more than the parts cost: a round takes about 0.9 us per 64 k,
+// a part (512 KB written and read back) 0.125 us from L2 and up to twice that from HBM, the second launch
+// 3 us: 2048 x 8192 x 10240 (12 tiles left for 74 pairs) 345 -> 281 us, 2048 x 8192 x 57344 (8 left) 1675 ->
+// 1592; with 54 left (2048 x 8192 x 8192) nothing is gained.
+static bool pp_split_pays(size_t tiles, size_t pairs, size_t k) {
+    const double rest = (double)(tiles % pairs);
+    return tiles > pairs && rest > 0 && 0.9 * (double)(k / 64) * (pairs - rest) / pairs > 2.0 * (0.125 * (pairs + rest) + 3.0);
+}
+
+// CTA pairs (512 weight rows x pair_bt tokens) or, with pair_bt == 0, one CTA per 128 rows x up to 256 tokens and k in
+// `slices`: whichever the modelled time in us says. A round of one-CTA tiles takes a fixed cost and a cost per 64 k that
+// grows with the tokens, slices cost a launch and their traffic; a round of pair tiles the same with its own costs, and up to
+// 14 % more when every pair is busy (power). Few tokens or rows leave most SMs without a pair tile, and whole rounds of tiles
+// of 256 tokens may leave the last one nearly empty; 1000 tokens x 28 tiles of 512 rows are 1.5 rounds for 74 pairs at 256
+// tokens and 1.9 at 208. The constants are a fit to 81 calls (129 to 1500 rows, 1024 x 1024 to 28672 x 8192), each with
+// eight choices forced in turn: predicted within 4 %, its choice 0.1 % behind the best on average and 3 % at worst. us before
+// (256 tokens, pairs only where each had a tile, slices only up to 128 tokens) / now: 200 x 8192 x 8192 72 / 44, 200 x 4096 x 14336
+// 119 / 41, 300 x 14336 x 4096 74 / 50, 700 x 8192 x 8192 144 / 100, 1000 x 2048 x 2048 23.6 / 19.5, 1000 x 14336 x 4096 119 / 110.
+struct PGChoice {
+    int pair_bt, slices;
+};
+static PGChoice pg_choose(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k, bool slices_ok) {
+    if (k < 1024 && m > 128)   // (shallower than what was measured: launches and drains)
+        return {ctx->prefill_pairs && (n + 511) / 512 * ((m + 255) / 256) >= (size_t)ctx->sm_count / 2 ? 256 : 0, 1};
+    const int sms = ctx->sm_count, kb = (int)(k / 64), bt = (int)std::min<size_t>((m + 15) / 16 * 16, 256);
+    const size_t tiles = (n + PG_BM - 1) / PG_BM * ((m + bt - 1) / bt);
+    PGChoice c = {0, 1};
+    double best = 1e30;
+    for (int s = 1; s <= 8 && s <= kb; ++s) {
+        const double mb = (double)s * m * n * 4e-6;
+        if (s > 1 && (!slices_ok || mb > 128.0)) break;
+        const double cost = 3.06 + (double)((tiles * s + sms - 1) / sms) * ((kb + s - 1) / s * (0.35 + 0.00089 * bt) + 1.55) + (s > 1 ? 2.35 + 0.176 * mb : 0.0);
+        if (cost < best) { best = cost; c.slices = s; }
+    }
+    if (!ctx->prefill_pairs || m <= 128) return c;
+    const size_t most = (size_t)sms / 2, chunks = (m + 255) / 256;
+    for (size_t ch = chunks; ch <= chunks + 3 && ch * 128 <= m + 127; ++ch) {
+        const size_t b = ((m + ch - 1) / ch + 15) / 16 * 16, t = (n + 511) / 512 * ((m + b - 1) / b);
+        const double tile = kb * (0.45 + 0.00102 * b) + 5.15 * b / 256, rest = (double)(t % most);
+        double cost = 3.62;
+        if (t <= most) cost += tile * (1.0 + 0.14 * t / most);
+        else if (pp_split_pays(t, most, k)) cost += tile * 1.14 * t / most + 0.125 * (most + rest) + 3.0;
+        else cost += tile * (1.14 * (t / most) + (rest > 0 ? 1.0 + 0.14 * rest / most : 0.0));
+        if (cost < best) { best = cost; c.pair_bt = (int)b; }
+    }
+    return c;
+}
+
 template <int KSUB>
 static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, const CUtensorMap &tm_a,
                                 const float *scales, float *out, PGParams p) {
     using G = PPGeom<KSUB>;
     p.n_tiles = (p.N + 511) / 512;
-    p.t_chunks = (p.M + 255) / 256;
+    p.t_chunks = (p.M + p.BT - 1) / p.BT;
     p.ksub = KSUB;
     p.k_blocks = p.K / (PG_BK * KSUB);
     p.ksplit = 1;
@@ -820,14 +869,10 @@ static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, con
     const int tiles = p.n_tiles * p.t_chunks;
     const int pairs = tiles < ctx->max_prefill_pairs ? tiles : ctx->max_prefill_pairs;
     cfg.gridDim = dim3(2 * pairs);
-    // Split the last round where that saves more than the parts cost: a round takes about 0.9 us per 64 k,
-    // a part (512 KB written and read back) 0.125 us from L2 and up to twice that from HBM, the second launch
-    // 3 us: 2048 x 8192 x 10240 (12 tiles left for 74 pairs) 345 -> 281 us, 2048 x 8192 x 57344 (8 left) 1675 ->
-    // 1592; with 54 left (2048 x 8192 x 8192) nothing is gained. Without memory for the parts, or inside a
-    // capture without an earlier call of the size, the last round stays whole.
+    // Without memory for the parts, or inside a capture without an earlier call of the size, the last round stays whole.
     const int rest = tiles % pairs;
     p.full_tiles = tiles;
-    if (tiles > pairs && rest > 0 && 0.9 * (p.K / 64) * (pairs - rest) / pairs > 2.0 * (0.125 * (pairs + rest) + 3.0)) {
+    if (pp_split_pays(tiles, pairs, p.K)) {
         if (ctx->gemm_ws.try_reserve((size_t)(pairs + rest) * 256 * 512 * sizeof(float), ctx->stream)) {
             p.full_tiles = tiles - rest;
             p.parts = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
@@ -840,36 +885,35 @@ static int launch_prefill_pairs(yscv_cuda_ctx *ctx, const CUtensorMap &tm_w, con
     ctx->launches++;
     if (p.full_tiles < tiles) {
         const int vec = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-        YSCV_CUDA_TRY(launch_pdl(pp_join_kernel, dim3((unsigned)rest, 32), dim3(128), 0, ctx->stream, p, pairs, vec, out));
+        YSCV_CUDA_TRY(launch_pdl(pp_join_kernel, dim3((unsigned)rest, (unsigned)(p.BT / 8)), dim3(128), 0, ctx->stream, p, pairs, vec, out));
         ctx->launches++;
     }
     snprintf(ctx->report_int4, sizeof(ctx->report_int4),
-             "int4_prefill_gemm m=%d n=%d k=%d: tcgen05 bf16 cta_group::2, pair tile 512 rows x 256 tokens, %d k per stage, "
-             "%d stages of %d KB per CTA, %d tiles on %d CTA pairs, %d split over k", p.M, p.N, p.K, KSUB * PG_BK, p.stages, G::STAGE / 1024,
+             "int4_prefill_gemm m=%d n=%d k=%d: tcgen05 bf16 cta_group::2, pair tile 512 rows x %d tokens, %d k per stage, "
+             "%d stages of %d KB per CTA, %d tiles on %d CTA pairs, %d split over k", p.M, p.N, p.K, p.BT, KSUB * PG_BK, p.stages, G::STAGE / 1024,
              tiles, pairs, tiles - p.full_tiles);
     ctx->last_kernel = "int4_prefill_gemm(tcgen05,bf16,cta_group::2)";
     return YSCV_CUDA_OK;
 }
 
 // act_bf16 != nullptr: the activations are already bf16 in the GEMM's k order (what the pre-pass
-// below writes; the decoder's norm and SwiGLU kernels can emit it): `act` and `scratch` are not used.
+// below writes; the decoder's norm and SwiGLU kernels can emit it): `act` and `scratch` are not used. `scratch` is the
+// context's, which may move.
 int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
                       float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16, int *parts) {
     PGParams p = {};
-    int rc_ws = 0;
     p.M = (int)m;
     p.N = (int)n;
     p.K = (int)k;
-    // Two 128-row weight tiles per CTA tile (256 rows x up to 256 tokens, the two accumulators
-    // filling all 512 TMEM columns, so the epilogue no longer overlaps the next tile) when that
-    // still gives every SM a tile: the activation tile, nine tenths of the L2 -> SM traffic, is
-    // then fetched once per 256 weight rows (2048 x 8192 x 8192: 918 -> 1121 TFLOP/s; 256 rows x
-    // 128 tokens with double-buffered accumulators measured 664: N = 128 MMAs read a third more
-    // shared memory per flop). Otherwise one weight tile x up to 256 tokens, accumulators
-    // double-buffered. One MMA tile per pass (N = BT, a multiple of 16).
-    const int m16 = (int)((m + 15) / 16 * 16);
+    const int m16 = (int)((m + 15) / 16 * 16), sms = ctx->sm_count;
+    const bool batch = int4_batch_bf16_wins(m, n, k, 32) && int4_batch_ready(ctx);   // up to 128 rows
+    const PGChoice choice = pg_choose(ctx, m, n, k, (m * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    const bool use_pairs = choice.pair_bt > 0 && !batch;
+    // Without the CTA pairs (switched off): two 128-row weight tiles per CTA tile (256 rows x up to 256 tokens, the two
+    // accumulators filling all 512 TMEM columns) when that still gives every SM a tile: the activation tile, nine tenths of
+    // the L2 -> SM traffic, is then fetched once per 256 weight rows (2048 x 8192 x 8192: 918 -> 1121 TFLOP/s).
     const size_t tiles2 = ((n + 2 * PG_BM - 1) / (2 * PG_BM)) * ((m + 255) / 256);
-    const int NA = (m16 > 128 && tiles2 >= (size_t)ctx->sm_count) ? 2 : 1;
+    const int NA = !ctx->prefill_pairs && m16 > 128 && tiles2 >= (size_t)sms ? 2 : 1;
     const int bt_max = 256;
     p.BT = m16 <= bt_max ? m16 : bt_max;
     p.NT = 1;
@@ -884,37 +928,22 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     p.stages = (227 * 1024 - 2 * p.ksub * NA * PG_BM * PG_BK * 2 - 1024) / p.stage_bytes;
     if (p.stages > 8) p.stages = 8;
     const int smem = 2 * p.ksub * NA * PG_BM * PG_BK * 2 + p.stages * p.stage_bytes + 256;
-    // A decode batch (one narrow token tile): cut K into slices so that the work items fill whole
-    // rounds of CTAs. Among 1..8 slices take the count with the shortest makespan
-    // (rounds of items / slices), as long as a slice keeps at least 512 k and the fp32 partial sums
-    // (written and read once per slice) stay below the bytes of the weights.
-    p.ksplit = 1;
-    {
-        const int base_tiles = p.n_tiles * p.t_chunks;
-        if (NA == 1 && p.t_chunks == 1 && p.BT <= 128 && (m * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-            const int sms = ctx->sm_count;
-            double best = (double)((base_tiles + sms - 1) / sms);
-            for (int sl = 2; sl <= 8; ++sl) {
-                if (p.k_blocks / sl < 8 / p.ksub) break;
-                if (16.0 * sl * (double)m > (double)k) break;
-                const double cost = (double)((base_tiles * sl + sms - 1) / sms) / sl + 0.02 * sl;
-                if (cost < best - 1e-9) { best = cost; p.ksplit = sl; }
-            }
-        }
-    }
+    p.ksplit = NA == 1 ? std::min(choice.slices, p.k_blocks) : 1;
     p.kb_per = (p.k_blocks + p.ksplit - 1) / p.ksplit;
     p.ksplit = (p.k_blocks + p.kb_per - 1) / p.kb_per;   // no empty slice (33 blocks in 8 slices of 5: seven slices)
     float *kernel_out = out;
-    const bool batch = int4_batch_bf16_wins(m, n, k, 32) && int4_batch_ready(ctx);   // up to 128 rows of a large matrix
-    if (p.ksplit > 1 && !batch) {
-        rc_ws = ctx->gemm_ws.reserve((size_t)p.ksplit * m * n * sizeof(float), ctx->stream);
-        if (rc_ws) return rc_ws;
-        kernel_out = reinterpret_cast<float *>(ctx->gemm_ws.ptr);
+    if (p.ksplit > 1 && !batch && !use_pairs) {
+        // the slices lie behind the activations (which are not there yet)
+        const size_t behind = act_bf16 ? 0 : (int4_prefill_scratch_bytes(m, k) + 255) / 256 * 256;
+        if (ctx->scratch.try_reserve(behind + (size_t)p.ksplit * m * n * sizeof(float), ctx->stream)) {
+            scratch = ctx->scratch.ptr;
+            kernel_out = reinterpret_cast<float *>(static_cast<unsigned char *>(scratch) + behind);
+        } else {   // inside a capture without an earlier call of the size, or no memory
+            p.ksplit = 1;
+            p.kb_per = p.k_blocks;
+        }
     }
-
-    // CTA pairs (512 weight rows x 256 tokens per pair) when every pair still gets a tile
-    const size_t pair_tiles = ((n + 511) / 512) * ((m + 255) / 256);
-    const bool use_pairs = ctx->prefill_pairs && NA == 2 && pair_tiles >= (size_t)(ctx->sm_count / 2);
+    if (use_pairs) p.BT = choice.pair_bt;
 
     const __nv_bfloat16 *abf = reinterpret_cast<const __nv_bfloat16 *>(act_bf16);
     if (!abf) {
@@ -931,10 +960,10 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     if (parts) *parts = 1;
 
     CUtensorMap tm_w, tm_a;
-    int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, (uint32_t)(NA * PG_BM), 32,
+    int rc = encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wq, n, k / 2, k / 2, (uint32_t)((use_pairs ? 2 : NA) * PG_BM), 32,
                        CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, abf, m, k, k * 2, use_pairs ? 128u : (uint32_t)p.BT, PG_BK,
+    rc = encode_2d(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, abf, m, k, k * 2, use_pairs ? (uint32_t)p.BT / 2 : (uint32_t)p.BT, PG_BK,
                    CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     if (use_pairs) {
