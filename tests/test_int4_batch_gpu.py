@@ -254,3 +254,26 @@ def test_prompt_tiles(m, n, k, form):
     for n0 in range(0, n, 512):
         assert float(diff[:, n0:n0 + 512].norm() / want[:, n0:n0 + 512].norm()) <= 8e-3, n0
     ctx.close()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,k", [(100, 256), (4736, 1280), (4800, 1536), (4737, 1792), (2048, 4352), (6000, 6912), (300, 8448), (4737, 6656)])
+def test_few_rows_depths(m, n, k):
+    """The few-row matmul where its last stage ends in half, and on both sides of the line between quantising the rows in the
+    kernel and before it: 21-bit blocks of 32 values (2^-22 of the block's maximum each, about four times its rms) and fp32 sums, 2e-6."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + k)
+    with torch.cuda.stream(stream):
+        packed, scales, w = _weights(g, n, k)
+        x = torch.randn(m, k, device="cuda", generator=g)
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+        ctx.int4_matmul_dev(h, x.data_ptr(), out.data_ptr(), m)
+        want = x.double() @ w.T
+    stream.synchronize()
+    assert ctx.device_status() == 0 and "int4_gemv_fast" in ctx.last_kernel()
+    assert torch.all(out[m] == 7.0)
+    assert float((out[:m].double() - want).norm() / want.norm()) <= 2e-6
+    ctx.close()

@@ -148,7 +148,7 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
             // (one size for every m up to 16, so that a call never outgrows what another one left)
             const size_t a_b = int4_gemv_scratch_bytes(16, k), b_b = int4_batch_exact_scratch_bytes(k);
             const size_t want = a_b > b_b ? a_b : b_b;
-            rc = batch || int4_gemv_uses_scratch(mc, k) ? ctx->scratch.reserve(want, ctx->stream) : ctx->scratch.reserve(want);
+            rc = batch || int4_gemv_uses_scratch(ctx, mc, n, k) ? ctx->scratch.reserve(want, ctx->stream) : ctx->scratch.reserve(want);
             if (rc) return rc;
         }
         if (batch) {
@@ -173,7 +173,7 @@ int int4_act_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, size_t m) 
     if (m == 0 || ((reinterpret_cast<uintptr_t>(w->d_packed) | reinterpret_cast<uintptr_t>(w->d_scales)) & 15)) return ACT_F32;
     if (m > 16) return !ctx->prefill_exact && int4_prefill_supported(m, n, k, gs) ? ACT_BF16 : ACT_F32;
     if (int4_batch_exact_wins(m, n, k, gs) && int4_batch_ready(ctx)) return ACT_TERMS;
-    return int4_gemv_fast_supported(m, n, k, gs) && int4_gemv_uses_scratch(m, k) ? ACT_DIGITS : ACT_F32;
+    return int4_gemv_fast_supported(m, n, k, gs) && int4_gemv_uses_scratch(ctx, m, n, k) && int4_gemv_digits_whole(m, k) ? ACT_DIGITS : ACT_F32;
 }
 
 int int4_form_parts(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, int form, size_t m) {

@@ -200,6 +200,9 @@ __device__ __forceinline__ void quantize_group_values(const float (&v)[8], unsig
     }
 }
 
+// Stages of a row of K values; the last one may reach past K
+__host__ __device__ inline int quant_stages(const QuantLayout &q, int K) { return (K + 32 * q.gs - 1) / (32 * q.gs); }
+
 // rows to visit per group, padding rows included
 __host__ __device__ inline int quant_slots(const QuantLayout &q) {
     return (q.mp <= 2) ? 2 : (q.ms > q.mc ? q.ms : q.mc);

@@ -118,20 +118,21 @@ int4_gemv_generic_kernel(const uint8_t *__restrict__ wq, const float *__restrict
 __global__ void __launch_bounds__(128)
 act_quant_kernel(const float *__restrict__ act, unsigned char *__restrict__ blobs, int M, int K,
                  QuantLayout q) {
+    const int groups = quant_stages(q, K) * q.gs;   // those past K, if any, are zero
     // programmatic dependent launch: the activations come from the predecessor, and the main kernel of
     // the previous call may still read the blobs
     pdl_wait();
     pdl_trigger();
     const int slots = quant_slots(q);
-    const int total = (K / 32) * slots;
+    const int total = groups * slots;
     const int t = threadIdx.x & 3;
     const int quads = (gridDim.x * blockDim.x) >> 2;
     const int rounds = (total + quads - 1) / quads;  // same trip count for every lane
     for (int r = 0; r < rounds; ++r) {
         const int item = r * quads + ((blockIdx.x * blockDim.x + threadIdx.x) >> 2);
         const bool valid = item < total;
-        const int Gabs = valid ? item % (K / 32) : 0, m = valid ? item / (K / 32) : 0;
-        quantize_group(m < M ? act + (size_t)m * K + Gabs * 32 + 8 * t : nullptr, blobs, q, Gabs, m,
+        const int Gabs = valid ? item % groups : 0, m = valid ? item / groups : 0;
+        quantize_group(m < M && Gabs * 32 < K ? act + (size_t)m * K + Gabs * 32 + 8 * t : nullptr, blobs, q, Gabs, m,
                        t, valid);
     }
 }
@@ -190,7 +191,7 @@ int4_gemv_fast_kernel(const __grid_constant__ CUtensorMap tm_w,
     if (r0 >= r1) return;
     const int rb_rows = g.tiles * 16;
     const int n_rb = (r1 - r0 + rb_rows - 1) / rb_rows;
-    const int k_stages = K / (GS * 32);
+    const int k_stages = (K + GS * 32 - 1) / (GS * 32);   // what lies past K reads as zeros (weights, scales, digits)
     const int total = n_rb * k_stages;
     const uint32_t ring_bytes = (uint32_t)g.stages * g.stage_bytes;
     float *red = reinterpret_cast<float *>(smem + ring_bytes);
@@ -199,7 +200,7 @@ int4_gemv_fast_kernel(const __grid_constant__ CUtensorMap tm_w,
     const uint32_t bar_empty = bar_full + 8 * 8;
     const uint32_t bar_act = bar_empty + 8 * 8;
     unsigned char *dig = smem + ring_bytes + 16 * 8 * 32 * 4 + 2 * 8 * 8 + 16;  // FUSEQ: resident blobs
-    float *act_s = reinterpret_cast<float *>(dig + (size_t)(K / (32 * GS)) * g.q.blob_bytes);
+    float *act_s = reinterpret_cast<float *>(dig + (size_t)k_stages * g.q.blob_bytes);
     // byte offset of the digit blob relative to the stage base (per-stage copy) or to `dig`
     const uint32_t b_off = FUSEQ ? 0u : (uint32_t)(g.w_bytes + g.s_bytes);
 
@@ -271,8 +272,8 @@ int4_gemv_fast_kernel(const __grid_constant__ CUtensorMap tm_w,
     // ---------------- consumers ----------------
     if constexpr (FUSEQ) {
         // quantise the activations while the first weight stages are in flight
-        const int slots = quant_slots(g.q);
-        const int items = (K / 32) * slots;
+        const int slots = quant_slots(g.q), groups = k_stages * GS;
+        const int items = groups * slots;
         constexpr int QUADS = FAST_CONSUMER_WARPS * 8;
         const int rounds = (items + QUADS - 1) / QUADS;
         const bool staged = g.act_bytes > 0;
@@ -281,12 +282,13 @@ int4_gemv_fast_kernel(const __grid_constant__ CUtensorMap tm_w,
         for (int r = 0; r < rounds; ++r) {
             const int item = r * QUADS + (tid >> 2);
             const bool valid = item < items;
-            const int Gabs = valid ? item % (K / 32) : 0, m = valid ? item / (K / 32) : 0;
+            const int Gabs = valid ? item % groups : 0, m = valid ? item / groups : 0;
             const size_t off = (size_t)m * K + Gabs * 32 + 8 * t;
+            const bool there = m < M && Gabs * 32 < K;
             if (staged)
-                quantize_group<true>(m < M && act_ok ? act_s + off : nullptr, dig, g.q, Gabs, m, t, valid);
+                quantize_group<true>(there && act_ok ? act_s + off : nullptr, dig, g.q, Gabs, m, t, valid);
             else
-                quantize_group<false>(m < M ? act + off : nullptr, dig, g.q, Gabs, m, t, valid);
+                quantize_group<false>(there ? act + off : nullptr, dig, g.q, Gabs, m, t, valid);
         }
         named_bar_sync(1, FAST_CONSUMER_WARPS * 32);
     }
@@ -454,15 +456,17 @@ int4_gemv_fast_kernel(const __grid_constant__ CUtensorMap tm_w,
 // ---------------------------------------------------------------------------
 
 static int padded_m(int m) { return m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : 16; }
-static int stage_groups(int mp, int k) { return (k % 512 == 0 && mp <= 4) ? 16 : 8; }
+// 512 k per stage for up to 4 rows, from 1536 on also where K ends in half a stage (with stages of 256 k / of 512: 1 row 2048 x
+// 768 3.5 / 3.5, 2048 x 4352 8.3 / 7.4, 2048 x 8448 13.2 / 9.5, 14336 x 8448 21.6 / 19.7; 4 rows 14336 x 1280 7.8 / 8.3, 6000 x 3328
+// 12.0 / 9.9, 2048 x 8448 13.3 / 10.7)
+static int stage_groups(int mp, int k) { return mp <= 4 && (k % 512 == 0 || k > 1536) ? 16 : 8; }
 
 size_t int4_gemv_scratch_bytes(size_t m, size_t k) {
     // worst case over every padded M up to the one requested
     size_t worst = 0;
     for (int mp = 1; mp <= padded_m((int)m); mp *= 2) {
-        const int gs = stage_groups(mp, (int)k);
-        const QuantLayout q = quant_layout(mp, gs);
-        const size_t b = (k / (32 * (size_t)gs)) * (size_t)q.blob_bytes;
+        const QuantLayout q = quant_layout(mp, stage_groups(mp, (int)k));
+        const size_t b = (size_t)quant_stages(q, (int)k) * (size_t)q.blob_bytes;
         worst = b > worst ? b : worst;
     }
     return worst + 256;
@@ -473,16 +477,15 @@ bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs) {
            m <= 16 && n >= 1 && n < (1u << 22) && k < (1u << 24);
 }
 
-// Largest resident digit copy the fused-quantisation variant keeps in shared memory.
-constexpr int FUSEQ_MAX_DIGIT_BYTES = 72 * 1024;
-// few activation rows: every CTA quantises them itself, no separate launch
-static bool fused_quant(int mp, int gs, int k) {
-    return mp <= 4 && (k / (32 * gs)) * quant_layout(mp, gs).blob_bytes <= FUSEQ_MAX_DIGIT_BYTES;
-}
-bool int4_gemv_uses_scratch(size_t m, size_t k) {
-    const int mp = padded_m((int)m);
-    return !fused_quant(mp, stage_groups(mp, (int)k), (int)k);
-}
+// Few and short activation rows: every CTA quantises them itself, no separate launch. That is work on the way to every CTA's
+// first product, so it pays up to 4500 values, 6800 where a CTA has more than 32 rows of weights to hide it behind (us per
+// call, in the kernel / in a launch of its own): 1 row 2048 x 4608 7.4 / 6.5, 2048 x 8192 10.5 / 8.9, 14336 x 4096
+// 10.5 / 11.7, 14336 x 8192 19.2 / 18.1, 28672 x 8192 38.7 / 33.3; 2 rows 2048 x 2048 4.3 / 5.2, 2048 x 2560 5.8 / 5.5, 14336 x 3072 9.3 /
+// 10.1, 28672 x 4096 21.5 / 20.2; 4 rows 2048 x 1024 3.8 / 4.0, 2048 x 4096 9.8 / 6.8, 14336 x 1536 8.5 / 8.8, 14336 x 4096 18.6 / 15.6.
+// (The digit planes of so many values are at most 56 KB.)
+static bool small_rows(const yscv_cuda_ctx *ctx, int n) { return (n + ctx->sm_count - 1) / ctx->sm_count <= 32; }
+static bool fused_quant(const yscv_cuda_ctx *ctx, int mp, int n, int k) { return mp <= 4 && mp * k <= (small_rows(ctx, n) ? 4500 : 6800); }
+bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) { return !fused_quant(ctx, padded_m((int)m), (int)n, (int)k); }
 
 template <int MP, int GS, int TP2, bool FUSEQ>
 static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
@@ -496,7 +499,7 @@ static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scale
     const int rb_rows = g.tiles * 16;
     g.w_bytes = rb_rows * GS * 16;
     g.s_bytes = rb_rows * GS * 4;
-    const int digit_bytes = FUSEQ ? (K / (32 * GS)) * q.blob_bytes : 0;
+    const int digit_bytes = FUSEQ ? quant_stages(q, K) * q.blob_bytes : 0;
     // stage the activations through TMA when they are small (M <= 2) and 16-byte aligned
     g.act_bytes = (FUSEQ && MP <= 2 && (size_t)M * K * 4 <= 32 * 1024 &&
                    (reinterpret_cast<uintptr_t>(act) & 15) == 0) ? M * K * 4 : 0;
@@ -562,10 +565,9 @@ template <int MP, int GS>
 static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
                           const float *act, float *out, int M, int N, int K, void *scratch) {
     const QuantLayout q = quant_layout(MP, GS);
-    const int rows_per_cta = (N + ctx->sm_count - 1) / ctx->sm_count;
-    const bool small = rows_per_cta <= 32;
+    const bool small = small_rows(ctx, N);
     if constexpr (MP <= 4) {
-        if (act && fused_quant(MP, GS, K)) {
+        if (act && fused_quant(ctx, MP, N, K)) {
             ctx->last_kernel = "int4_gemv_fast(imma,tma,fused-quant)";
             return small ? launch_fast<MP, GS, 2, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q)
                          : launch_fast<MP, GS, 8, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q);
@@ -573,7 +575,7 @@ static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *sc
     }
     unsigned char *blobs = reinterpret_cast<unsigned char *>(scratch);
     if (act) {
-        const int items = (K / 32) * quant_slots(q);
+        const int items = quant_stages(q, K) * q.gs * quant_slots(q);
         YSCV_CUDA_TRY(launch_pdl(act_quant_kernel, dim3((items * 4 + 127) / 128), dim3(128), 0, ctx->stream, act, blobs, M, K, q));
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
@@ -604,6 +606,8 @@ QuantLayout int4_gemv_layout(size_t m, size_t k) {
     const int mp = padded_m((int)m);
     return quant_layout(mp, stage_groups(mp, (int)k));
 }
+// The digit planes have no padding groups, which only the library's own pass writes
+bool int4_gemv_digits_whole(size_t m, size_t k) { return k % (stage_groups(padded_m((int)m), (int)k) * 32) == 0; }
 int int4_gemv_digits(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const void *digits, float *out, size_t m, size_t n, size_t k) {
     return int4_gemv_fast(ctx, wq, scales, nullptr, out, m, n, k, const_cast<void *>(digits));
 }
@@ -631,7 +635,7 @@ static int launch_scratch_variant(yscv_cuda_ctx *ctx, const uint8_t *wq, const f
                                   unsigned char *blobs) {
     const QuantLayout q = quant_layout(MP, GS);
     const int rows_per_cta = (N + ctx->sm_count - 1) / ctx->sm_count;
-    const int items = (K / 32) * quant_slots(q);
+    const int items = quant_stages(q, K) * q.gs * quant_slots(q);
     YSCV_CUDA_TRY(launch_pdl(act_quant_kernel, dim3((items * 4 + 127) / 128), dim3(128), 0, ctx->stream, act, blobs, M, K, q));
     YSCV_CUDA_TRY(cudaGetLastError());
     ctx->launches++;

@@ -14,7 +14,7 @@ namespace yscv {
 // int4_gemv.cu
 bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs);
 size_t int4_gemv_scratch_bytes(size_t m, size_t k);
-bool int4_gemv_uses_scratch(size_t m, size_t k);
+bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k);
 // fp32 matmul out[m][n] = sum_k x[m][k] w[n][k] for m > 8 as three TF32 products per fp32 product
 // on the tensor cores (f32_gemm_tf32x3.cu)
 bool f32_gemm_tc_supported(const float *d_w, const float *d_x, size_t m, size_t n, size_t k);
@@ -26,6 +26,7 @@ int int4_gemv_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, c
 // the same with digit planes that the caller wrote (ActForm ACT_DIGITS, act_out())
 int int4_gemv_digits(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const void *digits, float *out, size_t m, size_t n, size_t k);
 QuantLayout int4_gemv_layout(size_t m, size_t k);
+bool int4_gemv_digits_whole(size_t m, size_t k);
 int int4_gemv_generic(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
                       const float *act, float *out, size_t m, size_t n, size_t k, size_t gs);
 
