@@ -308,6 +308,22 @@ __device__ __forceinline__ void quantize_activation(const float *act_s, unsigned
     cons_sync();
 }
 
+// Eight activations k .. k + 7 per lane, straight from registers into the digit planes. All lanes of a warp call it
+// together; the caller's barrier publishes the planes.
+__device__ __forceinline__ void quantize_registers(const float (&v)[8], unsigned char *dig, int k) {
+    quantize_group_values(v, dig, quant_layout(1, DS_GS), k / 32, 0, (k / 8) & 3, true);
+}
+__device__ __forceinline__ void ldcg8(const float *p, float (&v)[8], bool aligned = true) {
+    if (!aligned) {   // (the caller's residual stream may lie anywhere)
+#pragma unroll
+        for (int t = 0; t < 8; ++t) v[t] = __ldcg(p + t);
+        return;
+    }
+    const float4 a = __ldcg(reinterpret_cast<const float4 *>(p)), b = __ldcg(reinterpret_cast<const float4 *>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
 struct RingPos {
     int slot;
     uint32_t phase;
@@ -405,12 +421,13 @@ __device__ __forceinline__ void consume_stages(const StepParams &p, const unsign
     }
 }
 
+// (row_scale: what the activations were not yet multiplied by, the inverse rms behind a norm.)
 // store: 0 out[row] = v; 1 out[row] = resid + v (resid fetched by the caller before the K loop);
 // 2 the block is gate tiles then up tiles of intermediate indices: out[i] = silu(gate_i) * up_i.
 // Rows (indices) of the block start at row_base; nothing at or past r1 is written.
 template <int TP2>
 __device__ __forceinline__ void finish_rows(const StepParams &p, float *red, int tiles, int row_base, int r1,
-                                            float *out, int store, const float (&acc)[2], float resid,
+                                            float *out, int store, const float (&acc)[2], float resid, float row_scale,
                                             unsigned int tp_tag, int tp_parity) {
     constexpr int GS = DS_GS;
     constexpr int KSL = (16 / TP2 < GS) ? 16 / TP2 : GS;
@@ -435,6 +452,8 @@ __device__ __forceinline__ void finish_rows(const StepParams &p, float *red, int
                 g += pg[0] + pg[1];
                 u += pu[0] + pu[1];
             }
+            g *= row_scale;
+            u *= row_scale;
             const float sg = 1.0f / (1.0f + expf(-g));
             if (my_row < r1) out[my_row] = (g * sg) * u;
         }
@@ -445,6 +464,7 @@ __device__ __forceinline__ void finish_rows(const StepParams &p, float *red, int
             const float *pp = red + ((ks * tiles + tl) * 2 + half) * 32 + q8 * 4;
             v += pp[0] + pp[1];
         }
+        v *= row_scale;
         // store 1 under tensor parallelism: v is this rank's partial sum over its K slice
         if (my_row < r1) {
             if (store == 1 && p.tp_size > 1) v = tp_reduce_row(p, my_row, v, tp_tag, tp_parity);
@@ -1344,6 +1364,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
     const unsigned int tp_seq = p.tp_size > 1 ? *p.tp_seq : 0u;
     const unsigned int tp_tag_base = tp_seq * (unsigned int)(2 * p.layers + 1);
     int tp_ar = 0;
+    float row_scale = 1.0f;
 
     // One matrix: for every K chunk, `stage_chunk(k0, klen)` leaves the activations of that
     // chunk in act_s and their digit planes in `dig`; then every row block of the CTA walks the
@@ -1379,16 +1400,16 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 if (n_rb > 1) { acc[0] = 0.0f; acc[1] = 0.0f; }
                 if (tiles == 1 && p.one_tile_16) {
                     consume_stages<1>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<1>(p, red, tiles, row_base, r1, out, store, acc, resid, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<1>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
                 } else if (tiles <= 2) {
                     consume_stages<2>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<2>(p, red, tiles, row_base, r1, out, store, acc, resid, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<2>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
                 } else if (!SIMPLE && tiles <= 4) {   // (small models have no 3- or 4-tile slab)
                     consume_stages<4>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<4>(p, red, tiles, row_base, r1, out, store, acc, resid, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<4>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
                 } else {
                     consume_stages<8>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<8>(p, red, tiles, row_base, r1, out, store, acc, resid, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<8>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
                 }
             }
         }
@@ -1450,12 +1471,34 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
     grid_barrier(p, epoch);
 
     // activation staging of the three kinds of GEMV input (each ends with the digit planes)
+    // x * gamma goes into the planes at once; the inverse rms, a factor of the whole row, meets the sums in the store
+    // (the reduction and a pass through shared memory were on the way to the first product, twice per layer)
+    const bool x_aligned = (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
     auto stage_normed = [&](const float *gamma) {
-        stage_norm(gamma);
-        quantize_activation(act_s, dig, H, false);
+        float ss = 0.0f;
+        for (int k = tid * 8; k < H; k += DS_CONSUMERS * 8) {   // (hidden % 512 == 0: whole warps)
+            float v[8], g[8];
+            ldcg8(p.x + k, v, x_aligned);
+            ldcg8(gamma + k, g);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                ss = fmaf(v[t], v[t], ss);
+                v[t] *= g[t];
+            }
+            quantize_registers(v, dig, k);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) misc[warp] = ss;
+        cons_sync();
+        float total = 0.0f;
+#pragma unroll
+        for (int w = 0; w < DS_CONSUMER_WARPS; ++w) total += misc[w];
+        row_scale = 1.0f / sqrtf(total / (float)H + p.eps);
     };
     // merge of the attention splits (the usual max-rescaling of a split softmax)
     auto stage_attention = [&]() {
+        row_scale = 1.0f;
         const int AW = p.n_q * p.d_head;
         if (!SIMPLE && p.attn_grouped) {
 #pragma unroll 4
@@ -1510,28 +1553,35 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
 #pragma unroll
                 for (int sp = 0; sp < 4; ++sp) wtab[tid * 4 + sp] = w[sp] * invL;
             }
-            // 4 x 512 elements per pass, their partial sums in registers across the barrier
-            for (int base = 0; base < AW; base += 4 * DS_CONSUMERS) {
-                float a[4][4];
+            // eight elements of a head per thread, their partial sums in registers across the barrier, straight into
+            // the digit planes (records start at multiples of d + 2 floats: 8-byte loads)
+            for (int base = 0; base < AW; base += 8 * DS_CONSUMERS) {
+                const int i = base + tid * 8;
+                const bool on = i < AW;   // (n_q * d_head % 512 == 0: whole warps)
+                const int hh = i / p.d_head, dd = i - hh * p.d_head;
+                const float *pp = p.attn + (size_t)hh * p.splits * (p.d_head + 2) + dd;
+                float2 a[4][4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int i = base + tid + j * DS_CONSUMERS;
-                    const int hh = i / p.d_head, dd = i - hh * p.d_head;
-                    const float *pp = p.attn + (size_t)hh * p.splits * (p.d_head + 2) + dd;
+                for (int sp = 0; sp < 4; ++sp) {
 #pragma unroll
-                    for (int sp = 0; sp < 4; ++sp)
-                        a[j][sp] = (i < AW && sp < p.splits) ? __ldcg(pp + (size_t)sp * (p.d_head + 2)) : 0.0f;
+                    for (int j = 0; j < 4; ++j)
+                        a[sp][j] = on && sp < p.splits ? __ldcg(reinterpret_cast<const float2 *>(pp + (size_t)sp * (p.d_head + 2)) + j)
+                                                       : make_float2(0.0f, 0.0f);
                 }
                 if (base == 0) cons_sync();  // the weight table is complete
+                if (on) {
+                    const float *w = wtab + hh * 4;
+                    float v[8];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int i = base + tid + j * DS_CONSUMERS;
-                    if (i < AW) {
-                        const float *w = wtab + (i / p.d_head) * 4;
-                        act_s[i] = fmaf(w[3], a[j][3], fmaf(w[2], a[j][2], fmaf(w[1], a[j][1], w[0] * a[j][0])));
+                    for (int j = 0; j < 4; ++j) {
+                        v[2 * j] = fmaf(w[3], a[3][j].x, fmaf(w[2], a[2][j].x, fmaf(w[1], a[1][j].x, w[0] * a[0][j].x)));
+                        v[2 * j + 1] = fmaf(w[3], a[3][j].y, fmaf(w[2], a[2][j].y, fmaf(w[1], a[1][j].y, w[0] * a[0][j].y)));
                     }
+                    quantize_registers(v, dig, i);
                 }
             }
+            cons_sync();
+            return;
         } else {
 #pragma unroll 4
             for (int i = tid; i < AW; i += DS_CONSUMERS) {
@@ -1564,9 +1614,16 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
     // the MLP activations [k0, k0 + klen): already silu(gate) * up (paired), or formed here
     auto stage_mlp = [&](int k0, int klen) {
         if (k0 > 0) cons_sync();  // every warp is done with the previous chunk's act_s and planes
+        row_scale = 1.0f;
         if (p.pair_gu) {
-#pragma unroll 4
-            for (int i = tid; i < klen; i += DS_CONSUMERS) act_s[i] = __ldcg(p.gu + k0 + i);
+#pragma unroll 2
+            for (int k = tid * 8; k < klen; k += DS_CONSUMERS * 8) {   // (chunks are whole stages of 512)
+                float v[8];
+                ldcg8(p.gu + k0 + k, v);
+                quantize_registers(v, dig, k);
+            }
+            cons_sync();
+            return;
         } else {
             for (int i0 = tid; i0 < klen; i0 += 12 * DS_CONSUMERS) {
                 float g[12], u[12];
@@ -1965,7 +2022,8 @@ extern "C" int yscv_cuda_decode_plan_create_ex(yscv_cuda_ctx *ctx, const yscv_cu
         kptr[n_layers + l] = layers[l].d_kscale;
         vptr[n_layers + l] = layers[l].d_vscale;
     }
-    const size_t attn_floats = (size_t)batch * n_q * (size_t)(grouped ? g_splits : splits) * (d_head + 2);
+    // (rounded up: what follows is read 16 bytes at a time)
+    const size_t attn_floats = ((size_t)batch * n_q * (size_t)(grouped ? g_splits : splits) * (d_head + 2) + 3) / 4 * 4;
     const size_t scratch_floats = (size_t)batch * (qkv_rows + 2 * inter + attn_w + 2 * (size_t)grid) + attn_floats;
 #define PLAN_TRY(expr)                                                                       \
     do {                                                                                     \
