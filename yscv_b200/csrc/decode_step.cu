@@ -689,6 +689,12 @@ __device__ __forceinline__ void attention_merge(const StepParams &p, int h, floa
     cons_sync();  // scratch is reused
 }
 
+// Splits in use: a CTA takes up to 128 keys in one pass, so a short context needs fewer than p.splits, and the merge behind
+// reads fewer records. (The batch form merges all of them.)
+__device__ __forceinline__ int used_splits(const StepParams &p, int pos) {
+    return p.batch > 1 ? p.splits : min(p.splits, (pos + 128) / 128);
+}
+
 // Attention of the one query of head h over positions 0 .. pos, the keys dealt in contiguous
 // chunks to p.splits CTAs per head: RoPE of the head's q and of its KV head's new k, cache
 // append (one CTA per KV head), then this CTA's chunk of scores, a local softmax and the
@@ -714,7 +720,9 @@ __device__ __forceinline__ void attention_head(const StepParams &p, int layer, i
     const size_t kv_stride = (size_t)p.n_kv * d;
     const float *kbase = kc + (size_t)kvh * d, *vbase = vc + (size_t)kvh * d;
     const int limit = pos + 1;
-    const int chunk = (limit + p.splits - 1) / p.splits;
+    const int S = used_splits(p, pos);
+    if (split >= S) return;
+    const int chunk = (limit + S - 1) / S;
     const int k0 = split * chunk, k1 = min(limit, k0 + chunk);   // this CTA's keys
     float *po = attn_o + ((size_t)h * p.splits + split) * (d + 2);
     if (k0 >= k1) {  // nothing for this split yet: the neutral element of the merge
@@ -949,7 +957,9 @@ __device__ __forceinline__ void attention_head_i8(const StepParams &p, int h, in
     const size_t kv_stride = (size_t)p.n_kv * d;   // bytes per cached row
     const int8_t *kbase = kc8 + (size_t)kvh * d, *vbase = vc8 + (size_t)kvh * d;
     const int limit = pos + 1;
-    const int chunk = (limit + p.splits - 1) / p.splits;
+    const int S = used_splits(p, pos);
+    if (split >= S) return;
+    const int chunk = (limit + S - 1) / S;
     const int k0 = split * chunk, k1 = min(limit, k0 + chunk);
     float *po = p.attn + ((size_t)h * p.splits + split) * (d + 2);
     if (k0 >= k1) {
@@ -1499,7 +1509,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
     // merge of the attention splits (the usual max-rescaling of a split softmax)
     auto stage_attention = [&]() {
         row_scale = 1.0f;
-        const int AW = p.n_q * p.d_head;
+        const int AW = p.n_q * p.d_head, S = used_splits(p, pos);
         if (!SIMPLE && p.attn_grouped) {
 #pragma unroll 4
             for (int i = tid; i < AW; i += DS_CONSUMERS) act_s[i] = __ldcg(p.attn_out + i);
@@ -1509,16 +1519,16 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
             if (tid < p.n_q) {
                 const float *pp = p.attn + (size_t)tid * p.splits * (p.d_head + 2) + p.d_head;
                 float M = -INFINITY;
-                for (int sp = 0; sp < p.splits; ++sp) M = fmaxf(M, __ldcg(pp + (size_t)sp * (p.d_head + 2)));
+                for (int sp = 0; sp < S; ++sp) M = fmaxf(M, __ldcg(pp + (size_t)sp * (p.d_head + 2)));
                 float L = 0.0f;
-                for (int sp = 0; sp < p.splits; ++sp) {
+                for (int sp = 0; sp < S; ++sp) {
                     const float m = __ldcg(pp + (size_t)sp * (p.d_head + 2));
                     const float w = m > -INFINITY ? expf(m - M) : 0.0f;
                     L = fmaf(w, __ldcg(pp + (size_t)sp * (p.d_head + 2) + 1), L);
                     wtab[tid * 16 + sp] = w;
                 }
                 const float invL = L > 0.0f ? 1.0f / L : 0.0f;
-                for (int sp = 0; sp < p.splits; ++sp) wtab[tid * 16 + sp] *= invL;
+                for (int sp = 0; sp < S; ++sp) wtab[tid * 16 + sp] *= invL;
             }
             cons_sync();
             for (int i = tid; i < AW; i += DS_CONSUMERS) {
@@ -1527,7 +1537,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 const float *w = wtab + hh * 16;
                 float acc = 0.0f;
 #pragma unroll 4
-                for (int sp = 0; sp < p.splits; ++sp) acc = fmaf(w[sp], __ldcg(pp + (size_t)sp * (p.d_head + 2)), acc);
+                for (int sp = 0; sp < S; ++sp) acc = fmaf(w[sp], __ldcg(pp + (size_t)sp * (p.d_head + 2)), acc);
                 act_s[i] = acc;
             }
         } else if (p.merge_table) {
@@ -1537,7 +1547,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 float m[4], e[4];
 #pragma unroll
                 for (int sp = 0; sp < 4; ++sp) {
-                    const bool on = sp < p.splits;
+                    const bool on = sp < S;
                     m[sp] = on ? __ldcg(pp + (size_t)sp * (p.d_head + 2)) : -INFINITY;
                     e[sp] = on ? __ldcg(pp + (size_t)sp * (p.d_head + 2) + 1) : 0.0f;
                 }
@@ -1565,7 +1575,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 for (int sp = 0; sp < 4; ++sp) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        a[sp][j] = on && sp < p.splits ? __ldcg(reinterpret_cast<const float2 *>(pp + (size_t)sp * (p.d_head + 2)) + j)
+                        a[sp][j] = on && sp < S ? __ldcg(reinterpret_cast<const float2 *>(pp + (size_t)sp * (p.d_head + 2)) + j)
                                                        : make_float2(0.0f, 0.0f);
                 }
                 if (base == 0) cons_sync();  // the weight table is complete
@@ -1590,7 +1600,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 float a[4], m[4], e[4];  // splits <= 4
 #pragma unroll
                 for (int sp = 0; sp < 4; ++sp) {
-                    const bool on = sp < p.splits;
+                    const bool on = sp < S;
                     a[sp] = on ? __ldcg(pp + (size_t)sp * (p.d_head + 2) + dd) : 0.0f;
                     m[sp] = on ? __ldcg(pp + (size_t)sp * (p.d_head + 2) + p.d_head) : -INFINITY;
                     e[sp] = on ? __ldcg(pp + (size_t)sp * (p.d_head + 2) + p.d_head + 1) : 0.0f;
