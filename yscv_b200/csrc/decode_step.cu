@@ -428,7 +428,7 @@ __device__ __forceinline__ void consume_stages(const StepParams &p, const unsign
 template <int TP2>
 __device__ __forceinline__ void finish_rows(const StepParams &p, float *red, int tiles, int row_base, int r1,
                                             float *out, int store, const float (&acc)[2], float resid, float row_scale,
-                                            unsigned int tp_tag, int tp_parity) {
+                                            unsigned int tp_tag, int tp_parity, bool more) {
     constexpr int GS = DS_GS;
     constexpr int KSL = (16 / TP2 < GS) ? 16 / TP2 : GS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -471,7 +471,7 @@ __device__ __forceinline__ void finish_rows(const StepParams &p, float *red, int
             out[my_row] = store == 1 ? resid + v : v;
         }
     }
-    cons_sync();  // `red` is reused by the next block
+    if (more) cons_sync();  // `red` is reused by the next block (behind the last one comes a grid barrier)
 }
 
 // Grouped attention, phase 1. CTA (kvh, split): RoPE of the group's queries and of the new key,
@@ -882,7 +882,7 @@ __device__ __forceinline__ void attention_head(const StepParams &p, int layer, i
         po[tid] = v;
     }
     if (tid == 0) { po[d] = mx; po[d + 1] = se; }
-    cons_sync();  // scratch is reused
+    if (qkv_base) cons_sync();  // scratch is reused by the next work item (else a grid barrier follows)
 }
 
 // ---- int8 KV cache (KvDtype::I8 of the reference, crates/yscv-onnx/src/runner/kv_cache.rs:44-90) ----
@@ -1410,16 +1410,16 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
                 if (n_rb > 1) { acc[0] = 0.0f; acc[1] = 0.0f; }
                 if (tiles == 1 && p.one_tile_16) {
                     consume_stages<1>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<1>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<1>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1, n_rb > 1);
                 } else if (tiles <= 2) {
                     consume_stages<2>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<2>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<2>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1, n_rb > 1);
                 } else if (!SIMPLE && tiles <= 4) {   // (small models have no 3- or 4-tile slab)
                     consume_stages<4>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<4>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<4>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1, n_rb > 1);
                 } else {
                     consume_stages<8>(p, smem, bar_full, bar_empty, dig, c, tiles, cs, ce, kps, cs, acc, dead);
-                    if (last) finish_rows<8>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1);
+                    if (last) finish_rows<8>(p, red, tiles, row_base, r1, out, store, acc, resid, row_scale, tp_tag, tp_ar & 1, n_rb > 1);
                 }
             }
         }
