@@ -116,10 +116,10 @@ void yscv_cuda_quant_stats_reset(void);
  * (crates/yscv-kernels/src/ops/int4_matmul.rs:548-605). */
 int yscv_cuda_ctx_set_int4_prefill_exact(yscv_cuda_ctx *ctx, int exact);
 /* Kernel-selection switch of the bf16 prefill GEMM: enable != 0 (the default) lets prefills
- * with at least one 512-row x 256-token tile per CTA pair run on CTA pairs (tcgen05
- * cta_group::2: each CTA dequantises 256 weight rows and stages half of the activation tile);
- * 0 keeps the one-CTA kernel. Same products, and the same summation order over k except for the
- * tiles of a last round that is split over k (the report says how many), which are added in parts. */
+ * run on CTA pairs where a modelled time favours them (tcgen05 cta_group::2, 512 rows x up to 256 tokens:
+ * each CTA dequantises 256 weight rows and stages half of the activation tile);
+ * 0 keeps the one-CTA kernel. Same products, and the same summation order over k except where k is split
+ * (tiles of a last round of pairs, slices of the one-CTA form; the report says), which is added in parts. */
 int yscv_cuda_ctx_set_int4_prefill_cta_pairs(yscv_cuda_ctx *ctx, int enable);
 /* Kernel-selection switch of the int8 GEMM, like the reference's environment gates on its
  * int8 paths (crates/yscv-onnx/src/runner/quant_stats.rs:68-71). The GEMM has a one-CTA kernel

@@ -393,8 +393,8 @@ int4_prefill_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_
 // Two CTAs on the two SMs of a TPC (a cluster of 2) share a tile of 512 weight rows x BT tokens (up to 256).
 // Each CTA dequantises its own 256 weight rows (two 128-row tiles, as the NA = 2 form above) and
 // stages HALF of the activation tile of a k block (BT / 2 tokens); the leader (cluster rank 0) issues
-// MMAs of M = 256, N = 256 that read both CTAs' shared memory and leave rows 0..127 in its own
-// TMEM and rows 128..255 in the peer's. Per k block an SM then pulls 8 KB of nibbles + 16 KB of
+// MMAs of M = 256, N = BT that read both CTAs' shared memory and leave rows 0..127 in its own
+// TMEM and rows 128..255 in the peer's. Per k block of 256 tokens an SM then pulls 8 KB of nibbles + 16 KB of
 // activations from L2 instead of 8 + 32 KB, and its tensor core reads half the activation bytes
 // from shared memory per flop: the two limits of the one-CTA form.
 //
@@ -440,7 +440,7 @@ __device__ __forceinline__ void pp_commit(uint32_t bar) {
 // pairs idle when few tiles remain (2048 x 8192 x 10240: 160 tiles on 74 pairs): the remaining tiles'
 // k blocks in one sequence, cut into equal ranges. A range is shorter than a tile, so it meets at most
 // two; the part of tile i (of the remaining ones) done by pair c is slot c + i of `parts`,
-// [256 tokens][512 rows] fp32, and pp_join_kernel adds a tile's parts in pair order.
+// [up to 256 tokens][512 rows] fp32, and pp_join_kernel adds a tile's parts in pair order.
 struct PPWalk {
     int t, full, pairs, kb, pair, u, u1;
     __device__ PPWalk(const PGParams &p, int pair_, int n_pairs, int tiles)
