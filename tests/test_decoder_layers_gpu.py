@@ -112,6 +112,48 @@ def test_step_attention_positions(tctx, n_q, n_kv, d, batch, kv_int8):
     dec.close()
 
 
+@pytest.mark.parametrize("n_q,n_kv", [(8, 2), (32, 4)])   # up to 16 and up to 4 key splits per head
+@pytest.mark.parametrize("kv_int8", [False, True])
+def test_one_launch_step_positions(tctx, n_q, n_kv, kv_int8):
+    """The one-launch step against the chain at positions where one more key split comes into use (128 keys each), with
+    the bounds above: the linears quantise their activations to 2^-22 of a group's maximum in both forms, but before or
+    after the norm's row factor, a few 1e-7 a linear."""
+    ctx, s = tctx
+    cfg = DecoderConfig(layers=2, hidden=512, mlp=1024, n_q=n_q, n_kv=n_kv, head_dim=64, vocab=300)
+    max_seq = 600
+    dec = Int4Decoder(ctx, cfg, 1, max_seq, s, seed=7, kv_int8=kv_int8)
+    assert dec.plan is not None and dec.layers is not None
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n_q)
+    with torch.cuda.stream(s):
+        caches = dec.kcache + dec.vcache
+        tables = dec.kscale + dec.vscale if kv_int8 else []
+        fill = [torch.randint(-127, 128, c.shape, dtype=torch.int8, device="cuda", generator=g) if kv_int8
+                else torch.randn(c.shape, device="cuda", generator=g) for c in caches]
+        fill += [0.005 + 0.01 * torch.rand(t.shape, device="cuda", generator=g) for t in tables]
+        for p in (0, 1, 127, 128, 129, 255, 256, 257, 383, 384, 385, 511, 512, 513, max_seq - 1):
+            res = []
+            for one in (True, False):
+                dec.one_launch = one
+                for dst, src in zip(caches + tables, fill):
+                    dst.copy_(src)
+                dec.pos.fill_(p)
+                dec.next_tokens.fill_(p % cfg.vocab)
+                lg = dec.forward(dec.next_tokens, 1).clone()
+                assert int(dec.pos.reshape(-1)[0]) == p + 1
+                res.append([lg] + [c[:, p].float().clone() for c in caches + tables])
+            s.synchronize()
+            assert ctx.device_status() == 0
+            a, b = res
+            assert float((a[0] - b[0]).norm() / b[0].norm()) <= (2e-3 if kv_int8 else 1e-5), p
+            for i, (x, y) in enumerate(zip(a[1:], b[1:])):
+                if kv_int8 and i < len(caches):   # a value on a rounding boundary
+                    assert float((x - y).abs().max()) <= 1, p
+                else:
+                    assert float((x - y).norm()) <= 1e-5 * float(y.norm()), p
+    dec.close()
+
+
 def test_workspace_of_another_size(tctx):
     """Without room for partial sums the matmuls join them; without room for the pass the call is refused."""
     ctx, s = tctx

@@ -45,12 +45,13 @@ class DecoderConfig:
     weight_std: float = 0.02
 
 
-# Steps of 2..8 sequences run as the operator chain from this hidden size on, as one launch below: the line lies
-# where the chain is the faster form eagerly too (a launch costs host time there). us per step, chain / one launch,
-# 200 cached positions, replayed and eager: hidden 512 (8 layers) batch 2 251 / 286 and 360 / 287, batch 8 318 / 351
-# and 442 / 351; 1024 (16 layers) batch 2 574 / 754 and 689 / 754, batch 8 713 / 884 and 846 / 884; 2048 (22
-# layers) batch 2 983 / 1363 and 1043 / 1362, batch 8 1252 / 1782 and 1320 / 1781. Longer caches favour the chain:
-# after 1500 positions 1427 / 2809 and 1494 / 2810 there. (Above 2048 the batch form has no plan.)
+# Steps of 2..8 sequences run as the operator chain from this hidden size on, as one launch below. us per step, chain / one
+# launch, 200 cached positions, replayed and eager: hidden 512 (8 layers) batch 2 211 / 275 and 226 / 275, batch 8 217 / 336
+# and 235 / 337; 1024 (16 layers) batch 2 486 / 787 and 533 / 788, batch 8 529 / 876 and 565 / 877; 2048 (22 layers) batch
+# 2 883 / 1344 and 933 / 1344, batch 8 965 / 1805 and 1015 / 1805, after 1500 positions 948 / 1593 and 1185 / 2801 replayed. The
+# line lay where the chain became the faster form eagerly too; with the layers behind one call it is ahead at 512 as well, by
+# 50 to 100 us, but there a step is one launch (about 60 for the chain) to programs that count on it, and one_launch = False
+# chooses the chain. (Above 2048 the batch form has no plan.)
 CHAIN_HIDDEN = 1024
 
 TINYLLAMA_1B = DecoderConfig(22, 2048, 5632, 32, 4, 64, 32000, 1e-5, 10000.0)
