@@ -63,6 +63,43 @@ def test_layers_against_single_operators(tctx, cfg, batch, prompt, kv_int8):
             assert float((a - b).norm() / b.norm()) <= 1.1e-2
 
 
+@pytest.mark.parametrize("batch", [2, 20])
+@pytest.mark.parametrize("kv_int8", [False, True])
+def test_a_decoder_given_other_tensors(tctx, batch, kv_int8):
+    """A pass reads the caches, gamma and weights that the decoder holds now, at an odd address of gamma too: equal bits
+    to a decoder that runs operator by operator on the same (up to 16 rows; above, the bound given above)."""
+    ctx, s = tctx
+    tokens = torch.randint(0, SMALL.vocab, (batch, 3), dtype=torch.int32, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    torch.cuda.synchronize()
+    one, other = (Int4Decoder(ctx, SMALL, batch, 140, s, seed=4, fused_step=False, kv_int8=kv_int8) for _ in range(2))
+    donor = Int4Decoder(ctx, SMALL, batch, 140, s, seed=5, fused_step=False, kv_int8=kv_int8)
+    other.layers = None
+    kept = []   # what the decoders held before stays allocated
+    with torch.cuda.stream(s):
+        gammas = [torch.rand(SMALL.hidden, device="cuda") + 0.5, (torch.rand(SMALL.hidden + 1, device="cuda") + 0.5)[1:]]
+        for step in ("nothing", "caches", "gamma", "weights", "odd gamma"):
+            got = []
+            for dec in (one, other):
+                kept.append((dec.kcache, dec.vcache, dec.gamma, dec.wqkv, dec.wo, dec.wgu, dec.wdown, *([dec.kscale, dec.vscale] if kv_int8 else [])))
+                if step == "caches":
+                    dec.kcache, dec.vcache = ([torch.zeros_like(c) for c in cs] for cs in (dec.kcache, dec.vcache))
+                    if kv_int8:
+                        dec.kscale, dec.vscale = ([torch.zeros_like(c) for c in cs] for cs in (dec.kscale, dec.vscale))
+                elif step == "weights":
+                    dec.wqkv, dec.wo, dec.wgu, dec.wdown = donor.wqkv, list(reversed(donor.wo)), donor.wgu, donor.wdown
+                elif "gamma" in step:
+                    dec.gamma = gammas[step == "odd gamma"]
+                dec.reset()
+                lg = dec.prefill(tokens).clone()
+                got.append([lg] + [c.clone() for c in (dec.kscale + dec.vscale if kv_int8 else dec.kcache + dec.vcache)])
+            s.synchronize()
+            for a, b in zip(*got):
+                assert torch.equal(a, b) if batch == 2 else float((a - b).norm() / b.norm()) <= 1.1e-2, step
+    assert ctx.device_status() == 0
+    for dec in (one, other, donor):
+        dec.close()
+
+
 HEADS = [  # n_q, n_kv, d: groups of 1 to 8 heads, both head sizes
     (8, 1, 64), (6, 6, 64), (12, 4, 64), (4, 2, 128), (8, 1, 128), (20, 4, 64)]
 

@@ -94,17 +94,13 @@ class Int4Decoder:
         self._bufs = {}
         self.graph = None
         stream.synchronize()
-        layers_of = [dict(qkv=self.wqkv[l].handle, o=self.wo[l].handle, gate_up=self.wgu[l].handle,
-                          down=self.wdown[l].handle, gamma_attn=self.gamma.data_ptr(),
-                          gamma_mlp=self.gamma.data_ptr(), kcache=self.kcache[l].data_ptr(),
-                          vcache=self.vcache[l].data_ptr(),
-                          kscale=self.kscale[l].data_ptr() if kv_int8 else None,
-                          vscale=self.vscale[l].data_ptr() if kv_int8 else None) for l in range(self.n_layers)]
+        layers_of = self._layers_of()
         # one GPU: the chain of a step or prompt pass as one library call (a collective between the operators
         # needs them one by one)
         self.layers = None
         if tp_size == 1 and self.n_layers > 0 and cfg.hidden % 8 == 0 and cfg.hidden <= 8192 and self.mlp_l % 8 == 0 and cfg.head_dim % 8 == 0:
             self.layers = ctx.decode_layers(layers_of)
+            self._layers_at = self._addresses()
         # batch 1: the whole single-token step as one persistent kernel per GPU, when the
         # shapes allow it (the library says which do). With tensor parallelism the ranks'
         # kernels exchange their partial sums through exchange regions mapped with CUDA IPC;
@@ -211,6 +207,31 @@ class Int4Decoder:
         return _Keep(*args, **kw)
 
     # ---- forward -------------------------------------------------------------------
+    def _layers_of(self):
+        """The layers as decode_plan() and decode_layers() take them."""
+        g, i8 = self.gamma.data_ptr(), self.kv_int8
+        return [dict(qkv=self.wqkv[l].handle, o=self.wo[l].handle, gate_up=self.wgu[l].handle, down=self.wdown[l].handle,
+                     gamma_attn=g, gamma_mlp=g, kcache=self.kcache[l].data_ptr(), vcache=self.vcache[l].data_ptr(),
+                     kscale=self.kscale[l].data_ptr() if i8 else None,
+                     vscale=self.vscale[l].data_ptr() if i8 else None) for l in range(self.n_layers)]
+
+    def _addresses(self):
+        """What a chain pass reads through self.layers. A program may give the decoder other caches, gammas or weights
+        between passes; 9 us for 22 layers, against 47 to write the array anew. (A plan and a captured graph keep
+        the addresses they were made with.)"""
+        caches = self.kcache + self.vcache + (self.kscale + self.vscale if self.kv_int8 else [])
+        weights = self.wqkv + self.wo + self.wgu + self.wdown
+        return self.gamma.data_ptr(), [t.data_ptr() for t in caches], [w.handle.handle for w in weights]
+
+    def _chain_layers(self):
+        """self.layers with today's addresses, or None where the pass has to go operator by operator."""
+        if self.layers is None or self.gamma.data_ptr() & 15:
+            return None
+        at = self._addresses()
+        if at != self._layers_at:
+            self.layers[:], self._layers_at = self.ctx.decode_layers(self._layers_of()), at
+        return self.layers
+
     def _buf(self, name, *shape, dtype=torch.float32):
         key = (name, shape, dtype)
         if key not in self._bufs:
@@ -231,14 +252,15 @@ class Int4Decoder:
         rows = B * seq
         qkv_w = (self.nq_l + 2 * self.nkv_l) * d
         x = self._buf("x", rows, H)
-        if self.layers is not None and not (self.one_launch and seq == 1):
+        layers = None if self.one_launch and seq == 1 else self._chain_layers()
+        if layers is not None:
             shape = (H, self.mlp_l, self.nq_l, self.nkv_l, d)
-            need = ctx.decoder_layers_workspace(self.layers, *shape, B, seq)
+            need = ctx.decoder_layers_workspace(layers, *shape, B, seq)
             ws = self._buf("layers", need, dtype=torch.uint8)
             last = self._buf("last", B, H)
             logits = self._buf("logits", B, c.vocab)
             ctx.embedding_dev(self.embedding.data_ptr(), c.vocab, H, tokens.data_ptr(), rows, x.data_ptr())
-            ctx.decoder_layers_dev(self.layers, *shape, self.max_seq, c.eps, c.rope_theta, self.kv_int8, B, seq, self.pos.data_ptr(),
+            ctx.decoder_layers_dev(layers, *shape, self.max_seq, c.eps, c.rope_theta, self.kv_int8, B, seq, self.pos.data_ptr(),
                                    x.data_ptr(), self.gamma.data_ptr(), last.data_ptr(), ws.data_ptr(), need)
             return self._head(last, logits, seq)
         h = self._buf("h", rows, H)
