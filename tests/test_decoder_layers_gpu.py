@@ -6,7 +6,7 @@ import torch
 
 import yscv_b200
 from yscv_b200 import synth
-from yscv_b200.decoder import DecoderConfig, Int4Decoder
+from yscv_b200.decoder import DecoderConfig, Int4Decoder, Int4Linear
 
 pytestmark = pytest.mark.gpu
 
@@ -98,6 +98,60 @@ def test_a_decoder_given_other_tensors(tctx, batch, kv_int8):
     assert ctx.device_status() == 0
     for dec in (one, other, donor):
         dec.close()
+
+
+def _repack(ctx, dec, layer, group, seed):
+    """Other random weights of the layer's shapes, packed in groups of `group`."""
+    for lins in (dec.wqkv, dec.wo, dec.wgu, dec.wdown):
+        n, k = lins[layer].n, lins[layer].k
+        w = torch.randn(n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(seed + n)) * 0.02
+        packed, scales = torch.empty(n, k // 2, dtype=torch.uint8, device="cuda"), torch.empty(n, k // group, device="cuda")
+        ctx.pack_int4_dev(w.data_ptr(), n, k, group, packed.data_ptr(), scales.data_ptr())
+        lins[layer] = Int4Linear(ctx, packed, scales, n, k, group)
+
+
+@pytest.mark.parametrize("mlp,batch", [(28672, 1), (8192, 2), (8192, 4), (5632, 9), (65536, 12), (5632, 24)])
+@pytest.mark.parametrize("groups", [(64, 32, 32), (32, 64, 32)])
+def test_layers_of_different_groups(tctx, mlp, batch, groups):
+    """Groups of 64 take fp32 activations, groups of 32 digit planes, fp16 terms, bf16 with k slices: the workspace holds
+    the largest form of any layer, nothing behind it is written, and the results are the single operators' (bound above; from
+    17 rows on those run in fp32, and each of 12 linears rounds weights and activations to bf16: 2^-8 * sqrt(24) = 1.9e-2)."""
+    ctx, s = tctx
+    cfg = DecoderConfig(layers=3, hidden=1024, mlp=mlp, n_q=8, n_kv=2, head_dim=64, vocab=300)
+    shape = (cfg.hidden, cfg.mlp, cfg.n_q, cfg.n_kv, cfg.head_dim)
+    dec = Int4Decoder(ctx, cfg, batch, 140, s, seed=8, fused_step=False)
+    largest = ctx.decoder_layers_workspace(dec.layers, *shape, batch, 1)
+    with torch.cuda.stream(s):
+        for l, group in enumerate(groups):
+            _repack(ctx, dec, l, group, 10 * l)
+        layers = ctx.decode_layers(dec._layers_of())
+        need = ctx.decoder_layers_workspace(layers, *shape, batch, 1)
+        assert need >= largest
+        x0 = torch.randn(batch, cfg.hidden, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+        x, last = x0.clone(), torch.empty(batch, cfg.hidden, device="cuda")
+        ws = torch.full((need + 4096,), 77, dtype=torch.uint8, device="cuda")
+        ctx.decoder_layers_dev(layers, *shape, 140, cfg.eps, cfg.rope_theta, False, batch, 1, dec.pos.data_ptr(), x.data_ptr(),
+                               dec.gamma.data_ptr(), last.data_ptr(), ws.data_ptr(), need)
+        assert bool((ws[need:] == 77).all())
+        got = []
+        tokens = torch.arange(batch, dtype=torch.int32, device="cuda")
+        for form in (dec.layers, None):
+            dec.layers = form
+            ctx.set_int4_prefill_exact(form is None)
+            dec.reset()
+            got.append(dec.forward(tokens, 1).clone())
+        # the direct call against the operators from the same residual rows
+        dec.embedding[:batch].copy_(x0)
+        dec.reset()
+        dec.forward(tokens, 1)
+        want = dec._buf("h", batch, cfg.hidden)
+        ctx.set_int4_prefill_exact(False)
+    s.synchronize()
+    assert ctx.device_status() == 0
+    tol = 1.9e-2 if batch > 16 else 1e-5
+    assert float((got[0] - got[1]).norm() / got[1].norm()) <= tol
+    assert float((last - want).norm() / want.norm()) <= tol
+    dec.close()
 
 
 HEADS = [  # n_q, n_kv, d: groups of 1 to 8 heads, both head sizes

@@ -24,7 +24,14 @@ struct Layout {
     int parts_qkv, parts_o, parts_gu, parts_down;
 };
 
-Layout layout(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer &l, const Shape &s, bool apart) {
+// What the form of a weight's activations depends on besides its shape, which check() makes the same in every layer
+bool alike(const yscv_cuda_int4_weight *a, const yscv_cuda_int4_weight *b) {
+    auto skew = [](const yscv_cuda_int4_weight *w) { return ((reinterpret_cast<uintptr_t>(w->d_packed) | reinterpret_cast<uintptr_t>(w->d_scales)) & 15) != 0; };
+    return a->group_size == b->group_size && skew(a) == skew(b);
+}
+
+// Room for the activations in every layer's form, and for the partial sums of the layer that leaves most
+Layout layout(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_layers, const Shape &s, bool apart) {
     const size_t m = s.rows();
     Layout o = {};
     size_t at = 0, act = 0;
@@ -33,16 +40,22 @@ Layout layout(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer &l, const Shape &
         at += (bytes + 255) / 256 * 256;
         return p;
     };
-    auto parts = [&](const yscv_cuda_int4_weight *w) {
+    auto fit = [&](const yscv_cuda_int4_weight *w, int &parts) {
         const int form = int4_act_form(ctx, w, m);
-        const size_t f32 = act_bytes(ACT_F32, m, w->k), own = act_bytes(form, m, w->k);
-        act = std::max(act, std::max(f32, own));
-        return apart ? int4_form_parts(ctx, w, form, m) : 1;
+        act = std::max(act, std::max(act_bytes(ACT_F32, m, w->k), act_bytes(form, m, w->k)));
+        // (run() may find the library's workspace there that was not to be had a moment ago)
+        if (int4_batch_exact_wins(m, w->m_w, w->k, w->group_size)) act = std::max(act, act_bytes(ACT_TERMS, m, w->k));
+        parts = std::max(parts, apart ? int4_form_parts(ctx, w, form, m) : 1);
     };
-    o.parts_qkv = parts(l.qkv);
-    o.parts_o = parts(l.o);
-    o.parts_gu = parts(l.gate_up);
-    o.parts_down = parts(l.down);
+    const yscv_cuda_decode_layer &l0 = layers[0];
+    for (size_t i = 0; i < n_layers; ++i) {
+        const yscv_cuda_decode_layer &l = layers[i];
+        if (i > 0 && alike(l.qkv, l0.qkv) && alike(l.o, l0.o) && alike(l.gate_up, l0.gate_up) && alike(l.down, l0.down)) continue;
+        fit(l.qkv, o.parts_qkv);
+        fit(l.o, o.parts_o);
+        fit(l.gate_up, o.parts_gu);
+        fit(l.down, o.parts_down);
+    }
     o.act = take(act);
     o.qkv = take(o.parts_qkv * m * s.qkv() * sizeof(float));
     o.q = take(o.parts_qkv > 1 ? m * s.n_q * s.d * sizeof(float) : 0);
@@ -136,7 +149,7 @@ int yscv_cuda_decoder_layers_workspace(yscv_cuda_ctx *ctx, const yscv_cuda_decod
     const int rc = check(ctx, layers, n_layers, s, 0);
     if (rc) return rc;
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
-    *bytes = batch * seq == 0 ? 0 : layout(ctx, layers[0], s, true).total;
+    *bytes = batch * seq == 0 ? 0 : layout(ctx, layers, n_layers, s, true).total;
     return YSCV_CUDA_OK;
 }
 
@@ -155,9 +168,9 @@ int yscv_cuda_decoder_layers_dev(yscv_cuda_ctx *ctx, const yscv_cuda_decode_laye
          reinterpret_cast<uintptr_t>(d_workspace)) & 15)
         return fail(YSCV_CUDA_ERR_UNSUPPORTED, "d_x, d_final_gamma, d_last and the workspace must be 16-byte aligned");
     YSCV_CUDA_TRY(cudaSetDevice(ctx->device));
-    Layout o = layout(ctx, layers[0], s, true);
+    Layout o = layout(ctx, layers, n_layers, s, true);
     // (room for partial sums is wanted only where the library can use its own workspace, which it may have got since)
-    if (o.total > workspace_bytes) o = layout(ctx, layers[0], s, false);
+    if (o.total > workspace_bytes) o = layout(ctx, layers, n_layers, s, false);
     if (o.total > workspace_bytes)
         return fail(YSCV_CUDA_ERR_BAD_ARG, "workspace of %zu bytes is too small: %zu needed", workspace_bytes, o.total);
     unsigned char *ws = static_cast<unsigned char *>(d_workspace);
