@@ -1,6 +1,10 @@
 """Host-side pieces of the C ABI that make no CUDA call: the packed-int4 container, the
 MatMulNBits nibble convention in both directions, the prepack gates, the empty weight table
 and the operator counters. CPU only."""
+import os
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -74,3 +78,15 @@ def test_quant_stats_start_at_zero_and_have_no_cpu_fallback():
     st = yscv_b200.quant_stats()
     assert set(st) == {n for n, _ in binding.QuantStats._fields_}
     assert all(v == 0 for v in st.values())
+
+
+def test_buffers_when_memory_runs_out(tmp_path):
+    """The library's device buffers, host code, built against a runtime that refuses memory on request: a call that works
+    on a buffer and asks for a larger one keeps the block it has when there is none."""
+    here = Path(__file__).resolve().parent
+    exe = tmp_path / "device_buffer_check"
+    include = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-Wall", "-I", str(include), "-o", str(exe), str(here / "device_buffer_check.cpp"),
+                    "-x", "c++", str(here.parent / "yscv_b200" / "csrc" / "device_buffer.cu")], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0, done.stdout

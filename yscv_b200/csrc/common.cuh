@@ -58,12 +58,13 @@ struct DeviceBuffer {
     // (asking the stream takes 0.15 us, which calls that launch one kernel and nothing else would feel)
     int reserve(size_t want);
     // The same for a buffer that a call can do without: false (and no error) where it would have to grow
-    // inside a capture or the memory is not there.
-    bool try_reserve(size_t want, cudaStream_t stream);
+    // inside a capture or the memory is not there. in_use: the caller works on the block that there is, which
+    // stays where the larger one is not to be had (contents do not move along).
+    bool try_reserve(size_t want, cudaStream_t stream, bool in_use = false);
     void release();
 
   private:
-    cudaError_t grow(size_t want);
+    cudaError_t grow(size_t want, bool in_use);
     bool note_capture(cudaStream_t stream);
 };
 

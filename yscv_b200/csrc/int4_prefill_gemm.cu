@@ -933,10 +933,11 @@ int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales
     p.ksplit = (p.k_blocks + p.kb_per - 1) / p.kb_per;   // no empty slice (33 blocks in 8 slices of 5: seven slices)
     float *kernel_out = out;
     if (p.ksplit > 1 && !batch && !use_pairs) {
-        // the slices lie behind the activations (which are not there yet)
+        // the slices lie behind the activations (which are not there yet, but have their place in `scratch`)
         const size_t behind = act_bf16 ? 0 : (int4_prefill_scratch_bytes(m, k) + 255) / 256 * 256;
-        if (ctx->scratch.try_reserve(behind + (size_t)p.ksplit * m * n * sizeof(float), ctx->stream)) {
-            scratch = ctx->scratch.ptr;
+        const bool room = ctx->scratch.try_reserve(behind + (size_t)p.ksplit * m * n * sizeof(float), ctx->stream, act_bf16 == nullptr);
+        scratch = ctx->scratch.ptr;
+        if (room) {
             kernel_out = reinterpret_cast<float *>(static_cast<unsigned char *>(scratch) + behind);
         } else {   // inside a capture without an earlier call of the size, or no memory
             p.ksplit = 1;
