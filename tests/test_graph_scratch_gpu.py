@@ -70,6 +70,34 @@ def test_replay_after_the_scratch_grew(batch, kv_int8):
     ctx.close()
 
 
+@pytest.mark.parametrize("m,k", [(1, 4608), (1, 6912), (1, 8192), (1, 8960), (2, 4352), (3, 2048), (4, 2304)])
+@pytest.mark.parametrize("n", [2048, 14336])
+def test_few_rows_in_a_graph_hold_no_scratch(m, k, n):
+    """Digit planes that fit a CTA: a captured call is one launch that quantises for itself, so that its replays are
+    independent of what other calls leave in the context's scratch, and its bits are those of the eager call."""
+    stream = torch.cuda.Stream()
+    ctx = yscv_b200.Context(0, stream=stream.cuda_stream)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    packed = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = torch.rand(n, k // 32, device="cuda", generator=g)
+    x, eager, replayed = torch.randn(m, k, device="cuda", generator=g), torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    torch.cuda.synchronize()
+    h = ctx.int4_weight_wrap(packed.data_ptr(), scales.data_ptr(), n, k, 32)
+    ctx.int4_matmul_dev(h, x.data_ptr(), eager.data_ptr(), m)
+    stream.synchronize()
+    before = ctx.launch_count()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        ctx.int4_matmul_dev(h, x.data_ptr(), replayed.data_ptr(), m)
+    assert ctx.launch_count() - before == 1 and "fused-quant" in ctx.last_kernel()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(eager, replayed)
+    assert ctx.device_status() == 0
+    del graph
+    ctx.close()
+
+
 def test_outgrown_buffers_are_given_back():
     """Without a graph nothing is kept: the memory in use after a call that outgrew the scratch is that of a
     context which made the larger call first; destroying a context returns what graphs made it keep."""

@@ -72,18 +72,25 @@ static int int4_matmul_dev(yscv_cuda_ctx *ctx, const uint8_t *d_packed, const fl
         const bool aligned = ((reinterpret_cast<uintptr_t>(d_packed) | reinterpret_cast<uintptr_t>(d_scales) |
                                reinterpret_cast<uintptr_t>(a)) & 15) == 0;
         const bool batch = aligned && int4_batch_exact_wins(mc, n, k, gs) && int4_batch_ready(ctx);
+        void *scratch = nullptr;
         if (aligned && (batch || int4_gemv_fast_supported(mc, n, k, gs))) {
             // (one size for every m up to 16, so that a call never outgrows what another one left)
             const size_t a_b = int4_gemv_scratch_bytes(16, k), b_b = int4_batch_exact_scratch_bytes(k);
             const size_t want = a_b > b_b ? a_b : b_b;
-            rc = batch || int4_gemv_uses_scratch(ctx, mc, n, k) ? ctx->scratch.reserve(want, ctx->stream) : ctx->scratch.reserve(want);
+            // A graph of a few rows holds no scratch where it can do without: the program may replay it beside other
+            // calls on the context, whose digit planes would lie in the same place (1 row 2048 x 8192 10.5 us, 8.9 with)
+            const bool uses = batch || int4_gemv_uses_scratch(ctx, mc, n, k);
+            const bool can_do_without = uses && !batch && int4_gemv_can_do_without_scratch(mc, k);
+            const bool alone = can_do_without && stream_capturing(ctx->stream);
+            rc = uses && !can_do_without ? ctx->scratch.reserve(want, ctx->stream) : ctx->scratch.reserve(want);
             if (rc) return rc;
+            if (!alone) scratch = ctx->scratch.ptr;
         }
         if (batch) {
-            rc = int4_batch_gemm(ctx, d_packed, d_scales, a, nullptr, o, mc, n, k, ctx->scratch.ptr);
+            rc = int4_batch_gemm(ctx, d_packed, d_scales, a, nullptr, o, mc, n, k, scratch);
             op_counters().int4_gemv_calls++;
         } else if (aligned && int4_gemv_fast_supported(mc, n, k, gs)) {
-            rc = int4_gemv_fast(ctx, d_packed, d_scales, a, o, mc, n, k, ctx->scratch.ptr);
+            rc = int4_gemv_fast(ctx, d_packed, d_scales, a, o, mc, n, k, scratch);
             op_counters().int4_gemv_calls++;
         } else {
             rc = int4_gemv_generic(ctx, d_packed, d_scales, a, o, mc, n, k, gs);

@@ -43,6 +43,8 @@ struct OpCounters {
 };
 OpCounters &op_counters();
 
+bool stream_capturing(cudaStream_t stream);
+
 // Grow-only device buffer owned by a context. A CUDA graph keeps the address that a captured call used, so a
 // buffer that was handed out inside a capture is not freed when a later call outgrows it: it goes to
 // `captured` and lives until release(). Such a buffer grows by half at least, so that what is kept stays below
@@ -65,7 +67,6 @@ struct DeviceBuffer {
 
   private:
     cudaError_t grow(size_t want, bool in_use);
-    bool note_capture(cudaStream_t stream);
 };
 
 }  // namespace yscv

@@ -6,7 +6,7 @@ namespace yscv {
 
 // Is the stream being captured? (A query that fails, as on the legacy stream while another thread captures,
 // is not this call's failure: the launch that follows reports it.)
-bool DeviceBuffer::note_capture(cudaStream_t stream) {
+bool stream_capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) {
         cudaGetLastError();
@@ -48,14 +48,14 @@ int DeviceBuffer::reserve(size_t want) {
 }
 
 int DeviceBuffer::reserve(size_t want, cudaStream_t stream) {
-    const bool capturing = note_capture(stream);
+    const bool capturing = stream_capturing(stream);
     const int rc = reserve(want);
     in_graph = in_graph || (capturing && rc == YSCV_CUDA_OK);
     return rc;
 }
 
 bool DeviceBuffer::try_reserve(size_t want, cudaStream_t stream, bool in_use) {
-    const bool capturing = note_capture(stream);
+    const bool capturing = stream_capturing(stream);
     if (want > bytes || !ptr) {
         if (capturing) return false;
         if (grow(want, in_use) != cudaSuccess) {

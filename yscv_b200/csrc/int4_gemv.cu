@@ -486,6 +486,12 @@ bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs) {
 static bool small_rows(const yscv_cuda_ctx *ctx, int n) { return (n + ctx->sm_count - 1) / ctx->sm_count <= 32; }
 static bool fused_quant(const yscv_cuda_ctx *ctx, int mp, int n, int k) { return mp <= 4 && mp * k <= (small_rows(ctx, n) ? 4500 : 6800); }
 bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) { return !fused_quant(ctx, padded_m((int)m), (int)n, (int)k); }
+// Longer rows that a CTA still can quantise, the planes resident in shared memory: for calls that should do without scratch
+bool int4_gemv_can_do_without_scratch(size_t m, size_t k) {
+    const int mp = padded_m((int)m);
+    const QuantLayout q = quant_layout(mp, stage_groups(mp, (int)k));
+    return mp <= 4 && (size_t)quant_stages(q, (int)k) * (size_t)q.blob_bytes <= 72 * 1024;
+}
 
 template <int MP, int GS, int TP2, bool FUSEQ>
 static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
@@ -560,14 +566,14 @@ static int launch_fast(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scale
     return YSCV_CUDA_OK;
 }
 
-// act == nullptr: the digit planes are in `scratch`
+// act == nullptr: the digit planes are in `scratch`. scratch == nullptr: there is none, every CTA quantises.
 template <int MP, int GS>
 static int launch_fast_tp(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales,
                           const float *act, float *out, int M, int N, int K, void *scratch) {
     const QuantLayout q = quant_layout(MP, GS);
     const bool small = small_rows(ctx, N);
     if constexpr (MP <= 4) {
-        if (act && fused_quant(ctx, MP, N, K)) {
+        if (act && (!scratch || fused_quant(ctx, MP, N, K))) {
             ctx->last_kernel = "int4_gemv_fast(imma,tma,fused-quant)";
             return small ? launch_fast<MP, GS, 2, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q)
                          : launch_fast<MP, GS, 8, true>(ctx, wq, scales, nullptr, act, out, M, N, K, q);
