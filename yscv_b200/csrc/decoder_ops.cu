@@ -1314,6 +1314,11 @@ int yscv_cuda_embedding_dev(yscv_cuda_ctx *ctx, const float *d_weight, size_t vo
 }  // extern "C"
 
 namespace yscv {
+// Name of an operator by the form it writes
+static const char *form_name(int form, const char *f32, const char *bf16, const char *digits, const char *terms) {
+    return form == ACT_BF16 ? bf16 : form == ACT_DIGITS ? digits : form == ACT_TERMS ? terms : f32;
+}
+
 // hidden % 8 == 0 and at most 8192, operands (and `pitch` floats) 16-byte aligned
 int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
               size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out) {
@@ -1331,7 +1336,7 @@ int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts,
                                          : pick(std::integral_constant<int, ACT_F32>());
     YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)out.slots()), dim3(threads), 0, ctx->stream, x, delta, parts, pitch, gamma, eps, (int)hidden,
                              row0, row_step, x_out, out));
-    DEC_EPILOGUE(ctx, out.form == ACT_F32 ? "add_rms_norm" : "add_rms_norm(bf16 activations out)");
+    DEC_EPILOGUE(ctx, form_name(out.form, "add_rms_norm", "add_rms_norm(bf16 activations out)", "add_rms_norm(digit planes out)", "add_rms_norm(fp16 terms out)"));
 }
 }  // namespace yscv
 
@@ -1566,7 +1571,7 @@ int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitc
                 : out.form == ACT_TERMS  ? swiglu_form_kernel<ACT_TERMS>
                                          : swiglu_form_kernel<ACT_F32>;
     YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(256), 0, ctx->stream, gate_up, parts, pitch, (int)visit, (int)inter, out));
-    DEC_EPILOGUE(ctx, out.form == ACT_F32 ? "swiglu" : "swiglu(bf16 activations out)");
+    DEC_EPILOGUE(ctx, form_name(out.form, "swiglu", "swiglu(bf16 activations out)", "swiglu(digit planes out)", "swiglu(fp16 terms out)"));
 }
 }  // namespace yscv
 
