@@ -106,12 +106,12 @@ gqa_decode_fused_kernel(DFParams p) {
     // ---- queries, new key and value ----
     const float *const row = p.qkv + (size_t)b * (p.n_q + 2 * p.n_kv) * D;
     auto load = [&](int i) {   // every part's load in flight
-        float4 y[8];
+        float4 y[INT4_MAX_PARTS];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) y[t] = t < p.parts ? *reinterpret_cast<const float4 *>(row + t * p.pitch + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = 0; t < INT4_MAX_PARTS; ++t) y[t] = t < p.parts ? *reinterpret_cast<const float4 *>(row + t * p.pitch + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         float4 x = y[0];
 #pragma unroll
-        for (int t = 1; t < 8; ++t)
+        for (int t = 1; t < INT4_MAX_PARTS; ++t)
             if (t < p.parts) { x.x += y[t].x; x.y += y[t].y; x.z += y[t].z; x.w += y[t].w; }
         return x;
     };
@@ -416,6 +416,7 @@ bool gqa_decode_fused_wins(const yscv_cuda_ctx *ctx, int form, bool kv_int8, siz
 template <typename KV>
 int gqa_decode_fused(yscv_cuda_ctx *ctx, const float *qkv, int parts, size_t pitch, size_t batch, size_t n_q, size_t n_kv, size_t d_head,
                      float theta, const int32_t *d_pos, KV *kcache, KV *vcache, float *kscale, float *vscale, size_t max_seq, const ActOut &out) {
+    if (parts > INT4_MAX_PARTS) return fail(YSCV_CUDA_ERR_BAD_ARG, "%d partial sums, at most %d", parts, INT4_MAX_PARTS);
     DFParams p = {qkv, parts, pitch, kcache, vcache, kscale, vscale, d_pos, (int)n_q, (int)n_kv, (int)max_seq, theta, ctx->d_status, out};
     auto pick = [&](auto dim) {
         constexpr int D = decltype(dim)::value;

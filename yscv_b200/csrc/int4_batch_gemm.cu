@@ -619,7 +619,7 @@ static int bg_split(const BGParams &p, int NA, int grid, int sms, bool slices_ok
     double best = 3.2 + (p.units + grid - 1) / grid * unit * (NA == 2 ? 1.75 : 1.0) + 2.0 * grid * NA * 128 * p.BT * 4 * mb;
     int slices = 0;
     const int tiles = (p.N + 127) / 128;
-    for (int s = 1; s <= 8 && s <= p.kb; ++s) {
+    for (int s = 1; s <= INT4_MAX_PARTS && s <= p.kb; ++s) {
         const double bytes = (double)s * p.M * p.N * 4;
         if (s > 1 && (!slices_ok || bytes > (double)ws_bytes)) break;
         const double rounds = (int)(((long long)tiles * s + sms - 1) / sms);

@@ -809,7 +809,7 @@ static PGChoice pg_choose(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k
     const size_t tiles = (n + PG_BM - 1) / PG_BM * ((m + bt - 1) / bt);
     PGChoice c = {0, 1};
     double best = 1e30;
-    for (int s = 1; s <= 8 && s <= kb; ++s) {
+    for (int s = 1; s <= INT4_MAX_PARTS && s <= kb; ++s) {
         const double mb = (double)s * m * n * 4e-6;
         if (s > 1 && (!slices_ok || mb > 128.0)) break;
         const double cost = 3.06 + (double)((tiles * s + sms - 1) / sms) * ((kb + s - 1) / s * (0.35 + 0.00089 * bt) + 1.55) + (s > 1 ? 2.35 + 0.176 * mb : 0.0);

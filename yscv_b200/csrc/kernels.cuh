@@ -37,6 +37,7 @@ size_t int4_prefill_scratch_bytes(size_t m, size_t k);
 int int4_prefill_gemm(yscv_cuda_ctx *ctx, const uint8_t *wq, const float *scales, const float *act,
                       float *out, size_t m, size_t n, size_t k, void *scratch, const void *act_bf16 = nullptr, int *parts = nullptr);
 
+constexpr int INT4_MAX_PARTS = 8;   // k slices of a matmul, and the parts that a kernel which adds them holds in registers
 int add_kslices(yscv_cuda_ctx *ctx, const float *parts, float *out, size_t elements, int slices);
 
 // int4_batch_gemm.cu: 3..128 activation rows, k % 128 == 0, 16-byte aligned operands. act_bf16 == nullptr:
