@@ -106,3 +106,31 @@ def test_rope_append_parts_and_alignment(tctx, oracle, n_q, n_kv, d, shift, i8):
                     assert np.abs(c - want).max() < 2e-5
             assert (cache[b, :p] == 0).all() and (cache[b, p + seq:] == 0).all()
         assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hidden", [8, 2040, 2048, 2056, 4088, 8192])
+@pytest.mark.parametrize("rows", [1, 2, 295, 296, 297, 600])
+def test_norm_forms_are_the_scalar_kernel(tctx, rows, hidden):
+    """Around two rows per SM and the sizes of the blocks: the bits of the kernel for operands at odd addresses, with and
+    without a delta, in place and not, to fp32 and to the bf16 of a following matmul."""
+    import torch
+    ctx, s = tctx
+    with torch.cuda.stream(s):
+        gen = torch.Generator(device="cuda").manual_seed(hidden + rows)
+        x, d = (torch.randn(rows * hidden, device="cuda", generator=gen) for _ in range(2))
+        g = torch.rand(hidden + 1, device="cuda", generator=gen)
+        for delta in (False, True):
+            xo = [torch.empty(rows * hidden + 1, device="cuda") for _ in range(2)]
+            no = [torch.empty(rows * hidden + 1, device="cuda") for _ in range(2)]
+            n16 = torch.empty(rows * hidden, dtype=torch.bfloat16, device="cuda")
+            inplace = x.clone()
+            dp = d.data_ptr() if delta else 0
+            g0 = g[1:].clone()
+            ctx.add_rms_norm_dev(x.data_ptr(), dp, g0.data_ptr(), 1e-5, rows, hidden, xo[0].data_ptr(), no[0].data_ptr())
+            ctx.add_rms_norm_dev(x.data_ptr(), dp, g[1:].data_ptr(), 1e-5, rows, hidden, xo[1].data_ptr() + 4, no[1].data_ptr() + 4)
+            ctx.add_rms_norm_act_dev(inplace.data_ptr(), dp, g0.data_ptr(), 1e-5, rows, hidden, inplace.data_ptr(), n16.data_ptr())
+            assert torch.equal(xo[0][:-1], xo[1][1:]) and torch.equal(no[0][:-1], no[1][1:])
+            assert torch.equal(inplace, xo[0][:-1])
+            assert torch.equal(n16.view(-1, 8), no[0][:-1].view(-1, 8)[:, ORDER].to(torch.bfloat16))
+    s.synchronize()
+    assert ctx.device_status() == 0

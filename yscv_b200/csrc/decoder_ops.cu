@@ -80,25 +80,31 @@ __device__ __forceinline__ void load8(const float *p, int parts, size_t pitch, f
 // Position of element e of a group of 8 in that order
 __device__ __forceinline__ int gemm_order_pos(int e) { return ((e & 3) << 1) | (e >> 2); }
 
-// x_out = x + delta (delta may be null), delta the sum of `parts` arrays `pitch` floats apart; the row normalised,
-// (x_out / sqrt(mean(x_out^2) + eps)) * gamma, in the form that the matmul behind it takes. Input row of block b:
-// row0 + b * row_step (blocks past the rows of `o` write padding).
+// x_out = x + delta (delta may be null), delta the sum of `parts` arrays `pitch` floats apart (one array without SUM); the
+// row normalised, (x_out / sqrt(mean(x_out^2) + eps)) * gamma, in the form that the matmul behind it takes. Input row of
+// block b: row0 + b * row_step (blocks past the rows of `o` write padding).
 //
-// Latency-bound for a decode batch (a block per row), bandwidth-bound for a prompt. A thread keeps eight consecutive
-// values in registers between the sum of squares and the scaling: one round trip with every load in
-// flight, 128-bit accesses, and what the activation forms want a lane to hold. The sum of squares goes through shared
-// memory so that its order is that of the kernel below (thread t: elements t, t + T, ...): the same result for every form and
-// alignment. With 32-bit accesses 2048 rows of 8192 to bf16 took 95 us, now 68 (4.3 TB/s); the passes it stands for
-// (partial sums added, conversion to digit planes) were launches of their own, 1.5 to 1.8 us each behind a decode batch.
-// T = 256 up to 2048 values, else 1024 (hidden <= 8 T). P pieces of eight per thread, T / P threads: one for a few rows,
-// more for a prompt, whose blocks then share an SM and keep the values in shared memory meanwhile.
-template <int FORM, int T, int P>
-__global__ void __launch_bounds__(T / P, P > 1 ? 1536 * P / T : 1)
+// Latency-bound for a few rows (a block per row), bandwidth-bound for many. A thread keeps its values in registers between
+// the sum of squares and the scaling: one round trip with every load in flight, 128-bit accesses, eight consecutive values
+// per lane where the form wants them, else four, so that an access of a warp is whole lines. The sum of squares goes through
+// shared memory so that its order is that of the kernel below (thread t: elements t, t + T, ...): the same result for every
+// form and alignment. T = 256 up to 2048 values, else 1024 (hidden <= 8 T).
+// FEW (up to two rows per SM, NORM_FEW): gamma is fetched before the reduction, a thread takes eight values. More: what counts
+// is rows per SM, so gamma comes late (28 to 32 registers instead of 40, six and more blocks of 256) and blocks of 512 take 16 values
+// per thread, two of them per SM in different phases. us, fp32 to fp32 / to bf16, warm caches: 1 x 2048 1.5 / 1.6, 1 x 8192 3.1 / 3.5,
+// 1024 x 2048 4.6 / 5.5 (with FEW 4.6 / 5.3; 512 x 2048 3.0 / 3.4, FEW 3.1 / 4.4), 300 x 4096 5.2 / 5.5 (FEW 5.9 / 6.3), 128 x 4096 2.7 / 2.7 (FEW 2.7 /
+// 2.8), 128 x 8192 from HBM 5.8 / 4.9 (FEW 5.1 / 4.5), 2048 x 8192 42.7 / 41.1 (4.9 TB/s of fp32 to bf16; FEW 49.9 / 46.9). The scalar
+// kernel below: 2.0, 3.7, 5.0, 8.2, 3.2, 5.9, 65. With the sum over parts left in for one part (72 registers) and blocks of 128 and 256
+// for more than 512 rows, 40 registers and spills, this took 10.0 / 8.9 at 1024 x 2048 and 20.5 / 17.5 at 513 x 8192 (now 9.5 / 10.9).
+constexpr size_t NORM_FEW = 2;
+template <int FORM, int T, bool SUM, bool FEW>
+__global__ void __launch_bounds__(FEW || T == 256 ? T : T / 2, FEW ? 1 : T == 256 ? 6 : 2)
 norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, const float *__restrict__ gamma, float eps, int hidden,
                  size_t row0, size_t row_step, float *x_out, ActOut o) {
     pdl_wait();
     pdl_trigger();
-    constexpr int TH = T / P;
+    constexpr int P = FEW || T == 256 ? 1 : 2, TH = T / P;      // P eights of values per thread
+    constexpr int W = FORM == ACT_F32 ? 4 : 8, N = P * 8 / W, Q = W / 4;   // N accesses of W values
     __shared__ float red[32];
     __shared__ __align__(16) float sm[8 * T];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
@@ -111,31 +117,59 @@ norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, co
         return;
     }
     const size_t base = (row0 + row * row_step) * hidden;
-    float v[8] = {};
+    float4 v[N * Q];
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        const int i = (tid + p * TH) * 8;
+    for (int p = 0; p < N; ++p) {
+        const int i = (tid + p * TH) * W;
         if (i < hidden) {   // (x not through the read-only path: x_out may be x)
-            const float4 a = *reinterpret_cast<const float4 *>(x + base + i), b = *reinterpret_cast<const float4 *>(x + base + i + 4);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-            if (delta) {
-                float d[8];
-                load8(delta + base + i, parts, pitch, d);
 #pragma unroll
-                for (int t = 0; t < 8; ++t) v[t] += d[t];
-            }
-            const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
-            *reinterpret_cast<float4 *>(sm + i) = lo;
-            *reinterpret_cast<float4 *>(sm + i + 4) = hi;
-            if (x_out) {
-                *reinterpret_cast<float4 *>(x_out + base + i) = lo;
-                *reinterpret_cast<float4 *>(x_out + base + i + 4) = hi;
+            for (int h = 0; h < Q; ++h) v[p * Q + h] = *reinterpret_cast<const float4 *>(x + base + i + 4 * h);
+        }
+    }
+    if (delta) {
+#pragma unroll
+        for (int p = 0; p < N; ++p) {
+            const int i = (tid + p * TH) * W;
+            if (i < hidden) {
+#pragma unroll
+                for (int h = 0; h < Q; ++h) {
+                    const float *src = delta + base + i + 4 * h;
+                    float4 d = __ldg(reinterpret_cast<const float4 *>(src));
+                    if constexpr (SUM) {
+#pragma unroll 4
+                        for (int s = 1; s < parts; ++s) {
+                            const float4 e = __ldg(reinterpret_cast<const float4 *>(src + s * pitch));
+                            d.x += e.x; d.y += e.y; d.z += e.z; d.w += e.w;
+                        }
+                    }
+                    float4 &y = v[p * Q + h];
+                    y.x += d.x; y.y += d.y; y.z += d.z; y.w += d.w;
+                }
             }
         }
     }
-    float g[8] = {};
-    if (P == 1 && tid * 8 < hidden) load8(gamma + tid * 8, 1, 0, g);
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+        const int i = (tid + p * TH) * W;
+        if (i < hidden) {
+#pragma unroll
+            for (int h = 0; h < Q; ++h) {
+                *reinterpret_cast<float4 *>(sm + i + 4 * h) = v[p * Q + h];
+                if (x_out) *reinterpret_cast<float4 *>(x_out + base + i + 4 * h) = v[p * Q + h];
+            }
+        }
+    }
+    float4 g[FEW ? N * Q : 1];
+    if constexpr (FEW) {
+#pragma unroll
+        for (int p = 0; p < N; ++p) {
+            const int i = (tid + p * TH) * W;
+            if (i < hidden) {
+#pragma unroll
+                for (int h = 0; h < Q; ++h) g[p * Q + h] = __ldg(reinterpret_cast<const float4 *>(gamma + i + 4 * h));
+            }
+        }
+    }
     __syncthreads();
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -156,18 +190,26 @@ norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, co
     for (int w = 0; w < T / 32; ++w) total += red[w];
     const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        const int i = (tid + p * TH) * 8;
+    for (int p = 0; p < N; ++p) {
+        const int i = (tid + p * TH) * W;
         const bool on = i < hidden;
-        if (P > 1 && on) {
-            load8(gamma + i, 1, 0, g);
-            const float4 a = *reinterpret_cast<const float4 *>(sm + i), b = *reinterpret_cast<const float4 *>(sm + i + 4);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        }
+        float n[W] = {};
+        if (on) {
 #pragma unroll
-        for (int t = 0; t < 8; ++t) v[t] = (v[t] * inv) * g[t];
-        store_act<FORM>(o, v, row, i, on);
+            for (int h = 0; h < Q; ++h) {
+                const float4 y = P > 1 ? *reinterpret_cast<const float4 *>(sm + i + 4 * h) : v[p * Q + h];
+                const float4 c = FEW ? g[p * Q + h] : __ldg(reinterpret_cast<const float4 *>(gamma + i + 4 * h));
+                n[4 * h] = (y.x * inv) * c.x;
+                n[4 * h + 1] = (y.y * inv) * c.y;
+                n[4 * h + 2] = (y.z * inv) * c.z;
+                n[4 * h + 3] = (y.w * inv) * c.w;
+            }
+        }
+        if constexpr (FORM == ACT_F32) {
+            if (on) *reinterpret_cast<float4 *>(static_cast<float *>(o.ptr) + (size_t)row * o.k + i) = make_float4(n[0], n[1], n[2], n[3]);
+        } else {
+            store_act<FORM>(o, n, row, i, on);
+        }
     }
 }
 
@@ -1322,13 +1364,17 @@ static const char *form_name(int form, const char *f32, const char *bf16, const 
 // hidden % 8 == 0 and at most 8192, operands (and `pitch` floats) 16-byte aligned
 int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
               size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out) {
-    const bool prompt = rows > 512 && (out.form == ACT_F32 || out.form == ACT_BF16);
-    const unsigned threads = hidden <= 2048 ? (prompt ? 128u : 256u) : (prompt ? 256u : 1024u);
+    const bool small = hidden <= 2048;
+    // (partial sums and the forms of up to 16 rows come with few rows)
+    const bool few = rows <= NORM_FEW * ctx->sm_count || parts > 1 || (out.form != ACT_F32 && out.form != ACT_BF16);
+    const unsigned threads = small ? 256u : few ? 1024u : 512u;
     auto pick = [&](auto form) {
         constexpr int F = decltype(form)::value;
-        if constexpr (F == ACT_F32 || F == ACT_BF16)
-            if (prompt) return hidden <= 2048 ? norm_form_kernel<F, 256, 2> : norm_form_kernel<F, 1024, 4>;
-        return hidden <= 2048 ? norm_form_kernel<F, 256, 1> : norm_form_kernel<F, 1024, 1>;
+        if constexpr (F == ACT_F32 || F == ACT_BF16) {
+            if (!few) return small ? norm_form_kernel<F, 256, false, false> : norm_form_kernel<F, 1024, false, false>;
+        }
+        if (parts > 1) return small ? norm_form_kernel<F, 256, true, true> : norm_form_kernel<F, 1024, true, true>;
+        return small ? norm_form_kernel<F, 256, false, true> : norm_form_kernel<F, 1024, false, true>;
     };
     auto kern = out.form == ACT_BF16     ? pick(std::integral_constant<int, ACT_BF16>())
                 : out.form == ACT_DIGITS ? pick(std::integral_constant<int, ACT_DIGITS>())
