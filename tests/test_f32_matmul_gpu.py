@@ -100,3 +100,21 @@ def test_argmax_over_partials(sctx):
         ctx.argmax_last_dev(logits.data_ptr(), 5, vocab, out.data_ptr())
     stream.synchronize()
     assert out.tolist() == [31999, 0, 12346, 31999, 31999]
+
+
+@pytest.mark.parametrize("n", [1, 9, 2499, 2500, 4095])
+@pytest.mark.parametrize("k", [4, 132, 1028])
+def test_few_weight_rows_are_the_same_sums(sctx, n, k):
+    """Up to 8 activation rows: fewer weight rows than fill the SMs take a kernel of their own; its columns are the bits of
+    those that the other kernel makes of the same rows in a larger matrix."""
+    ctx, s = sctx
+    with torch.cuda.stream(s):
+        g = torch.Generator(device="cuda").manual_seed(n * k)
+        w, x = torch.randn(4099, k, device="cuda", generator=g), torch.randn(8, k, device="cuda", generator=g)
+        for m in range(1, 9):
+            few, many = torch.full((m, n), float("nan"), device="cuda"), torch.empty(m, 4099, device="cuda")
+            ctx.f32_matmul_dev(w.data_ptr(), x.data_ptr(), m, n, k, few.data_ptr())
+            ctx.f32_matmul_dev(w.data_ptr(), x.data_ptr(), m, 4099, k, many.data_ptr())
+            assert torch.equal(few, many[:, :n])
+    s.synchronize()
+    assert ctx.device_status() == 0

@@ -1122,6 +1122,48 @@ attention_combine_kernel(const float *__restrict__ part, int n_splits, int d, in
     }
 }
 
+// out[m][n] = sum_k x[m][k] * w[n][k]; one warp per weight row, up to MT x rows per pass. For few weight rows, where what
+// counts is how many warps share the weights: with two and four rows per warp (the kernel below, which takes over where the
+// rows fill the SMs; its sums are the same) 3 x 300 x 512 takes 2.9 us and here 1.9, 4 x 1000 x 4096 12.7 and 7.3, 8 x 1000 x 4096
+// 20.1 and 14.5, from HBM 1 x 3000 x 4096 15.6 and 12.6, 3 x 3000 x 4096 23.8 and 16.2; the other way 1 x 4096 x 4096 17.1 and
+// 21.9, 4 x 4096 x 4096 24.3 and 28.0, 8 x 3000 x 4096 30.1 and 32.4, 5 x 6000 x 1024 10.6 and 15.9.
+template <int MT>
+__global__ void __launch_bounds__(256)
+f32_matmul_rows_kernel(const float *__restrict__ w, const float *__restrict__ x, float *__restrict__ out, int m0, int M, int N, int K) {
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31;
+    const int wpb = blockDim.x >> 5;
+    const int mt = min(MT, M - m0);
+    for (int n = blockIdx.x * wpb + (threadIdx.x >> 5); n < N; n += gridDim.x * wpb) {
+        const float4 *wr = reinterpret_cast<const float4 *>(w + (size_t)n * K);
+        float acc[MT];
+#pragma unroll
+        for (int i = 0; i < MT; ++i) acc[i] = 0.0f;
+#pragma unroll 4
+        for (int c = lane; c < K / 4; c += 32) {
+            const float4 wv = __ldg(wr + c);
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                if (i < mt) {
+                    const float4 xv = __ldg(reinterpret_cast<const float4 *>(x + (size_t)(m0 + i) * K) + c);
+                    acc[i] = fmaf(wv.x, xv.x, acc[i]);
+                    acc[i] = fmaf(wv.y, xv.y, acc[i]);
+                    acc[i] = fmaf(wv.z, xv.z, acc[i]);
+                    acc[i] = fmaf(wv.w, xv.w, acc[i]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            float v = acc[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && i < mt) out[(size_t)(m0 + i) * N + n] = v;
+        }
+    }
+}
+
 // out[m][n] = sum_k x[m][k] * w[n][k] for m <= MT: one warp per R weight rows, which share the x rows it reads.
 // Bound by the weights' HBM stream: enough loads in flight per warp (R rows, unrolled) and one pass whatever m.
 // The weights skip L1, which holds the x rows. With a row per warp, four loads in flight and a pass per 4 x rows
@@ -1726,6 +1768,16 @@ int yscv_cuda_f32_matmul_dev(yscv_cuda_ctx *ctx, const float *d_w, const float *
         YSCV_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
         ctx->last_kernel = "f32_matmul(tiled)";
+        return YSCV_CUDA_OK;
+    }
+    if (n < (m <= 4 ? 4096u : 2500u)) {
+        const unsigned blocks = (unsigned)((n + 7) / 8);
+        for (size_t m0 = 0; m0 < m; m0 += 4) {
+            YSCV_CUDA_TRY(launch_pdl(f32_matmul_rows_kernel<4>, dim3(blocks), dim3(256), 0, ctx->stream, d_w, d_x, d_out, (int)m0, (int)m, (int)n, (int)k));
+            YSCV_CUDA_TRY(cudaGetLastError());
+            ctx->launches++;
+        }
+        ctx->last_kernel = "f32_matmul";
         return YSCV_CUDA_OK;
     }
     // one pass over the weights: rows per warp and unroll with enough loads in flight for the registers that m takes
