@@ -204,6 +204,7 @@ f32_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
     pdl_trigger();
 
     FTWalk walk(p);
+    const int stages_k = p.K / FT_BK;            // (odd: the last unit is one stage)
     int tile, k0, k1;
     bool alive = true;
     if (warp == FT_PRODUCER) {
@@ -213,7 +214,7 @@ f32_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
             uint32_t ph = 0;
             while (alive && walk.next(tile, k0, k1)) {
                 const int nt = tile / p.t_chunks, tc = tile - nt * p.t_chunks;
-                for (int s = 2 * k0; s < 2 * k1; ++s) {
+                for (int s = 2 * k0; s < min(2 * k1, stages_k); ++s) {
                     alive = mbar_wait(empty + st * 8, ph ^ 1u, status);
                     if (!alive) break;
                     const uint32_t dst = base + (uint32_t)st * p.stage_bytes, bar = full + st * 8;
@@ -238,8 +239,8 @@ f32_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
         int st = 0, ring = 0, buf = 0;
         uint32_t ph = 0, rph = 0, bph = 0;
         while (alive && walk.next(tile, k0, k1)) {
-            for (int s = 2 * k0; s < 2 * k1; ++s) {
-                const bool first = (s & 1) == 0;     // a unit's first stage starts an accumulator
+            for (int s = 2 * k0; s < min(2 * k1, stages_k); ++s) {
+                const bool first = (s & 1) == 0, last = !first || s + 1 == stages_k;   // a unit's first stage starts an accumulator
                 const int slot = a * RING + ring;
                 alive = __all_sync(0xffffffffu, (!first || mbar_wait(tempty + buf * 8, bph ^ 1u, status)) &&
                                                     mbar_wait(full + st * 8, ph, status) && mbar_wait(afull + slot * 8, rph, status));
@@ -257,12 +258,12 @@ f32_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
                     }
                     ft_commit(empty + st * 8);
                     ft_commit(mdone + slot * 8);
-                    if (!first) ft_commit(tfull + buf * 8);
+                    if (last) ft_commit(tfull + buf * 8);
                 }
                 __syncwarp();
                 if (++st == p.stages) { st = 0; ph ^= 1u; }
                 if (++ring == RING) { ring = 0; rph ^= 1u; }
-                if (!first && ++buf == 2) { buf = 0; bph ^= 1u; }
+                if (last && ++buf == 2) { buf = 0; bph ^= 1u; }
             }
         }
     } else if (warp >= FT_SPLIT0 && warp < FT_PRODUCER) {
@@ -276,7 +277,7 @@ f32_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_co
         int st = 0, ring = 0;
         uint32_t ph = 0, rph = 0;
         while (alive && walk.next(tile, k0, k1)) {
-            for (int s = 2 * k0; s < 2 * k1; ++s) {
+            for (int s = 2 * k0; s < min(2 * k1, stages_k); ++s) {
                 const int slot = a * RING + ring;
                 alive = mbar_wait(full + st * 8, ph, status);
                 if (!alive) break;
@@ -415,7 +416,7 @@ int f32_gemm_tc(yscv_cuda_ctx *ctx, const float *d_w, const float *d_x, size_t m
     const int m16 = (int)((m + 15) / 16 * 16), sms = ctx->sm_count;
     p.BT = m16 <= FT_BT_MAX ? m16 : FT_BT_MAX;
     p.t_chunks = (p.M + p.BT - 1) / p.BT;
-    p.kb = (p.K + FT_UNIT - 1) / FT_UNIT;   // (k % 64 == 32: the last unit's second stage lies past the edge and reads zeros)
+    p.kb = (p.K + FT_UNIT - 1) / FT_UNIT;
     const int tiles1 = (p.N + FT_BM - 1) / FT_BM * p.t_chunks, tiles2 = (p.N + 2 * FT_BM - 1) / (2 * FT_BM) * p.t_chunks;
     const int NA = p.BT <= FT_BT_MAX / 2 && (long long)tiles2 * p.kb >= 8ll * sms ? 2 : 1;
     const int tiles = NA == 2 ? tiles2 : tiles1;
