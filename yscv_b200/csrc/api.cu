@@ -108,7 +108,7 @@ int int4_act_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, size_t m) 
     if (m == 0 || ((reinterpret_cast<uintptr_t>(w->d_packed) | reinterpret_cast<uintptr_t>(w->d_scales)) & 15)) return ACT_F32;
     if (m > 16) return !ctx->prefill_exact && int4_prefill_supported(m, n, k, gs) ? ACT_BF16 : ACT_F32;
     if (int4_batch_exact_wins(m, n, k, gs) && int4_batch_ready(ctx)) return ACT_TERMS;
-    return int4_gemv_fast_supported(m, n, k, gs) && int4_gemv_uses_scratch(ctx, m, n, k) && int4_gemv_digits_whole(m, k) ? ACT_DIGITS : ACT_F32;
+    return int4_gemv_fast_supported(m, n, k, gs) && int4_gemv_wants_digits(ctx, m, n, k) && int4_gemv_digits_whole(m, k) ? ACT_DIGITS : ACT_F32;
 }
 
 int int4_form_parts(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, int form, size_t m) {

@@ -478,14 +478,26 @@ bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs) {
 }
 
 // Few and short activation rows: every CTA quantises them itself, no separate launch. That is work on the way to every CTA's
-// first product, so it pays up to 4500 values, 6800 where a CTA has more than 32 rows of weights to hide it behind (us per
-// call, in the kernel / in a launch of its own): 1 row 2048 x 4608 7.4 / 6.5, 2048 x 8192 10.5 / 8.9, 14336 x 4096
-// 10.5 / 11.7, 14336 x 8192 19.2 / 18.1, 28672 x 8192 38.7 / 33.3; 2 rows 2048 x 2048 4.3 / 5.2, 2048 x 2560 5.8 / 5.5, 14336 x 3072 9.3 /
-// 10.1, 28672 x 4096 21.5 / 20.2; 4 rows 2048 x 1024 3.8 / 4.0, 2048 x 4096 9.8 / 6.8, 14336 x 1536 8.5 / 8.8, 14336 x 4096 18.6 / 15.6.
+// first product, so it pays only up to a line, which lies where a launch of its own is the faster call, host time included (us
+// per call one after another, in the kernel / in a launch of its own; inside a capture the first form is taken anyway):
+//   up to 32 rows of weights per CTA: 1 row 2048 x 4096 6.4 / 6.3, 4608 7.4 / 6.7, 8192 10.5 / 9.0; 2 rows 2048 x 2048 4.6 / 6.2, 2560 5.8 / 6.3,
+//   3072 6.3 / 6.2, 4096 7.4 / 6.6; 4 rows 2048 x 1280 5.0 / 6.3, 2048 5.9 / 6.3, 2560 7.0 / 6.3, 4096 9.9 / 6.9;
+//   more, which hide it better: 1 row 14336 x 4096 9.5 / 9.7, 5632 12.4 / 11.8 (weights from HBM 12.7 / 13.8), 8192 16.7 / 15.2; 2 rows 14336 x 3072
+//   8.7 / 8.7, 4096 10.4 / 10.2 (11.8 / 12.0); 4 rows 6144 x 1536 6.3 / 6.3, 2048 7.5 / 6.9, 14336 x 1536 7.9 / 7.8 (8.6 / 9.1), 4096 16.9 / 13.7.
 // (The digit planes of so many values are at most 56 KB.)
 static bool small_rows(const yscv_cuda_ctx *ctx, int n) { return (n + ctx->sm_count - 1) / ctx->sm_count <= 32; }
-static bool fused_quant(const yscv_cuda_ctx *ctx, int mp, int n, int k) { return mp <= 4 && mp * k <= (small_rows(ctx, n) ? 4500 : 6800); }
+static bool fused_quant(const yscv_cuda_ctx *ctx, int mp, int n, int k) {
+    if (mp > 4) return false;
+    return mp * k <= (!small_rows(ctx, n) ? 6800 : mp == 1 ? 4500 : mp == 2 ? 5200 : 8200);
+}
 bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) { return !fused_quant(ctx, padded_m((int)m), (int)n, (int)k); }
+// Where the operator in front should write digit planes, which costs it little and no launch: from where a launch of its own
+// is ahead inside a graph, where launches are close (us in the kernel / in a launch of its own: 1 row 2048 x 4608 7.4 / 6.2; 2 rows 2048 x 2048
+// 4.3 / 4.9, 2560 5.7 / 5.2; 4 rows 2048 x 1024 3.8 / 4.1, 1280 5.0 / 4.5, 14336 x 1536 7.7 / 7.4)
+bool int4_gemv_wants_digits(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) {
+    const int mp = padded_m((int)m);
+    return mp > 4 || mp * (int)k > (small_rows(ctx, (int)n) ? 4500 : 6800);
+}
 // Longer rows that a CTA still can quantise, the planes resident in shared memory: for calls that should do without scratch
 bool int4_gemv_can_do_without_scratch(size_t m, size_t k) {
     const int mp = padded_m((int)m);

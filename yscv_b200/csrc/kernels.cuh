@@ -15,6 +15,7 @@ namespace yscv {
 bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs);
 size_t int4_gemv_scratch_bytes(size_t m, size_t k);
 bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k);
+bool int4_gemv_wants_digits(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k);
 bool int4_gemv_can_do_without_scratch(size_t m, size_t k);   // scratch == nullptr then
 // fp32 matmul out[m][n] = sum_k x[m][k] w[n][k] for m > 8 as three TF32 products per fp32 product
 // on the tensor cores (f32_gemm_tf32x3.cu)
