@@ -203,6 +203,40 @@ def test_step_attention_positions(tctx, n_q, n_kv, d, batch, kv_int8):
     dec.close()
 
 
+@pytest.mark.parametrize("n_q,n_kv,d,batch,kv_int8,one,three", [
+    # CTAs per sequence and KV head 8, 4, 2, 1, with a grid that fills the machine's two CTAs per SM or not
+    (32, 4, 64, 2, False, 600, 640), (32, 4, 64, 8, False, 1200, 1240), (32, 4, 64, 12, False, 400, 440), (32, 4, 64, 24, False, 300, 340),
+    (32, 4, 64, 40, False, 200, 240), (32, 4, 64, 64, False, 400, 440), (32, 4, 64, 2, True, 300, 340), (32, 4, 64, 48, True, 130, 170),
+    (16, 16, 64, 8, False, 200, 240), (16, 2, 128, 10, False, 1200, 1240), (16, 2, 128, 40, False, 400, 440), (8, 2, 128, 95, False, 400, 440),
+    (16, 2, 128, 16, True, 200, 240)])
+def test_longest_cache_of_the_one_attention_kernel(tctx, n_q, n_kv, d, batch, kv_int8, one, three):
+    """On both sides of the line: two launches more, and the same step over a nearly full cache within the bounds above."""
+    ctx, s = tctx
+    cfg = DecoderConfig(layers=1, hidden=256, mlp=256, n_q=n_q, n_kv=n_kv, head_dim=d, vocab=300)
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    out, launches = [], []
+    with torch.cuda.stream(s):
+        tokens = torch.randint(0, cfg.vocab, (batch,), dtype=torch.int32, device="cuda", generator=g)
+        shape = (batch, one, n_kv, d)
+        fill = [torch.randint(-127, 128, shape, dtype=torch.int8, device="cuda", generator=g) if kv_int8 else torch.randn(shape, device="cuda", generator=g)
+                for _ in range(2)]
+        scales = [0.005 + 0.01 * torch.rand(batch, one, device="cuda", generator=g) for _ in range(2)]
+        for max_seq in (one, three):
+            dec = Int4Decoder(ctx, cfg, batch, max_seq, s, seed=6, fused_step=False, kv_int8=kv_int8)
+            for dst, src in zip(dec.kcache + dec.vcache + (dec.kscale + dec.vscale if kv_int8 else []), fill + scales):
+                dst[:, :one].copy_(src)
+            dec.pos.fill_(one - 1)
+            before = ctx.launch_count()
+            out.append(dec.forward(tokens, 1).clone())
+            launches.append(ctx.launch_count() - before)
+            s.synchronize()
+            dec.close()
+    assert launches[1] - launches[0] == 2
+    assert ctx.device_status() == 0
+    tol = 1.1e-2 if batch > 16 else 1e-5
+    assert float((out[0] - out[1]).norm() / out[1].norm()) <= (max(tol, 2e-3) if kv_int8 else tol)
+
+
 @pytest.mark.parametrize("n_q,n_kv", [(8, 2), (32, 4)])   # up to 16 and up to 4 key splits per head
 @pytest.mark.parametrize("kv_int8", [False, True])
 def test_one_launch_step_positions(tctx, n_q, n_kv, kv_int8):

@@ -401,16 +401,42 @@ static int df_ctas(const yscv_cuda_ctx *ctx, size_t pairs) {
     while (C < 8 && pairs * C * 2 <= (size_t)2 * ctx->sm_count) C *= 2;
     return C;
 }
-// Where it gains: while a CTA's share of the cache is short. A long one takes chunk after chunk, where the three
-// kernels spread it over the machine (and read int8 rows on the tensor cores). us per step, this / three kernels: 1B shape, f32, 8
-// sequences 200 / 800 / 1500 keys 977 / 1034, 1078 / 1119, 1198 / 1205; 32: 50 / 200 / 800 keys 920 / 1083, 1012 / 1113, 1435 / 1418;
-// 64: 50 / 400 keys 1089 / 1246, 1588 / 1601; 2: 400 / 1500 keys 921 / 947, 1110 / 963; int8, 32: 30 / 200 / 400 keys 926 / 1024,
-// 1026 / 1067, 1189 / 1104. Heads of 128 in f32 gain as long as the grid fills the machine (4 layers of the 70B shape, 64
-// sequences 300 / 2048 keys 1833 / 1875, 2961 / 3150; 16: 1000 keys 1555 / 1636; 2: 2048 keys 1423 / 1404).
+// The longest cache that this kernel takes. A CTA walks its share of the keys chunk after chunk, where the three kernels spread long
+// ones over the machine and read int8 rows on the tensor cores; the host knows the cache's length and not the position, so the line lies
+// where a full cache is even. It depends on the CTAs that share a sequence's keys, on how much of the machine's two CTAs per
+// SM the grid fills (the three kernels gain by what it leaves empty), and on the heads of a group (eight are computed whatever
+// there are). us per layer of a step, full cache, this / three kernels (about 5000 points, 1 to 148 sequences, caches of 130 to 8192):
+//   f32, 32 / 4 heads of 64: 2 sequences 600 keys 37.7 / 37.1, 1600 45.9 / 37.6; 8: 200 34.9 / 37.2, 1200 43.6 / 44.1, 2100 51.2 / 48.6; 12: 400 48.4 /
+//   49.7, 1200 60.9 / 56.3; 16: 800 55.7 / 56.0; 24: 300 43.9 / 46.4, 600 53.2 / 50.6; 32: 600 53.9 / 54.0, 1200 73.0 / 65.5; 48: 200 49.9 / 49.6, 400
+//   62.1 / 56.6; 64: 400 63.4 / 63.5. 16 / 16 heads of 64, 8 sequences: 200 34.9 / 35.0, 400 42.8 / 40.0.
+//   f32, 64 / 8 heads of 128: 4: 400 57.2 / 55.1 (clusters of eight, 82 KB a CTA: a grid of more than 200 does not fit at once), 8192 190 / 148;
+//   8: 8192 209 / 240; 9: 1200 116 / 100; 19: 400 77.8 / 78.7, 2100 211 / 164; 37: 2100 216 / 267; 40: 800 181 / 156; 64: 2100 389 / 425.
+//   32 / 8: 16: 1600 114 / 117; 64: 600 143 / 142, 2100 376 / 345. 32 / 32, 8: 400 83.0 / 83.0, 2100 216 / 190.
+//   int8: 32 / 4 heads of 64, 8: 300 35.9 / 35.8, 800 40.5 / 37.3; 32: 130 39.7 / 42.3, 300 46.2 / 44.2; 64 / 8 of 128, 2: 200 44.0 / 44.5, 600 50.5 / 44.6;
+//   64: 130 80.1 / 70.3.
+static size_t df_longest(const yscv_cuda_ctx *ctx, bool kv_int8, size_t pairs, size_t group, size_t d_head) {
+    const size_t C = df_ctas(ctx, pairs), ctas = pairs * C, slots = (size_t)2 * ctx->sm_count, waves = (ctas + slots - 1) / slots;
+    const size_t fill = 100 * ctas / (slots * waves);   // % of the slots of its waves
+    if (kv_int8) {
+        if (d_head == 128) return group == 1 ? 0 : C == 8 ? 200 : C == 4 ? 130 : 0;
+        return C == 8 ? 300 : C == 4 ? 200 : C == 2 || (group >= 3 && waves == 1) ? 130 : 0;
+    }
+    if (d_head == 64) {
+        const bool full = fill >= 80;
+        if (group >= 4) return waves > 2 ? 0 : waves == 2 ? 400 : (C == 8 ? 600 : C == 4 ? 400 : C == 2 ? 300 : 200) * (full ? 2 : 1);
+        if (waves > 1 || (C == 1 && group == 1)) return 0;
+        return C == 8 ? (full ? 600 : 400) : C == 4 ? (full ? 400 : 200) : full ? 200 : 130;
+    }
+    if (C == 8) return ctas <= 64 ? 400 : ctas <= 128 ? 600 : ctas <= 200 ? (group >= 4 ? 1200 : 600) : 0;
+    if (C == 4 && ctas > 256) return 200;
+    if (waves > 2 || (waves == 2 && group < 4)) return 0;
+    if (group >= 8) return fill >= 85 ? (size_t)-1 : fill >= 75 ? 2000 : waves == 2 ? 200 : fill >= 60 ? 600 : 400;
+    if (group >= 4) return waves == 2 ? (fill >= 85 ? 600 : fill >= 75 ? 300 : 130) : fill >= 85 ? 1600 : fill >= 75 ? 800 : fill >= 60 ? 400 : 300;
+    return fill >= 85 ? (group > 1 ? 600 : 200) : fill >= 75 ? 200 : 130;
+}
 bool gqa_decode_fused_wins(const yscv_cuda_ctx *ctx, int form, bool kv_int8, size_t batch, size_t n_q, size_t n_kv, size_t d_head, size_t max_seq) {
     if ((d_head != 64 && d_head != 128) || n_q / n_kv > DF_HB || n_kv * d_head > 4096 || n_kv > 65535 || batch > 65000 || form == ACT_TERMS) return false;
-    const size_t C = df_ctas(ctx, batch * n_kv);
-    return max_seq <= 200 * C || (d_head == 128 && !kv_int8 && batch * n_kv * C >= (size_t)ctx->sm_count);
+    return max_seq <= df_longest(ctx, kv_int8, batch * n_kv, n_q / n_kv, d_head);
 }
 
 template <typename KV>
