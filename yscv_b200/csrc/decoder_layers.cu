@@ -4,7 +4,8 @@
 // single calls cannot is hand results over as they are: an operator writes the activations in the form that the
 // matmul behind it takes (act_forms.cuh), and a matmul whose k was cut into slices leaves them for the operator behind
 // it to add. A launch of a small decode batch is 1.5 to 2 us of latency whatever it does: 32 sequences at the 1B shape
-// (22 layers) had 15 launches per layer, 8 sequences 13; now 7 (9 over long caches).
+// (22 layers) had 15 launches per layer, 8 sequences 13; now 8: norm, QKV, attention, output, norm, gate/up, SwiGLU, down
+// (10 with RoPE, split and merge apart over long caches, and one more behind a matmul whose tiles several CTAs share).
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -103,7 +104,7 @@ int run(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_layer
         const yscv_cuda_decode_layer &l = layers[i];
         KV *kc = static_cast<KV *>(l.d_kcache), *vc = static_cast<KV *>(l.d_vcache);
         ActOut a = act_out(int4_act_form(ctx, l.qkv, m), m, H, act);
-        if ((rc = norm_form(ctx, x, delta, parts, m * H, l.d_gamma_attn, eps, m, 0, 1, H, x, a))) return rc;
+        if ((rc = norm_form(ctx, x, delta, parts, m * H, l.d_gamma_attn, eps, m, 0, 1, H, x, a, true))) return rc;
         parts = o.parts_qkv;
         if ((rc = int4_matmul_form(ctx, l.qkv, a, qkv, &parts))) return rc;
         const int form = int4_act_form(ctx, l.o, m);
@@ -125,17 +126,17 @@ int run(yscv_cuda_ctx *ctx, const yscv_cuda_decode_layer *layers, size_t n_layer
         parts = o.parts_o;
         if ((rc = int4_matmul_form(ctx, l.o, a, down, &parts))) return rc;
         a = act_out(int4_act_form(ctx, l.gate_up, m), m, H, act);
-        if ((rc = norm_form(ctx, x, down, parts, m * H, l.d_gamma_mlp, eps, m, 0, 1, H, x, a))) return rc;
+        if ((rc = norm_form(ctx, x, down, parts, m * H, l.d_gamma_mlp, eps, m, 0, 1, H, x, a, true))) return rc;
         parts = o.parts_gu;
         if ((rc = int4_matmul_form(ctx, l.gate_up, a, gu, &parts))) return rc;
         a = act_out(int4_act_form(ctx, l.down, m), m, s.inter, act);
-        if ((rc = swiglu_form(ctx, gu, parts, m * 2 * s.inter, m, s.inter, a))) return rc;
+        if ((rc = swiglu_form(ctx, gu, parts, m * 2 * s.inter, m, s.inter, a, true))) return rc;
         parts = o.parts_down;
         if ((rc = int4_matmul_form(ctx, l.down, a, down, &parts))) return rc;
         delta = down;
     }
     // the final norm of the last position of every sequence
-    return norm_form(ctx, x, delta, parts, m * H, final_gamma, eps, s.batch, s.seq - 1, s.seq, H, nullptr, act_out(ACT_F32, s.batch, H, last));
+    return norm_form(ctx, x, delta, parts, m * H, final_gamma, eps, s.batch, s.seq - 1, s.seq, H, nullptr, act_out(ACT_F32, s.batch, H, last), true);
 }
 
 }  // namespace

@@ -63,13 +63,11 @@ __global__ void embedding_kernel(const float *__restrict__ w, const int32_t *__r
     for (int i = threadIdx.x; i < dim / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// Eight consecutive values, with SUM the sum of `parts` arrays `pitch` floats apart, added in that order
-template <bool SUM>
+// Eight consecutive values that are the sum of `parts` arrays `pitch` floats apart, added in that order
 __device__ __forceinline__ void load8(const float *p, int parts, size_t pitch, float (&v)[8]) {
     const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    if constexpr (!SUM) return;
 #pragma unroll 4
     for (int s = 1; s < parts; ++s) {
         const float4 *q = reinterpret_cast<const float4 *>(p + s * pitch);
@@ -82,42 +80,33 @@ __device__ __forceinline__ void load8(const float *p, int parts, size_t pitch, f
 // Position of element e of a group of 8 in that order
 __device__ __forceinline__ int gemm_order_pos(int e) { return ((e & 3) << 1) | (e >> 2); }
 
-// x_out = x + delta (delta may be null), delta the sum of `parts` arrays `pitch` floats apart (one array without SUM); the
-// row normalised, (x_out / sqrt(mean(x_out^2) + eps)) * gamma, in the form that the matmul behind it takes. Input row of
-// block b: row0 + b * row_step (blocks past the rows of `o` write padding).
+// x_out = x + delta (delta may be null), the row normalised, (x_out / sqrt(mean(x_out^2) + eps)) * gamma, as fp32 or as the
+// bf16 activations of the matmul behind it. Input row of block b: row0 + b * row_step.
 //
 // Latency-bound for a few rows (a block per row), bandwidth-bound for many. A thread keeps its values in registers between
 // the sum of squares and the scaling: one round trip with every load in flight, 128-bit accesses, eight consecutive values
 // per lane where the form wants them, else four, so that an access of a warp is whole lines. The sum of squares goes through
-// shared memory so that its order is that of the kernel below (thread t: elements t, t + T, ...): the same result for every
+// shared memory so that its order is that of the scalar kernel below (thread t: elements t, t + T, ...): the same result for every
 // form and alignment. T = 256 up to 2048 values, else 1024 (hidden <= 8 T).
 // FEW (up to two rows per SM, NORM_FEW): gamma is fetched before the reduction, a thread takes eight values. More: what counts
 // is rows per SM, so gamma comes late (28 to 32 registers instead of 40, six and more blocks of 256) and blocks of 512 take 16 values
 // per thread, two of them per SM in different phases. us, fp32 to fp32 / to bf16, warm caches: 1 x 2048 1.5 / 1.6, 1 x 8192 3.1 / 3.5,
 // 1024 x 2048 4.6 / 5.5 (with FEW 4.6 / 5.3; 512 x 2048 3.0 / 3.4, FEW 3.1 / 4.4), 300 x 4096 5.2 / 5.5 (FEW 5.9 / 6.3), 128 x 4096 2.7 / 2.7 (FEW 2.7 /
 // 2.8), 128 x 8192 from HBM 5.8 / 4.9 (FEW 5.1 / 4.5), 2048 x 8192 42.7 / 41.1 (4.9 TB/s of fp32 to bf16; FEW 49.9 / 46.9). The scalar
-// kernel below: 2.0, 3.7, 5.0, 8.2, 3.2, 5.9, 65. With the sum over parts left in for one part (72 registers) and blocks of 128 and 256
+// kernel: 2.0, 3.7, 5.0, 8.2, 3.2, 5.9, 65. With a sum over parts left in for one part (72 registers) and blocks of 128 and 256
 // for more than 512 rows, 40 registers and spills, this took 10.0 / 8.9 at 1024 x 2048 and 20.5 / 17.5 at 513 x 8192 (now 9.5 / 10.9).
 constexpr size_t NORM_FEW = 2;
-template <int FORM, int T, bool SUM, bool FEW>
+template <bool BF16, int T, bool FEW>
 __global__ void __launch_bounds__(FEW || T == 256 ? T : T / 2, FEW ? 1 : T == 256 ? 6 : 2)
-norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, const float *__restrict__ gamma, float eps, int hidden,
-                 size_t row0, size_t row_step, float *x_out, ActOut o) {
+norm_rows_kernel(const float *x, const float *delta, const float *__restrict__ gamma, float eps, int hidden, size_t row0, size_t row_step,
+                 float *x_out, ActOut o) {
     pdl_wait();
     pdl_trigger();
-    constexpr int P = FEW || T == 256 ? 1 : 2, TH = T / P;      // P eights of values per thread
-    constexpr int W = FORM == ACT_F32 ? 4 : 8, N = P * 8 / W, Q = W / 4;   // N accesses of W values
+    constexpr int P = FEW || T == 256 ? 1 : 2, TH = T / P;                 // P eights of values per thread
+    constexpr int W = BF16 ? 8 : 4, N = P * 8 / W, Q = W / 4;   // N accesses of W values
     __shared__ float red[32];
     __shared__ __align__(16) float sm[8 * T];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-    if (FORM == ACT_DIGITS && row >= o.rows) {
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const int i = (tid + p * TH) * 8;
-            store_act_padding(o, row, i < hidden ? i : 0, i < hidden);
-        }
-        return;
-    }
     const size_t base = (row0 + row * row_step) * hidden;
     float4 v[N * Q];
 #pragma unroll
@@ -135,15 +124,7 @@ norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, co
             if (i < hidden) {
 #pragma unroll
                 for (int h = 0; h < Q; ++h) {
-                    const float *src = delta + base + i + 4 * h;
-                    float4 d = __ldg(reinterpret_cast<const float4 *>(src));
-                    if constexpr (SUM) {
-#pragma unroll 4
-                        for (int s = 1; s < parts; ++s) {
-                            const float4 e = __ldg(reinterpret_cast<const float4 *>(src + s * pitch));
-                            d.x += e.x; d.y += e.y; d.z += e.z; d.w += e.w;
-                        }
-                    }
+                    const float4 d = __ldg(reinterpret_cast<const float4 *>(delta + base + i + 4 * h));
                     float4 &y = v[p * Q + h];
                     y.x += d.x; y.y += d.y; y.z += d.z; y.w += d.w;
                 }
@@ -194,9 +175,8 @@ norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, co
 #pragma unroll
     for (int p = 0; p < N; ++p) {
         const int i = (tid + p * TH) * W;
-        const bool on = i < hidden;
-        float n[W] = {};
-        if (on) {
+        if (i < hidden) {
+            float n[W];
 #pragma unroll
             for (int h = 0; h < Q; ++h) {
                 const float4 y = P > 1 ? *reinterpret_cast<const float4 *>(sm + i + 4 * h) : v[p * Q + h];
@@ -206,13 +186,72 @@ norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, co
                 n[4 * h + 2] = (y.z * inv) * c.z;
                 n[4 * h + 3] = (y.w * inv) * c.w;
             }
-        }
-        if constexpr (FORM == ACT_F32) {
-            if (on) *reinterpret_cast<float4 *>(static_cast<float *>(o.ptr) + (size_t)row * o.k + i) = make_float4(n[0], n[1], n[2], n[3]);
-        } else {
-            store_act<FORM>(o, n, row, i, on);
+            if constexpr (BF16) store_act<ACT_BF16>(o, n, row, i, true);
+            else *reinterpret_cast<float4 *>(static_cast<float *>(o.ptr) + (size_t)row * o.k + i) = make_float4(n[0], n[1], n[2], n[3]);
         }
     }
+}
+
+// The same between two matmuls of a chain of few rows: delta the sum of `parts` arrays `pitch` floats apart, the row in any
+// form (blocks past the rows of `o` write padding), eight consecutive values per thread. One part takes it too: what it has
+// over the kernel above are registers, 72 for 40, which keep its blocks from moving in beside the CTAs of the matmul in front, on as
+// many SMs as there are rows, where they would hold up the CTAs of the matmul behind, which fetch their first weights early (1B
+// shape, us per step with this one / with the loop taken out: 4 sequences 967 / 1007, 9 1275 / 1360, 16 1286 / 1377, 64 1160 / 1233).
+template <int FORM, int T>
+__global__ void __launch_bounds__(T, 1)   // (without the 1 the compiler keeps to 44 registers)
+norm_form_kernel(const float *x, const float *delta, int parts, size_t pitch, const float *__restrict__ gamma, float eps, int hidden,
+                 size_t row0, size_t row_step, float *x_out, ActOut o) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float red[32];
+    __shared__ __align__(16) float sm[8 * T];
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, i = tid * 8;
+    const bool on = i < hidden;
+    if (FORM == ACT_DIGITS && row >= o.rows) {
+        store_act_padding(o, row, on ? i : 0, on);
+        return;
+    }
+    const size_t base = (row0 + row * row_step) * hidden;
+    float v[8] = {};
+    if (on) {   // (x not through the read-only path: x_out may be x)
+        const float4 a = *reinterpret_cast<const float4 *>(x + base + i), b = *reinterpret_cast<const float4 *>(x + base + i + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        if (delta) {
+            float d[8];
+            load8(delta + base + i, parts, pitch, d);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v[t] += d[t];
+        }
+        const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+        *reinterpret_cast<float4 *>(sm + i) = lo;
+        *reinterpret_cast<float4 *>(sm + i + 4) = hi;
+        if (x_out) {
+            *reinterpret_cast<float4 *>(x_out + base + i) = lo;
+            *reinterpret_cast<float4 *>(x_out + base + i + 4) = hi;
+        }
+    }
+    float g[8] = {};
+    if (on) load8(gamma + i, 1, 0, g);
+    __syncthreads();
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int e = tid + j * T;
+        const float y = e < hidden ? sm[e] : 0.0f;
+        ss = fmaf(y, y, ss);
+    }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, s);
+    if (lane == 0) red[tid >> 5] = ss;
+    __syncthreads();
+    float total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) total += red[w];
+    const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) v[t] = (v[t] * inv) * g[t];
+    store_act<FORM>(o, v, row, i, on);
 }
 
 // The same for operands that are not 16-byte aligned and rows that are no multiple of 8, up to 16384
@@ -324,8 +363,9 @@ swiglu_kernel(const float *__restrict__ gu, void *__restrict__ out, int rows, in
 }
 // The same for partial sums and for the forms of up to 16 rows. (In the place of the kernel above, one part, fp32 or bf16 out: 1 x
 // 28672 1.8 us for 1.66, 128 x 5632 2.8 for 2.2, 2048 x 1024 5.5 for 4.3, 2048 x 28672 to bf16 94 for 83; without the loop over
-// parts still up to 18 % more, 128 x 14336 3.9 for 3.3: whole warps and the general store.)
-template <int FORM, bool SUM>
+// parts still up to 18 % more, 128 x 14336 3.9 for 3.3: whole warps and the general store. Between two matmuls of few rows it stays all
+// the same, as told at norm_form_kernel: a step of 40 sequences 1106 us, 1114 with the other.)
+template <int FORM>
 __global__ void __launch_bounds__(256)
 swiglu_form_kernel(const float *__restrict__ gu, int parts, size_t pitch, int rows, int inter, ActOut o) {
     pdl_wait();
@@ -341,8 +381,8 @@ swiglu_form_kernel(const float *__restrict__ gu, int parts, size_t pitch, int ro
             }
             float g[8] = {}, u[8] = {}, n[8];
             if (on) {
-                load8<SUM>(gu + (size_t)r * 2 * inter + c * 8, parts, pitch, g);
-                load8<SUM>(gu + (size_t)r * 2 * inter + inter + c * 8, parts, pitch, u);
+                load8(gu + (size_t)r * 2 * inter + c * 8, parts, pitch, g);
+                load8(gu + (size_t)r * 2 * inter + inter + c * 8, parts, pitch, u);
             }
 #pragma unroll
             for (int t = 0; t < 8; ++t) n[t] = swiglu_one(g[t], u[t]);
@@ -1435,26 +1475,31 @@ static const char *form_name(int form, const char *f32, const char *bf16, const 
 
 // hidden % 8 == 0 and at most 8192, operands (and `pitch` floats) 16-byte aligned
 int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
-              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out) {
-    const bool small = hidden <= 2048;
-    // (partial sums and the forms of up to 16 rows come with few rows)
-    const bool few = rows <= NORM_FEW * ctx->sm_count || parts > 1 || (out.form != ACT_F32 && out.form != ACT_BF16);
-    const unsigned threads = small ? 256u : few ? 1024u : 512u;
+              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out, bool between) {
+    const bool small = hidden <= 2048, few = rows <= NORM_FEW * ctx->sm_count;
+    const char *name = form_name(out.form, "add_rms_norm", "add_rms_norm(bf16 activations out)", "add_rms_norm(digit planes out)", "add_rms_norm(fp16 terms out)");
+    if (parts == 1 && (out.form == ACT_F32 || out.form == ACT_BF16) && !(between && few)) {
+        auto pick = [&](auto bf16) {
+            constexpr bool B = decltype(bf16)::value;
+            return few ? (small ? norm_rows_kernel<B, 256, true> : norm_rows_kernel<B, 1024, true>)
+                       : (small ? norm_rows_kernel<B, 256, false> : norm_rows_kernel<B, 1024, false>);
+        };
+        auto kern = out.form == ACT_BF16 ? pick(std::true_type()) : pick(std::false_type());
+        YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)rows), dim3(small ? 256u : few ? 1024u : 512u), 0, ctx->stream, x, delta, gamma, eps, (int)hidden,
+                                 row0, row_step, x_out, out));
+        DEC_EPILOGUE(ctx, name);
+    }
     auto pick = [&](auto form) {
         constexpr int F = decltype(form)::value;
-        if constexpr (F == ACT_F32 || F == ACT_BF16) {
-            if (!few) return small ? norm_form_kernel<F, 256, false, false> : norm_form_kernel<F, 1024, false, false>;
-        }
-        if (parts > 1) return small ? norm_form_kernel<F, 256, true, true> : norm_form_kernel<F, 1024, true, true>;
-        return small ? norm_form_kernel<F, 256, false, true> : norm_form_kernel<F, 1024, false, true>;
+        return small ? norm_form_kernel<F, 256> : norm_form_kernel<F, 1024>;
     };
     auto kern = out.form == ACT_BF16     ? pick(std::integral_constant<int, ACT_BF16>())
                 : out.form == ACT_DIGITS ? pick(std::integral_constant<int, ACT_DIGITS>())
                 : out.form == ACT_TERMS  ? pick(std::integral_constant<int, ACT_TERMS>())
                                          : pick(std::integral_constant<int, ACT_F32>());
-    YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)out.slots()), dim3(threads), 0, ctx->stream, x, delta, parts, pitch, gamma, eps, (int)hidden,
-                             row0, row_step, x_out, out));
-    DEC_EPILOGUE(ctx, form_name(out.form, "add_rms_norm", "add_rms_norm(bf16 activations out)", "add_rms_norm(digit planes out)", "add_rms_norm(fp16 terms out)"));
+    YSCV_CUDA_TRY(launch_pdl(kern, dim3((unsigned)out.slots()), dim3(small ? 256u : 1024u), 0, ctx->stream, x, delta, parts, pitch, gamma, eps,
+                             (int)hidden, row0, row_step, x_out, out));
+    DEC_EPILOGUE(ctx, name);
 }
 }  // namespace yscv
 
@@ -1465,7 +1510,7 @@ static int add_rms_norm_impl(yscv_cuda_ctx *ctx, const float *x, const float *de
     const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(gamma) |
                            reinterpret_cast<uintptr_t>(x_out) | reinterpret_cast<uintptr_t>(normed);
     if (hidden % 8 == 0 && hidden <= 8192 && (ptrs & 15) == 0)
-        return norm_form(ctx, x, delta, 1, 0, gamma, eps, rows, 0, 1, hidden, x_out, act_out(ACT ? ACT_BF16 : ACT_F32, rows, hidden, normed));
+        return norm_form(ctx, x, delta, 1, 0, gamma, eps, rows, 0, 1, hidden, x_out, act_out(ACT ? ACT_BF16 : ACT_F32, rows, hidden, normed), false);
     // eight elements per thread: 256 threads are enough up to 2048, 1024 up to 8192; sixteen up to 16384
     const unsigned threads = hidden <= 2048 ? 256u : 1024u;
     auto kern = hidden <= 8192 ? add_rms_norm_kernel<ACT, 8> : hidden <= 16384 ? add_rms_norm_kernel<ACT, 16> : add_rms_norm_long_kernel<ACT>;
@@ -1682,23 +1727,19 @@ int yscv_cuda_gqa_attention_i8_dev(yscv_cuda_ctx *ctx, const float *d_q, size_t 
 
 namespace yscv {
 // inter % 8 == 0, operands (and `pitch` floats) 16-byte aligned
-int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out) {
+int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out, bool between) {
     const size_t visit = out.slots();
     const dim3 grid((unsigned)((inter / 8 + 255) / 256), (unsigned)(visit < 32768 ? visit : 32768));
     const char *name = form_name(out.form, "swiglu", "swiglu(bf16 activations out)", "swiglu(digit planes out)", "swiglu(fp16 terms out)");
-    if (parts == 1 && (out.form == ACT_F32 || out.form == ACT_BF16)) {
+    if (parts == 1 && (out.form == ACT_F32 || out.form == ACT_BF16) && !(between && rows <= NORM_FEW * ctx->sm_count)) {
         auto plain = out.form == ACT_BF16 ? swiglu_kernel<true> : swiglu_kernel<false>;
         YSCV_CUDA_TRY(launch_pdl(plain, grid, dim3(256), 0, ctx->stream, gate_up, out.ptr, (int)rows, (int)inter));
         DEC_EPILOGUE(ctx, name);
     }
-    auto pick = [&](auto form) {
-        constexpr int F = decltype(form)::value;
-        return parts > 1 ? swiglu_form_kernel<F, true> : swiglu_form_kernel<F, false>;
-    };
-    auto kern = out.form == ACT_BF16     ? pick(std::integral_constant<int, ACT_BF16>())
-                : out.form == ACT_DIGITS ? pick(std::integral_constant<int, ACT_DIGITS>())
-                : out.form == ACT_TERMS  ? pick(std::integral_constant<int, ACT_TERMS>())
-                                         : pick(std::integral_constant<int, ACT_F32>());
+    auto kern = out.form == ACT_BF16     ? swiglu_form_kernel<ACT_BF16>
+                : out.form == ACT_DIGITS ? swiglu_form_kernel<ACT_DIGITS>
+                : out.form == ACT_TERMS  ? swiglu_form_kernel<ACT_TERMS>
+                                         : swiglu_form_kernel<ACT_F32>;
     YSCV_CUDA_TRY(launch_pdl(kern, grid, dim3(256), 0, ctx->stream, gate_up, parts, pitch, (int)visit, (int)inter, out));
     DEC_EPILOGUE(ctx, name);
 }
@@ -1708,7 +1749,7 @@ template <bool ACT>
 static int swiglu_impl(yscv_cuda_ctx *ctx, const float *gate_up, size_t rows, size_t inter, void *out) {
     if (rows * inter == 0) return YSCV_CUDA_OK;
     if (inter % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-        return swiglu_form(ctx, gate_up, 1, 0, rows, inter, act_out(ACT ? ACT_BF16 : ACT_F32, rows, inter, out));
+        return swiglu_form(ctx, gate_up, 1, 0, rows, inter, act_out(ACT ? ACT_BF16 : ACT_F32, rows, inter, out), false);
     } else {
         const size_t total = rows * (inter / (ACT ? 8 : 1));
         const unsigned blocks = (unsigned)((total + 255) / 256 < 65535 ? (total + 255) / 256 : 65535);

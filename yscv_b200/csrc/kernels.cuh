@@ -65,8 +65,8 @@ int int4_matmul_form(yscv_cuda_ctx *ctx, const yscv_cuda_int4_weight *w, const A
 
 // decoder_ops.cu, the operators between the matmuls. Inputs that are `parts` partial sums lie `pitch` floats apart.
 int norm_form(yscv_cuda_ctx *ctx, const float *x, const float *delta, int parts, size_t pitch, const float *gamma, float eps,
-              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out);
-int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out);
+              size_t rows, size_t row0, size_t row_step, size_t hidden, float *x_out, const ActOut &out, bool between);
+int swiglu_form(yscv_cuda_ctx *ctx, const float *gate_up, int parts, size_t pitch, size_t rows, size_t inter, const ActOut &out, bool between);
 template <typename KV>
 int rope_append_form(yscv_cuda_ctx *ctx, const float *qkv, int parts, size_t pitch, float *q_out, size_t q_out_stride, size_t batch,
                      size_t seq, size_t n_q, size_t n_kv, size_t d_head, float theta, const int32_t *d_pos, KV *kcache, KV *vcache,
