@@ -644,6 +644,7 @@ void yscv_cuda_decode_plan_free(yscv_cuda_decode_plan *plan);
  * (row b * seq + s at position *d_pos + s) and is overwritten; the caches are
  * [batch][max_seq][n_kv][d_head] (kv_int8: int8 with scale tables [batch][max_seq]); d_last
  * [batch][hidden] receives RMSNorm(final residual) * final_gamma of every sequence's last position.
+ * Layers may differ in the group size and alignment of their weights, not in their shapes.
  * _workspace says how many bytes of device memory a pass needs (its first call may allocate the
  * library's own workspace, so ask outside a capture); passes that overlap need one each. hidden, inter and
  * d_head must be multiples of 8, hidden at most 8192, d_x, the gammas, d_last and the workspace 16-byte aligned

@@ -1376,8 +1376,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const StepPa
     int tp_ar = 0;
     float row_scale = 1.0f;
 
-    // One matrix: for every K chunk, `stage_chunk(k0, klen)` leaves the activations of that
-    // chunk in act_s and their digit planes in `dig`; then every row block of the CTA walks the
+    // One matrix: for every K chunk, `stage_chunk(k0, klen)` leaves the digit planes of its activations in `dig`
+    // (act_s is used on the way by some); then every row block of the CTA walks the
     // chunk's stages. (More than one chunk only with a single row block: the accumulators then
     // live across the chunks.)
     auto gemv = [&](int mi, float *out, int store, auto &&stage_chunk) {
