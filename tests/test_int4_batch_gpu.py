@@ -258,7 +258,7 @@ def test_prompt_tiles(m, n, k, form):
 
 @pytest.mark.parametrize("m", [1, 2, 3, 4])
 @pytest.mark.parametrize("n,k", [(100, 256), (4736, 1280), (4800, 1536), (4737, 1792), (2048, 4352), (6000, 6912), (300, 8448), (4737, 6656),
-                                 (2048, 2048), (2048, 2304), (2048, 2560), (2048, 2816), (2048, 4608)])
+                                 (2048, 2048), (2048, 2304), (2048, 2560), (2048, 3584), (2048, 4608), (2500, 4096), (19000, 3840)])
 def test_few_rows_depths(m, n, k):
     """The few-row matmul where its last stage ends in half, and on both sides of the line between quantising the rows in the
     kernel and before it: 21-bit blocks of 32 values (2^-22 of the block's maximum each, about four times its rms) and fp32 sums, 2e-6."""

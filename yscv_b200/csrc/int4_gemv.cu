@@ -479,16 +479,20 @@ bool int4_gemv_fast_supported(size_t m, size_t n, size_t k, size_t gs) {
 
 // Few and short activation rows: every CTA quantises them itself, no separate launch. That is work on the way to every CTA's
 // first product, so it pays only up to a line, which lies where a launch of its own is the faster call, host time included (us
-// per call one after another, in the kernel / in a launch of its own; inside a capture the first form is taken anyway):
-//   up to 32 rows of weights per CTA: 1 row 2048 x 4096 6.4 / 6.3, 4608 7.4 / 6.7, 8192 10.5 / 9.0; 2 rows 2048 x 2048 4.6 / 6.2, 2560 5.8 / 6.3,
-//   3072 6.3 / 6.2, 4096 7.4 / 6.6; 4 rows 2048 x 1280 5.0 / 6.3, 2048 5.9 / 6.3, 2560 7.0 / 6.3, 4096 9.9 / 6.9;
-//   more, which hide it better: 1 row 14336 x 4096 9.5 / 9.7, 5632 12.4 / 11.8 (weights from HBM 12.7 / 13.8), 8192 16.7 / 15.2; 2 rows 14336 x 3072
-//   8.7 / 8.7, 4096 10.4 / 10.2 (11.8 / 12.0); 4 rows 6144 x 1536 6.3 / 6.3, 2048 7.5 / 6.9, 14336 x 1536 7.9 / 7.8 (8.6 / 9.1), 4096 16.9 / 13.7.
+// per call, one after another through up to 16 matrices, in the kernel / in a launch of its own; inside a capture the first form
+// is taken anyway):
+//   up to 16 rows of weights per CTA: 1 row 1500 x 4096 6.4 / 6.4, 4608 7.4 / 6.7; 2 rows 2048 x 2560 5.7 / 6.4, 3072 6.3 / 6.4, 3584 6.8 / 6.5, 4096 7.3 / 6.7; 4
+//   rows 2048 x 1280 5.0 / 6.4, 2048 5.8 / 6.3, 2304 7.3 / 6.4;
+//   up to 128: 1 row 4500 x 5632 8.3 / 8.9, 6656 9.6 / 9.7, 8192 10.8 / 10.7, 14336 x 8192 18.5 / 17.9; 2 rows 4500 x 3072 6.5 / 7.2, 4096 7.7 / 8.1, 11008 x 4096
+//   10.6 / 12.1, 4608 12.5 / 12.5, 14336 x 4096 11.5 / 12.4; 4 rows 14336 x 2048 11.2 / 11.4, 2304 12.9 / 12.5;
+//   more: 1 row 28672 x 6656 26.4, 8192 37.6 / 32.6; 2 rows 28672 x 3584 15.8 / 18.1, 4096 20.7 / 19.9; 4 rows 28672 x 2048 17.5 / 17.4, 2304 20.3 / 19.6.
 // (The digit planes of so many values are at most 56 KB.)
 static bool small_rows(const yscv_cuda_ctx *ctx, int n) { return (n + ctx->sm_count - 1) / ctx->sm_count <= 32; }
 static bool fused_quant(const yscv_cuda_ctx *ctx, int mp, int n, int k) {
     if (mp > 4) return false;
-    return mp * k <= (!small_rows(ctx, n) ? 6800 : mp == 1 ? 4500 : mp == 2 ? 5200 : 8200);
+    const int per = (n + ctx->sm_count - 1) / ctx->sm_count;   // weight rows of a CTA
+    if (per <= 16) return mp * k <= (mp == 1 ? 4500 : mp == 2 ? 6200 : 8200);
+    return mp * k <= (mp == 1 ? 6800 : per <= 128 ? 8200 : 7700);
 }
 bool int4_gemv_uses_scratch(const yscv_cuda_ctx *ctx, size_t m, size_t n, size_t k) { return !fused_quant(ctx, padded_m((int)m), (int)n, (int)k); }
 // Where the operator in front should write digit planes, which costs it little and no launch: from where a launch of its own
