@@ -172,12 +172,12 @@ HEADS = [  # n_q, n_kv, d: groups of 1 to 8 heads, both head sizes
 @pytest.mark.parametrize("n_q,n_kv,d", HEADS)
 @pytest.mark.parametrize("batch", [2, 7, 40])
 @pytest.mark.parametrize("kv_int8", [False, True])
-def test_step_attention_positions(tctx, n_q, n_kv, d, batch, kv_int8):
+@pytest.mark.parametrize("max_seq", [196, 126])   # the shorter one keeps one and two CTAs per sequence in the one kernel
+def test_step_attention_positions(tctx, n_q, n_kv, d, batch, kv_int8, max_seq):
     """One step at positions around the chunks and the CTAs' shares of the one-kernel attention, against the three
     kernels; the appended rows; a sequence whose cache holds a NaN and an infinity; a position past the cache."""
     ctx, s = tctx
     cfg = DecoderConfig(layers=1, hidden=256, mlp=256, n_q=n_q, n_kv=n_kv, head_dim=d, vocab=300)
-    max_seq = 196
     dec = Int4Decoder(ctx, cfg, batch, max_seq, s, seed=6, fused_step=False, kv_int8=kv_int8)
     layers = dec.layers
     g = torch.Generator(device="cuda")
@@ -193,7 +193,7 @@ def test_step_attention_positions(tctx, n_q, n_kv, d, batch, kv_int8):
         bad[batch - 1, 0].fill_(float("nan"))
         caches = dec.kcache + dec.vcache
         tables = dec.kscale + dec.vscale if kv_int8 else []
-        for p in (0, 1, 23, 24, 25, 63, 64, 65, 127, 128, 129, max_seq - 1, max_seq):
+        for p in [q for q in (0, 1, 23, 24, 25, 63, 64, 65, 127, 128, 129) if q < max_seq - 1] + [max_seq - 1, max_seq]:
             res = []
             for form in (layers, None):
                 dec.layers = form
